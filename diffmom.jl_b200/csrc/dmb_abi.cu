@@ -105,6 +105,7 @@ dmb_status dmb_ctx_destroy(dmb_ctx *c) {
     c->aca.release();
     dmb::tc_release(c);
     dmb::oz_release(c);
+    dmb::oz64_release(c);
     dmb::local_release(c);
     dmb::far_release(c);
     for (auto &e : c->kt_pool) cudaEventDestroy(e);

@@ -1344,9 +1344,12 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
     if (use_tc) {
       dmb::tc_ldlt_update_c64(c, N, r0, c_hi, jcol, K, (float2 *)F, (const float2 *)Wb, NBW, woff, slot);
     } else if constexpr (std::is_same<C, double2>::value) {
-      // complex128 factor: the FP64-pipe GEMM (128 x 64 tiles, lower triangle)
-      dmb::zgemm64_lower_update(c, rest, c_hi - r0, K, (const double2 *)Wb + r0 * NBW + woff, NBW,
-                                (const double2 *)F + r0 * N + jcol, N, (double2 *)F + r0 * N + r0, N);
+      const double2 *Wk = (const double2 *)Wb + r0 * NBW + woff, *Lk = (const double2 *)F + r0 * N + jcol;
+      if (dmb::oz64_available(c, K) && dmb::oz64_reserve(c, rest, c_hi - r0, K, slot))
+        dmb::oz64_lower_update(c, rest, c_hi - r0, K, Wk, NBW, Lk, N, (double2 *)F + r0 * N + r0, N, slot, err);
+      else
+        // the FP64-pipe GEMM (128 x 64 tiles, lower triangle)
+        dmb::zgemm64_lower_update(c, rest, c_hi - r0, K, Wk, NBW, Lk, N, (double2 *)F + r0 * N + r0, N);
     } else {
       dim3 g(blocks_for(rest, 64), blocks_for(c_hi - r0, 64));
       DMB_LAUNCH(c, k_ldlt_update<C>, g, 256, 0, N, r0, c_hi, jcol, K, F, Wb, NBW, woff, 0, (C *)nullptr, err);
@@ -1468,6 +1471,7 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
   DMB_CUDA(cudaMemcpyAsync(&h_err, err, 4, cudaMemcpyDeviceToHost, c->stream));
   DMB_CUDA(cudaStreamSynchronize(c->stream));
   DMB_REQUIRE(!(h_err & 4u), DMB_ERR_TIMEOUT, "factorisation: a panel-step wait expired");
+  DMB_REQUIRE(!(h_err & 8u), DMB_ERR_TIMEOUT, "int8 tensor-core update: a pipeline wait expired");
   DMB_REQUIRE(h_err == 0, DMB_ERR_BREAKDOWN, "near-field factorisation broke down: zero or non-finite pivot");
   if (use_tc)
     DMB_REQUIRE(dmb::tc_error_word(c) == 0, DMB_ERR_TIMEOUT, "tensor-core update: a pipeline wait expired");

@@ -165,6 +165,13 @@ struct FarTileState {
   DevBuf d_panels, d_cnt, d_tasks, d_job, d_err;
 };
 
+// Operand planes, scales and residue planes of the complex128 factor updates on
+// the INT8 tensor cores (dmb_oz64.cu), one set per issuing stream.
+struct Oz64State {
+  DevBuf planes[3], scale[3], res[3];
+  bool attr = false;
+};
+
 struct dmb_ctx {
   int device = 0;
   // operator of dmb_gmres / dmb_matvec: 0 the resident dense Z, 1 the
@@ -233,6 +240,7 @@ struct dmb_ctx {
   DevBuf d_dinv;      // Jacobi inverse diagonal
   DevBuf d_W;         // LDL^T panel workspace
   DevBuf d_flags;     // triangular-solve progress flags / error word
+  Oz64State oz64;
   double nnz_ratio = 0;
   bool pc_valid = false;
 
@@ -413,6 +421,14 @@ void zgemm64_sub(dmb_ctx *c, bool a_transposed, int64_t M, int64_t R, int64_t K,
                  const double2 *B, int64_t ldb, double2 *Y, int64_t ldy);
 void zgemm64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int64_t K, const double2 *W, int64_t ldw,
                           const double2 *Lrows, int64_t ldl, double2 *F, int64_t ldf);
+// the same update on the INT8 tensor cores (dmb_oz64.cu), K 256 or 1024, with
+// the buffers of `slot`; err gets bit 8 when a pipeline wait expires.
+// oz64_reserve: false when the buffers cannot be allocated
+bool oz64_available(dmb_ctx *c, int K);
+bool oz64_reserve(dmb_ctx *c, int64_t M, int64_t C, int K, int slot);
+void oz64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int K, const double2 *W, int64_t ldw, const double2 *L,
+                       int64_t ldl, double2 *F, int64_t ldf, int slot, unsigned *err);
+void oz64_release(dmb_ctx *c);
 unsigned read_err_word(dmb_ctx *c);  // error word of the triangular solves (bit 2: a wait expired)
 void matvec_dev(dmb_ctx *c, const void *x, void *y, int64_t nrhs);  // device buffers, c128
 void conj_dev(dmb_ctx *c, double2 *x, int64_t count);
