@@ -8,16 +8,13 @@
 //     symmetric), so it is factored as L D L^T -- unit lower L, diagonal D, no
 //     pivoting -- which has the same inverse as the reference's UMFPACK LU up to
 //     rounding, at half the flops.  Right-looking, panel width NB = 64:
-//       k_ldlt_diag    one CTA factors the 64x64 diagonal block and writes the
-//                      inverse of its unit-lower factor (used twice: by the panel
-//                      and by the triangular solves);
-//       k_ldlt_panel   L21 D1 = A21 L11^-T as a small GEMM with that inverse,
-//                      L21 = (L21 D1) D1^-1, rows in parallel;
-//       k_ldlt_update  trailing update A22 -= (L21 D1) L21^T on lower tiles
-//                      (FP64 SIMT for complex128 factors, FP32 SIMT or the
-//                      tensor-core kernel for complex64 factors); inside a
-//                      256-wide panel its first CTA then factors the next
-//                      diagonal block, so that block needs no launch of its own.
+//       k_ldlt_mid64   complex128: a 256-wide panel (four diagonal blocks, their
+//                      panel rows and the updates between them) in one launch;
+//       k_ldlt_first, k_ldlt_step  complex64: one launch per 64 columns (strip
+//                      update, next diagonal block, its panel rows);
+//     and updates A22 -= (L21 D1) L21^T after every 256 and 1,024 columns
+//     (complex128: int8 residue products, dmb_oz64.cu, or the FP64 pipe;
+//     complex64: the tensor-core kernels of dmb_tc.cu or FP32 units).
 //     A zero or non-finite pivot stops with DMB_ERR_BREAKDOWN.
 //   * apply (NearFieldOperator, :1034-1054): L y = x, z = y / D, L^T x = z as
 //     one kernel per sweep.  Each CTA draws a ticket (block row, launch order),
@@ -144,84 +141,6 @@ __global__ void k_diag_inv(int64_t N, const ZC *__restrict__ Z, const double *__
 // applies both updates: L = L_0 L_1 ... with L_k = I + l_k e_k^T, so
 // X = ... (I - l_1 e_1^T)(I - l_0 e_0^T), and row k of X is final once steps
 // 0..k-1 have run.  One barrier pair per step covers both.
-template <class C>
-__device__ __forceinline__ void ldlt_diag_block(int64_t N, int64_t j, int b, C *__restrict__ F,
-                                                C *__restrict__ Linv, unsigned *__restrict__ err, C *colk) {
-  C *rowk = colk + NB;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  C a[4][4], x[4][4];
-#pragma unroll
-  for (int p = 0; p < 4; p++)
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      int i = ty + 16 * p, c = tx + 16 * q;
-      a[p][q] = (i < b && c <= i) ? F[(j + i) * N + j + c] : czero<C>();
-      x[p][q] = (i == c) ? cone<C>() : czero<C>();
-    }
-  for (int k = 0; k < b; k++) {
-    const int kq = k >> 4;
-    if (tx == (k & 15)) {
-#pragma unroll
-      for (int p = 0; p < 4; p++)
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-          if (q == kq) colk[ty + 16 * p] = a[p][q];
-    }
-    if (ty == (k & 15)) {
-#pragma unroll
-      for (int p = 0; p < 4; p++)
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-          if (p == kq) rowk[tx + 16 * q] = x[p][q];
-    }
-    __syncthreads();
-    const C d = colk[k];
-    const double ad = (double)cabsv(d);
-    if (!(ad > 0.0) || !isfinite(ad)) {
-      if (threadIdx.x == 0) atomicOr(err, 2u);
-      return;  // uniform: every thread read the same pivot
-    }
-    const C inv_d = cdiv(cone<C>(), d);
-    C l[4], xr[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      l[q] = cmul(colk[tx + 16 * q], inv_d);
-      xr[q] = rowk[tx + 16 * q];
-    }
-    // warp-uniform skips: row blocks entirely at or above k, column blocks of
-    // the block entirely left of k, and columns of X right of k (row k of X
-    // is zero there) hold nothing to update
-#pragma unroll
-    for (int p = 0; p < 4; p++) {
-      if (16 * p + 15 <= k) continue;
-      const int i = ty + 16 * p;
-      const C ci = colk[i];
-      const C lik = cmul(ci, inv_d);
-#pragma unroll
-      for (int q = 0; q <= p; q++) {
-        if (16 * q + 15 < k) continue;
-        const int c = tx + 16 * q;
-        if (c > k && c <= i) a[p][q] = csub(a[p][q], cmul(ci, l[q]));
-        if (c == k && i > k) a[p][q] = lik;  // L entry of column k
-      }
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        if (16 * q > k) continue;
-        if (i > k) x[p][q] = csub(x[p][q], cmul(lik, xr[q]));
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int p = 0; p < 4; p++)
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      int i = ty + 16 * p, c = tx + 16 * q;
-      if (i < b && c <= i) F[(j + i) * N + j + c] = a[p][q];
-      Linv[i * NB + c] = x[p][q];
-    }
-}
-
 // 1 / x for a positive normal float: the hardware approximation refined by
 // one Newton-Raphson step, r <- r (2 - x r)
 __device__ __forceinline__ float rcp_nr(float x) {
@@ -229,6 +148,29 @@ __device__ __forceinline__ float rcp_nr(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r * fmaf(-x, r, 2.f);
 }
+// the same for doubles: two Newton-Raphson steps
+__device__ __forceinline__ double rcp_nr(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  r = fma(r, fma(-x, r, 1.0), r);
+  return fma(r, fma(-x, r, 1.0), r);
+}
+// 1 / d of a pivot: conj(d) / |d|^2; FP64 pivots whose |d|^2 leaves the
+// normal range are divided by Smith's algorithm
+__device__ __forceinline__ float2 pivot_inverse(float2 d) {
+  const float rd = rcp_nr(fmaf(d.x, d.x, d.y * d.y));
+  return make_float2(d.x * rd, -d.y * rd);
+}
+__device__ __forceinline__ double2 pivot_inverse(double2 d) {
+  const double d2 = fma(d.x, d.x, d.y * d.y);
+  if (d2 > 1e-290 && d2 < 1e290) {
+    const double rd = rcp_nr(d2);
+    return make_double2(d.x * rd, -d.y * rd);
+  }
+  return cdiv(make_double2(1.0, 0.0), d);
+}
+__device__ __forceinline__ float2 cneg(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ double2 cneg(double2 a) { return make_double2(-a.x, -a.y); }
 __device__ __forceinline__ float2 csel(bool p, float2 a, float2 b) { return make_float2(p ? a.x : b.x, p ? a.y : b.y); }
 
 // Elimination of the 16 x 16 diagonal sub-block at s0 by one warp, all in
@@ -244,7 +186,7 @@ __device__ __forceinline__ float2 csel(bool p, float2 a, float2 b) { return make
 // zero, non-finite or outside the FP32 normal range (|d| below ~1e-19 or above
 // ~1e19) is a breakdown (false, uniform over the warp, decided after the 16
 // steps).
-__device__ __forceinline__ bool elim16_warp(float2 (*A)[65], float2 (*Xs)[17], int s0, int lane) {
+__device__ __forceinline__ bool elim16_warp(float2 (*A)[65], float2 (*Xs)[17], int s0, int lane, float2 *, float2 *) {
   const unsigned FULL = 0xffffffffu;
   const int c = lane & 15, ih = lane >> 4;
   float2 a[8], x[8];
@@ -296,16 +238,152 @@ __device__ __forceinline__ bool elim16_warp(float2 (*A)[65], float2 (*Xs)[17], i
 }
 
 
-// Blocked form of ldlt_diag_block for complex64 blocks (same results up to
-// rounding): four 16-wide sub-panels; warp 0 eliminates the 16 x 16 diagonal
-// sub-block in registers (elim16_warp, which also forms its unit-lower
-// inverse), then the CTA computes the sub-panel below it (up to three rows
-// per thread, accumulated together) and the trailing update (four columns per
-// thread).  The 64 x 64 inverse is assembled from the four 16 x 16 inverses
-// by recursive doubling (16-wide pairs, then the 32-wide halves), each phase
-// a small product with several independent sums per thread.
-// Rows and columns at or beyond b are padded with the identity (D = 1, L = 0).
-constexpr size_t DIAG_BLOCKED_SMEM = sizeof(float2) * (2 * 64 * 65 + 64 * 17 + 4 * 16 * 17 + 16) + 16;
+// The plain form for complex128 blocks with a pivot outside the range of the
+// fast one below: entry by entry in shared memory, pivots divided by Smith's
+// algorithm.  A zero or non-finite pivot is a breakdown.
+__device__ __noinline__ bool elim16_any(double2 (*A)[68], double2 (*Xs)[17], int s0, int lane, double2 *dinv) {
+  for (int e = lane; e < 256; e += 32) Xs[e >> 4][e & 15] = make_double2((e >> 4) == (e & 15) ? 1.0 : 0.0, 0.0);
+  __syncwarp();
+  for (int k = 0; k < 16; k++) {
+    const double2 d = A[s0 + k][s0 + k];
+    const double ad = cabsv(d);
+    if (!(ad > 0.0) || !isfinite(ad)) return false;
+    const double2 inv_d = cdiv(make_double2(1.0, 0.0), d);
+    double2 v[8], x[8];
+#pragma unroll
+    for (int m = 0; m < 8; m++) {
+      const int e = lane + 32 * m, i = e >> 4, c = e & 15;
+      const double2 l = cmul(A[s0 + i][s0 + k], inv_d);
+      v[m] = c == k ? l : csub(A[s0 + i][s0 + c], cmul(l, A[s0 + c][s0 + k]));
+      x[m] = csub(Xs[i][c], cmul(l, Xs[k][c]));
+    }
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < 8; m++) {
+      const int e = lane + 32 * m, i = e >> 4, c = e & 15;
+      if (i <= k) continue;
+      if (c >= k && c <= i) A[s0 + i][s0 + c] = v[m];
+      Xs[i][c] = x[m];
+    }
+    if (lane == 0) dinv[k] = inv_d;
+    __syncwarp();
+  }
+  return true;
+}
+
+// The same for complex128 blocks (lanes and rows as above).  A double takes
+// two shuffles, so column k and row k of X go through shared memory (buf: 48
+// values).  Bound by the latency of the chain pivot -> reciprocal -> next
+// pivot, so that chain is kept to itself: every lane forms the next pivot
+// a_{k+1,k+1} - a_{k+1,k}^2 / d from the column of this step and inverts it
+// while the block's updates and their exchange run.  The L entry of column k
+// and the update of the columns right of it are one multiply-add with a
+// per-lane factor.  dinv receives the reciprocal pivots.
+__device__ __forceinline__ bool elim16_warp(double2 (*A)[68], double2 (*Xs)[17], int s0, int lane, double2 *buf,
+                                            double2 *dinv) {
+  const unsigned FULL = 0xffffffffu;
+  const int c = lane & 15, ih = lane >> 4;
+  double2 *colb = buf, *rowb = buf + 16, *diag = buf + 32;
+  double2 a[8], x[8];
+#pragma unroll
+  for (int m = 0; m < 8; m++) {
+    const int i = ih + 2 * m;
+    a[m] = (c <= i) ? A[s0 + i][s0 + c] : A[s0 + c][s0 + i];
+    x[m] = (i == c) ? make_double2(1.0, 0.0) : make_double2(0.0, 0.0);
+    if (c == 0) colb[i] = a[m];
+    if (c == 1 && i == 1) diag[0] = a[m];
+  }
+  if (ih == 0) rowb[c] = x[0];
+  __syncwarp();
+  bool ok = true;
+  double2 d = colb[0];
+#pragma unroll 2
+  for (int k = 0; k < 16; k++) {
+    const double d2 = fma(d.x, d.x, d.y * d.y);
+    ok = ok && d2 > 1e-290 && d2 < 1e290;
+    const double rd = rcp_nr(d2);
+    const double2 inv_d = make_double2(d.x * rd, -d.y * rd);
+    const double2 akc = colb[c], xk = rowb[c], an = colb[min(k + 1, 15)], dn = diag[0];
+    double2 aik[8];
+#pragma unroll
+    for (int m = 0; m < 8; m++) aik[m] = colb[ih + 2 * m];
+    __syncwarp();
+    d = csub(dn, cmul(cmul(an, an), inv_d));
+    if (lane == 0) dinv[k] = inv_d;
+    const double2 f = c > k ? cneg(cmul(akc, inv_d)) : inv_d, xf = cneg(cmul(inv_d, xk));
+#pragma unroll
+    for (int m = 0; m < 8; m++) {
+      const int i = ih + 2 * m;
+      double2 u = c > k ? a[m] : make_double2(0.0, 0.0), v = x[m];
+      cfma(u, aik[m], f);
+      cfma(v, aik[m], xf);
+      if (i > k && c >= k) a[m] = u;
+      if (i > k) x[m] = v;
+      if (c == k + 1) colb[i] = a[m];
+      if (i == k + 1) rowb[c] = x[m];
+      if (i == k + 2 && c == k + 2) diag[0] = a[m];
+    }
+    __syncwarp();
+  }
+  if (!__all_sync(FULL, ok)) return elim16_any(A, Xs, s0, lane, dinv);
+#pragma unroll
+  for (int m = 0; m < 8; m++) {
+    const int i = ih + 2 * m;
+    if (c <= i) A[s0 + i][s0 + c] = a[m];
+    Xs[i][c] = x[m];
+  }
+  return true;
+}
+
+// (cr, ci) += a b on an 8 x 8 tile by FP64 matrix instructions: a[row lane / 4]
+// [k lane % 4], b[k lane % 4][col lane / 4]; the accumulators hold columns
+// 2 (lane % 4) + {0, 1} of row lane / 4
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+__device__ __forceinline__ void zmma(double (&cr)[2], double (&ci)[2], double2 a, double2 b) {
+  dmma(cr, a.x, b.x);
+  dmma(ci, a.x, b.y);
+  dmma(cr, -a.y, b.y);
+  dmma(ci, a.y, b.x);
+}
+
+// Shared memory of a diagonal tile's factorisation: the tile A, the sub-panel
+// Wp, the inverses Xd of its 16 x 16 diagonal blocks, its inverse LI.  The
+// leading dimension of complex128 tiles suits the FP64 matrix instruction's
+// fragments (8 rows x 4 columns of 16 bytes without bank conflicts).
+template <class C> struct DiagSmem {
+  static constexpr int LD = sizeof(C) == 16 ? 68 : 65;
+  static constexpr size_t bytes = sizeof(C) * (2 * 64 * LD + 64 * 17 + 4 * 16 * 17 + 16) + 16;
+  C (*A)[LD];
+  C (*Wp)[17];
+  C (*Xd)[16][17];
+  C (*LI)[LD];
+  C *dinv;
+  int *bad;
+  __device__ explicit DiagSmem(unsigned char *smem) {
+    C *p = reinterpret_cast<C *>(smem);
+    A = reinterpret_cast<C(*)[LD]>(p);
+    Wp = reinterpret_cast<C(*)[17]>(p + 64 * LD);
+    Xd = reinterpret_cast<C(*)[16][17]>(p + 64 * LD + 64 * 17);
+    LI = reinterpret_cast<C(*)[LD]>(p + 64 * LD + 64 * 17 + 4 * 16 * 17);
+    dinv = p + 2 * 64 * LD + 64 * 17 + 4 * 16 * 17;
+    bad = reinterpret_cast<int *>(dinv + 16);
+  }
+};
+
+// Blocked factorisation of a 64 x 64 diagonal tile: four 16-wide sub-panels;
+// warp 0 eliminates the 16 x 16 diagonal sub-block in registers (elim16_warp,
+// which also forms its unit-lower inverse), then the CTA computes the sub-panel
+// below it and the trailing update (complex64: up to three rows, four columns
+// per thread; complex128: 8 x 8 tiles of matrix instructions per warp).  The
+// 64 x 64 inverse is assembled from the four 16 x 16 inverses by recursive
+// doubling (16-wide pairs, then the 32-wide halves), each phase a small product
+// with several independent sums per thread.  Rows and columns at or beyond b
+// are padded with the identity (D = 1, L = 0).
+constexpr size_t DIAG_BLOCKED_SMEM = DiagSmem<float2>::bytes;
 
 // The diagonal tile as the blocked factorisation expects it in shared memory:
 // lower triangle of F at (j, j), zeros above, identity padding beyond b.
@@ -401,24 +479,26 @@ __device__ __forceinline__ void diag_tile_update_smem(int64_t N, int64_t j, int 
 // four 16 x 16 diagonal blocks.  loaded: the tile is already in shared memory
 // (diag_tile_load, possibly updated by diag_tile_update_smem).  Returns false
 // after a breakdown (uniform).
-__device__ bool ldlt_diag_phase1(int64_t N, int64_t j, int b, float2 *__restrict__ F, unsigned *__restrict__ err,
+template <class C>
+__device__ bool ldlt_diag_phase1(int64_t N, int64_t j, int b, C *__restrict__ F, unsigned *__restrict__ err,
                                  unsigned char *smem, bool loaded) {
-  float2(*A)[65] = reinterpret_cast<float2(*)[65]>(smem);
-  float2(*Wp)[17] = reinterpret_cast<float2(*)[17]>(smem + sizeof(float2) * 64 * 65);
-  float2(*Xd)[16][17] = reinterpret_cast<float2(*)[16][17]>(smem + sizeof(float2) * (64 * 65 + 64 * 17));
-  float2 *dinv = reinterpret_cast<float2 *>(smem + sizeof(float2) * (2 * 64 * 65 + 64 * 17 + 4 * 16 * 17));
-  volatile int *bad = reinterpret_cast<volatile int *>(dinv + 16);
+  DiagSmem<C> sm(smem);
+  auto A = sm.A;
+  auto Wp = sm.Wp;
+  auto Xd = sm.Xd;
+  C *dinv = sm.dinv;
+  volatile int *bad = sm.bad;
   const int t = threadIdx.x;  // 256 threads
   if (!loaded) {
-    float2 v[16];
+    C v[16];
 #pragma unroll
     for (int m = 0; m < 16; m++) {
       const int e = t + 256 * m, i = e >> 6, c = e & 63;
-      v[m] = make_float2(0.f, 0.f);
+      v[m] = czero<C>();
       if (i < b && c < b) {
         if (c <= i) v[m] = F[(j + i) * N + j + c];
       } else if (i == c) {
-        v[m] = make_float2(1.f, 0.f);
+        v[m] = cone<C>();
       }
     }
 #pragma unroll
@@ -432,7 +512,7 @@ __device__ bool ldlt_diag_phase1(int64_t N, int64_t j, int b, float2 *__restrict
   for (int s = 0; s < 4; s++) {
     const int s0 = 16 * s;
     if (t < 32) {
-      if (!elim16_warp(A, Xd[s], s0, t)) {  // uniform over the warp
+      if (!elim16_warp(A, Xd[s], s0, t, &Wp[0][0], dinv)) {  // uniform over the warp
         if (t == 0) {
           atomicOr(err, 2u);
           *bad = 1;
@@ -443,26 +523,60 @@ __device__ bool ldlt_diag_phase1(int64_t N, int64_t j, int b, float2 *__restrict
     if (*bad) return false;  // uniform
     if (s == 3) break;
     const int nr = 48 - s0;
+    if constexpr (sizeof(C) == 16) {
+      // FP64 matrix instructions on 8 x 8 tiles: W = A21 X^T (12, 8 or 4
+      // tiles), L21 = W / D, then the lower tiles of A22 -= W L21^T (21, 10
+      // or 3); a warp takes every eighth tile
+      const int warp = t >> 5, l4 = t & 3, l8 = (t & 31) >> 2, n8 = nr / 8;
+      for (int q = warp; q < 2 * n8; q += 8) {
+        const int r = s0 + 16 + 8 * (q >> 1), cj = 8 * (q & 1);
+        double wr[2] = {0.0, 0.0}, wi[2] = {0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < 16; k += 4)
+          if (k < cj + 8) zmma(wr, wi, A[r + l8][s0 + k + l4], Xd[s][cj + l8][k + l4]);
+#pragma unroll
+        for (int u = 0; u < 2; u++) Wp[r + l8][cj + 2 * l4 + u] = make_double2(wr[u], wi[u]);
+      }
+      __syncthreads();
+      for (int e = t; e < nr * 16; e += blockDim.x) {
+        const int r = s0 + 16 + (e >> 4), c = e & 15;
+        A[r][s0 + c] = cmul(Wp[r][c], dinv[c]);
+      }
+      __syncthreads();
+      for (int q = warp; q < n8 * (n8 + 1) / 2; q += 8) {
+        int ti = 0, tj = q;
+        while (tj > ti) tj -= ++ti;  // tile (ti, tj), row by row of the lower triangle
+        const int r = s0 + 16 + 8 * ti, cc = s0 + 16 + 8 * tj;
+        double ur[2] = {0.0, 0.0}, ui[2] = {0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < 16; k += 4) zmma(ur, ui, Wp[r + l8][k + l4], A[cc + l8][s0 + k + l4]);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          C &v = A[r + l8][cc + 2 * l4 + u];
+          v = csub(v, make_double2(ur[u], ui[u]));
+        }
+      }
+      __syncthreads();
+      continue;
+    }
     // 1 / D of the 16 pivots; sub-panel W = A21 X^T with up to three outputs
     // per thread accumulated together
     if (t < 16) {
-      const float2 dd = A[s0 + t][s0 + t];
-      const float rd = rcp_nr(fmaf(dd.x, dd.x, dd.y * dd.y));
-      dinv[t] = make_float2(dd.x * rd, -dd.y * rd);
+      dinv[t] = pivot_inverse(A[s0 + t][s0 + t]);
     }
     {
-      float2 acc[3];
+      C acc[3];
       int rr[3];
       const int c = t & 15;
 #pragma unroll
       for (int u = 0; u < 3; u++) {
-        acc[u] = make_float2(0.f, 0.f);
+        acc[u] = czero<C>();
         rr[u] = s0 + 16 + (t >> 4) + 16 * u;
       }
 #pragma unroll
       for (int k = 0; k < 16; k++) {
         if (k <= c) {
-          const float2 xk = Xd[s][c][k];
+          const C xk = Xd[s][c][k];
 #pragma unroll
           for (int u = 0; u < 3; u++)
             if (rr[u] < 64) cfma(acc[u], A[rr[u]][s0 + k], xk);
@@ -484,10 +598,10 @@ __device__ bool ldlt_diag_phase1(int64_t N, int64_t j, int b, float2 *__restrict
       for (int e = t; e < nr * ncq; e += blockDim.x) {
         const int i = s0 + 16 + e / ncq, j0 = s0 + 16 + 4 * (e % ncq);
         if (j0 > i) continue;
-        float2 acc[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        C acc[4] = {czero<C>(), czero<C>(), czero<C>(), czero<C>()};
 #pragma unroll
         for (int k = 0; k < 16; k++) {
-          const float2 w = Wp[i][k];
+          const C w = Wp[i][k];
 #pragma unroll
           for (int q = 0; q < 4; q++) cfma(acc[q], w, A[min(j0 + q, 63)][s0 + k]);
         }
@@ -508,24 +622,26 @@ __device__ bool ldlt_diag_phase1(int64_t N, int64_t j, int b, float2 *__restrict
 // Phase 2: the unit-lower inverse of the factored tile (L in shared memory)
 // by recursive doubling from the four 16 x 16 inverses of phase 1, and its
 // store to Linv.
-__device__ void ldlt_diag_phase2(float2 *__restrict__ Linv, unsigned char *smem, bool skip_diag_blocks = false) {
-  float2(*A)[65] = reinterpret_cast<float2(*)[65]>(smem);
-  float2(*Wp)[17] = reinterpret_cast<float2(*)[17]>(smem + sizeof(float2) * 64 * 65);
-  float2(*Xd)[16][17] = reinterpret_cast<float2(*)[16][17]>(smem + sizeof(float2) * (64 * 65 + 64 * 17));
-  float2(*LI)[65] = reinterpret_cast<float2(*)[65]>(smem + sizeof(float2) * (64 * 65 + 64 * 17 + 4 * 16 * 17));
+template <class C>
+__device__ void ldlt_diag_phase2(C *__restrict__ Linv, unsigned char *smem, bool skip_diag_blocks = false) {
+  DiagSmem<C> sm(smem);
+  auto A = sm.A;
+  auto Wp = sm.Wp;
+  auto Xd = sm.Xd;
+  auto LI = sm.LI;
   const int t = threadIdx.x;
   // Linv by recursive doubling: 16-level pairs, then the 32-level block
   //   [[X0, 0], [-X1 L10 X0, X1]]
   for (int e = t; e < 64 * 64; e += blockDim.x) {
     const int i = e >> 6, c = e & 63;
-    LI[i][c] = ((i >> 4) == (c >> 4)) ? Xd[i >> 4][i & 15][c & 15] : make_float2(0.f, 0.f);
+    LI[i][c] = ((i >> 4) == (c >> 4)) ? Xd[i >> 4][i & 15][c & 15] : czero<C>();
   }
   // phase A: T_h = L[32h+16.., 32h..] Xd[2h] (two 16 x 16 products, 2 outputs per thread)
   {
 #pragma unroll
     for (int u = 0; u < 2; u++) {
       const int e = t + 256 * u, h = e >> 8, r = (e >> 4) & 15, c = e & 15;
-      float2 p0 = make_float2(0.f, 0.f), p1 = make_float2(0.f, 0.f);
+      C p0 = czero<C>(), p1 = czero<C>();
 #pragma unroll
       for (int k = 0; k < 16; k += 2) {
         cfma(p0, A[32 * h + 16 + r][32 * h + k], Xd[2 * h][k][c]);
@@ -540,14 +656,14 @@ __device__ void ldlt_diag_phase2(float2 *__restrict__ Linv, unsigned char *smem,
 #pragma unroll
     for (int u = 0; u < 2; u++) {
       const int e = t + 256 * u, h = e >> 8, r = (e >> 4) & 15, c = e & 15;
-      float2 p0 = make_float2(0.f, 0.f), p1 = make_float2(0.f, 0.f);
+      C p0 = czero<C>(), p1 = czero<C>();
 #pragma unroll
       for (int k = 0; k < 16; k += 2) {
         if (k <= r) cfma(p0, Xd[2 * h + 1][r][k], Wp[32 * h + k][c]);
         if (k + 1 <= r) cfma(p1, Xd[2 * h + 1][r][k + 1], Wp[32 * h + k + 1][c]);
       }
-      const float2 acc = cadd(p0, p1);
-      LI[32 * h + 16 + r][32 * h + c] = make_float2(-acc.x, -acc.y);
+      const C acc = cadd(p0, p1);
+      LI[32 * h + 16 + r][32 * h + c] = cneg(acc);
     }
   }
   __syncthreads();
@@ -556,11 +672,11 @@ __device__ void ldlt_diag_phase2(float2 *__restrict__ Linv, unsigned char *smem,
   // Wp[32 + r][c - 16] for c >= 16)
   {
     const int c = t & 31, r0 = t >> 5;  // rows r0, r0 + 8, r0 + 16, r0 + 24
-    float2 p[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    C p[4] = {czero<C>(), czero<C>(), czero<C>(), czero<C>()};
 #pragma unroll
     for (int k = 0; k < 32; k++) {
       if (k >= c) {
-        const float2 x = LI[k][c];
+        const C x = LI[k][c];
 #pragma unroll
         for (int q = 0; q < 4; q++) cfma(p[q], A[32 + r0 + 8 * q][k], x);
       }
@@ -577,109 +693,22 @@ __device__ void ldlt_diag_phase2(float2 *__restrict__ Linv, unsigned char *smem,
   // phase D: LI[32 + r][c] = -X_b U, X_b = LI[32.., 32..] lower (k <= r)
   {
     const int c = t & 31, r0 = t >> 5;
-    float2 p[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    C p[4] = {czero<C>(), czero<C>(), czero<C>(), czero<C>()};
 #pragma unroll
     for (int k = 0; k < 32; k++) {
-      const float2 u = c < 16 ? Wp[k][c] : Wp[32 + k][c - 16];
+      const C u = c < 16 ? Wp[k][c] : Wp[32 + k][c - 16];
 #pragma unroll
       for (int q = 0; q < 4; q++)
         if (k <= r0 + 8 * q) cfma(p[q], LI[32 + r0 + 8 * q][32 + k], u);
     }
 #pragma unroll
-    for (int q = 0; q < 4; q++) LI[32 + r0 + 8 * q][c] = make_float2(-p[q].x, -p[q].y);
+    for (int q = 0; q < 4; q++) LI[32 + r0 + 8 * q][c] = cneg(p[q]);
   }
   __syncthreads();
   // (skip_diag_blocks: the 16 x 16 diagonal blocks were stored already)
   for (int e = t; e < 64 * 64; e += blockDim.x)
     if (!skip_diag_blocks || (e >> 10) != ((e & 63) >> 4)) Linv[e] = LI[e >> 6][e & 63];
   __syncthreads();
-}
-
-// Blocked form of ldlt_diag_block for complex64 blocks: phase 1 (with the
-// 16 x 16 inverses), the store of L and D, phase 2.
-__device__ void ldlt_diag_blocked(int64_t N, int64_t j, int b, float2 *__restrict__ F, float2 *__restrict__ Linv,
-                                  unsigned *__restrict__ err, unsigned char *smem, bool loaded = false) {
-  if (!ldlt_diag_phase1(N, j, b, F, err, smem, loaded)) return;
-  ldlt_diag_phase2(Linv, smem);
-}
-template <class C>
-__global__ void __launch_bounds__(256) k_ldlt_diag(int64_t N, int64_t j, int b, C *__restrict__ F,
-                                                   C *__restrict__ Linv, unsigned *__restrict__ err) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  if constexpr (std::is_same<C, float2>::value)
-    ldlt_diag_blocked(N, j, b, F, Linv, err, smem_raw);
-  else
-    ldlt_diag_block<C>(N, j, b, F, Linv, err, reinterpret_cast<C *>(smem_raw));
-}
-
-// Panel: W = A21 Linv^T (row r: W[r][c] = sum_{k<=c} A21[r][k] Linv[c][k]),
-// then L21 = W D^-1, for the 64 rows from r0.  Reads go through L2 (the
-// fused step kernel reads blocks written by another CTA of the same launch).
-// a_in_smem: the A21 tile is already in As (ldlt_strip_update_smem)
-template <class C>
-__device__ __forceinline__ void ldlt_panel_rows(int64_t N, int64_t j, int b, int64_t r0, C *__restrict__ F,
-                                                const C *__restrict__ Linv, C *__restrict__ W, int wstride,
-                                                int woff, unsigned char *smem_raw, bool a_in_smem = false) {
-  C(*As)[NB + 1] = reinterpret_cast<C(*)[NB + 1]>(smem_raw);
-  C(*Li)[NB + 1] = reinterpret_cast<C(*)[NB + 1]>(smem_raw + sizeof(C) * NB * (NB + 1));
-  C *dg = reinterpret_cast<C *>(smem_raw + 2 * sizeof(C) * NB * (NB + 1));
-  if (a_in_smem) {
-    C vl[16];
-#pragma unroll
-    for (int m = 0; m < 16; m++) vl[m] = __ldcg(Linv + threadIdx.x + 256 * m);
-#pragma unroll
-    for (int m = 0; m < 16; m++) {
-      const int e = threadIdx.x + 256 * m;
-      Li[e / NB][e % NB] = vl[m];
-    }
-  } else {
-    // 256 threads: all 32 loads of a thread in flight before the shared stores
-    C va[16], vl[16];
-#pragma unroll
-    for (int m = 0; m < 16; m++) {
-      const int e = threadIdx.x + 256 * m, rr = e / NB, k = e % NB;
-      const int64_t r = r0 + rr;
-      va[m] = (r < N && k < b) ? __ldcg(F + r * N + j + k) : czero<C>();
-      vl[m] = __ldcg(Linv + rr * NB + k);
-    }
-#pragma unroll
-    for (int m = 0; m < 16; m++) {
-      const int e = threadIdx.x + 256 * m;
-      As[e / NB][e % NB] = va[m];
-      Li[e / NB][e % NB] = vl[m];
-    }
-  }
-  if (threadIdx.x < b) dg[threadIdx.x] = __ldcg(F + (j + threadIdx.x) * N + j + threadIdx.x);
-  __syncthreads();
-  // thread (c, rq) owns column c of rows rq, rq + 4, ..., rq + 60: sixteen
-  // independent accumulators per Linv entry
-  const int c = threadIdx.x & 63, rq = threadIdx.x >> 6;
-  if (c >= b) return;
-  C acc[16];
-#pragma unroll
-  for (int t = 0; t < 16; t++) acc[t] = czero<C>();
-  for (int k = 0; k <= c; k++) {
-    const C lk = Li[c][k];
-#pragma unroll
-    for (int t = 0; t < 16; t++) cfma(acc[t], As[rq + 4 * t][k], lk);
-  }
-  const C inv = cdiv(cone<C>(), dg[c]);
-#pragma unroll
-  for (int t = 0; t < 16; t++) {
-    const int64_t r = r0 + rq + 4 * t;
-    if (r < N) {
-      W[r * wstride + woff + c] = acc[t];
-      F[r * N + j + c] = cmul(acc[t], inv);
-    }
-  }
-}
-
-template <class C>
-__global__ void __launch_bounds__(256) k_ldlt_panel(int64_t N, int64_t j, int b, C *__restrict__ F,
-                                                    const C *__restrict__ Linv, C *__restrict__ W, int wstride,
-                                                    int woff) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  ldlt_panel_rows<C>(N, j, b, j + b + (int64_t)blockIdx.x * NB, F, Linv, W, wstride, woff, smem_raw);
 }
 
 // Panel rows of the fused step by blocked forward substitution, W L11^T =
@@ -865,39 +894,29 @@ __device__ __forceinline__ void ldlt_strip_update_smem(int64_t N, int64_t r0, in
     }
 }
 
-// Trailing / strip update on tiles (grid.x row tiles, grid.y column tiles from
-// r_lo; tiles entirely above the diagonal exit at once).
-//
-// diag_b > 0: the CTA of tile (0, 0) -- the diagonal block at r_lo, which is
-// the next panel's -- factors that block right after updating it
-// (ldlt_diag_block, Linv_next), while the other CTAs finish the strip.
+// Trailing update of a complex64 factor on FP32 units (grid.x row tiles, grid.y
+// column tiles from r_lo; tiles entirely above the diagonal exit at once).
 template <class C>
 __global__ void __launch_bounds__(256) k_ldlt_update(int64_t N, int64_t r_lo, int64_t c_hi, int64_t jcol, int K,
                                                      C *__restrict__ F, const C *__restrict__ W, int wstride,
-                                                     int woff, int diag_b, C *__restrict__ Linv_next,
-                                                     unsigned *__restrict__ err) {
+                                                     int woff) {
   __shared__ C Ws[16][65];
   __shared__ C Ls[16][65];
   const int64_t r0 = r_lo + (int64_t)blockIdx.x * 64, c0 = r_lo + (int64_t)blockIdx.y * 64;
   if (r0 >= N || c0 >= c_hi || c0 > r0 + 63) return;
   ldlt_tile_update<C>(N, r0, c0, c_hi, jcol, K, F, W, wstride, woff, Ws, Ls);
-  if (diag_b > 0 && blockIdx.x == 0 && blockIdx.y == 0) {
-    __syncthreads();  // the tile's writes are visible to the whole CTA
-    ldlt_diag_block<C>(N, r_lo, diag_b, F, Linv_next, err, &Ws[0][0]);
-  }
 }
 
-// One panel step inside a 256-wide middle panel, fused: strip update of the
+// One panel step inside a 256-wide middle panel (complex64), fused: strip update of the
 // columns [r_lo, c_hi) by the panel at jcol; the CTA holding ticket 0 updates
 // the next diagonal block (tile (0, 0)), factors it and publishes its inverse
 // (sync[1]); every other CTA of column tile 0 then runs the next panel on its
 // own rows (W at woff_next, L21 = W D^-1).  Tickets are drawn in launch order,
 // so the CTA that the others wait for is already running; the wait is bounded
 // (error bit 4 on expiry).
-template <class C>
 __global__ void __launch_bounds__(256) k_ldlt_step(int64_t N, int64_t r_lo, int64_t c_hi, int64_t jcol, int K,
-                                                   C *__restrict__ F, C *__restrict__ W, int wstride, int woff,
-                                                   int woff_next, int nb_next, C *__restrict__ Linv_next,
+                                                   float2 *__restrict__ F, float2 *__restrict__ W, int wstride, int woff,
+                                                   int woff_next, int nb_next, float2 *__restrict__ Linv_next,
                                                    unsigned *__restrict__ sync, unsigned *__restrict__ err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned s_ticket;
@@ -910,50 +929,41 @@ __global__ void __launch_bounds__(256) k_ldlt_step(int64_t N, int64_t r_lo, int6
   const int ct = (int)(t % nct);
   const int64_t r0 = r_lo + rt * 64, c0 = r_lo + (int64_t)ct * 64;
   if (r0 >= N || c0 > r0 + 63) return;
-  C(*Ws)[65] = reinterpret_cast<C(*)[65]>(smem_raw);
-  C(*Ls)[65] = reinterpret_cast<C(*)[65]>(smem_raw + sizeof(C) * 16 * 65);
+  float2(*Ws)[65] = reinterpret_cast<float2(*)[65]>(smem_raw);
+  float2(*Ls)[65] = reinterpret_cast<float2(*)[65]>(smem_raw + sizeof(float2) * 16 * 65);
   if (t == 0) {
     // the next diagonal tile: loaded once, updated and factored in shared
     // memory (complex64); the update's K chunks are staged in the space of
     // the tile's inverse
-    if constexpr (std::is_same<C, float2>::value) {
-      float2(*A)[65] = reinterpret_cast<float2(*)[65]>(smem_raw);
-      float2(*St)[16][65] =
-          reinterpret_cast<float2(*)[16][65]>(smem_raw + sizeof(float2) * (64 * 65 + 64 * 17 + 4 * 16 * 17));
-      diag_tile_load(N, r_lo, nb_next, F, A);
-      diag_tile_update_smem(N, r_lo, nb_next, jcol, K, F, W, wstride, woff, A, St);
-      // L, D and the 16 x 16 diagonal blocks of the inverse are published
-      // first (the panel rows need only them); the rest of the tile's
-      // inverse, for the solves, is formed while the panel rows run
-      const bool ok = ldlt_diag_phase1(N, r_lo, nb_next, F, err, smem_raw, true);
-      if (ok) {
-        float2(*Xd)[16][17] = reinterpret_cast<float2(*)[16][17]>(smem_raw + sizeof(float2) * (64 * 65 + 64 * 17));
-        for (int e = threadIdx.x; e < 4 * 256; e += 256) {
-          const int s = e >> 8, i = (e >> 4) & 15, c = e & 15;
-          Linv_next[(16 * s + i) * NB + 16 * s + c] = Xd[s][i][c];
-        }
+    float2(*A)[65] = reinterpret_cast<float2(*)[65]>(smem_raw);
+    float2(*St)[16][65] =
+        reinterpret_cast<float2(*)[16][65]>(smem_raw + sizeof(float2) * (64 * 65 + 64 * 17 + 4 * 16 * 17));
+    diag_tile_load(N, r_lo, nb_next, F, A);
+    diag_tile_update_smem(N, r_lo, nb_next, jcol, K, F, W, wstride, woff, A, St);
+    // L, D and the 16 x 16 diagonal blocks of the inverse are published
+    // first (the panel rows need only them); the rest of the tile's
+    // inverse, for the solves, is formed while the panel rows run
+    const bool ok = ldlt_diag_phase1(N, r_lo, nb_next, F, err, smem_raw, true);
+    if (ok) {
+      float2(*Xd)[16][17] = reinterpret_cast<float2(*)[16][17]>(smem_raw + sizeof(float2) * (64 * 65 + 64 * 17));
+      for (int e = threadIdx.x; e < 4 * 256; e += 256) {
+        const int s = e >> 8, i = (e >> 4) & 15, c = e & 15;
+        Linv_next[(16 * s + i) * NB + 16 * s + c] = Xd[s][i][c];
       }
-      __threadfence();
-      __syncthreads();
-      if (threadIdx.x == 0) atomicExch(&sync[1], 1u);
-      if (ok) ldlt_diag_phase2(Linv_next, smem_raw, true);
-    } else {
-      ldlt_tile_update<C>(N, r0, c0, c_hi, jcol, K, F, W, wstride, woff, Ws, Ls);
-      __syncthreads();
-      ldlt_diag_block<C>(N, r_lo, nb_next, F, Linv_next, err, reinterpret_cast<C *>(smem_raw));
-      __threadfence();
-      __syncthreads();
-      if (threadIdx.x == 0) atomicExch(&sync[1], 1u);
     }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) atomicExch(&sync[1], 1u);
+    if (ok) ldlt_diag_phase2(Linv_next, smem_raw, true);
     return;
   }
   if (ct != 0) {
-    ldlt_tile_update<C>(N, r0, c0, c_hi, jcol, K, F, W, wstride, woff, Ws, Ls);
+    ldlt_tile_update<float2>(N, r0, c0, c_hi, jcol, K, F, W, wstride, woff, Ws, Ls);
     return;
   }
   // column 0: the strip tile is the next panel's A21 tile; it stays in
   // shared memory for the panel rows after the diagonal block is published
-  ldlt_strip_update_smem<C>(N, r0, c0, nb_next, jcol, K, F, W, wstride, woff, smem_raw);
+  ldlt_strip_update_smem<float2>(N, r0, c0, nb_next, jcol, K, F, W, wstride, woff, smem_raw);
   if (threadIdx.x == 0) {
     long long it = 0;
     int ok = 1;
@@ -970,10 +980,7 @@ __global__ void __launch_bounds__(256) k_ldlt_step(int64_t N, int64_t r_lo, int6
   }
   __syncthreads();
   if (!s_ok) return;
-  if constexpr (std::is_same<C, float2>::value)
-    ldlt_panel_rows_blk(N, r_lo, nb_next, r0, F, Linv_next, W, wstride, woff_next, smem_raw);
-  else
-    ldlt_panel_rows<C>(N, r_lo, nb_next, r0, F, Linv_next, W, wstride, woff_next, smem_raw, true);
+  ldlt_panel_rows_blk(N, r_lo, nb_next, r0, F, Linv_next, W, wstride, woff_next, smem_raw);
 }
 
 // The first 64-wide block of a middle panel (complex64), one launch: the
@@ -981,7 +988,7 @@ __global__ void __launch_bounds__(256) k_ldlt_step(int64_t N, int64_t r_lo, int6
 // L, D and the 16 x 16 inverse blocks, then forms the rest of the inverse
 // (phase 2); every other CTA loads its 64 rows of the block column, waits for
 // the publication (bounded, error bit 4 on expiry) and runs its panel rows
-// by blocked forward substitution.  Replaces k_ldlt_diag + k_ldlt_panel.
+// by blocked forward substitution.
 __global__ void __launch_bounds__(256) k_ldlt_first(int64_t N, int64_t j, int b, float2 *__restrict__ F,
                                                     float2 *__restrict__ Linv, float2 *__restrict__ W, int wstride,
                                                     int woff, unsigned *__restrict__ sync,
@@ -1041,6 +1048,279 @@ __global__ void __launch_bounds__(256) k_ldlt_first(int64_t N, int64_t j, int b,
   __syncthreads();
   if (!s_ok) return;
   ldlt_panel_rows_blk(N, j, b, r0, F, Linv, W, wstride, woff, smem_raw);
+}
+
+// ---------------------------------------------------------------------------
+// A 256-wide middle panel of a complex128 factor in one launch, driven by data
+// flow.  The CTA that draws ticket r owns the 64-row tile r (rows J + 64 r ..)
+// of the panel's four 64-wide block columns s:
+//   * r > s: T = A_rs - sum_{q<s} W_rq L_sq^T as soon as tile s has published
+//     its L_sq; then, once tile s has published its factored diagonal block,
+//     W_rs L_ss^T = T by forward substitution with the inverses of the 16 x 16
+//     blocks (each warp alone on 8 rows), L_rs = W_rs D_s^-1;
+//   * r < 4: after each block column its own diagonal tile is updated by
+//     W_rs L_rs^T; the last of these updates goes straight to the tile's
+//     factorisation (r = s).
+// The chain is then, per 64 columns, one factorisation, one substitution and
+// one 64 x 64 x 64 update on a single SM; everything else runs while others
+// wait.  Tickets are drawn in launch order and a CTA waits only for tiles 0-3,
+// which started before it; the waits are bounded (error bit 4).
+// The products are FP64 matrix instructions (mma.sync m8n8k4, full FP64
+// multiply-adds; 37.0 TFLOP/s measured against 33.1 for FMA), which leave the
+// shared-memory pipe idle enough to sit at the FP64 rate with eight warps.
+// Measured: 220 us a panel of 7,680 rows; before, a launch with the 64-column
+// strip update and the next diagonal block (105-130 us) and one with its panel
+// rows (17-28 us) per 64 columns.
+// ---------------------------------------------------------------------------
+// spin until *flag is set (one thread); false on expiry
+__device__ __forceinline__ bool wait_word(volatile unsigned *flag, unsigned *err) {
+  long long it = 0;
+  while (*flag == 0u) {
+    if (++it > SPIN_LIMIT) {
+      atomicOr(err, 4u);
+      return false;
+    }
+    __nanosleep(32);
+  }
+  __threadfence();
+  return true;
+}
+
+constexpr int MID_WORDS = 24;  // per middle panel: ticket, diagonal flags [4], row flags [4][4]
+
+__global__ void __launch_bounds__(256, 1) k_ldlt_mid64(int64_t N, int64_t J, int w, double2 *__restrict__ F,
+                                                       double2 *__restrict__ Linv, double2 *__restrict__ W,
+                                                       int wstride, unsigned *sync, unsigned *err) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ unsigned s_ticket;
+  __shared__ int s_ok;
+  constexpr int LD = DiagSmem<double2>::LD;
+  DiagSmem<double2> sm(smem_raw);
+  double2(*As)[LD] = sm.A;
+  double2(*Ls)[LD] = sm.LI;
+  double2 *dinv = &sm.Wp[0][0];  // 64 reciprocal pivots
+  unsigned *diag_flag = sync + 1, *row_flag = sync + 5;
+  if (threadIdx.x == 0) s_ticket = atomicAdd(sync, 1u);
+  __syncthreads();
+  const int rt = (int)s_ticket;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, l4 = lane & 3, l8 = lane >> 2;
+  const int nsb = (w + 63) / 64;
+  const int64_t r0 = J + 64 * (int64_t)rt;
+  const int nr = (int)min((int64_t)64, N - r0);
+  // wait for a flag, the whole CTA (uniform result)
+  auto wait = [&](unsigned *flag) {
+    if (t == 0) s_ok = wait_word(flag, err) ? 1 : 0;
+    __syncthreads();
+    const bool ok = s_ok != 0;
+    __syncthreads();
+    return ok;
+  };
+  auto publish = [&](unsigned *flag) {
+    __threadfence();
+    __syncthreads();
+    if (t == 0) atomicExch(flag, 1u);
+  };
+  // T[64][LD] <- G rows (row r at G + r ld), zero outside nrow x ncol
+  auto stage = [&](double2(*T)[LD], const double2 *G, int64_t ld, int nrow, int ncol) {
+    double2 v[16];
+#pragma unroll
+    for (int m = 0; m < 16; m++) {
+      const int e = t + 256 * m, i = e >> 6, c = e & 63;
+      v[m] = (i < nrow && c < ncol) ? __ldcg(G + i * ld + c) : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+    for (int m = 0; m < 16; m++) {
+      const int e = t + 256 * m;
+      T[e >> 6][e & 63] = v[m];
+    }
+  };
+  // rows 16 (warp / 2) .., columns 32 (warp % 2) .. of a 64 x 64 product
+  const int wr = 16 * (warp >> 1), wc = 32 * (warp & 1);
+  for (int s = 0; s < nsb && s <= rt; s++) {
+    const int64_t jc = J + 64 * s;
+    const int b = (int)min((int64_t)64, J + w - jc);
+    if (s == rt) {
+      // the diagonal tile (updated by the steps below, or untouched for r = 0)
+      if (s == 0) {
+        stage(As, F + jc * N + jc, N, b, b);
+        __syncthreads();
+      }
+      for (int e = t; e < 64 * 64; e += 256) {  // lower part, identity beyond b
+        const int i = e >> 6, c = e & 63;
+        if (i >= b || c >= b) As[i][c] = make_double2(i == c ? 1.0 : 0.0, 0.0);
+        else if (c > i) As[i][c] = make_double2(0.0, 0.0);
+      }
+      double2 *Lb = Linv + (jc / 64) * 4096;
+      const bool ok = ldlt_diag_phase1(N, jc, b, F, err, smem_raw, true);
+      if (ok)
+        for (int e = t; e < 4 * 256; e += 256) {
+          const int q = e >> 8, i = (e >> 4) & 15, c = e & 15;
+          Lb[(16 * q + i) * 64 + 16 * q + c] = sm.Xd[q][i][c];
+        }
+      publish(diag_flag + s);
+      if (ok) ldlt_diag_phase2(Lb, smem_raw, true);
+      return;
+    }
+    // acc = -A_rs + sum_q W_rq L_sq^T
+    double cr[2][4][2], ci[2][4][2];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const int rr = wr + 8 * i + l8, cc = wc + 8 * j + 2 * l4 + u;
+          const double2 v = (rr < nr && cc < b) ? __ldcg(F + (r0 + rr) * N + jc + cc) : make_double2(0.0, 0.0);
+          cr[i][j][u] = -v.x;
+          ci[i][j][u] = -v.y;
+        }
+    for (int q = 0; q < s; q++) {
+      if (!wait(row_flag + 4 * s + q)) return;
+      stage(As, W + r0 * wstride + 64 * q, wstride, nr, 64);
+      stage(Ls, F + jc * N + J + 64 * q, N, b, 64);
+      __syncthreads();
+#pragma unroll 4
+      for (int k = 0; k < 64; k += 4) {
+        double2 a[2], l[4];
+#pragma unroll
+        for (int i = 0; i < 2; i++) a[i] = As[wr + 8 * i + l8][k + l4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) l[j] = Ls[wc + 8 * j + l8][k + l4];
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) zmma(cr[i][j], ci[i][j], a[i], l[j]);
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+          As[wr + 8 * i + l8][wc + 8 * j + 2 * l4 + u] = make_double2(-cr[i][j][u], -ci[i][j][u]);
+    if (!wait(diag_flag + s)) return;
+    stage(Ls, F + jc * N + jc, N, b, b);
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      const int e = t + 256 * m, q = e >> 8, i = (e >> 4) & 15, c = e & 15;
+      sm.Xd[q][i][c] = __ldcg(Linv + (jc / 64) * 4096 + (16 * q + i) * 64 + 16 * q + c);
+    }
+    __syncthreads();
+    if (t < b) dinv[t] = pivot_inverse(Ls[t][t]);
+    // W_rs: 8 rows per warp, 16 columns at a time
+    double2(*Tw)[LD] = As + 8 * warp;
+#pragma unroll 1
+    for (int q = 0; q < 4; q++) {
+      if (16 * q >= b) break;  // uniform
+      double tr[2][2], ti[2][2];
+      if (q > 0) {
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+          for (int u = 0; u < 2; u++) {
+            const double2 v = Tw[l8][16 * q + 8 * n + 2 * l4 + u];
+            tr[n][u] = v.x;
+            ti[n][u] = v.y;
+          }
+        for (int k = 0; k < 16 * q; k += 4) {
+          const double2 a = cneg(Tw[l8][k + l4]);
+#pragma unroll
+          for (int n = 0; n < 2; n++) zmma(tr[n], ti[n], a, Ls[16 * q + 8 * n + l8][k + l4]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+          for (int u = 0; u < 2; u++)
+            Tw[l8][16 * q + 8 * n + 2 * l4 + u] = make_double2(tr[n][u], ti[n][u]);
+        __syncwarp();
+      }
+#pragma unroll
+      for (int n = 0; n < 2; n++) tr[n][0] = tr[n][1] = ti[n][0] = ti[n][1] = 0.0;
+#pragma unroll
+      for (int k = 0; k < 16; k += 4) {
+        const double2 a = Tw[l8][16 * q + k + l4];
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+          if (k < 8 * n + 8) zmma(tr[n], ti[n], a, sm.Xd[q][8 * n + l8][k + l4]);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int n = 0; n < 2; n++)
+#pragma unroll
+        for (int u = 0; u < 2; u++) Tw[l8][16 * q + 8 * n + 2 * l4 + u] = make_double2(tr[n][u], ti[n][u]);
+      __syncwarp();
+    }
+    __syncthreads();
+    const bool below = rt < nsb;   // tiles of the panel's diagonal part keep L_rs for their own update
+    const bool last = rt == s + 1;  // the factorisation of this tile comes next
+#pragma unroll 4
+    for (int m = 0; m < 16; m++) {
+      const int e = t + 256 * m, i = e >> 6, c = e & 63;
+      const double2 v = c < b ? As[i][c] : make_double2(0.0, 0.0);
+      const double2 l = c < b ? cmul(v, dinv[c]) : make_double2(0.0, 0.0);
+      if (i < nr && c < b) {
+        W[(r0 + i) * wstride + 64 * s + c] = v;
+        F[(r0 + i) * N + jc + c] = l;
+      }
+      if (below) Ls[i][c] = l;
+    }
+    if (!below) {
+      __syncthreads();
+      continue;
+    }
+    if (last) __syncthreads();  // published after the update, when the stores have drained
+    else publish(row_flag + 4 * rt + s);
+    // the own diagonal tile -= W_rs L_rs^T, 36 lower 8 x 8 tiles: warp v < 4
+    // takes row tile 7 - v, columns 0-4, warp 4 + v the rest of that row tile
+    // and row tile v (nine tiles per SM quarter)
+    {
+      const int v = warp & 3;
+      const int nt = warp < 4 ? 5 : 4;
+      double ur[5][2], ui[5][2];
+      int ti[5], tj[5];
+      double2 fd[5][2];
+#pragma unroll
+      for (int x = 0; x < 5; x++) {
+        ur[x][0] = ur[x][1] = ui[x][0] = ui[x][1] = 0.0;
+        if (warp < 4) {
+          ti[x] = 7 - v;
+          tj[x] = x;
+        } else {
+          ti[x] = x < 3 - v ? 7 - v : v;
+          tj[x] = x < 3 - v ? 5 + x : x - (3 - v);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const int i = 8 * ti[x] + l8, c = 8 * tj[x] + 2 * l4 + u;
+          fd[x][u] = (x < nt && i < nr && c <= i) ? __ldcg(F + (r0 + i) * N + r0 + c) : make_double2(0.0, 0.0);
+        }
+      }
+#pragma unroll 4
+      for (int k = 0; k < 64; k += 4) {
+#pragma unroll
+        for (int x = 0; x < 5; x++)
+          if (x < nt) zmma(ur[x], ui[x], As[8 * ti[x] + l8][k + l4], Ls[8 * tj[x] + l8][k + l4]);
+      }
+      if (last) publish(row_flag + 4 * rt + s);
+      else __syncthreads();
+#pragma unroll
+      for (int x = 0; x < 5; x++) {
+        if (x >= nt) continue;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const int i = 8 * ti[x] + l8, c = 8 * tj[x] + 2 * l4 + u;
+          if (i >= nr || c > i) continue;
+          const double2 d = csub(fd[x][u], make_double2(ur[x][u], ui[x][u]));
+          if (last) As[i][c] = d;
+          else __stcg(F + (r0 + i) * N + r0 + c, d);
+        }
+      }
+      __syncthreads();
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1264,22 +1544,19 @@ __global__ void k_scale_vec(int64_t N, int64_t R, const double2 *__restrict__ d,
   x[i] = cmul(x[i], d[i % N]);
 }
 
-template <class C> size_t diag_smem() {
-  return std::is_same<C, float2>::value ? DIAG_BLOCKED_SMEM : sizeof(C) * 2 * NB;
-}
+// the complex64 panel steps: panel rows or the diagonal tile
+constexpr size_t STEP_SMEM = std::max(sizeof(float2) * (2 * NB * (NB + 1) + NB), DIAG_BLOCKED_SMEM);
 
 template <class C> void set_smem_attrs() {
   static bool done = false;
   if (done) return;
-  size_t panel = sizeof(C) * (2 * NB * (NB + 1) + NB);
-  DMB_CUDA(cudaFuncSetAttribute(k_ldlt_panel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)panel));
-  DMB_CUDA(cudaFuncSetAttribute(k_ldlt_diag<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)diag_smem<C>()));
-  DMB_CUDA(cudaFuncSetAttribute(k_ldlt_step<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)std::max(panel, diag_smem<C>())));
-  if constexpr (std::is_same<C, float2>::value)
-    DMB_CUDA(cudaFuncSetAttribute(k_ldlt_first, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)std::max(panel, diag_smem<C>())));
+  if constexpr (std::is_same<C, float2>::value) {
+    DMB_CUDA(cudaFuncSetAttribute(k_ldlt_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STEP_SMEM));
+    DMB_CUDA(cudaFuncSetAttribute(k_ldlt_first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STEP_SMEM));
+  } else {
+    DMB_CUDA(cudaFuncSetAttribute(k_ldlt_mid64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)DiagSmem<double2>::bytes));
+  }
   DMB_CUDA(cudaFuncSetAttribute(k_trsv_fwd<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(2 * sizeof(C) * NB * NB)));
   DMB_CUDA(cudaFuncSetAttribute(k_trsv_bwd<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1288,11 +1565,11 @@ template <class C> void set_smem_attrs() {
 }
 
 // Three-level right-looking LDL^T.  Block columns of NBW = 1024 are factored
-// as 256-wide middle panels, each made of four 64-wide panels (diagonal block,
-// panel, SIMT strip updates inside the 256 columns).  After each middle panel
-// the rest of the 1024-wide block column receives one K = 256 update, and after
-// the block column the whole trailing matrix receives one K = 1024 update --
-// both on the tensor cores for complex64 factors.
+// as 256-wide middle panels (complex128: one launch; complex64: one launch per
+// 64 columns).  After each middle panel the rest of the 1024-wide block column
+// receives one K = 256 update, and after the block column the whole trailing
+// matrix receives one K = 1024 update -- on the tensor cores (complex64: split
+// operands, complex128: int8 residues).
 //
 // Lookahead (details at update_block_column / update_trailing): the next
 // panel's latency-bound diagonal/panel/strip kernels run on the main stream
@@ -1310,7 +1587,10 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
   c->d_dinv.ensure(sizeof(C) * (size_t)nblk * NB * NB);  // Linv blocks
   // err word, then two words (ticket, ready flag) per panel step
   // (then two more per 64-block for the first block of each middle panel)
-  c->d_flags.ensure(std::max<size_t>(64, 4 * (4 + 4 * (size_t)nblk)));
+  // (complex128: MID_WORDS per middle panel)
+  const size_t flag_words = 4 + (std::is_same<C, float2>::value ? 4 * (size_t)nblk
+                                                                : MID_WORDS * (size_t)((N + NBO - 1) / NBO));
+  c->d_flags.ensure(std::max<size_t>(64, 4 * flag_words));
   if (!c->stream2 || !c->stream3) {
     // the panel chain (context stream) first, then the lookahead updates,
     // then auxiliary work (right-hand sides, int8 operand planes), which only
@@ -1326,13 +1606,7 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
   unsigned *err = c->d_flags.as<unsigned>();
   C *Linv = c->d_dinv.as<C>();
   unsigned *step_sync = err + 4;
-  DMB_CUDA(cudaMemsetAsync(err, 0, 4 * (4 + 4 * (size_t)nblk), c->stream));
-  // the fused panel step (strip + next diagonal block + next panel) for
-  // complex64 factors; complex128 factors keep separate launches (their
-  // 134 KB panel staging would allow one CTA per SM)
-  const bool fuse_step = std::is_same<C, float2>::value;
-  const size_t sm_panel = sizeof(C) * (2 * NB * (NB + 1) + NB);
-  const size_t sm_step = std::max(sm_panel, diag_smem<C>());  // panel rows or the diagonal block
+  DMB_CUDA(cudaMemsetAsync(err, 0, 4 * flag_words, c->stream));
   const bool use_tc = std::is_same<C, float2>::value && dmb::tc_available(c);
   // trailing update F[r][cc] -= W[r][woff..woff+K) L[cc][jcol..jcol+K) on
   // rows >= r0, columns [r0, c_hi); slot: the packed-operand buffers of the
@@ -1352,7 +1626,7 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
         dmb::zgemm64_lower_update(c, rest, c_hi - r0, K, Wk, NBW, Lk, N, (double2 *)F + r0 * N + r0, N);
     } else {
       dim3 g(blocks_for(rest, 64), blocks_for(c_hi - r0, 64));
-      DMB_LAUNCH(c, k_ldlt_update<C>, g, 256, 0, N, r0, c_hi, jcol, K, F, Wb, NBW, woff, 0, (C *)nullptr, err);
+      DMB_LAUNCH(c, k_ldlt_update<C>, g, 256, 0, N, r0, c_hi, jcol, K, F, Wb, NBW, woff);
     }
     // algorithmic work: K complex MACs per updated lower-triangle entry
     const double cols = (double)(c_hi - r0), rows = (double)rest;
@@ -1427,38 +1701,25 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
     const int64_t J2E = std::min<int64_t>(N, J2 + NBW);
     for (int64_t J = J2; J < J2E; J += NBO) {
       const int64_t JE = std::min<int64_t>(J2E, J + NBO);
-      // diag_done / panel_done: the previous step's kernel already factored
-      // this diagonal block / ran this panel
-      bool diag_done = false, panel_done = false;
-      for (int64_t j = J; j < JE; j += NB) {
-        const int b = (int)std::min<int64_t>(NB, N - j);
-        C *Lblk = Linv + (j / NB) * NB * NB;
-        const int64_t rest = N - j - b;
-        if constexpr (std::is_same<C, float2>::value) {
-          if (!diag_done) {  // the first block of the middle panel: factor + panel rows in one launch
-            DMB_LAUNCH(c, k_ldlt_first, 1 + blocks_for(std::max<int64_t>(rest, 0), NB), 256, sm_step, N, j, b, F,
-                       Lblk, Wb, NBW, (int)(j - J2), step_sync + 2 * nblk + 2 * (j / NB), err);
-            diag_done = panel_done = true;
-          }
-        }
-        if (!diag_done) DMB_LAUNCH(c, k_ldlt_diag<C>, 1, 256, diag_smem<C>(), N, j, b, F, Lblk, err);
-        if (rest <= 0) break;
-        if (!panel_done)
-          DMB_LAUNCH(c, k_ldlt_panel<C>, blocks_for(rest, NB), 256, sm_panel, N, j, b, F, Lblk, Wb, NBW,
-                     (int)(j - J2));
-        diag_done = panel_done = false;
-        if (j + b < JE) {  // strip update inside the middle panel, fused with the next diagonal block
-          const int nb_next = (int)std::min<int64_t>(NB, N - (j + b));
-          dim3 g(blocks_for(rest, 64), blocks_for(JE - (j + b), 64));
-          if (fuse_step) {
-            DMB_LAUNCH(c, k_ldlt_step<C>, g.x * g.y, 256, sm_step, N, j + b, JE, j, b, F, Wb, NBW,
-                       (int)(j - J2), (int)(j + b - J2), nb_next, Lblk + NB * NB, step_sync + 2 * (j / NB), err);
-            panel_done = true;
+      if constexpr (std::is_same<C, double2>::value) {
+        DMB_LAUNCH(c, k_ldlt_mid64, blocks_for(N - J, NB), 256, DiagSmem<double2>::bytes, N, J, (int)(JE - J), F, Linv,
+                   Wb + (J - J2), NBW, step_sync + MID_WORDS * (J / NBO), err);
+      } else {
+        // the first block: factor and panel rows in one launch; then, per
+        // block, the strip update by the previous one, its diagonal tile and
+        // its panel rows
+        for (int64_t j = J; j < JE; j += NB) {
+          const int b = (int)std::min<int64_t>(NB, N - j);
+          C *Lblk = Linv + (j / NB) * NB * NB;
+          if (j == J) {
+            DMB_LAUNCH(c, k_ldlt_first, 1 + blocks_for(N - j - b, NB), 256, STEP_SMEM, N, j, b, F, Lblk, Wb, NBW,
+                       (int)(j - J2), step_sync + 2 * nblk + 2 * (j / NB), err);
           } else {
-            DMB_LAUNCH(c, k_ldlt_update<C>, g, 256, 0, N, j + b, JE, j, b, F, Wb, NBW, (int)(j - J2), nb_next,
-                       Lblk + NB * NB, err);
+            const int64_t p = j - NB;  // the previous block
+            const dim3 g(blocks_for(N - j, 64), blocks_for(JE - j, 64));
+            DMB_LAUNCH(c, k_ldlt_step, g.x * g.y, 256, STEP_SMEM, N, j, JE, p, NB, F, Wb, NBW, (int)(p - J2),
+                       (int)(j - J2), b, Lblk, step_sync + 2 * (p / NB), err);
           }
-          diag_done = true;
         }
       }
       update_block_column(JE, J2E, J, (int)(JE - J), Wb, (int)(J - J2));
