@@ -85,7 +85,7 @@ dmb_status dmb_ctx_destroy(dmb_ctx *c) {
     DevBuf *bufs[] = {&c->d_xyz, &c->d_tri, &c->d_tcache, &c->d_rwg_slot, &c->d_tplus,
                       &c->d_tminus, &c->d_vpo, &c->d_vmo, &c->d_len, &c->d_ap, &c->d_am,
                       &c->d_slot_rwg, &c->d_slot_side, &c->d_wq, &c->d_centers, &c->d_adj_off,
-                      &c->d_adj_nb, &c->d_near_rec, &c->d_near_val, &c->d_near_entry_mn,
+                      &c->d_adj_nb, &c->d_near_pair, &c->d_near_val, &c->d_near_entry_mn,
                       &c->d_near_entry_off, &c->d_near_row_off, &c->d_near_row_ent, &c->d_near_row_col,
                       &c->d_near_entry_sum, &c->d_Z, &c->d_F, &c->d_dinv, &c->d_W,
                       &c->d_flags, &c->d_li_idx, &c->d_li_cnt, &c->d_li_inv, &c->d_net, &c->d_V,

@@ -258,145 +258,133 @@ __device__ double analytic_1overR(const double P[3], const double V1[3], const d
   return log_sum - ah * atan_sum;
 }
 
-// Greens.jl:189-201 compensated exprel series, 18 terms
-__device__ double2 green_exprel(double2 z) {
-  double2 term = make_double2(1.0, 0.0), total = term, corr = make_double2(0.0, 0.0);
-  for (int order = 1; order <= 18; order++) {
-    double2 zs = make_double2(z.x / (order + 1), z.y / (order + 1));
-    term = cmul(term, zs);
-    double2 ct = csub(term, corr);
-    double2 upd = cadd(total, ct);
-    corr = csub(csub(upd, total), ct);
-    total = upd;
+// Near terms of one ordered pair of triangles, for all of its (test slot,
+// source slot) records at once: the self term (ta == tb, EFIE.jl:534-606) or an
+// edge-adjacent one (ta outer, tb analytic, EFIE.jl:611-684).  Both are sums
+// over outer points a and inner points b of a kernel times f_i(a) . f_j(b) and
+// of the kernel alone, so eight moments about the triangles' centroids (as for
+// the far pairs) serve the nine records; static and smooth parts add up in
+// them.  Only the scalar part of an adjacent static term has a moment of its
+// own (the analytic integral instead of the 7-point sum).  Eight lanes share a
+// pair, lane a its outer point a, and are summed by shuffles.  Bound by the FP64
+// pipe (square roots, divisions, the logarithms and arctangents of the analytic
+// integral); one thread per record, which evaluated every kernel value nine
+// times, took 540 us for 7,200 triangles and 145 us for the smallest mesh.
+struct NearMoments {
+  double v[17];  // m0 re im, ma[3] re im, mb[3] re im, mab re im, scalar re (its im is m0's)
+};
+
+// (exp(-ikR) - 1) / R without cancellation: exp(-iy) - 1 = -2 sin(y/2)
+// (sin(y/2) + i cos(y/2)) (Greens.jl:364-400 switches to a series below |kR| =
+// 0.5 for the same reason); R -> 0: -ik
+__device__ __forceinline__ double2 smooth_kernel(double R, double k) {
+  if (R == 0.0) return make_double2(0.0, -k);
+  double sn, cs;
+  sincos(0.5 * k * R, &sn, &cs);
+  const double f = -2.0 * sn / R;
+  return make_double2(f * sn, f * cs);
+}
+
+__device__ __forceinline__ void near_pair_moments(const TriCache &A, const TriCache &B, bool self, int a, int nq,
+                                                  const double *__restrict__ wq_std, const double *__restrict__ wq_hi,
+                                                  double k, NearMoments &mo) {
+#pragma unroll
+  for (int i = 0; i < 17; i++) mo.v[i] = 0.0;
+  // add outer point la with weight w: kernel sums g0 and gb (about B's centroid)
+  auto add = [&](const double (&la)[3], double w, const double2 g0, const double2 (&gb)[3]) {
+    mo.v[0] += w * g0.x;
+    mo.v[1] += w * g0.y;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      mo.v[2 + 2 * c] += w * g0.x * la[c];
+      mo.v[3 + 2 * c] += w * g0.y * la[c];
+      mo.v[8 + 2 * c] += w * gb[c].x;
+      mo.v[9 + 2 * c] += w * gb[c].y;
+      mo.v[14] += w * gb[c].x * la[c];
+      mo.v[15] += w * gb[c].y * la[c];
+    }
+  };
+  // smooth part: the 7-point rule for self terms, else the standard rule
+  if (a < (self ? 7 : nq)) {
+    const double(*pa)[3] = self ? A.qph : A.qp;
+    const double(*pb)[3] = self ? B.qph : B.qp;
+    const double *wq = self ? wq_hi : wq_std;
+    const int nb = self ? 7 : nq;
+    const double la[3] = {pa[a][0] - A.cen[0], pa[a][1] - A.cen[1], pa[a][2] - A.cen[2]};
+    double2 g0 = make_double2(0, 0), gb[3] = {g0, g0, g0};
+    for (int b = 0; b < nb; b++) {
+      const double dx = pa[a][0] - pb[b][0], dy = pa[a][1] - pb[b][1], dz = pa[a][2] - pb[b][2];
+      const double2 g = cscale(smooth_kernel(sqrt(dx * dx + dy * dy + dz * dz), k), wq[b]);
+      g0 = cadd(g0, g);
+#pragma unroll
+      for (int c = 0; c < 3; c++) gb[c] = cadd(gb[c], cscale(g, pb[b][c] - B.cen[c]));
+    }
+    const double w = DMB_INV_FOUR_PI * wq[a] * (2 * A.area) * (2 * B.area);
+    mo.v[16] += w * g0.x;
+    add(la, w, g0, gb);
   }
-  return total;
-}
-
-// Greens.jl:381-400 _greens_smooth_unchecked: (exp(-ikR)-1)/(4 pi R)
-__device__ double2 greens_smooth(const double r[3], const double rp[3], double k) {
-  double dx = r[0] - rp[0], dy = r[1] - rp[1], dz = r[2] - rp[2];
-  double R = hypot(hypot(dx, dy), dz);
-  double2 q = make_double2(0.0, -k);
-  if (R == 0.0) return cscale(q, DMB_INV_FOUR_PI);
-  double2 z = make_double2(0.0, -k * R);
-  if (hypot(z.x, z.y) <= 0.5) return cmul(cscale(q, DMB_INV_FOUR_PI), green_exprel(z));
-  double sh = sin(0.5 * z.y);
-  double2 em1 = make_double2(0.0 - 2.0 * (sh * sh), sin(z.y));
-  return cscale(em1, DMB_INV_FOUR_PI / R);
-}
-
-__device__ __forceinline__ void fval(const TriCache &T, int slot, const double r[3], double f[3]) {
-  double s = T.s[slot];
-  f[0] = s * (r[0] - T.p[slot][0]);
-  f[1] = s * (r[1] - T.p[slot][1]);
-  f[2] = s * (r[2] - T.p[slot][2]);
-}
-__device__ __forceinline__ double dot3(const double a[3], const double b[3]) {
-  return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
-}
-
-// one near record: self (ta == tb) or edge-adjacent (ta outer, tb analytic)
-__device__ double2 near_value(const NearRec rc, const TriCache *__restrict__ tc, int nq,
-                              const double *__restrict__ wq_std, const double *__restrict__ wq_hi, double k,
-                              double inv_k2) {
-  const TriCache &A = tc[rc.ta];
-  const TriCache &B = tc[rc.tb];
-  double dvm = A.dv[rc.ia], dvn = B.dv[rc.ib];
-  double dvmn = dvm * dvn * inv_k2;
-  double inv4pi = DMB_INV_FOUR_PI;
-  double vr = 0, vi = 0;
-  if (rc.ta == rc.tb) {
-    // _self_cell_cached (EFIE.jl:534-606)
-    double Am = A.area;
-    double2 vs = make_double2(0, 0);
-    for (int a = 0; a < 7; a++) {
-      double fm[3];
-      fval(A, rc.ia, A.qph[a], fm);
-      for (int b = 0; b < 7; b++) {
-        double fn[3];
-        fval(A, rc.ib, A.qph[b], fn);
-        double2 Gs = greens_smooth(A.qph[a], A.qph[b], k);
-        double fd = dot3(fm, fn);
-        double2 vp = cscale(Gs, fd), sp = cscale(Gs, dvmn);
-        double wt = wq_hi[a] * wq_hi[b] * (2 * Am) * (2 * Am);
-        vs = cadd(vs, cscale(csub(vp, sp), wt));
-      }
+  // static part: outer 7-point rule, inner 1/R in closed form
+  if (a < 7) {
+    const double la[3] = {A.qph[a][0] - A.cen[0], A.qph[a][1] - A.cen[1], A.qph[a][2] - A.cen[2]};
+    const double S = analytic_1overR(A.qph[a], B.v[0], B.v[1], B.v[2]);
+    double2 g0 = make_double2(self ? S : 0.0, 0.0), gb[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) gb[c] = make_double2(self ? S * la[c] : 0.0, 0.0);
+    for (int b = 0; b < 7; b++) {
+      const double dx = A.qph[a][0] - B.qph[b][0], dy = A.qph[a][1] - B.qph[b][1], dz = A.qph[a][2] - B.qph[b][2];
+      const double R = sqrt(dx * dx + dy * dy + dz * dz);
+      if (R == 0.0) continue;
+      const double w = wq_hi[b] * (2 * B.area) / R;
+      // self: f_j(a) S + sum (f_j(b) - f_j(a)) / R; adjacent: sum f_j(b) / R
+      if (!self) g0.x += w;
+#pragma unroll
+      for (int c = 0; c < 3; c++) gb[c].x += w * (B.qph[b][c] - (self ? A.qph[a][c] : B.cen[c]));
     }
-    double vg = 0.0;
-    for (int a = 0; a < 7; a++) {
-      double fm[3], fna[3];
-      fval(A, rc.ia, A.qph[a], fm);
-      fval(A, rc.ib, A.qph[a], fna);
-      double S = analytic_1overR(A.qph[a], A.v[0], A.v[1], A.v[2]);
-      double inner = inv4pi * S;
-      double scl = dvmn * inner;
-      double lead = dot3(fm, fna) * inner;
-      double rem = 0.0;
-      for (int b = 0; b < 7; b++) {
-        double dx = A.qph[a][0] - A.qph[b][0], dy = A.qph[a][1] - A.qph[b][1],
-               dz = A.qph[a][2] - A.qph[b][2];
-        double R = hypot(hypot(dx, dy), dz);
-        if (R == 0.0) continue;
-        double fn[3];
-        fval(A, rc.ib, A.qph[b], fn);
-        double df[3] = {fn[0] - fna[0], fn[1] - fna[1], fn[2] - fna[2]};
-        rem += dot3(fm, df) * (inv4pi / R) * wq_hi[b] * (2 * Am);
-      }
-      double ow = wq_hi[a] * (2 * Am);
-      vg += ((lead + rem) - scl) * ow;
-    }
-    vr = vs.x + vg;
-    vi = vs.y;
-  } else {
-    // _adjacent_cell_cached (EFIE.jl:611-684): smooth part on the standard
-    // rule, singular part with outer 7-point rule on A, analytic on B.
-    double Am = A.area, An = B.area;
-    double2 vs = make_double2(0, 0);
-    for (int a = 0; a < nq; a++) {
-      double fm[3];
-      fval(A, rc.ia, A.qp[a], fm);
-      for (int b = 0; b < nq; b++) {
-        double fn[3];
-        fval(B, rc.ib, B.qp[b], fn);
-        double2 Gs = greens_smooth(A.qp[a], B.qp[b], k);
-        double2 vp = cscale(Gs, dot3(fm, fn)), sp = cscale(Gs, dvmn);
-        double wt = wq_std[a] * wq_std[b] * (2 * Am) * (2 * An);
-        vs = cadd(vs, cscale(csub(vp, sp), wt));
-      }
-    }
-    double vg = 0.0;
-    for (int a = 0; a < 7; a++) {
-      double fm[3];
-      fval(A, rc.ia, A.qph[a], fm);
-      double S = analytic_1overR(A.qph[a], B.v[0], B.v[1], B.v[2]);
-      double inner = inv4pi * S;
-      double scl = dvmn * inner;
-      double vsg = 0.0;
-      for (int b = 0; b < 7; b++) {
-        double dx = A.qph[a][0] - B.qph[b][0], dy = A.qph[a][1] - B.qph[b][1],
-               dz = A.qph[a][2] - B.qph[b][2];
-        double R = hypot(hypot(dx, dy), dz);
-        if (R == 0.0) continue;
-        double fn[3];
-        fval(B, rc.ib, B.qph[b], fn);
-        vsg += dot3(fm, fn) * (inv4pi / R) * wq_hi[b] * (2 * An);
-      }
-      double ow = wq_hi[a] * (2 * Am);
-      vg += (vsg - scl) * ow;
-    }
-    vr = vs.x + vg;
-    vi = vs.y;
+    const double w = DMB_INV_FOUR_PI * wq_hi[a] * (2 * A.area);
+    mo.v[16] += w * S;
+    add(la, w, g0, gb);
   }
-  return make_double2(vr, vi);
 }
 
-__global__ void k_near_values(int64_t nrec, const NearRec *__restrict__ recs,
-                              const TriCache *__restrict__ tc, int nq, const double *__restrict__ wq_std,
-                              const double *__restrict__ wq_hi, double k, double inv_k2,
-                              double2 *__restrict__ vals) {
-  int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nrec) return;
-  vals[r] = near_value(recs[r], tc, nq, wq_std, wq_hi, k, inv_k2);
+__device__ __forceinline__ void near_pair(const NearPair &np, int lane8, const TriCache *__restrict__ tc, int nq,
+                                          const double *__restrict__ wq_std, const double *__restrict__ wq_hi, double k,
+                                          double inv_k2, double2 *__restrict__ vals) {
+  const TriCache &A = tc[np.ta], &B = tc[np.tb];
+  NearMoments mo;
+  near_pair_moments(A, B, np.ta == np.tb, lane8, nq, wq_std, wq_hi, k, mo);
+#pragma unroll
+  for (int i = 0; i < 17; i++)
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) mo.v[i] += __shfl_xor_sync(0xffffffffu, mo.v[i], o);
+  for (int e = lane8; e < 9; e += 8) {
+    const int r = np.rec[e];
+    if (r < 0) continue;
+    const int i = e / 3, j = e % 3;
+    const double *pi = A.pl[i], *pj = B.pl[j];
+    const double ss = A.s[i] * B.s[j], sc = A.dv[i] * B.dv[j] * inv_k2;
+    const double pp = pi[0] * pj[0] + pi[1] * pj[1] + pi[2] * pj[2];
+    double2 v;
+    v.x = ss * (mo.v[14] - (mo.v[2] * pj[0] + mo.v[4] * pj[1] + mo.v[6] * pj[2]) -
+                (mo.v[8] * pi[0] + mo.v[10] * pi[1] + mo.v[12] * pi[2]) + pp * mo.v[0]) -
+          sc * mo.v[16];
+    v.y = ss * (mo.v[15] - (mo.v[3] * pj[0] + mo.v[5] * pj[1] + mo.v[7] * pj[2]) -
+                (mo.v[9] * pi[0] + mo.v[11] * pi[1] + mo.v[13] * pi[2]) + pp * mo.v[1]) -
+          sc * mo.v[1];
+    vals[r] = v;
+  }
+}
+
+// eight lanes per pair; lanes beyond the last pair repeat it without writing
+__global__ void __launch_bounds__(128) k_near_values(int64_t npair, const NearPair *__restrict__ pairs,
+                                                     const TriCache *__restrict__ tc, int nq,
+                                                     const double *__restrict__ wq_std,
+                                                     const double *__restrict__ wq_hi, double k, double inv_k2,
+                                                     double2 *__restrict__ vals) {
+  const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  NearPair np = pairs[min(p, npair - 1)];
+  if (p >= npair)
+    for (int e = 0; e < 9; e++) np.rec[e] = -1;
+  near_pair(np, threadIdx.x & 7, tc, nq, wq_std, wq_hi, k, inv_k2, vals);
 }
 
 // sum the records of each near entry in fixed order, add to Z[m][n], Z[n][m]
@@ -429,16 +417,16 @@ __global__ void k_near_add(int64_t nent, const int2 *__restrict__ mn, const int6
 }
 
 // Near terms of many surfaces in one launch each (uneven surface batches):
-// thread -> (surface, record / entry) through the jobs' prefix offsets.
+// thread -> (surface, triangle pair / entry) through the jobs' prefix offsets.
 struct NearJob {
-  const NearRec *recs;
+  const NearPair *pairs;
   const TriCache *tc;
   const double *wq;       // 7 standard + 7 high-order weights
   double2 *vals;
   const int2 *mn;
   const int64_t *eoff;
   void *Z;
-  int64_t N, rec0, ent0;  // first record / entry of the surface in the batch
+  int64_t N, pair0, ent0;  // first pair / entry of the surface in the batch
   double k, inv_k2, omega_mu0;
   int nq;
 };
@@ -447,18 +435,20 @@ __device__ __forceinline__ int near_job_of(const NearJob *jobs, int njobs, int64
   int lo = 0, hi = njobs - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) / 2;
-    if ((entries ? jobs[mid].ent0 : jobs[mid].rec0) <= g) lo = mid;
+    if ((entries ? jobs[mid].ent0 : jobs[mid].pair0) <= g) lo = mid;
     else hi = mid - 1;
   }
   return lo;
 }
 
-__global__ void k_near_values_batched(const NearJob *__restrict__ jobs, int njobs, int64_t total) {
-  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= total) return;
+__global__ void __launch_bounds__(128) k_near_values_batched(const NearJob *__restrict__ jobs, int njobs,
+                                                             int64_t total) {
+  const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3, g = min(p, total - 1);
   const NearJob &jb = jobs[near_job_of(jobs, njobs, g, false)];
-  const int64_t r = g - jb.rec0;
-  jb.vals[r] = near_value(jb.recs[r], jb.tc, jb.nq, jb.wq, jb.wq + 7, jb.k, jb.inv_k2);
+  NearPair np = jb.pairs[g - jb.pair0];
+  if (p >= total)
+    for (int e = 0; e < 9; e++) np.rec[e] = -1;
+  near_pair(np, threadIdx.x & 7, jb.tc, jb.nq, jb.wq, jb.wq + 7, jb.k, jb.inv_k2, jb.vals);
 }
 
 template <class ZC>
@@ -538,25 +528,34 @@ void build_host_topology(dmb_ctx *c) {
   }
   // near records: self pairs and ordered adjacent pairs, canonical m <= n
   struct Key {
-    int32_t m, n, ta, tb, ia, ib;
+    int32_t m, n, ta, tb, ia, ib, pair;
   };
   std::vector<Key> keys;
+  std::vector<NearPair> npairs;
   keys.reserve(12 * nt);
-  for (int64_t t = 0; t < nt; t++)
+  npairs.reserve(4 * nt);
+  auto new_pair = [&](int64_t ta, int64_t tb) {
+    npairs.push_back({(int)ta, (int)tb, {-1, -1, -1, -1, -1, -1, -1, -1, -1}});
+    return (int32_t)npairs.size() - 1;
+  };
+  for (int64_t t = 0; t < nt; t++) {
+    const int32_t pr = new_pair(t, t);
     for (int i = 0; i < 3; i++)
       for (int j = 0; j < 3; j++) {
         int32_t m = slot_rwg[3 * t + i], n = slot_rwg[3 * t + j];
         if (m < 0 || n < 0 || m > n) continue;
-        keys.push_back({m, n, (int32_t)t, (int32_t)t, i, j});
+        keys.push_back({m, n, (int32_t)t, (int32_t)t, i, j, pr});
       }
+  }
   for (int64_t ta = 0; ta < nt; ta++)
     for (int32_t q = c->adj_off[ta]; q < c->adj_off[ta + 1]; q++) {
       int32_t tb = c->adj_nb[q];
+      const int32_t pr = new_pair(ta, tb);
       for (int i = 0; i < 3; i++)
         for (int j = 0; j < 3; j++) {
           int32_t m = slot_rwg[3 * ta + i], n = slot_rwg[3 * tb + j];
           if (m < 0 || n < 0 || m > n) continue;
-          keys.push_back({m, n, (int32_t)ta, tb, i, j});
+          keys.push_back({m, n, (int32_t)ta, tb, i, j, pr});
         }
     }
   std::sort(keys.begin(), keys.end(), [](const Key &a, const Key &b) {
@@ -567,18 +566,18 @@ void build_host_topology(dmb_ctx *c) {
     if (a.ia != b.ia) return a.ia < b.ia;
     return a.ib < b.ib;
   });
-  std::vector<NearRec> recs(keys.size());
   std::vector<int2> ent;
   std::vector<int64_t> eoff;
   for (size_t i = 0; i < keys.size(); i++) {
-    recs[i] = {keys[i].ta, keys[i].tb, keys[i].ia, keys[i].ib};
+    npairs[keys[i].pair].rec[3 * keys[i].ia + keys[i].ib] = (int)i;
     if (i == 0 || keys[i].m != keys[i - 1].m || keys[i].n != keys[i - 1].n) {
       ent.push_back(make_int2(keys[i].m, keys[i].n));
       eoff.push_back((int64_t)i);
     }
   }
   eoff.push_back((int64_t)keys.size());
-  c->n_near_rec = (int64_t)recs.size();
+  c->n_near_rec = (int64_t)keys.size();
+  c->n_near_pair = keys.empty() ? 0 : (int64_t)npairs.size();
   c->n_near_entry = (int64_t)ent.size();
 
   auto up = [&](DevBuf &b, const void *src, size_t bytes) {
@@ -609,14 +608,14 @@ void build_host_topology(dmb_ctx *c) {
       }
     }
   }
-  up(c->d_near_rec, recs.data(), recs.size() * sizeof(NearRec));
+  up(c->d_near_pair, npairs.data(), npairs.size() * sizeof(NearPair));
   up(c->d_near_entry_mn, ent.data(), ent.size() * sizeof(int2));
   up(c->d_near_entry_off, eoff.data(), eoff.size() * sizeof(int64_t));
   up(c->d_near_row_off, roff.data(), roff.size() * sizeof(int64_t));
   up(c->d_near_row_ent, rent.data(), rent.size() * 4);
   up(c->d_near_row_col, rcol.data(), rcol.size() * 4);
   c->d_near_entry_sum.ensure(std::max<size_t>(16, ent.size() * sizeof(double2)));
-  c->d_near_val.ensure(std::max<size_t>(16, recs.size() * sizeof(double2)));
+  c->d_near_val.ensure(std::max<size_t>(16, keys.size() * sizeof(double2)));
   up(c->d_slot_rwg, slot_rwg.data(), slot_rwg.size() * 4);
   up(c->d_slot_side, slot_side.data(), slot_side.size() * 4);
   c->d_tcache.ensure(sizeof(TriCache) * std::max<int64_t>(nt, 1));
@@ -676,8 +675,8 @@ void ensure_cache(dmb_ctx *c, int quad_order) {
 void near_values(dmb_ctx *c, double k, double inv_k2) {
   if (c->n_near_rec == 0) return;
   const double *dwq = c->d_wq.as<double>();
-  DMB_LAUNCH(c, k_near_values, (unsigned)((c->n_near_rec + 127) / 128), 128, 0, c->n_near_rec,
-             c->d_near_rec.as<NearRec>(), c->d_tcache.as<TriCache>(), c->nq, dwq, dwq + 7, k, inv_k2,
+  DMB_LAUNCH(c, k_near_values, (unsigned)((8 * c->n_near_pair + 127) / 128), 128, 0, c->n_near_pair,
+             c->d_near_pair.as<NearPair>(), c->d_tcache.as<TriCache>(), c->nq, dwq, dwq + 7, k, inv_k2,
              c->d_near_val.as<double2>());
 }
 
@@ -761,11 +760,11 @@ double assemble_batch(const std::vector<dmb_ctx *> &cs, double k, double eta0, i
   DMB_CUDA(cudaEventRecord(e0, c0->stream));
   far_tiles_batched(cs, T, f64, k, inv_k2, omega_mu0, bufs.far_jobs, bufs.far_tasks, bufs.far_err);
   std::vector<NearJob> jobs;
-  int64_t nrec = 0, nent = 0;
+  int64_t npair = 0, nent = 0;
   for (dmb_ctx *c : cs) {
     if (c->n_near_rec == 0) continue;
     NearJob jb;
-    jb.recs = c->d_near_rec.as<NearRec>();
+    jb.pairs = c->d_near_pair.as<NearPair>();
     jb.tc = c->d_tcache.as<TriCache>();
     jb.wq = c->d_wq.as<double>();
     jb.vals = c->d_near_val.as<double2>();
@@ -773,14 +772,14 @@ double assemble_batch(const std::vector<dmb_ctx *> &cs, double k, double eta0, i
     jb.eoff = c->d_near_entry_off.as<int64_t>();
     jb.Z = c->d_Z.p;
     jb.N = c->n;
-    jb.rec0 = nrec;
+    jb.pair0 = npair;
     jb.ent0 = nent;
     jb.k = k;
     jb.inv_k2 = inv_k2;
     jb.omega_mu0 = omega_mu0;
     jb.nq = c->nq;
     jobs.push_back(jb);
-    nrec += c->n_near_rec;
+    npair += c->n_near_pair;
     nent += c->n_near_entry;
   }
   if (!jobs.empty()) {
@@ -788,8 +787,8 @@ double assemble_batch(const std::vector<dmb_ctx *> &cs, double k, double eta0, i
     DMB_CUDA(cudaMemcpyAsync(bufs.near_jobs.p, jobs.data(), jobs.size() * sizeof(NearJob), cudaMemcpyHostToDevice,
                              c0->stream));
     const int nj = (int)jobs.size();
-    DMB_LAUNCH(c0, k_near_values_batched, (unsigned)((nrec + 127) / 128), 128, 0, bufs.near_jobs.as<NearJob>(), nj,
-               nrec);
+    DMB_LAUNCH(c0, k_near_values_batched, (unsigned)((8 * npair + 127) / 128), 128, 0, bufs.near_jobs.as<NearJob>(),
+               nj, npair);
     if (f64)
       DMB_LAUNCH(c0, k_near_add_batched<double2>, (unsigned)((nent + 255) / 256), 256, 0,
                  bufs.near_jobs.as<NearJob>(), nj, nent);

@@ -100,10 +100,12 @@ struct TriCache {
   double pl[3][3];    // opposite vertex minus centroid
 };
 
-// near-field record: one (near triangle pair, test slot, source slot)
-struct NearRec {
-  int ta, tb;     // ta == tb: self; otherwise ta outer (test), tb analytic (source)
-  int ia, ib;     // slots
+// one ordered pair of near triangles (ta == tb: self; otherwise ta outer, tb
+// analytic) and, per (test slot, source slot), the record its value goes to
+// (-1: none)
+struct NearPair {
+  int ta, tb;
+  int rec[9];
 };
 
 // H-matrix operator of dmb_aca_build (dmb_aca.cu).  Blocks are kept in task
@@ -219,12 +221,12 @@ struct dmb_ctx {
   // adjacency + near records
   std::vector<int32_t> adj_off, adj_nb;
   DevBuf d_adj_off, d_adj_nb;
-  DevBuf d_near_rec, d_near_val, d_near_entry_mn, d_near_entry_off;
+  DevBuf d_near_pair, d_near_val, d_near_entry_mn, d_near_entry_off;
   // the near entries touching each RWG row (CSR, entry order) and the summed
   // value of each entry: the matrix-free product gathers its near part per
   // row in a fixed order (no atomics)
   DevBuf d_near_row_off, d_near_row_ent, d_near_row_col, d_near_entry_sum;
-  int64_t n_near_rec = 0, n_near_entry = 0;
+  int64_t n_near_rec = 0, n_near_pair = 0, n_near_entry = 0;
 
   // impedance matrix (row-major == column-major since Z is symmetric)
   DevBuf d_Z;
