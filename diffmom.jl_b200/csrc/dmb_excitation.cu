@@ -266,50 +266,115 @@ __global__ void k_pattern_rhs(int64_t N, const TriCache *__restrict__ tc, const 
   V[n] = acc;
 }
 
-// radiation matrix G (3*NO x N, row-major) for directions rh
-__global__ void k_radiation(int64_t N, int64_t NO, const TriCache *__restrict__ tc, const int *__restrict__ rslot,
-                            int nq, const double *__restrict__ wq, const double *__restrict__ rh, double k,
-                            double eta0, double2 *__restrict__ G) {
-  int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int64_t q = blockIdx.y;
-  if (n >= N) return;
-  double r0 = rh[3 * q], r1 = rh[3 * q + 1], r2 = rh[3 * q + 2];
-  double rn2 = r0 * r0 + r1 * r1 + r2 * r2;
-  double2 c0 = make_double2(0, 0), c1 = c0, c2 = c0;
-  for (int s = 0; s < 2; s++) {
-    int sl = rslot[2 * n + s];
-    const TriCache &T = tc[sl / 3];
-    int i = sl % 3;
-    for (int qs = 0; qs < nq; qs++) {
-      double f0 = T.s[i] * (T.qp[qs][0] - T.p[i][0]);
-      double f1 = T.s[i] * (T.qp[qs][1] - T.p[i][1]);
-      double f2 = T.s[i] * (T.qp[qs][2] - T.p[i][2]);
-      double wt = wq[qs] * 2 * T.area;
-      double arg = k * (r0 * T.qp[qs][0] + r1 * T.qp[qs][1] + r2 * T.qp[qs][2]);
-      double sn, cs;
-      sincos(arg, &sn, &cs);
-      double2 ph = make_double2(wt * cs, wt * sn);
-      c0 = cadd(c0, cscale(ph, f0));
-      c1 = cadd(c1, cscale(ph, f1));
-      c2 = cadd(c2, cscale(ph, f2));
+// ---------------------------------------------------------------------------
+// Far field E(d) = i k eta0 / (4 pi) d x (d x C(d)) / |d|^2, C(d) = sum over
+// quadrature points w 2A J(r) exp(ik d . r) (radiation_vectors times the
+// currents, FarField.jl:425-611).  The current J of a triangle's points is the
+// sum of its three basis functions, so a direction needs one phase per point (3
+// Nt) instead of one per basis function and point (6 N = 9 Nt), and no matrix
+// of 3 NO x N radiation vectors (67 MB for 181 directions of 7,680 functions,
+// whose product with one column ran on nine CTAs: 2.8 ms of a solve's 49).
+// ---------------------------------------------------------------------------
+// points pos[3][P] and weighted currents cur[r][3][P], P = nq nt
+__global__ void k_point_currents(int nt, int nq, int64_t N, const TriCache *__restrict__ tc,
+                                 const double *__restrict__ wq, const double2 *__restrict__ I,
+                                 double *__restrict__ pos, double2 *__restrict__ cur) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t r = blockIdx.y, P = (int64_t)nq * nt;
+  if (t >= nt) return;
+  const TriCache &T = tc[t];
+  double2 x[3];
+#pragma unroll
+  for (int i = 0; i < 3; i++) x[i] = T.rwg[i] >= 0 ? cscale(I[r * N + T.rwg[i]], T.s[i]) : make_double2(0, 0);
+  for (int q = 0; q < nq; q++) {
+    const double w = wq[q] * 2 * T.area;
+    const int64_t p = (int64_t)q * nt + t;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      double2 j = make_double2(0, 0);
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+        if (T.rwg[i] >= 0) j = cadd(j, cscale(x[i], T.qp[q][c] - T.p[i][c]));
+      cur[(r * 3 + c) * P + p] = cscale(j, w);
+      if (r == 0) pos[c * P + p] = T.qp[q][c];
     }
   }
-  // rh x (rh x C) / |rh|^2 = (rh (rh.C) - C |rh|^2) / |rh|^2
-  double2 d = cadd(cadd(cscale(c0, r0), cscale(c1, r1)), cscale(c2, r2));
-  double2 v0 = cscale(csub(cscale(d, r0), cscale(c0, rn2)), 1.0 / rn2);
-  double2 v1 = cscale(csub(cscale(d, r1), cscale(c1, rn2)), 1.0 / rn2);
-  double2 v2 = cscale(csub(cscale(d, r2), cscale(c2, rn2)), 1.0 / rn2);
-  double2 pref = make_double2(0, k * eta0 * DMB_INV_FOUR_PI);
-  G[(3 * q + 0) * N + n] = cmul(pref, v0);
-  G[(3 * q + 1) * N + n] = cmul(pref, v1);
-  G[(3 * q + 2) * N + n] = cmul(pref, v2);
+}
+
+// partial sums of C over the points of chunk blockIdx.y for D directions and Q
+// columns: part[chunk][r NO + d][3].  D Q = 4: four directions share a point's
+// loads for one column, four columns share a phase otherwise.
+template <int D, int Q>
+__global__ void __launch_bounds__(128) k_farfield_part(int64_t P, int64_t chunk, int64_t NO, int64_t R,
+                                                       const double *__restrict__ rh, double k,
+                                                       const double *__restrict__ pos, const double2 *__restrict__ cur,
+                                                       double2 *__restrict__ part) {
+  __shared__ double2 red[4][12];
+  const int64_t d0 = (int64_t)blockIdx.x * D, r0 = (int64_t)blockIdx.z * Q;
+  double kd[D][3];
+#pragma unroll
+  for (int d = 0; d < D; d++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) kd[d][c] = k * rh[3 * min(d0 + d, NO - 1) + c];
+  double2 acc[4][3];
+#pragma unroll
+  for (int u = 0; u < 4; u++) acc[u][0] = acc[u][1] = acc[u][2] = make_double2(0, 0);
+  const int64_t p1 = min(P, (blockIdx.y + 1) * chunk);
+  for (int64_t p = blockIdx.y * chunk + threadIdx.x; p < p1; p += 128) {
+    const double x = pos[p], y = pos[P + p], z = pos[2 * P + p];
+    double2 j[Q][3];
+#pragma unroll
+    for (int q = 0; q < Q; q++)
+#pragma unroll
+      for (int c = 0; c < 3; c++) j[q][c] = cur[(min(r0 + q, R - 1) * 3 + c) * P + p];
+#pragma unroll
+    for (int d = 0; d < D; d++) {
+      double2 ph;
+      sincos(kd[d][0] * x + kd[d][1] * y + kd[d][2] * z, &ph.y, &ph.x);
+#pragma unroll
+      for (int q = 0; q < Q; q++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) cfma(acc[d * Q + q][c], ph, j[q][c]);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 4; u++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const double2 v = warp_sum2(acc[u][c]);
+      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][3 * u + c] = v;
+    }
+  __syncthreads();
+  if (threadIdx.x < 12) {
+    const int u = threadIdx.x / 3, c = threadIdx.x % 3;
+    const int64_t d = d0 + u / Q, r = r0 + u % Q;
+    if (d < NO && r < R)
+      part[((blockIdx.y * R + r) * NO + d) * 3 + c] =
+          cadd(cadd(red[0][threadIdx.x], red[1][threadIdx.x]), cadd(red[2][threadIdx.x], red[3][threadIdx.x]));
+  }
+}
+
+// the chunks' sums in order, and d x (d x C) / |d|^2 = (d (d . C) - C |d|^2) / |d|^2
+__global__ void k_farfield_sum(int nchunk, int64_t NO, int64_t R, const double *__restrict__ rh, double k, double eta0,
+                               const double2 *__restrict__ part, double2 *__restrict__ E) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= NO * R) return;
+  double2 C[3] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
+  for (int h = 0; h < nchunk; h++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) C[c] = cadd(C[c], part[(h * NO * R + e) * 3 + c]);
+  const double *d = rh + 3 * (e % NO);
+  const double n2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+  const double2 dc = cadd(cadd(cscale(C[0], d[0]), cscale(C[1], d[1])), cscale(C[2], d[2]));
+  const double2 pref = make_double2(0, k * eta0 * DMB_INV_FOUR_PI);
+#pragma unroll
+  for (int c = 0; c < 3; c++) E[3 * e + c] = cmul(pref, cscale(csub(cscale(dc, d[c]), cscale(C[c], n2)), 1.0 / n2));
 }
 
 // Monostatic far field: for incidence r the field of current column I_r in
 // the direction -k_hat_r (one CTA per incidence, block reduction over RWGs),
 // E (3 complex per r) and sigma_r = 4 pi |E|^2 / |E0_r|^2 (Diagnostics.jl:460-474).
-__global__ void __launch_bounds__(256) k_monostatic(int64_t N, const TriCache *__restrict__ tc,
-                                                    const int *__restrict__ rslot, int nq,
+__global__ void __launch_bounds__(256) k_monostatic(int64_t N, int nt, const TriCache *__restrict__ tc, int nq,
                                                     const double *__restrict__ wq, const double *__restrict__ kv,
                                                     const double *__restrict__ E0s, double k, double eta0,
                                                     const double2 *__restrict__ I, double2 *__restrict__ E,
@@ -321,22 +386,30 @@ __global__ void __launch_bounds__(256) k_monostatic(int64_t N, const TriCache *_
   const double r0 = -kx / kn, r1 = -ky / kn, r2 = -kz / kn;
   double2 c0 = make_double2(0, 0), c1 = c0, c2 = c0;
   const double2 *Ir = I + r * N;
-  for (int64_t n = threadIdx.x; n < N; n += blockDim.x) {
-    const double2 in = Ir[n];
-    for (int s = 0; s < 2; s++) {
-      const int sl = rslot[2 * n + s];
-      const TriCache &T = tc[sl / 3];
-      const int i = sl % 3;
-      for (int qs = 0; qs < nq; qs++) {
-        const double wt = wq[qs] * 2 * T.area * T.s[i];
-        const double arg = k * (r0 * T.qp[qs][0] + r1 * T.qp[qs][1] + r2 * T.qp[qs][2]);
-        double sn, cs;
-        sincos(arg, &sn, &cs);
-        const double2 ph = cmul(make_double2(wt * cs, wt * sn), in);
-        c0 = cadd(c0, cscale(ph, T.qp[qs][0] - T.p[i][0]));
-        c1 = cadd(c1, cscale(ph, T.qp[qs][1] - T.p[i][1]));
-        c2 = cadd(c2, cscale(ph, T.qp[qs][2] - T.p[i][2]));
-      }
+  // one phase per quadrature point: the current of a triangle's points is the
+  // sum of its basis functions (1,024 incidences of 10,680 functions: 0.64 ms
+  // with a phase per function and point)
+  for (int t = threadIdx.x; t < nt; t += blockDim.x) {
+    const TriCache &T = tc[t];
+    double2 x[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) x[i] = T.rwg[i] >= 0 ? cscale(Ir[T.rwg[i]], T.s[i]) : make_double2(0, 0);
+    for (int qs = 0; qs < nq; qs++) {
+      const double wt = wq[qs] * 2 * T.area;
+      const double arg = k * (r0 * T.qp[qs][0] + r1 * T.qp[qs][1] + r2 * T.qp[qs][2]);
+      double sn, cs;
+      sincos(arg, &sn, &cs);
+      const double2 ph = make_double2(wt * cs, wt * sn);
+      double2 j[3] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+        if (T.rwg[i] >= 0) {
+#pragma unroll
+          for (int c = 0; c < 3; c++) j[c] = cadd(j[c], cscale(x[i], T.qp[qs][c] - T.p[i][c]));
+        }
+      cfma(c0, ph, j[0]);
+      cfma(c1, ph, j[1]);
+      cfma(c2, ph, j[2]);
     }
   }
   c0 = warp_sum2(c0);
@@ -367,36 +440,6 @@ __global__ void __launch_bounds__(256) k_monostatic(int64_t N, const TriCache *_
     const double e0 = E0s[r];
     sigma[r] = 4.0 * 3.14159265358979323846 * (cabs2(v0) + cabs2(v1) + cabs2(v2)) / (e0 * e0);
   }
-}
-
-// C (M x R col-major) = A (M x K row-major) B (K x R col-major)
-__global__ void __launch_bounds__(256) k_gemm_rc(int64_t M, int64_t K, int64_t R, const double2 *__restrict__ A,
-                                                 const double2 *__restrict__ B, double2 *__restrict__ C) {
-  __shared__ double2 As[16][65];
-  __shared__ double2 Bs[16][65];
-  int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  int64_t m0 = (int64_t)blockIdx.x * 64, r0 = (int64_t)blockIdx.y * 64;
-  double2 acc[4][4];
-  for (int i = 0; i < 4; i++)
-    for (int j = 0; j < 4; j++) acc[i][j] = make_double2(0, 0);
-  for (int64_t k0 = 0; k0 < K; k0 += 16) {
-    for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-      int kk = e & 15, mm = e >> 4;
-      int64_t m = m0 + mm, kx = k0 + kk, r = r0 + mm;
-      As[kk][mm] = (m < M && kx < K) ? A[m * K + kx] : make_double2(0, 0);
-      Bs[kk][mm] = (r < R && kx < K) ? B[r * K + kx] : make_double2(0, 0);
-    }
-    __syncthreads();
-    for (int kk = 0; kk < 16; kk++)
-      for (int i = 0; i < 4; i++)
-        for (int j = 0; j < 4; j++) acc[i][j] = cadd(acc[i][j], cmul(As[kk][ty + 16 * i], Bs[kk][tx + 16 * j]));
-    __syncthreads();
-  }
-  for (int i = 0; i < 4; i++)
-    for (int j = 0; j < 4; j++) {
-      int64_t m = m0 + ty + 16 * i, r = r0 + tx + 16 * j;
-      if (m < M && r < R) C[r * M + m] = acc[i][j];
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -554,17 +597,34 @@ void rhs_plane_waves_async(dmb_ctx *c, const double *kvecs, const double *E0s, c
 void farfield_dev(dmb_ctx *c, const double *rhat, int64_t NO, double k, double eta0, int quad_order,
                   const double *I_dev, int64_t nrhs, double *E_dev) {
   ensure_cache(c, quad_order);
-  const int64_t N = c->n;
-  DevBuf dr, G;
-  dr.ensure(24 * NO);
-  G.ensure(sizeof(double2) * 3 * NO * N);
-  DMB_CUDA(cudaMemcpyAsync(dr.p, rhat, 24 * NO, cudaMemcpyHostToDevice, c->stream));
-  dim3 g(blocks_for(N, 128), (unsigned)NO);
-  DMB_LAUNCH(c, k_radiation, g, 128, 0, N, NO, c->d_tcache.as<TriCache>(), c->d_rwg_slot.as<int>(), c->nq,
-             c->d_wq.as<double>(), dr.as<double>(), k, eta0, G.as<double2>());
-  dim3 g2(blocks_for(3 * NO, 64), blocks_for(nrhs, 64));
-  DMB_LAUNCH(c, k_gemm_rc, g2, 256, 0, 3 * NO, N, nrhs, G.as<double2>(), (const double2 *)I_dev,
-             (double2 *)E_dev);
+  const int64_t N = c->n, P = (int64_t)c->nq * c->nt;
+  // columns at most 256 at a time (the workspace stays below 50 MB per 4,000
+  // points); the points in enough chunks to occupy the GPU, at least 512 each
+  const int64_t cols = std::min<int64_t>(nrhs, 256);
+  const int64_t groups = cols > 1 ? NO * ((cols + 3) / 4) : (NO + 3) / 4;
+  const int64_t nchunk = std::max<int64_t>(1, std::min((P + 511) / 512, (8 * (int64_t)c->sm_count + groups - 1) / groups));
+  const int64_t chunk = (P + nchunk - 1) / nchunk;
+  // workspace of the context: directions, points, currents, partial sums
+  const size_t off_pos = sizeof(double) * 3 * NO, off_cur = (off_pos + sizeof(double) * 3 * P + 15) / 16 * 16,
+               off_part = off_cur + sizeof(double2) * 3 * P * cols;
+  c->d_far.ensure(off_part + sizeof(double2) * 3 * NO * cols * nchunk);
+  char *base = c->d_far.as<char>();
+  double *dr = (double *)base, *pos = (double *)(base + off_pos);
+  double2 *cur = (double2 *)(base + off_cur), *part = (double2 *)(base + off_part);
+  DMB_CUDA(cudaMemcpyAsync(dr, rhat, 24 * NO, cudaMemcpyHostToDevice, c->stream));
+  for (int64_t r = 0; r < nrhs; r += cols) {
+    const int64_t nr = std::min(cols, nrhs - r);
+    DMB_LAUNCH(c, k_point_currents, dim3(blocks_for(c->nt, 128), (unsigned)nr), 128, 0, (int)c->nt, c->nq, N,
+               c->d_tcache.as<TriCache>(), c->d_wq.as<double>(), (const double2 *)I_dev + r * N, pos, cur);
+    if (nr > 1)
+      DMB_LAUNCH(c, (k_farfield_part<1, 4>), dim3((unsigned)NO, (unsigned)nchunk, (unsigned)((nr + 3) / 4)), 128, 0, P,
+                 chunk, NO, nr, dr, k, pos, cur, part);
+    else
+      DMB_LAUNCH(c, (k_farfield_part<4, 1>), dim3((unsigned)((NO + 3) / 4), (unsigned)nchunk), 128, 0, P, chunk, NO,
+                 nr, dr, k, pos, cur, part);
+    DMB_LAUNCH(c, k_farfield_sum, blocks_for(NO * nr, 128), 128, 0, (int)nchunk, NO, nr, dr, k, eta0, part,
+               (double2 *)E_dev + 3 * NO * r);
+  }
   DMB_CUDA(cudaStreamSynchronize(c->stream));
 }
 
@@ -624,8 +684,7 @@ void monostatic_dev(dmb_ctx *c, int64_t R, double k, double eta0, int quad_order
                     double *E_dev, double *sigma_dev) {
   ensure_cache(c, quad_order);
   const double *dk = (const double *)((const char *)c->d_small.p + 64), *de = dk + 3 * R;
-  DMB_LAUNCH(c, k_monostatic, (unsigned)R, 256, 0, c->n, c->d_tcache.as<TriCache>(), c->d_rwg_slot.as<int>(),
-             c->nq, c->d_wq.as<double>(), dk, de, k, eta0, (const double2 *)I_dev, (double2 *)E_dev, sigma_dev);
+  DMB_LAUNCH(c, k_monostatic, (unsigned)R, 256, 0, c->n, (int)c->nt, c->d_tcache.as<TriCache>(), c->nq, c->d_wq.as<double>(), dk, de, k, eta0, (const double2 *)I_dev, (double2 *)E_dev, sigma_dev);
 }
 
 void prepare_operator(dmb_ctx *c, double k, double eta0, int quad_order) {

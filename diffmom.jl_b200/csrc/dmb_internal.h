@@ -257,6 +257,7 @@ struct dmb_ctx {
 
   // resident solution of dmb_solve_resident / dmb_solve_resident_many
   DevBuf d_rhs, d_sol, d_mono;
+  DevBuf d_far;       // far-field workspace
   int64_t sol_r = 0;
   // small persistent scratch (counters, plane-wave parameters): the solve path
   // allocates nothing after its first call
