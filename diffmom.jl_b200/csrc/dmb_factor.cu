@@ -16,12 +16,11 @@
 //     (complex128: int8 residue products, dmb_oz64.cu, or the FP64 pipe;
 //     complex64: the tensor-core kernels of dmb_tc.cu or FP32 units).
 //     A zero or non-finite pivot stops with DMB_ERR_BREAKDOWN.
-//   * apply (NearFieldOperator, :1034-1054): L y = x, z = y / D, L^T x = z as
-//     one kernel per sweep.  Each CTA draws a ticket (block row, launch order),
-//     accumulates the contributions of already-solved block rows in registers as
-//     their flags appear, then multiplies by the precomputed inverse of its
-//     diagonal block.  Every wait is bounded: on expiry the kernel sets an error
-//     bit and returns; the host raises DMB_ERR_TIMEOUT.
+//   * apply (NearFieldOperator, :1034-1054): L y = x, z = y / D, L^T x = z; up
+//     to seven columns by one data-flow launch per sweep (k_sweep_fwd /
+//     k_sweep_bwd, 256-row blocks and their inverses), more columns by panels.
+//     Every wait is bounded: on expiry the kernel sets an error bit and returns;
+//     the host raises DMB_ERR_TIMEOUT.
 #include <algorithm>
 #include <type_traits>
 #include <cmath>
@@ -1323,213 +1322,6 @@ __global__ void __launch_bounds__(256, 1) k_ldlt_mid64(int64_t N, int64_t J, int
   }
 }
 
-// ---------------------------------------------------------------------------
-// ticket-ordered triangular solves (one right-hand side per grid.y)
-// ---------------------------------------------------------------------------
-// wait until flag[cb] is set; return how many consecutive flags from cb on are
-// set (>= 1), or 0 when the wait expired (error bit 4 recorded)
-__device__ int wait_flags(const volatile unsigned *fl, int cb, int limit, unsigned *err, long long spin_limit) {
-  long long it = 0;
-  while (fl[cb] == 0u) {
-    if (++it > spin_limit) {
-      atomicOr(err, 4u);
-      return 0;
-    }
-    if (*((volatile unsigned *)err) & 4u) return 0;
-    __nanosleep(64);
-  }
-  int r = cb + 1;
-  while (r < limit && fl[r] != 0u) r++;
-  return r - cb;
-}
-
-// 64 x 64 matrix (shared memory, row stride NB) times a 64-vector (shared
-// memory) with four threads per output: thread (o = tid >> 2, part = tid & 3)
-// sums 16 terms, two shuffles combine the parts.  TR: the matrix is read
-// transposed (output o takes column o).  Every thread returns the sum of its
-// output.
-template <class FC, bool TR>
-__device__ __forceinline__ double2 gemv64_quad(const FC *__restrict__ M, const double2 *__restrict__ v) {
-  const int o = threadIdx.x >> 2, part = threadIdx.x & 3;
-  double2 a = make_double2(0, 0), b = make_double2(0, 0);
-#pragma unroll
-  for (int k = 0; k < 16; k += 2) {
-    const int c0 = part * 16 + k, c1 = c0 + 1;
-    cfma(a, to_d2(TR ? M[c0 * NB + o] : M[o * NB + c0]), v[c0]);
-    cfma(b, to_d2(TR ? M[c1 * NB + o] : M[o * NB + c1]), v[c1]);
-  }
-  a = cadd(a, b);
-  a.x += __shfl_xor_sync(0xffffffffu, a.x, 1);
-  a.y += __shfl_xor_sync(0xffffffffu, a.y, 1);
-  a.x += __shfl_xor_sync(0xffffffffu, a.x, 2);
-  a.y += __shfl_xor_sync(0xffffffffu, a.y, 2);
-  return a;
-}
-
-// L y = x (x overwritten), L unit lower.  256 threads = 4 row groups x 64
-// columns; while earlier block rows are streamed each thread accumulates its
-// 16 rows across all solved block rows in registers, and those partial sums
-// are reduced before the last wait.  The L block of the last dependency
-// (block row t-1) and the inverse diagonal block are staged in shared memory
-// before any wait, so the critical path after the last flag is one L2 read of
-// y_{t-1} into shared memory and two 64 x 64 products on chip (four threads
-// per row, two shuffles each).
-template <class FC>
-__global__ void __launch_bounds__(256) k_trsv_fwd(int64_t N, const FC *__restrict__ F, const FC *__restrict__ Linv,
-                                                  double2 *x, unsigned *flags, unsigned *tickets, unsigned *err,
-                                                  long long spin_limit) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  FC *Lp = reinterpret_cast<FC *>(smem_raw);
-  FC *Li = Lp + NB * NB;
-  __shared__ double2 acc[NB];
-  __shared__ double2 ys[NB];
-  __shared__ double2 part[2][NB];
-  __shared__ int s_t, s_n;
-  const int nblk = (int)((N + NB - 1) / NB);
-  const int rhs = blockIdx.y;
-  double2 *xr = x + (int64_t)rhs * N;
-  unsigned *fl = flags + (int64_t)rhs * nblk;
-  if (threadIdx.x == 0) s_t = (int)atomicAdd(tickets + rhs, 1u);
-  __syncthreads();
-  const int t = s_t;
-  const int64_t r0 = (int64_t)t * NB;
-  const int bs = (int)(N - r0 < NB ? N - r0 : NB);
-  const int col = threadIdx.x & 63, rg = threadIdx.x >> 6, half = (threadIdx.x >> 5) & 1;
-  // stage Linv_tt and, for t > 0, L[r0.., (t-1)*NB..]
-  const FC *Lit = Linv + (int64_t)t * NB * NB;
-  for (int e = threadIdx.x; e < NB * NB; e += 256) {
-    Li[e] = Lit[e];
-    int row = e >> 6, cc = e & 63;
-    if (t > 0) Lp[e] = row < bs ? F[(r0 + row) * N + (int64_t)(t - 1) * NB + cc] : FC{};
-  }
-  double2 p[16];
-#pragma unroll
-  for (int i = 0; i < 16; i++) p[i] = make_double2(0, 0);
-  int cb = 0;
-  while (cb < t - 1) {
-    if (threadIdx.x == 0) s_n = wait_flags(fl, cb, t - 1, err, spin_limit);
-    __syncthreads();
-    const int n = s_n;
-    __syncthreads();
-    if (n == 0) return;
-    __threadfence();
-    for (int q = cb; q < cb + n; q++) {
-      const int64_t c0 = (int64_t)q * NB;
-      const double2 yv = __ldcg(xr + c0 + col);
-#pragma unroll
-      for (int i = 0; i < 16; i++) {
-        int row = rg + 4 * i;
-        if (row < bs) cfma(p[i], to_d2(F[(r0 + row) * N + c0 + col]), yv);
-      }
-    }
-    cb += n;
-  }
-  // acc = x_t - (streamed block rows), before the last wait
-  if (threadIdx.x < NB) acc[threadIdx.x] = threadIdx.x < bs ? xr[r0 + threadIdx.x] : make_double2(0, 0);
-#pragma unroll
-  for (int i = 0; i < 16; i++) {
-    double2 v = warp_sum2(p[i]);
-    if ((threadIdx.x & 31) == 0) part[half][rg + 4 * i] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < NB) acc[threadIdx.x] = csub(acc[threadIdx.x], cadd(part[0][threadIdx.x], part[1][threadIdx.x]));
-  if (t > 0) {
-    if (threadIdx.x == 0) s_n = wait_flags(fl, t - 1, t, err, spin_limit);
-    __syncthreads();
-    if (s_n == 0) return;
-    __threadfence();
-    if (threadIdx.x < NB) ys[threadIdx.x] = __ldcg(xr + (int64_t)(t - 1) * NB + threadIdx.x);
-    __syncthreads();
-    const double2 v = gemv64_quad<FC, false>(Lp, ys);
-    if ((threadIdx.x & 3) == 0) acc[threadIdx.x >> 2] = csub(acc[threadIdx.x >> 2], v);
-  }
-  __syncthreads();
-  // y_t = Linv_tt acc
-  const double2 y = gemv64_quad<FC, false>(Li, acc);
-  if ((threadIdx.x & 3) == 0 && (threadIdx.x >> 2) < bs) xr[r0 + (threadIdx.x >> 2)] = y;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) atomicExch(fl + t, 1u);
-}
-
-// L^T x = z (x overwritten), block rows bottom-up; flags indexed by ticket
-// (ticket 0 = last block row).  Thread (rq, col) handles column col of the
-// solved block rows' L entries, rows rq + 4i.  The L block of the last
-// dependency (block row t+1) and Linv_tt are staged before any wait.
-template <class FC>
-__global__ void __launch_bounds__(256) k_trsv_bwd(int64_t N, const FC *__restrict__ F, const FC *__restrict__ Linv,
-                                                  double2 *x, unsigned *flags, unsigned *tickets, unsigned *err,
-                                                  long long spin_limit) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  FC *Lp = reinterpret_cast<FC *>(smem_raw);
-  FC *Li = Lp + NB * NB;
-  __shared__ double2 acc[NB];
-  __shared__ double2 part[4][NB];
-  __shared__ int s_t, s_n;
-  const int nblk = (int)((N + NB - 1) / NB);
-  const int rhs = blockIdx.y;
-  double2 *xr = x + (int64_t)rhs * N;
-  unsigned *fl = flags + (int64_t)rhs * nblk;
-  if (threadIdx.x == 0) s_t = (int)atomicAdd(tickets + rhs, 1u);
-  __syncthreads();
-  const int tk = s_t;
-  const int t = nblk - 1 - tk;
-  const int64_t r0 = (int64_t)t * NB;
-  const int bs = (int)(N - r0 < NB ? N - r0 : NB);
-  const int col = threadIdx.x & 63, rq = threadIdx.x >> 6;
-  const FC *Lit = Linv + (int64_t)t * NB * NB;
-  const int64_t cl0 = (int64_t)(t + 1) * NB;  // last dependency block row
-  const int cls = tk > 0 ? (int)(N - cl0 < NB ? N - cl0 : NB) : 0;
-  for (int e = threadIdx.x; e < NB * NB; e += 256) {
-    Li[e] = Lit[e];
-    int r = e >> 6, cc = e & 63;
-    if (tk > 0) Lp[e] = (r < cls && cc < bs) ? F[(cl0 + r) * N + r0 + cc] : FC{};
-  }
-  double2 s = make_double2(0, 0);
-  int q0 = 0;
-  while (q0 < tk - 1) {
-    if (threadIdx.x == 0) s_n = wait_flags(fl, q0, tk - 1, err, spin_limit);
-    __syncthreads();
-    const int n = s_n;
-    __syncthreads();
-    if (n == 0) return;
-    __threadfence();
-    for (int q = q0; q < q0 + n; q++) {
-      const int cb = nblk - 1 - q;
-      const int64_t c0 = (int64_t)cb * NB;
-      const int cbs = (int)(N - c0 < NB ? N - c0 : NB);
-      if (col < bs)
-        for (int r = rq; r < cbs; r += 4) cfma(s, to_d2(F[(c0 + r) * N + r0 + col]), __ldcg(xr + c0 + r));
-    }
-    q0 += n;
-  }
-  if (tk > 0) {
-    if (threadIdx.x == 0) s_n = wait_flags(fl, tk - 1, tk, err, spin_limit);
-    __syncthreads();
-    if (s_n == 0) return;
-    __threadfence();
-    for (int r = rq; r < cls; r += 4) cfma(s, to_d2(Lp[r * NB + col]), __ldcg(xr + cl0 + r));
-  }
-  part[rq][col] = s;
-  if (threadIdx.x < NB) acc[threadIdx.x] = threadIdx.x < bs ? xr[r0 + threadIdx.x] : make_double2(0, 0);
-  __syncthreads();
-  if (threadIdx.x < NB)
-    acc[threadIdx.x] = csub(acc[threadIdx.x], cadd(cadd(part[0][threadIdx.x], part[1][threadIdx.x]),
-                                                   cadd(part[2][threadIdx.x], part[3][threadIdx.x])));
-  __syncthreads();
-  // x_t = Linv_tt^T acc: x[c] = sum_r Linv[r][c] acc[r]
-  s = make_double2(0, 0);
-  for (int r = rq; r < NB; r += 4) cfma(s, to_d2(Li[r * NB + col]), acc[r]);
-  part[rq][col] = s;
-  __syncthreads();
-  if (threadIdx.x < bs)
-    xr[r0 + threadIdx.x] = cadd(cadd(part[0][threadIdx.x], part[1][threadIdx.x]),
-                                cadd(part[2][threadIdx.x], part[3][threadIdx.x]));
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) atomicExch(fl + tk, 1u);
-}
-
 template <class FC>
 __global__ void k_scale_by_dinv(int64_t N, int64_t R, const FC *__restrict__ F, double2 *__restrict__ x) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1557,10 +1349,6 @@ template <class C> void set_smem_attrs() {
     DMB_CUDA(cudaFuncSetAttribute(k_ldlt_mid64, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)DiagSmem<double2>::bytes));
   }
-  DMB_CUDA(cudaFuncSetAttribute(k_trsv_fwd<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(2 * sizeof(C) * NB * NB)));
-  DMB_CUDA(cudaFuncSetAttribute(k_trsv_bwd<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(2 * sizeof(C) * NB * NB)));
   done = true;
 }
 
@@ -1736,36 +1524,6 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
   DMB_REQUIRE(h_err == 0, DMB_ERR_BREAKDOWN, "near-field factorisation broke down: zero or non-finite pivot");
   if (use_tc)
     DMB_REQUIRE(dmb::tc_error_word(c) == 0, DMB_ERR_TIMEOUT, "tensor-core update: a pipeline wait expired");
-}
-
-void ldlt_solve_blocked_c64(dmb_ctx *c, const float2 *F, double2 *x, int64_t R);
-
-template <class C> void ldlt_solve(dmb_ctx *c, const C *F, double2 *x, int64_t R) {
-  if constexpr (std::is_same<C, float2>::value) {
-    // complex64 factor, one right-hand side: blocked sweeps with the 1024-row
-    // block inverses (the flag-ordered sweeps below run a few columns
-    // concurrently and are faster from two on)
-    if (R == 1) {
-      ldlt_solve_blocked_c64(c, F, x, R);
-      return;
-    }
-  }
-  const int64_t N = c->n;
-  const int nblk = (int)((N + NB - 1) / NB);
-  const size_t flag_words = (size_t)R * nblk + R;
-  c->d_flags.ensure(std::max<size_t>(64, 4 * (flag_words + 2)));
-  unsigned *err = c->d_flags.as<unsigned>();
-  unsigned *tickets = err + 1;
-  unsigned *flags = tickets + R;
-  const C *Linv = c->d_dinv.as<C>();
-  dim3 g(nblk, (unsigned)R);
-  DMB_CUDA(cudaMemsetAsync(err, 0, 4 * (flag_words + 1), c->stream));
-  set_smem_attrs<C>();
-  const size_t sm = 2 * sizeof(C) * NB * NB;
-  DMB_LAUNCH(c, k_trsv_fwd<C>, g, 256, sm, N, F, Linv, x, flags, tickets, err, c->spin_limit);
-  DMB_LAUNCH(c, k_scale_by_dinv<C>, blocks_for(N * R, 256), 256, 0, N, R, F, x);
-  DMB_CUDA(cudaMemsetAsync(tickets, 0, 4 * flag_words, c->stream));
-  DMB_LAUNCH(c, k_trsv_bwd<C>, g, 256, sm, N, F, Linv, x, flags, tickets, err, c->spin_limit);
 }
 
 // ---------------------------------------------------------------------------
@@ -1960,24 +1718,25 @@ template <class C> void forward_block(dmb_ctx *c, const C *F, int64_t o0, int64_
   }
 }
 
-// Inverses of the 1024-row diagonal blocks of the unit lower factor by
-// recursive doubling from the 64 x 64 block inverses of the factorisation:
-// for consecutive s-blocks A, B inside one outer block,
+// Inverses of the OB-row diagonal blocks of the unit lower factor (OB = 1024
+// for the tensor-core sweeps, 256 for the few-column ones) by recursive
+// doubling from the 64 x 64 block inverses of the factorisation: for
+// consecutive s-blocks A, B inside one outer block,
 //   [A 0; C B]^-1 = [A^-1 0; -B^-1 C A^-1  B^-1],
-// s = 64, 128, 256, 512, all pairs of a level in one launch per product.
+// s = 64, 128, .. OB / 2, all pairs of a level in one launch per product.
 // X (column-major, leading dimension N; outer block o occupies rows o0..o1 and
 // block-local columns 0..o1-o0) receives the inverses.
 
 // X <- the 64-block inverses on the diagonal of every outer block, 0 elsewhere
-__global__ void k_inv_init(int64_t N, const float2 *__restrict__ Linv, double2 *__restrict__ X) {
+template <int OB, class FC>
+__global__ void k_inv_init(int64_t N, const FC *__restrict__ Linv, double2 *__restrict__ X) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N * TP_OUTER) return;
+  if (i >= N * OB) return;
   const int64_t col = i / N, r = i % N;  // consecutive threads: consecutive rows
-  const int64_t o0 = r - r % TP_OUTER;
+  const int64_t o0 = r - r % OB;
   double2 v = make_double2(0.0, 0.0);
   if (o0 + col < N && (o0 + col) / NB == r / NB) {
-    const float2 l = Linv[(r / NB) * NB * NB + (r % NB) * NB + (o0 + col) % NB];
-    v = make_double2(l.x, l.y);
+    v = to_d2(Linv[(r / NB) * NB * NB + (r % NB) * NB + (o0 + col) % NB]);
   }
   X[col * N + r] = v;
 }
@@ -1993,14 +1752,14 @@ template <> __device__ __forceinline__ double2 inv_conv<double2>(double2 v) { re
 // 64 x 64 output tiles (grid.x), FP32 SIMT with 16-deep shared stages
 // TC: the arithmetic of the products (float2 for the tensor-core sweeps'
 // inverses, double2 for the one-RHS sweeps')
-template <int STEP, class TC = float2>
-__global__ void __launch_bounds__(256) k_inv_level(int64_t N, int s, const float2 *__restrict__ F,
+template <int STEP, int OB, class FC, class TC>
+__global__ void __launch_bounds__(256) k_inv_level(int64_t N, int s, const FC *__restrict__ F,
                                                    double2 *__restrict__ X, TC *__restrict__ T) {
   __shared__ TC As[16][65];
   __shared__ TC Bs[16][65];
-  const int ppo = TP_OUTER / (2 * s);
-  const int64_t o0 = (int64_t)(blockIdx.y / ppo) * TP_OUTER;
-  const int64_t o1 = min(N, o0 + TP_OUTER);
+  const int ppo = OB / (2 * s);
+  const int64_t o0 = (int64_t)(blockIdx.y / ppo) * OB;
+  const int64_t o1 = min(N, o0 + OB);
   const int64_t i0 = o0 + 2 * (int64_t)s * (blockIdx.y % ppo);
   const int64_t a0 = i0, b0 = i0 + s;
   if (b0 >= o1) return;  // no B block in this slot
@@ -2024,8 +1783,8 @@ __global__ void __launch_bounds__(256) k_inv_level(int64_t N, int s, const float
       if (STEP == 1) {
         const int kk = e & 15, rr = e >> 4;  // k fastest: F rows and X columns are k-contiguous
         const int k = k0 + kk, i = 64 * ti + rr, j = 64 * tj + rr;
-        const float2 f = (k < k_hi && i < sb) ? F[(b0 + i) * N + a0 + k] : make_float2(0.f, 0.f);
-        As[kk][rr] = inv_conv<TC>(make_double2(f.x, f.y));
+        const FC f = (k < k_hi && i < sb) ? F[(b0 + i) * N + a0 + k] : czero<FC>();
+        As[kk][rr] = inv_conv<TC>(to_d2(f));
         const double2 x = (k < k_hi) ? X[(a0 - o0 + j) * N + a0 + k] : make_double2(0.0, 0.0);
         Bs[kk][rr] = inv_conv<TC>(x);
       } else {
@@ -2068,28 +1827,26 @@ __global__ void __launch_bounds__(256) k_inv_level(int64_t N, int s, const float
 // Pack the complex64 factor for the tensor-core sweeps (once per
 // factorisation): L'' and (L^T)'', and the inverses of the 1024-row diagonal
 // blocks of L (recursive doubling, k_inv_init / k_inv_level).
-// The 1024-row block inverses of L (once per factorisation): FP32 products
-// into d_trsm_id for the tensor-core sweeps (which round them to TF32
-// anyway), FP64 products into d_sv_inv for the one-RHS sweeps (as accurate as
-// substitution with the stored 64-block inverses).
-template <class TC> void prepare_block_inverses(dmb_ctx *c, const float2 *F) {
-  constexpr bool f64 = std::is_same<TC, double2>::value;
-  uint64_t &ver = f64 ? c->f_inv64 : c->f_inv;
+// The block inverses of L (once per factorisation): 1024-row ones by FP32
+// products into d_trsm_id for the tensor-core sweeps (which round them to TF32
+// anyway), 256-row ones by FP64 products into d_sv_inv for the few-column
+// sweeps (as accurate as substitution with the stored 64-block inverses).
+template <int OB, class FC, class TC>
+void prepare_block_inverses(dmb_ctx *c, const FC *F, DevBuf &dst, uint64_t &ver) {
   if (ver == c->f_version) return;
   const int64_t N = c->n;
-  DevBuf &dst = f64 ? c->d_sv_inv : c->d_trsm_id;
-  dst.ensure(sizeof(double2) * N * TP_OUTER);
+  dst.ensure(sizeof(double2) * N * OB);
   double2 *Xid = dst.as<double2>();
-  const int64_t nout = (N + TP_OUTER - 1) / TP_OUTER;
-  // scratch for the products T: (pair slots) x s x s <= nout x 1024 x 256
-  c->d_trsm_t.ensure(sizeof(TC) * nout * TP_OUTER * (TP_OUTER / 4));
+  const int64_t nout = (N + OB - 1) / OB;
+  // scratch for the products T: (pair slots) x s x s <= nout x OB x OB / 4
+  c->d_trsm_t.ensure(sizeof(TC) * nout * OB * (OB / 4));
   TC *T = c->d_trsm_t.as<TC>();
-  DMB_LAUNCH(c, k_inv_init, blocks_for(N * TP_OUTER, 256), 256, 0, N, c->d_dinv.as<float2>(), Xid);
-  for (int s = NB; s < TP_OUTER; s *= 2) {
+  DMB_LAUNCH(c, (k_inv_init<OB, FC>), blocks_for(N * OB, 256), 256, 0, N, c->d_dinv.as<FC>(), Xid);
+  for (int s = NB; s < OB && s < N; s *= 2) {
     const int nt = (s + 63) / 64;
-    dim3 g((unsigned)(nt * nt), (unsigned)(nout * (TP_OUTER / (2 * s))));
-    DMB_LAUNCH(c, (k_inv_level<1, TC>), g, 256, 0, N, s, F, Xid, T);
-    DMB_LAUNCH(c, (k_inv_level<2, TC>), g, 256, 0, N, s, F, Xid, T);
+    dim3 g((unsigned)(nt * nt), (unsigned)(nout * (OB / (2 * s))));
+    DMB_LAUNCH(c, (k_inv_level<1, OB, FC, TC>), g, 256, 0, N, s, F, Xid, T);
+    DMB_LAUNCH(c, (k_inv_level<2, OB, FC, TC>), g, 256, 0, N, s, F, Xid, T);
   }
   ver = c->f_version;
 }
@@ -2099,7 +1856,7 @@ void prepare_packed_factor(dmb_ctx *c, const float2 *F) {
   const int64_t N = c->n;
   trsm_panel_attrs<float2>();
   dmb::tc_trsm_pack_factor(c, F, N);
-  prepare_block_inverses<float2>(c, F);
+  prepare_block_inverses<TP_OUTER, float2, float2>(c, F, c->d_trsm_id, c->f_inv);
   double2 *Xid = c->d_trsm_id.as<double2>();
   const int64_t nout = (N + TP_OUTER - 1) / TP_OUTER;
   for (int64_t o = 0; o < nout; o++) {
@@ -2110,116 +1867,225 @@ void prepare_packed_factor(dmb_ctx *c, const float2 *F) {
 }
 
 // ---------------------------------------------------------------------------
-// One-RHS sweeps of a complex64 factor with the 1024-row block inverses X_o:
-//   forward, o = 0, 1, ...:  a = b_o - L[o, <o] y;   y_o = X_o a
-//   backward, o = last..0:   a = z_o - L[>o, o]^T x; x_o = X_o^T a
-// Eleven block steps per sweep at N = 10,680, each two or three launches of
-// bandwidth-bound products (L read once per sweep, X_o once); no waits
-// between CTAs, fixed summation order.
+// Triangular sweeps for one to seven right-hand sides (one per grid.y), L and
+// its transpose, by data flow over 256-row blocks:
+//   forward,  o = 0..last: a_o = b_o - L[o, <o] y,       y_o = X_o a_o
+//   backward, o = last..0: a_o = y_o / D - L[>o, o]^T x, x_o = X_o^T a_o
+// with X_o the inverse of L's diagonal block.  A CTA owns 16 rows (forward) or
+// columns (backward) of a block: it streams its part of L block by block as the
+// blocks of y (x) are published, publishes its 16 values of a_o, and, once all
+// of a_o is there, its 16 values of X_o a_o.  The next block's part of L and
+// the part of X_o are loaded ahead of the waits, so a block costs two flag round
+// trips and two short on-chip sums; the stream of L runs beside that chain
+// over all SMs.  CTAs take their slices in ticket order and wait only on
+// earlier tickets; every wait is bounded (error bit 4).  All sums in a fixed
+// order.  Bound by the chain, about 6 us a block, up to N = 10,000 and by the
+// read of L above.  (Chains of 64-row blocks on one CTA each took 8 us a block:
+// 1.39 ms a sweep at N = 10,680, complex128.)
 // ---------------------------------------------------------------------------
-constexpr int SV_IC = 64;  // rows per partial-sum chunk of the column products
+constexpr int SV = 256;  // rows per block
+constexpr int SW = 16;   // rows per CTA
 
-// y[i] = (SUB ? b[i] - s : s), s = sum_j M[i ld + j] v[j], i < rows: a warp per row
-template <class MC, bool SUB>
-__global__ void __launch_bounds__(256) k_sv_rowdot(int rows, int cols, const MC *__restrict__ M, int64_t ld,
-                                                   const double2 *__restrict__ v, const double2 *__restrict__ b,
-                                                   double2 *__restrict__ y) {
-  const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (i >= rows) return;
-  const MC *Mi = M + (int64_t)i * ld;
-  // four loads in flight per lane (one warp per row leaves few warps)
-  double2 a0 = make_double2(0, 0), a1 = make_double2(0, 0), a2 = make_double2(0, 0), a3 = make_double2(0, 0);
-  int j = lane;
-  for (; j + 96 < cols; j += 128) {
-    cfma(a0, to_d2(Mi[j]), v[j]);
-    cfma(a1, to_d2(Mi[j + 32]), v[j + 32]);
-    cfma(a2, to_d2(Mi[j + 64]), v[j + 64]);
-    cfma(a3, to_d2(Mi[j + 96]), v[j + 96]);
+// wait until *cnt reaches want (thread 0); false on expiry or another CTA's
+__device__ __forceinline__ bool wait_count(volatile unsigned *cnt, unsigned want, unsigned *err, long long limit) {
+  long long it = 0;
+  while (*cnt < want) {
+    if (++it > limit) {
+      atomicOr(err, 4u);
+      return false;
+    }
+    if ((it & 15) == 0) {
+      if (*((volatile unsigned *)err) & 4u) return false;
+      if (it > 64) __nanosleep(20);
+    }
   }
-  for (; j < cols; j += 32) cfma(a0, to_d2(Mi[j]), v[j]);
-  a0 = warp_sum2(cadd(cadd(a0, a1), cadd(a2, a3)));
-  if (lane == 0) y[i] = SUB ? csub(b[i], a0) : a0;
+  __threadfence();
+  return true;
 }
 
-// part[chunk][j] = sum over the chunk's rows i of M[i ld + j] v[i], j < ncols
-// (chunk = blockIdx.y, SV_IC rows; consecutive threads read consecutive j)
+__device__ __forceinline__ unsigned sweep_slices(int64_t N, int64_t o) {  // CTAs of block o
+  return (unsigned)((min((int64_t)SV, N - o * SV) + SW - 1) / SW);
+}
+
+// Rows r, r + 1 of a warp against the 256 vector values v (lane + 32 j):
+// the matrix values m0, m1 are in registers already
 template <class MC>
-__global__ void __launch_bounds__(256) k_sv_colpart(int nrows, int ncols, const MC *__restrict__ M, int64_t ld,
-                                                    const double2 *__restrict__ v, double2 *__restrict__ part) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= ncols) return;
-  const int i0 = blockIdx.y * SV_IC, i1 = min(nrows, i0 + SV_IC);
-  double2 a0 = make_double2(0, 0), a1 = make_double2(0, 0);
-  int i = i0;
-  for (; i + 1 < i1; i += 2) {
-    cfma(a0, to_d2(M[(int64_t)i * ld + j]), v[i]);
-    cfma(a1, to_d2(M[(int64_t)(i + 1) * ld + j]), v[i + 1]);
+__device__ __forceinline__ void rows2_fma(const MC (&m0)[8], const MC (&m1)[8], const double2 *v, int n, int lane,
+                                          double2 &s0, double2 &s1) {
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const double2 y = lane + 32 * j < n ? __ldcg(v + lane + 32 * j) : make_double2(0.0, 0.0);
+    cfma(s0, to_d2(m0[j]), y);
+    cfma(s1, to_d2(m1[j]), y);
   }
-  if (i < i1) cfma(a0, to_d2(M[(int64_t)i * ld + j]), v[i]);
-  part[(int64_t)blockIdx.y * ncols + j] = cadd(a0, a1);
 }
 
-// y[j] = (sub ? b[j] - s : s), s = the chunks' partial sums in order
-__global__ void k_sv_colsum(int ncols, int nchunks, const double2 *__restrict__ part, const double2 *__restrict__ b,
-                            int sub, double2 *__restrict__ y) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= ncols) return;
-  double2 s = make_double2(0, 0);
-  for (int q = 0; q < nchunks; q++) s = cadd(s, part[(int64_t)q * ncols + j]);
-  y[j] = sub ? csub(b[j], s) : s;
+// sum of the 16 row groups (threads t with equal t & 15) -> red[0][t & 15]'s
+// total on threads below 16
+__device__ __forceinline__ double2 cols_sum(double2 v, double2 (*red)[SW]) {
+  const int t = threadIdx.x;
+  v.x += __shfl_xor_sync(0xffffffffu, v.x, 16);
+  v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
+  __syncthreads();
+  if ((t & 31) < 16) red[t >> 5][t & 15] = v;
+  __syncthreads();
+  double2 s = make_double2(0.0, 0.0);
+  if (t < 16)
+#pragma unroll
+    for (int g = 0; g < 8; g++) s = cadd(s, red[g][t]);
+  return s;
 }
 
-void ldlt_solve_blocked_c64(dmb_ctx *c, const float2 *F, double2 *x, int64_t R) {
-  const int64_t N = c->n;
-  prepare_block_inverses<double2>(c, F);
+template <class FC>
+__global__ void __launch_bounds__(256, 2) k_sweep_fwd(int64_t N, const FC *__restrict__ F,
+                                                      const double2 *__restrict__ X, double2 *x, double2 *abuf,
+                                                      unsigned *tickets, unsigned *acnt, unsigned *ycnt, unsigned *err,
+                                                      long long limit) {
+  __shared__ double2 red[8][SW];
+  __shared__ int s_t, s_ok;
+  const int rhs = blockIdx.y, t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int64_t nblk = (N + SV - 1) / SV;
+  x += rhs * N;
+  abuf += rhs * N;
+  acnt += rhs * nblk;
+  ycnt += rhs * nblk;
+  if (t == 0) s_t = (int)atomicAdd(tickets + rhs, 1u);
+  __syncthreads();
+  const int64_t r0 = (int64_t)s_t * SW, o = r0 / SV, o0 = o * SV;
+  const int i = (int)((r0 - o0) / SW), nr = (int)min((int64_t)SW, N - r0);
+  auto wait = [&](unsigned *cnt, unsigned want) {
+    if (t == 0) s_ok = wait_count(cnt, want, err, limit) ? 1 : 0;
+    __syncthreads();
+    const bool ok = s_ok != 0;
+    __syncthreads();
+    return ok;
+  };
+  const int64_t ra = r0 + 2 * warp;  // this warp's rows ra, ra + 1
+  double2 s0 = make_double2(0.0, 0.0), s1 = s0;
+  for (int64_t p = 0; p < o; p++) {
+    FC m0[8], m1[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      m0[j] = ra < N ? F[ra * N + p * SV + lane + 32 * j] : czero<FC>();
+      m1[j] = ra + 1 < N ? F[(ra + 1) * N + p * SV + lane + 32 * j] : czero<FC>();
+    }
+    if (!wait(ycnt + p, SV / SW)) return;
+    rows2_fma(m0, m1, x + p * SV, SV, lane, s0, s1);
+  }
+  s0 = warp_sum2(s0);
+  s1 = warp_sum2(s1);
+  if (lane < 2 && 2 * warp + lane < nr)
+    __stcg(abuf + ra + lane, csub(x[ra + lane], lane == 0 ? s0 : s1));
+  // X_o: column r0 + c of the inverse's rows, k = g + 16 j <= row
+  const int c = t & 15, g = t >> 4;
+  double2 xv[16];
+#pragma unroll
+  for (int j = 0; j < 16; j++)
+    xv[j] = (j <= i && c < nr) ? X[(int64_t)(g + 16 * j) * N + r0 + c] : make_double2(0.0, 0.0);
+  __syncthreads();
+  if (t == 0) {
+    __threadfence();
+    atomicAdd(acnt + o, 1u);
+  }
+  if (!wait(acnt + o, sweep_slices(N, o))) return;
+  double2 v = make_double2(0.0, 0.0);
+#pragma unroll
+  for (int j = 0; j < 16; j++)
+    if (j <= i && g + 16 * j < N - o0) cfma(v, xv[j], __ldcg(abuf + o0 + g + 16 * j));
+  v = cols_sum(v, red);
+  if (t < nr) __stcg(x + r0 + t, v);
+  __syncthreads();
+  if (t == 0) {
+    __threadfence();
+    atomicAdd(ycnt + o, 1u);
+  }
+}
+
+template <class FC>
+__global__ void __launch_bounds__(256, 2) k_sweep_bwd(int64_t N, const FC *__restrict__ F,
+                                                      const double2 *__restrict__ X, double2 *x, double2 *abuf,
+                                                      unsigned *tickets, unsigned *acnt, unsigned *xcnt, unsigned *err,
+                                                      long long limit) {
+  __shared__ double2 red[8][SW];
+  __shared__ int s_t, s_ok;
+  const int rhs = blockIdx.y, t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int64_t nblk = (N + SV - 1) / SV;
+  x += rhs * N;
+  abuf += rhs * N;
+  acnt += rhs * nblk;
+  xcnt += rhs * nblk;
+  if (t == 0) s_t = (int)atomicAdd(tickets + rhs, 1u);
+  __syncthreads();
+  const int64_t r0 = ((N + SW - 1) / SW - 1 - s_t) * SW, o = r0 / SV, o0 = o * SV;
+  const int nr = (int)min((int64_t)SW, N - r0), w = (int)min((int64_t)SV, N - o0);
+  auto wait = [&](unsigned *cnt, unsigned want) {
+    if (t == 0) s_ok = wait_count(cnt, want, err, limit) ? 1 : 0;
+    __syncthreads();
+    const bool ok = s_ok != 0;
+    __syncthreads();
+    return ok;
+  };
+  const int c = t & 15, g = t >> 4;  // column r0 + c, rows g + 16 j of a block
+  double2 v = make_double2(0.0, 0.0);
+  for (int64_t p = nblk - 1; p > o; p--) {
+    const int n = (int)min((int64_t)SV, N - p * SV);
+    FC m[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++)
+      m[j] = (g + 16 * j < n && c < nr) ? F[(p * SV + g + 16 * j) * N + r0 + c] : czero<FC>();
+    if (!wait(xcnt + p, sweep_slices(N, p))) return;
+#pragma unroll
+    for (int j = 0; j < 16; j++)
+      if (g + 16 * j < n) cfma(v, to_d2(m[j]), __ldcg(x + p * SV + g + 16 * j));
+  }
+  v = cols_sum(v, red);
+  if (t < nr) {
+    const int64_t r = r0 + t;
+    __stcg(abuf + r, csub(cdiv(x[r], to_d2(F[r * N + r])), v));
+  }
+  // X_o^T: outputs ra, ra + 1 of a warp, the inverse's columns of these rows
+  const int64_t ra = r0 + 2 * warp;
+  double2 m0[8], m1[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const int k = lane + 32 * j;
+    m0[j] = (ra < N && k < w) ? X[(ra - o0) * N + o0 + k] : make_double2(0.0, 0.0);
+    m1[j] = (ra + 1 < N && k < w) ? X[(ra + 1 - o0) * N + o0 + k] : make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  if (t == 0) {
+    __threadfence();
+    atomicAdd(acnt + o, 1u);
+  }
+  if (!wait(acnt + o, sweep_slices(N, o))) return;
+  double2 s0 = make_double2(0.0, 0.0), s1 = s0;
+  rows2_fma(m0, m1, abuf + o0, w, lane, s0, s1);
+  s0 = warp_sum2(s0);
+  s1 = warp_sum2(s1);
+  if (lane < 2 && 2 * warp + lane < nr) __stcg(x + ra + lane, lane == 0 ? s0 : s1);
+  __syncthreads();
+  if (t == 0) {
+    __threadfence();
+    atomicAdd(xcnt + o, 1u);
+  }
+}
+
+template <class C> void ldlt_solve(dmb_ctx *c, const C *F, double2 *x, int64_t R) {
+  const int64_t N = c->n, nblk = (N + SV - 1) / SV;
+  prepare_block_inverses<SV, C, double2>(c, F, c->d_sv_inv, c->f_inv64);
   const double2 *X = c->d_sv_inv.as<double2>();
-  const int64_t nout = (N + TP_OUTER - 1) / TP_OUTER;
-  const int max_chunks = (int)std::max<int64_t>((N + SV_IC - 1) / SV_IC, 1);
-  c->d_sv_acc.ensure(sizeof(double2) * TP_OUTER);
-  c->d_sv_part.ensure(sizeof(double2) * (size_t)max_chunks * TP_OUTER);
-  double2 *acc = c->d_sv_acc.as<double2>(), *part = c->d_sv_part.as<double2>();
-  for (int64_t r = 0; r < R; r++) {
-    double2 *xr = x + r * N;
-    for (int64_t o = 0; o < nout; o++) {  // forward
-      const int64_t o0 = o * TP_OUTER;
-      const int w = (int)std::min<int64_t>(TP_OUTER, N - o0);
-      const double2 *a = xr + o0;
-      if (o0 > 0) {
-        DMB_LAUNCH(c, (k_sv_rowdot<float2, true>), blocks_for((int64_t)w * 32, 256), 256, 0, w, (int)o0,
-                   F + o0 * N, N, xr, xr + o0, acc);
-        a = acc;
-      }
-      const int nch = (w + SV_IC - 1) / SV_IC;
-      // y_o[i] = sum_k X_o[i][k] a[k]; X_o column k is contiguous: X[k N + o0 + i]
-      DMB_LAUNCH(c, k_sv_colpart<double2>, dim3(blocks_for(w, 256), (unsigned)nch), 256, 0, w, w, X + o0, N, a,
-                 part);
-      DMB_LAUNCH(c, k_sv_colsum, blocks_for(w, 256), 256, 0, w, nch, part, (const double2 *)nullptr, 0, xr + o0);
-    }
-    DMB_LAUNCH(c, k_scale_by_dinv<float2>, blocks_for(N, 256), 256, 0, N, (int64_t)1, F, xr);
-    for (int64_t o = nout - 1; o >= 0; o--) {  // backward
-      const int64_t o0 = o * TP_OUTER, o1 = std::min<int64_t>(N, o0 + TP_OUTER);
-      const int w = (int)(o1 - o0);
-      const double2 *a = xr + o0;
-      if (o1 < N) {
-        // a[c] = z[o0 + c] - sum_{i >= o1} L[i][o0 + c] x[i]
-        const int nr = (int)(N - o1), nch = (nr + SV_IC - 1) / SV_IC;
-        DMB_LAUNCH(c, k_sv_colpart<float2>, dim3(blocks_for(w, 256), (unsigned)nch), 256, 0, nr, w,
-                   F + o1 * N + o0, N, xr + o1, part);
-        DMB_LAUNCH(c, k_sv_colsum, blocks_for(w, 256), 256, 0, w, nch, part, xr + o0, 1, acc);
-        a = acc;
-      }
-      // x_o[k] = sum_i X_o[i][k] a[i] = sum_i X[k N + o0 + i] a[i]: a warp per output
-      if (a == acc) {
-        DMB_LAUNCH(c, (k_sv_rowdot<double2, false>), blocks_for((int64_t)w * 32, 256), 256, 0, w, w, X + o0, N, a,
-                   (const double2 *)nullptr, xr + o0);
-      } else {
-        // the last block reads and writes x_o: go through the scratch vector
-        DMB_CUDA(cudaMemcpyAsync(acc, xr + o0, sizeof(double2) * w, cudaMemcpyDeviceToDevice, c->stream));
-        DMB_LAUNCH(c, (k_sv_rowdot<double2, false>), blocks_for((int64_t)w * 32, 256), 256, 0, w, w, X + o0, N,
-                   acc, (const double2 *)nullptr, xr + o0);
-      }
-    }
-  }
+  c->d_sv_acc.ensure(sizeof(double2) * 2 * N * R);
+  double2 *abuf = c->d_sv_acc.as<double2>();
+  // the error word, a ticket counter per column and sweep, four counters per
+  // block, column
+  const size_t words = 1 + 2 * R + 4 * R * nblk;
+  c->d_flags.ensure(std::max<size_t>(64, 4 * words));
+  unsigned *err = c->d_flags.as<unsigned>(), *tickets = err + 1, *cnt = tickets + 2 * R;
+  DMB_CUDA(cudaMemsetAsync(err, 0, 4 * words, c->stream));
+  const dim3 g((unsigned)((N + SW - 1) / SW), (unsigned)R);
+  DMB_LAUNCH(c, k_sweep_fwd<C>, g, 256, 0, N, F, X, x, abuf, tickets, cnt, cnt + R * nblk, err, c->spin_limit);
+  DMB_LAUNCH(c, k_sweep_bwd<C>, g, 256, 0, N, F, X, x, abuf + N * R, tickets + R, cnt + 2 * R * nblk,
+             cnt + 3 * R * nblk, err, c->spin_limit);
 }
 
 template <class C> void ldlt_solve_batched(dmb_ctx *c, const C *F, double2 *X, int64_t R) {
@@ -2346,6 +2212,16 @@ void nf_factor_resident(dmb_ctx *c, int kind, int precision) {
   c->pc_kind = kind;
   c->pc_prec = precision;
   c->pc_valid = true;
+}
+
+// what applications of the factor keep per factor, made now: a captured
+// iteration replayed with a later factor does not make it
+void pc_prepare_dev(dmb_ctx *c, int64_t nrhs) {
+  if (c->pc_kind != DMB_PRECOND_NF_LU || nrhs >= 8) return;
+  if (c->pc_prec == DMB_PREC_FP64)
+    prepare_block_inverses<SV, double2, double2>(c, c->d_F.as<double2>(), c->d_sv_inv, c->f_inv64);
+  else
+    prepare_block_inverses<SV, float2, double2>(c, c->d_F.as<float2>(), c->d_sv_inv, c->f_inv64);
 }
 
 void pc_apply_dev(dmb_ctx *c, double *x, int64_t nrhs) {

@@ -300,8 +300,8 @@ struct dmb_ctx {
   uint64_t f_version = 0;        // bumped by every LDL^T factorisation
   uint64_t f_packed = ~0ull;     // factor version packed for the batched triangular solves
   uint64_t f_inv = ~0ull;        // factor version whose 1024-row block inverses are in d_trsm_id
-  uint64_t f_inv64 = ~0ull;      // ... whose FP64-product block inverses are in d_sv_inv
-  DevBuf d_sv_acc, d_sv_part, d_sv_inv;  // the blocked one-RHS sweeps: scratch and block inverses
+  uint64_t f_inv64 = ~0ull;      // ... whose 256-row block inverses (FP64 products) are in d_sv_inv
+  DevBuf d_sv_acc, d_sv_inv;     // the few-column sweeps: scratch and block inverses
   // inputs of the current host topology (build_host_topology)
   bool topo_valid = false;
   std::vector<int32_t> topo_tri, topo_tplus, topo_tminus;
@@ -437,6 +437,7 @@ void matvec_dev(dmb_ctx *c, const void *x, void *y, int64_t nrhs);  // device bu
 void conj_dev(dmb_ctx *c, double2 *x, int64_t count);
 void nf_build(dmb_ctx *c, double cutoff, int kind);
 void pc_apply_dev(dmb_ctx *c, double *x, int64_t nrhs);             // in place, c128 device
+void pc_prepare_dev(dmb_ctx *c, int64_t nrhs);  // per-factor operands of pc_apply_dev
 void rhs_plane_waves_dev(dmb_ctx *c, const double *kvecs, const double *E0s, const double *pols,
                          int64_t R, int quad_order, double *V_dev);
 void rhs_plane_waves_async(dmb_ctx *c, const double *kvecs, const double *E0s, const double *pols, int64_t R,

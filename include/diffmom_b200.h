@@ -140,9 +140,8 @@ const char *dmb_version(void);
  * meets the tolerance.  0 stops exactly where Krylov.gmres stops (iteration
  * counts of the reference). */
 #define DMB_OPT_TRUE_RESIDUAL 8
-/* DMB_OPT_SPIN_LIMIT: polls a waiting CTA of the chained triangular sweeps
- * (complex128 factors, and 2-7 right-hand sides of complex64 ones) makes
- * before it gives up; the call then fails with DMB_ERR_TIMEOUT and the context
+/* DMB_OPT_SPIN_LIMIT: polls a waiting CTA of the data-flow triangular sweeps
+ * (one to seven right-hand sides) makes before it gives up; the call then fails with DMB_ERR_TIMEOUT and the context
  * stays usable.  A negative value restores the default (2e7 polls, seconds);
  * small values exercise the timeout path without any GPU fault. */
 #define DMB_OPT_SPIN_LIMIT 9
