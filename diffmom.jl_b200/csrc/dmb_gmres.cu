@@ -23,48 +23,81 @@ namespace {
 
 unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
-// h[r][i] = <V_i(r), w(r)> for i in [0, j]
-__global__ void k_dots(int64_t N, int64_t R, int j, int64_t vstride, const double2 *__restrict__ V,
-                       const double2 *__restrict__ w, double2 *__restrict__ h, int hld) {
-  __shared__ double2 red[32];
-  int i = blockIdx.x;
-  int64_t r = blockIdx.y;
+// One Arnoldi step is five launches (few systems are launch- and latency-bound:
+// ten launches with single-thread accumulations took 84 us a step at 9,720
+// unknowns, 90 basis vectors): twice k_dots / k_cgs_update, then k_arnoldi_next.
+// Reductions leave partial sums that the next kernel's CTAs add up in order,
+// each for itself, so nothing waits on one last CTA.
+
+// hp[r][i][s] = part s (of gridDim.z) of <V_i(r), w(r)>; zeroes the count of
+// active systems for the end of the step
+__global__ void __launch_bounds__(256) k_dots(int64_t N, int64_t vstride, const double2 *__restrict__ V,
+                                              const double2 *__restrict__ w, double2 *__restrict__ hp,
+                                              unsigned *__restrict__ active) {
+  __shared__ double2 red[8];
+  const int i = blockIdx.x, s = blockIdx.z, S = gridDim.z;
+  const int64_t r = blockIdx.y, n0 = N * s / S, n1 = N * (s + 1) / S;
   const double2 *vi = V + (int64_t)i * vstride + r * N;
   const double2 *wr = w + r * N;
   double re = 0, im = 0;
-  for (int64_t n = threadIdx.x; n < N; n += blockDim.x) {
-    double2 a = vi[n], b = wr[n];
+#pragma unroll 4
+  for (int64_t n = n0 + threadIdx.x; n < n1; n += 256) {
+    const double2 a = vi[n], b = wr[n];
     re = fma(a.x, b.x, fma(a.y, b.y, re));
     im = fma(a.x, b.y, fma(-a.y, b.x, im));
   }
-  double2 v = warp_sum2(make_double2(re, im));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x / 32] = v;
+  const double2 v = warp_sum2(make_double2(re, im));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    v = threadIdx.x < blockDim.x / 32 ? red[threadIdx.x] : make_double2(0, 0);
-    v = warp_sum2(v);
-    if (threadIdx.x == 0) h[r * hld + i] = v;
+  if (threadIdx.x == 0) {
+    double2 t = red[0];
+    for (int q = 1; q < 8; q++) t = cadd(t, red[q]);
+    hp[(r * gridDim.x + i) * S + s] = t;
+    if (i == 0 && r == 0 && s == 0) *active = 0;
   }
-  (void)j;
 }
 
-// w(r) -= sum_i h[r][i] V_i(r); H[r][:, j] += h
-__global__ void k_cgs_update(int64_t N, int64_t R, int j, int64_t vstride, const double2 *__restrict__ V,
-                             const double2 *__restrict__ h, int hld, double2 *__restrict__ w) {
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= N * R) return;
-  int64_t r = idx / N, n = idx % N;
-  double2 acc = w[idx];
-  for (int i = 0; i <= j; i++) acc = csub(acc, cmul(h[r * hld + i], V[(int64_t)i * vstride + r * N + n]));
-  w[idx] = acc;
-}
-
-__global__ void k_hacc(int64_t R, int j, const double2 *__restrict__ h, int hld, double2 *__restrict__ H,
-                       int kcap) {
-  int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  double2 *Hr = H + r * (int64_t)(kcap + 1) * kcap + (int64_t)j * (kcap + 1);
-  for (int i = 0; i <= j; i++) Hr[i] = cadd(Hr[i], h[r * hld + i]);
+// w(r) -= sum_{i < m} h_i V_i(r), h_i the sum of hp's S parts; the first CTA of
+// a system adds h to column m - 1 of its H; np (if not null): per CTA the
+// partial sum of |w|^2
+constexpr int UPD_T = 64, UPD_H = 512;  // threads per CTA, coefficients per shared pass
+__global__ void __launch_bounds__(UPD_T) k_cgs_update(int64_t N, int m, int S, int64_t vstride,
+                                                      const double2 *__restrict__ V, const double2 *__restrict__ hp,
+                                                      double2 *__restrict__ w, double2 *__restrict__ H, int kcap,
+                                                      double *__restrict__ np) {
+  __shared__ double2 h[UPD_H];
+  __shared__ double red[UPD_T / 32];
+  const int64_t r = blockIdx.y, n = (int64_t)blockIdx.x * UPD_T + threadIdx.x;
+  double2 *Hr = H + r * (int64_t)(kcap + 1) * kcap + (int64_t)(m - 1) * (kcap + 1);
+  double2 acc = n < N ? w[r * N + n] : make_double2(0, 0);
+  for (int i0 = 0; i0 < m; i0 += UPD_H) {
+    const int ni = min(UPD_H, m - i0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < ni; i += UPD_T) {
+      const double2 *p = hp + (r * m + i0 + i) * S;
+      double2 t = p[0];
+      for (int s = 1; s < S; s++) t = cadd(t, p[s]);
+      h[i] = t;
+      if (blockIdx.x == 0) Hr[i0 + i] = cadd(Hr[i0 + i], t);
+    }
+    __syncthreads();
+    if (n < N) {
+      const double2 *v = V + (int64_t)i0 * vstride + r * N + n;
+#pragma unroll 8
+      for (int i = 0; i < ni; i++) acc = csub(acc, cmul(h[i], v[(int64_t)i * vstride]));
+    }
+  }
+  if (n < N) w[r * N + n] = acc;
+  if (np) {
+    const double s = warp_sum(n < N ? cabs2(acc) : 0.0);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = red[0];
+      for (int q = 1; q < UPD_T / 32; q++) t += red[q];
+      np[r * gridDim.x + blockIdx.x] = t;
+    }
+  }
 }
 
 __global__ void k_norms(int64_t N, const double2 *__restrict__ w, double *__restrict__ out) {
@@ -124,76 +157,125 @@ __global__ void k_init_state(int64_t R, const double *__restrict__ nrm, double t
   gr[0] = make_double2(nrm[r], 0);
 }
 
-// Givens update of column j for every active system
-__global__ void k_givens(int64_t R, int j, int kcap, double2 *__restrict__ H, const double *__restrict__ hnext,
-                         double *__restrict__ cs, double2 *__restrict__ sn, double2 *__restrict__ g,
-                         SysState *__restrict__ st, unsigned *__restrict__ active) {
-  int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  SysState s = st[r];
-  if (s.done >= 2) return;
-  double2 *Hc = H + r * (int64_t)(kcap + 1) * kcap + (int64_t)j * (kcap + 1);
-  double *c = cs + r * (int64_t)kcap;
-  double2 *sv = sn + r * (int64_t)kcap;
-  double2 *gr = g + r * (int64_t)(kcap + 1);
-  Hc[j + 1] = make_double2(hnext[r], 0);
-  // previous rotations: [c s; -conj(s) c]
+// Givens update of column j of one system by one thread; col: the column's
+// first j entries in shared memory, rotated by the rotations rc, rs (shared)
+__device__ void givens_column(int j, double hnext, double2 *col, const double *rc, const double2 *rs,
+                              double2 *__restrict__ Hc, double *__restrict__ c, double2 *__restrict__ sv,
+                              double2 *__restrict__ gr, SysState &s) {
+  // the rotations [c s; -conj(s) c] in order; only the running entry b feeds
+  // the next one
+  double2 a = col[0];
   for (int i = 0; i < j; i++) {
-    double2 a = Hc[i], b = Hc[i + 1];
-    Hc[i] = cadd(cscale(a, c[i]), cmul(sv[i], b));
-    Hc[i + 1] = csub(cscale(b, c[i]), cmul(cconj(sv[i]), a));
+    const double2 b = col[i + 1];
+    col[i] = cadd(cscale(a, rc[i]), cmul(rs[i], b));
+    a = csub(cscale(b, rc[i]), cmul(cconj(rs[i]), a));
   }
-  double2 a = Hc[j], b = Hc[j + 1];
-  double na = hypot(a.x, a.y), nb = hypot(b.x, b.y);
+  const double na = hypot(a.x, a.y), nb = fabs(hnext);
   double cc;
   double2 ss, rho;
   if (nb == 0.0) {
     cc = 1.0; ss = make_double2(0, 0); rho = a;
   } else if (na == 0.0) {
-    cc = 0.0; ss = cdiv(cconj(b), make_double2(nb, 0)); rho = make_double2(nb, 0);
+    cc = 0.0; ss = make_double2(hnext / nb, 0); rho = make_double2(nb, 0);
   } else {
-    double t = hypot(na, nb);
-    double2 sa = cscale(a, 1.0 / na);
+    const double t = hypot(na, nb);
+    const double2 sa = cscale(a, 1.0 / na);
     cc = na / t;
-    ss = cscale(cmul(sa, cconj(b)), 1.0 / t);
+    ss = cscale(sa, hnext / t);
     rho = cscale(sa, t);
   }
   c[j] = cc;
   sv[j] = ss;
   Hc[j] = rho;
   Hc[j + 1] = make_double2(0, 0);
-  double2 gj = gr[j];
+  const double2 gj = gr[j], gn = cscale(cmul(cconj(ss), gj), -1.0);
   gr[j] = cscale(gj, cc);
-  gr[j + 1] = cscale(cmul(cconj(ss), gj), -1.0);
+  gr[j + 1] = gn;
   s.kx = j + 1;
-  s.resid_x = hypot(gr[j + 1].x, gr[j + 1].y);
+  s.resid_x = hypot(gn.x, gn.y);
   if (s.done == 0) {
     s.k = j + 1;
     s.resid = s.resid_x;
     if (s.resid <= s.eps) s.done = 1;
-    else if (hnext[r] == 0.0) s.done = 2;  // lucky breakdown: exact solution in the space
+    else if (hnext == 0.0) s.done = 2;  // lucky breakdown: exact solution in the space
     if (!isfinite(s.resid)) s.done = 3;
   }
-  st[r] = s;
-  if (!s.done) atomicAdd(active, 1u);
 }
 
-// y = R^-1 g (back substitution, per system), stored in y[r][i]
-__global__ void k_backsolve(int64_t R, int kcap, const double2 *__restrict__ H, const double2 *__restrict__ g,
-                            const SysState *__restrict__ st, double2 *__restrict__ y) {
-  int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  int k = st[r].k;
+// End of an Arnoldi step: the norm of w from its partial sums, V_{j+1} = w /
+// norm, and (a system's first CTA) the Givens update of column j
+constexpr int NXT_T = 128, NXT_J = 512;  // rotations of a longer column stay in global memory
+__global__ void __launch_bounds__(NXT_T) k_arnoldi_next(int64_t N, int j, int kcap, int nparts,
+                                                        const double *__restrict__ np, const double2 *__restrict__ w,
+                                                        double2 *__restrict__ Vn, double2 *__restrict__ H,
+                                                        double *__restrict__ cs, double2 *__restrict__ sn,
+                                                        double2 *__restrict__ g, SysState *__restrict__ st,
+                                                        unsigned *__restrict__ active) {
+  __shared__ double red[NXT_T / 32];
+  __shared__ double2 col[NXT_J + 1], rs[NXT_J];
+  __shared__ double rc[NXT_J];
+  const int64_t r = blockIdx.y;
+  double s = 0;
+  for (int p = threadIdx.x; p < nparts; p += NXT_T) s += np[r * nparts + p];
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  double2 *Hc = H + r * (int64_t)(kcap + 1) * kcap + (int64_t)j * (kcap + 1);
+  const bool first = blockIdx.x == 0, staged = j <= NXT_J;
+  if (first && staged) {
+    for (int i = threadIdx.x; i <= j; i += NXT_T) {
+      col[i] = Hc[i];
+      if (i < j) {
+        rc[i] = cs[r * (int64_t)kcap + i];
+        rs[i] = sn[r * (int64_t)kcap + i];
+      }
+    }
+  }
+  __syncthreads();
+  s = red[0];
+  for (int q = 1; q < NXT_T / 32; q++) s += red[q];
+  const double nrm = sqrt(s);
+  const int64_t n = (int64_t)blockIdx.x * NXT_T + threadIdx.x;
+  if (n < N) Vn[r * N + n] = nrm > 0 ? cscale(w[r * N + n], 1.0 / nrm) : make_double2(0, 0);
+  if (!first) return;
+  if (threadIdx.x == 0) {
+    SysState ss = st[r];
+    if (ss.done < 2) {
+      double *c = cs + r * (int64_t)kcap;
+      double2 *sv = sn + r * (int64_t)kcap, *gr = g + r * (int64_t)(kcap + 1);
+      if (staged) givens_column(j, nrm, col, rc, rs, Hc, c, sv, gr, ss);
+      else givens_column(j, nrm, Hc, c, sv, Hc, c, sv, gr, ss);
+      st[r] = ss;
+      if (!ss.done) atomicAdd(active, 1u);
+    }
+  }
+  __syncthreads();
+  if (staged)
+    for (int i = threadIdx.x; i < j; i += NXT_T) Hc[i] = col[i];
+}
+
+// y = R^-1 g, stored in y[r][i]: a CTA per system, column by column (the
+// next column is on its way while the current one is subtracted)
+__global__ void __launch_bounds__(128) k_backsolve(int kcap, const double2 *__restrict__ H,
+                                                   const double2 *__restrict__ g, const SysState *__restrict__ st,
+                                                   double2 *__restrict__ y) {
+  const int64_t r = blockIdx.x;
+  const int k = st[r].k, t = threadIdx.x;
   const double2 *Hr = H + r * (int64_t)(kcap + 1) * kcap;
   const double2 *gr = g + r * (int64_t)(kcap + 1);
   double2 *yr = y + r * (int64_t)kcap;
+  for (int i = t; i < kcap; i += 128) yr[i] = i < k ? gr[i] : make_double2(0, 0);
+  __syncthreads();
   for (int i = k - 1; i >= 0; i--) {
-    double2 v = gr[i];
-    for (int l = i + 1; l < k; l++) v = csub(v, cmul(Hr[(int64_t)l * (kcap + 1) + i], yr[l]));
-    double2 d = Hr[(int64_t)i * (kcap + 1) + i];
-    yr[i] = (d.x == 0 && d.y == 0) ? make_double2(0, 0) : cdiv(v, d);
+    const double2 *Hi = Hr + (int64_t)i * (kcap + 1);
+    const double2 d = Hi[i], hv = t < i ? Hi[t] : make_double2(0, 0);
+    const double2 v = yr[i];
+    const double2 yi = (d.x == 0 && d.y == 0) ? make_double2(0, 0) : cdiv(v, d);
+    __syncthreads();
+    if (t == 0) yr[i] = yi;
+    if (t < i) yr[t] = csub(yr[t], cmul(hv, yi));
+    for (int l = t + 128; l < i; l += 128) yr[l] = csub(yr[l], cmul(Hi[l], yi));
+    __syncthreads();
   }
-  for (int i = k; i < kcap; i++) yr[i] = make_double2(0, 0);
 }
 
 // x(r) += sum_i y[r][i] V_i(r)
@@ -294,9 +376,13 @@ void gmres_dev(dmb_ctx *c, const double *b_dev, double *x_dev, int64_t R, double
   if (prod_resid) c->d_Wraw.ensure(vec_bytes * kcap);
   double2 *Wraw = prod_resid ? c->d_Wraw.as<double2>() : nullptr;
   c->d_work.ensure(vec_bytes * 2);
-  // layout: H[R][(k+1)k] g[R][k+1] sn[R][k] hb[R][k+1] y[R][k] | cs[R][k] nrm[2R] | st[R] | active
-  size_t small = sizeof(double2) * R * ((size_t)(kcap + 1) * kcap + 2 * (kcap + 1) + 2 * kcap) +
-                 sizeof(double) * R * (kcap + 3) + sizeof(SysState) * R + 64;
+  // layout: H[R][(k+1)k] g[R][k+1] sn[R][k] hb[R][k+1][parts] y[R][k] | cs[R][k] nrm[3R] norm parts[R][..] |
+  // st[R] | active
+  constexpr int DOT_PARTS = 8;
+  const int64_t hb_len = std::max<int64_t>(R * (kcap + 1), std::min<int64_t>(R * (kcap + 1) * DOT_PARTS,
+                                                                            4 * (int64_t)c->sm_count));
+  size_t small = sizeof(double2) * (R * ((size_t)(kcap + 1) * kcap + (kcap + 1) + 2 * kcap) + hb_len) +
+                 sizeof(double) * R * (kcap + 3 + blocks_for(N, UPD_T)) + sizeof(SysState) * R + 64;
   c->d_H.ensure(small);
   double2 *V = c->d_V.as<double2>();
   double2 *w = c->d_work.as<double2>();
@@ -305,11 +391,12 @@ void gmres_dev(dmb_ctx *c, const double *b_dev, double *x_dev, int64_t R, double
   double2 *g = H + R * (int64_t)(kcap + 1) * kcap;
   double2 *sn = g + R * (int64_t)(kcap + 1);
   double2 *hb = sn + R * (int64_t)kcap;
-  double2 *ybuf = hb + R * (int64_t)(kcap + 1);
+  double2 *ybuf = hb + hb_len;
   double *cs = (double *)(ybuf + R * (int64_t)kcap);
   double *nrm = cs + R * (int64_t)kcap;   // [0,R) Krylov norms, [R,2R) ||b||, [2R,3R) ||b - Z x||
   double *tnrm = nrm + 2 * R;
-  SysState *st = (SysState *)(nrm + 3 * R);
+  double *npart = nrm + 3 * R;            // partial sums of |w|^2
+  SysState *st = (SysState *)(npart + R * blocks_for(N, UPD_T));
   unsigned *active = (unsigned *)(st + R);
   const double2 *b = (const double2 *)b_dev;
   double2 *x = (double2 *)x_dev;
@@ -397,15 +484,16 @@ void gmres_dev(dmb_ctx *c, const double *b_dev, double *x_dev, int64_t R, double
       apply_operator(c, precond_kind, side, Vj, w, flex ? Zv + (int64_t)jj * vstride : tmp, R, prod_resid);
       if (prod_resid)
         DMB_CUDA(cudaMemcpyAsync(Wraw + (int64_t)jj * vstride, w, vec_bytes, cudaMemcpyDeviceToDevice, c->stream));
+      // parts per dot product: enough CTAs for the GPU when there are few
+      const int S = (int)std::max<int64_t>(1, std::min<int64_t>(DOT_PARTS, 4 * c->sm_count / ((jj + 1) * R)));
+      const unsigned ub = blocks_for(N, UPD_T);
       for (int pass = 0; pass < 2; pass++) {
-        DMB_LAUNCH(c, k_dots, dim3(jj + 1, (unsigned)R), 256, 0, N, R, jj, vstride, V, w, hb, kcap + 1);
-        DMB_LAUNCH(c, k_cgs_update, blocks_for(N * R, 256), 256, 0, N, R, jj, vstride, V, hb, kcap + 1, w);
-        DMB_LAUNCH(c, k_hacc, blocks_for(R, 128), 128, 0, R, jj, hb, kcap + 1, H, kcap);
+        DMB_LAUNCH(c, k_dots, dim3(jj + 1, (unsigned)R, (unsigned)S), 256, 0, N, vstride, V, w, hb, active);
+        DMB_LAUNCH(c, k_cgs_update, dim3(ub, (unsigned)R), UPD_T, 0, N, jj + 1, S, vstride, V, hb, w, H, kcap,
+                   pass == 1 ? npart : nullptr);
       }
-      DMB_LAUNCH(c, k_norms, (unsigned)R, 256, 0, N, w, nrm);
-      DMB_LAUNCH(c, k_scale_cols, blocks_for(N * R, 256), 256, 0, N, R, nrm, w, V + (int64_t)(jj + 1) * vstride);
-      DMB_CUDA(cudaMemsetAsync(active, 0, 4, c->stream));
-      DMB_LAUNCH(c, k_givens, blocks_for(R, 128), 128, 0, R, jj, kcap, H, nrm, cs, sn, g, st, active);
+      DMB_LAUNCH(c, k_arnoldi_next, dim3(blocks_for(N, NXT_T), (unsigned)R), NXT_T, 0, N, jj, kcap, (int)ub, npart, w,
+                 V + (int64_t)(jj + 1) * vstride, H, cs, sn, g, st, active);
     };
     // iterations j0 .. j0 + nb - 1, directly or as a captured graph
     auto run_block = [&](int j0, int nb) {
@@ -477,7 +565,7 @@ void gmres_dev(dmb_ctx *c, const double *b_dev, double *x_dev, int64_t R, double
       // same Arnoldi process (its Krylov space kept) with its threshold
       // lowered by the factor the true residual still needs, margin 2.
       while (h_active == 0 && left_recheck) {
-        DMB_LAUNCH(c, k_backsolve, blocks_for(R, 128), 128, 0, R, kcap, H, g, st, ybuf);
+        DMB_LAUNCH(c, k_backsolve, (unsigned)R, 128, 0, kcap, H, g, st, ybuf);
         DMB_CUDA(cudaMemcpyAsync(tmp, x, vec_bytes, cudaMemcpyDeviceToDevice, c->stream));
         DMB_LAUNCH(c, k_combine, blocks_for(N * R, 256), 256, 0, N, R, j, vstride, V, ybuf, kcap, tmp);
         matvec_dev(c, tmp, w, R);
@@ -515,7 +603,7 @@ void gmres_dev(dmb_ctx *c, const double *b_dev, double *x_dev, int64_t R, double
     }
     // solution update from this cycle
     j_last = j;
-    DMB_LAUNCH(c, k_backsolve, blocks_for(R, 128), 128, 0, R, kcap, H, g, st, ybuf);
+    DMB_LAUNCH(c, k_backsolve, (unsigned)R, 128, 0, kcap, H, g, st, ybuf);
     if (flex) {
       DMB_LAUNCH(c, k_combine, blocks_for(N * R, 256), 256, 0, N, R, j, vstride, Zv, ybuf, kcap, x);
     } else {

@@ -18,26 +18,55 @@ namespace {
 // ---------------------------------------------------------------------------
 // matvec
 // ---------------------------------------------------------------------------
-// y = Z x for one right-hand side: one warp per row, 16-byte loads.
-template <class ZC>
-__global__ void k_gemv(int64_t N, const ZC *__restrict__ Z, const double2 *__restrict__ x,
+// y = Z x for one right-hand side: RW rows per warp, RW U matrix loads per
+// lane in flight.  HBM-bound.  Two rows per warp (x loaded once for both, half
+// as many rows streamed at a time) from 640 MB on, one below, where two leave
+// SMs without warps: complex64 9,720 unknowns 128 us against 184 with one row
+// (171 before), 4,693 49 against 45; complex128 7,680 139 against 158 (224
+// before), 4,720 64 against 60 (78 before).
+__device__ __forceinline__ void gemv_fma(double2 z, double2 v, double &re, double &im) {
+  re = fma(z.x, v.x, re);
+  re = fma(-z.y, v.y, re);
+  im = fma(z.x, v.y, im);
+  im = fma(z.y, v.x, im);
+}
+template <class ZC, int RW, int U>
+__global__ void __launch_bounds__(256) k_gemv(int64_t N, const ZC *__restrict__ Z, const double2 *__restrict__ x,
                        double2 *__restrict__ y) {
-  int64_t row = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  int lane = threadIdx.x & 31;
+  // rows RW warp .. of this warp; x is loaded once for its rows
+  const int64_t row = ((int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * RW;
+  const int lane = threadIdx.x & 31;
   if (row >= N) return;
-  const ZC *zr = Z + row * N;
-  double re = 0, im = 0;
-  for (int64_t n = lane; n < N; n += 32) {
-    double2 z = to_d2(zr[n]);
-    double2 v = x[n];
-    re = fma(z.x, v.x, re);
-    re = fma(-z.y, v.y, re);
-    im = fma(z.x, v.y, im);
-    im = fma(z.y, v.x, im);
+  const ZC *zr[RW];
+  double re[RW], im[RW];
+#pragma unroll
+  for (int q = 0; q < RW; q++) {
+    zr[q] = Z + min(row + q, N - 1) * N;
+    re[q] = im[q] = 0;
   }
-  re = warp_sum(re);
-  im = warp_sum(im);
-  if (lane == 0) y[row] = make_double2(re, im);
+  int64_t n = lane;
+  for (; n + 32 * (U - 1) < N; n += 32 * U) {
+    ZC z[U][RW];
+    double2 v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+#pragma unroll
+      for (int q = 0; q < RW; q++) z[u][q] = zr[q][n + 32 * u];
+      v[u] = x[n + 32 * u];
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int q = 0; q < RW; q++) gemv_fma(to_d2(z[u][q]), v[u], re[q], im[q]);
+  }
+  for (; n < N; n += 32)
+#pragma unroll
+    for (int q = 0; q < RW; q++) gemv_fma(to_d2(zr[q][n]), x[n], re[q], im[q]);
+#pragma unroll
+  for (int q = 0; q < RW; q++) {
+    const double a = warp_sum(re[q]), b = warp_sum(im[q]);
+    if (lane == 0 && row + q < N) y[row + q] = make_double2(a, b);
+  }
 }
 
 // Y = Z X for R right-hand sides (X, Y column-major N x R), SIMT tiles with
@@ -392,11 +421,13 @@ void matvec_dev(dmb_ctx *c, const void *x, void *y, int64_t nrhs) {
     return;
   }
   if (nrhs == 1) {
-    unsigned g = blocks_for(N, 8);
+    const bool two = N * N * (c->z_prec == DMB_PREC_FP64 ? 16 : 8) >= (int64_t)640 << 20;
+    const unsigned g = blocks_for(N, two ? 16 : 8);
+    auto gemv = [&](auto kernel, auto *Z) { DMB_LAUNCH(c, kernel, g, 256, 0, N, Z, xd, yd); };
     if (c->z_prec == DMB_PREC_FP64)
-      DMB_LAUNCH(c, k_gemv<double2>, g, 256, 0, N, c->d_Z.as<double2>(), xd, yd);
+      two ? gemv(k_gemv<double2, 2, 4>, c->d_Z.as<double2>()) : gemv(k_gemv<double2, 1, 16>, c->d_Z.as<double2>());
     else
-      DMB_LAUNCH(c, k_gemv<float2>, g, 256, 0, N, c->d_Z.as<float2>(), xd, yd);
+      two ? gemv(k_gemv<float2, 2, 4>, c->d_Z.as<float2>()) : gemv(k_gemv<float2, 1, 16>, c->d_Z.as<float2>());
   } else if (c->z_prec == DMB_PREC_FP64 && nrhs >= 16) {
     zgemm64_zx(c, c->d_Z.as<double2>(), xd, yd, N, nrhs);
   } else if (nrhs < 32 || c->z_prec == DMB_PREC_FP64) {
