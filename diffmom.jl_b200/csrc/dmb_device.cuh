@@ -98,3 +98,39 @@ __device__ __forceinline__ double warp_max(double v) {
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
+
+// sin(kR), cos(kR) from those of k Rc and the Taylor series of the short
+// remainder d = k (R - Rc); a remainder above 0.75 (coarse meshes) takes the
+// direct evaluation.  Series terms through d^16 / d^17: the first omitted
+// term is below 1e-18 at |d| = 0.75.
+__device__ __forceinline__ void phase_exp(double k, double R, double Rc, double s0, double c0, double &sn,
+                                          double &cs) {
+  const double d = k * (R - Rc);
+  if (fabs(d) > 0.75) {
+    sincos(k * R, &sn, &cs);
+    return;
+  }
+  const double u = d * d;
+  double cd = 1.0 / 20922789888000.0;  // 1/16!
+  cd = fma(cd, u, -1.0 / 87178291200.0);
+  cd = fma(cd, u, 1.0 / 479001600.0);
+  cd = fma(cd, u, -1.0 / 3628800.0);
+  cd = fma(cd, u, 1.0 / 40320.0);
+  cd = fma(cd, u, -1.0 / 720.0);
+  cd = fma(cd, u, 1.0 / 24.0);
+  cd = fma(cd, u, -0.5);
+  cd = fma(cd, u, 1.0);
+  double sd = 1.0 / 355687428096000.0;  // 1/17!
+  sd = fma(sd, u, -1.0 / 1307674368000.0);
+  sd = fma(sd, u, 1.0 / 6227020800.0);
+  sd = fma(sd, u, -1.0 / 39916800.0);
+  sd = fma(sd, u, 1.0 / 362880.0);
+  sd = fma(sd, u, -1.0 / 5040.0);
+  sd = fma(sd, u, 1.0 / 120.0);
+  sd = fma(sd, u, -1.0 / 6.0);
+  sd = fma(sd, u, 1.0);
+  sd *= d;
+  // angle sum: (c0 + i s0)(cd + i sd)
+  cs = fma(c0, cd, -s0 * sd);
+  sn = fma(s0, cd, c0 * sd);
+}

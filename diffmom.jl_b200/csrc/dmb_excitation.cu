@@ -459,7 +459,9 @@ __device__ __forceinline__ bool tri_adjacent2(const int *__restrict__ off, const
   return false;
 }
 
-// Ys[3ta+i] = sum_{tb far from ta} sum_j block(ta,tb)[i][j] Xs[3tb+j]
+// Ys[3ta+i] = sum_{tb far from ta} sum_j block(ta,tb)[i][j] Xs[3tb+j]: the
+// product that needs no workspace beyond its slot vectors
+// (dmb_matvec_free_noalloc)
 __global__ void __launch_bounds__(256) k_mf_far(int nt, int nq, const TriCache *__restrict__ tc,
                                                 const int *__restrict__ aoff, const int *__restrict__ anb,
                                                 double k, double inv_k2, const double2 *__restrict__ Xs,
@@ -526,6 +528,149 @@ __global__ void __launch_bounds__(256) k_mf_far(int nt, int nq, const TriCache *
     for (int w = 0; w < 8; w++) s = cadd(s, red[w][threadIdx.x]);
     Ys[3 * ta + threadIdx.x] = s;
   }
+}
+
+// The same product with a workspace, as sums over quadrature points: y_i of a
+// test triangle is w [s_i (r - p_i) . A(r) - dv_i phi(r) / k^2] summed over its
+// points, A and phi the potentials of the source points' weighted currents and
+// charges (the contribution of a point pair is one Green value times four
+// complex numbers; the 3 x 3 blocks and their moments are never formed).  A
+// thread holds QT points of one test triangle; the source triangles of a chunk
+// pass through shared memory, read as broadcasts.  The phase of the centroid
+// distance is taken once per triangle pair (phase_exp).  Bound by the FP64 pipe.
+// Chunks give the parallelism; their partial sums are added in order.
+constexpr int MF_TB = 32;     // source triangles per shared tile
+constexpr int MF_F = 11;      // per source point: position, current (3 complex), charge (complex)
+
+// source points of every triangle: src[(q MF_F + f) nt + t]
+__global__ void k_mf_sources(int nt, int nq, const TriCache *__restrict__ tc, const double2 *__restrict__ x,
+                             double *__restrict__ src) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nt) return;
+  const TriCache &T = tc[t];
+  double2 xs[3], rho = make_double2(0, 0);
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const double2 v = T.rwg[i] >= 0 ? x[T.rwg[i]] : make_double2(0, 0);
+    xs[i] = T.rwg[i] >= 0 ? cscale(v, T.s[i]) : v;
+    if (T.rwg[i] >= 0) rho = cadd(rho, cscale(v, T.dv[i]));
+  }
+  for (int q = 0; q < nq; q++) {
+    double *o = src + (int64_t)q * MF_F * nt + t;
+    const double w = T.w2a[q];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      double2 j = make_double2(0, 0);
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+        if (T.rwg[i] >= 0) j = cadd(j, cscale(xs[i], T.qp[q][c] - T.p[i][c]));
+      o[(int64_t)c * nt] = T.qp[q][c];
+      o[(int64_t)(3 + 2 * c) * nt] = w * j.x;
+      o[(int64_t)(4 + 2 * c) * nt] = w * j.y;
+    }
+    o[(int64_t)9 * nt] = w * rho.x;
+    o[(int64_t)10 * nt] = w * rho.y;
+  }
+}
+
+template <int NQ, int QT>
+__global__ void __launch_bounds__(128) k_mf_points(int nt, int chunk, const TriCache *__restrict__ tc,
+                                                   const int *__restrict__ aoff, const int *__restrict__ anb, double k,
+                                                   double inv_k2, const double *__restrict__ src,
+                                                   double2 *__restrict__ part) {
+  __shared__ double S[NQ * MF_F][MF_TB];
+  __shared__ double cen[3][MF_TB];
+  const int ta = blockIdx.x * 128 + threadIdx.x, q0 = blockIdx.z * QT;
+  const bool live = ta < nt;
+  const TriCache &A = tc[live ? ta : nt - 1];
+  double r[QT][3];
+  double2 acc[QT][4];
+#pragma unroll
+  for (int q = 0; q < QT; q++) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) r[q][c] = A.qp[min(q0 + q, NQ - 1)][c];
+#pragma unroll
+    for (int c = 0; c < 4; c++) acc[q][c] = make_double2(0, 0);
+  }
+  const double ca0 = A.cen[0], ca1 = A.cen[1], ca2 = A.cen[2];
+  // edge neighbours: three at once, further ones (edges shared by more than
+  // two triangles) from the list
+  const int a0 = aoff[live ? ta : nt - 1], a1 = aoff[(live ? ta : nt - 1) + 1];
+  const int n0 = a1 > a0 ? anb[a0] : -1, n1 = a1 > a0 + 1 ? anb[a0 + 1] : -1, n2 = a1 > a0 + 2 ? anb[a0 + 2] : -1;
+  const int b1 = min(nt, (int)(blockIdx.y + 1) * chunk);
+  for (int t0 = blockIdx.y * chunk; t0 < b1; t0 += MF_TB) {
+    const int nb = min(MF_TB, b1 - t0);
+    __syncthreads();
+    for (int e = threadIdx.x; e < NQ * MF_F * MF_TB; e += 128) {
+      const int f = e / MF_TB, b = e % MF_TB;
+      S[f][b] = b < nb ? src[(int64_t)f * nt + t0 + b] : 0.0;
+    }
+    if (threadIdx.x < 3 * MF_TB) {
+      const int c = threadIdx.x / MF_TB, b = threadIdx.x % MF_TB;
+      cen[c][b] = b < nb ? tc[t0 + b].cen[c] : 0.0;
+    }
+    __syncthreads();
+    for (int b = 0; b < nb; b++) {
+      const int tb = t0 + b;
+      bool near = tb == ta || tb == n0 || tb == n1 || tb == n2;
+      for (int e = a0 + 3; e < a1; e++) near |= anb[e] == tb;
+      if (near) continue;
+      const double cx = ca0 - cen[0][b], cy = ca1 - cen[1][b], cz = ca2 - cen[2][b];
+      const double Rc = sqrt(cx * cx + cy * cy + cz * cz);
+      double s0, c0;
+      sincos(k * Rc, &s0, &c0);
+#pragma unroll
+      for (int p = 0; p < NQ; p++) {
+        const double *v = &S[p * MF_F][b];
+        const double x = v[0], y = v[MF_TB], z = v[2 * MF_TB];
+#pragma unroll
+        for (int q = 0; q < QT; q++) {
+          const double dx = r[q][0] - x, dy = r[q][1] - y, dz = r[q][2] - z;
+          const double R2 = dx * dx + dy * dy + dz * dz, rinv = rsqrt(R2);
+          double sn, cs;
+          phase_exp(k, R2 * rinv, Rc, s0, c0, sn, cs);
+          const double2 g = make_double2(rinv * cs, -rinv * sn);
+#pragma unroll
+          for (int c = 0; c < 4; c++)
+            cfma(acc[q][c], g, make_double2(v[(3 + 2 * c) * MF_TB], v[(4 + 2 * c) * MF_TB]));
+        }
+      }
+    }
+  }
+  if (!live) return;
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    double2 y = make_double2(0, 0);
+#pragma unroll
+    for (int q = 0; q < QT; q++) {
+      if (q0 + q >= NQ) continue;
+      const double w = A.w2a[q0 + q] * DMB_INV_FOUR_PI;
+#pragma unroll
+      for (int c = 0; c < 3; c++) y = cadd(y, cscale(acc[q][c], w * A.s[i] * (r[q][c] - A.p[i][c])));
+      y = csub(y, cscale(acc[q][3], w * A.dv[i] * inv_k2));
+    }
+    part[((int64_t)(blockIdx.z * gridDim.y + blockIdx.y) * nt + ta) * 3 + i] = y;
+  }
+}
+
+// y[m] = -i w (its two slots' partial sums in order + its near entries in order)
+__global__ void k_mf_collect(int64_t N, int nt, int nparts, const int *__restrict__ rslot,
+                             const double2 *__restrict__ part, const int64_t *__restrict__ roff,
+                             const int *__restrict__ rent, const int *__restrict__ rcol,
+                             const double2 *__restrict__ esum, const double2 *__restrict__ x, double w,
+                             double2 *__restrict__ y) {
+  const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= N) return;
+  const int64_t sp = rslot[2 * m], sm = rslot[2 * m + 1];
+  double2 a = make_double2(0, 0), b = a, near = a;
+#pragma unroll 4
+  for (int p = 0; p < nparts; p++) {
+    a = cadd(a, part[(int64_t)p * 3 * nt + sp]);
+    b = cadd(b, part[(int64_t)p * 3 * nt + sm]);
+  }
+  for (int64_t q = roff[m]; q < roff[m + 1]; q++) near = cadd(near, cmul(esum[rent[q]], x[rcol[q]]));
+  const double2 v = cadd(cadd(a, b), near);
+  y[m] = make_double2(w * v.y, -w * v.x);
 }
 
 __global__ void k_mf_gather(int64_t N, const int *__restrict__ rslot, const double2 *__restrict__ Ys,
@@ -698,26 +843,32 @@ void prepare_operator(dmb_ctx *c, double k, double eta0, int quad_order) {
 
 void matvec_free_dev(dmb_ctx *c, const double *x, double *y) {
   DMB_REQUIRE(c->cache_valid && c->k != 0.0, DMB_ERR_STATE, "operator not prepared");
-  const int64_t N = c->n, nt = c->nt;
-  DevBuf xs, ys;
-  xs.ensure(sizeof(double2) * 3 * nt);
-  ys.ensure(sizeof(double2) * 3 * nt);
-  DMB_CUDA(cudaMemsetAsync(xs.p, 0, sizeof(double2) * 3 * nt, c->stream));
-  DMB_LAUNCH(c, k_scatter_slots, blocks_for(N, 256), 256, 0, N, c->d_rwg_slot.as<int>(), (const double2 *)x,
-             xs.as<double2>());
-  DMB_LAUNCH(c, k_mf_far, (unsigned)nt, 256, 0, (int)nt, c->nq, c->d_tcache.as<TriCache>(),
-             c->d_adj_off.as<int>(), c->d_adj_nb.as<int>(), c->k, 1.0 / (c->k * c->k), xs.as<double2>(),
-             ys.as<double2>());
-  DMB_LAUNCH(c, k_mf_gather, blocks_for(N, 256), 256, 0, N, c->d_rwg_slot.as<int>(), ys.as<double2>(),
-             (double2 *)y);
-  if (c->n_near_entry > 0) {
+  const int64_t N = c->n;
+  const int nt = (int)c->nt, nq = c->nq, qt = std::min(nq, 4), nz = (nq + qt - 1) / qt;
+  // source chunks (multiples of the shared tile) for about four CTAs per SM
+  const int gx = (nt + 127) / 128, want = std::max(1, (4 * c->sm_count + gx * nz - 1) / (gx * nz));
+  const int chunk = std::max(MF_TB, (nt + want - 1) / want / MF_TB * MF_TB), nchunk = (nt + chunk - 1) / chunk;
+  const size_t src_bytes = sizeof(double) * MF_F * nq * nt;
+  c->d_mf.ensure(src_bytes + sizeof(double2) * 3 * nt * nchunk * nz + 16);
+  double *src = c->d_mf.as<double>();
+  double2 *part = (double2 *)(c->d_mf.as<char>() + (src_bytes + 15) / 16 * 16);
+  const double2 *xd = (const double2 *)x;
+  DMB_LAUNCH(c, k_mf_sources, blocks_for(nt, 128), 128, 0, nt, nq, c->d_tcache.as<TriCache>(), xd, src);
+  const dim3 g((unsigned)gx, (unsigned)nchunk, (unsigned)nz);
+  auto far = [&](auto kernel) {
+    DMB_LAUNCH(c, kernel, g, 128, 0, nt, chunk, c->d_tcache.as<TriCache>(), c->d_adj_off.as<int>(),
+               c->d_adj_nb.as<int>(), c->k, 1.0 / (c->k * c->k), src, part);
+  };
+  if (nq == 1) far(k_mf_points<1, 1>);
+  else if (nq == 3) far(k_mf_points<3, 3>);
+  else if (nq == 4) far(k_mf_points<4, 4>);
+  else far(k_mf_points<7, 4>);
+  if (c->n_near_entry > 0)
     DMB_LAUNCH(c, k_near_entry_sum, blocks_for(c->n_near_entry, 256), 256, 0, c->n_near_entry,
                c->d_near_entry_off.as<int64_t>(), c->d_near_val.as<double2>(), c->d_near_entry_sum.as<double2>());
-    DMB_LAUNCH(c, k_mf_near_rows, blocks_for(N, 256), 256, 0, N, c->d_near_row_off.as<int64_t>(),
-               c->d_near_row_ent.as<int>(), c->d_near_row_col.as<int>(), c->d_near_entry_sum.as<double2>(),
-               (const double2 *)x, (double2 *)y);
-  }
-  DMB_LAUNCH(c, k_times_minus_i_w, blocks_for(N, 256), 256, 0, N, c->k * c->eta0, (double2 *)y);
+  DMB_LAUNCH(c, k_mf_collect, blocks_for(N, 128), 128, 0, N, nt, nchunk * nz, c->d_rwg_slot.as<int>(), part,
+             c->d_near_row_off.as<int64_t>(), c->d_near_row_ent.as<int>(), c->d_near_row_col.as<int>(),
+             c->d_near_entry_sum.as<double2>(), xd, c->k * c->eta0, (double2 *)y);
   DMB_CUDA(cudaStreamSynchronize(c->stream));
 }
 

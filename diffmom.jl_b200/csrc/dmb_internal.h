@@ -258,6 +258,7 @@ struct dmb_ctx {
   // resident solution of dmb_solve_resident / dmb_solve_resident_many
   DevBuf d_rhs, d_sol, d_mono;
   DevBuf d_far;       // far-field workspace
+  DevBuf d_mf;        // matrix-free product workspace
   int64_t sol_r = 0;
   // small persistent scratch (counters, plane-wave parameters): the solve path
   // allocates nothing after its first call
