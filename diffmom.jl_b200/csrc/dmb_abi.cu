@@ -95,6 +95,9 @@ dmb_status dmb_ctx_destroy(dmb_ctx *c) {
     c->d_sol.release();
     c->d_mono.release();
     c->d_far.release();
+    for (DevBuf &b : c->d_io) b.release();
+    for (DevBuf &b : c->d_tmp) b.release();
+    dmb::hostcopy_release(c);
     c->d_mf.release();
     c->d_trsm_id.release();
     c->d_Wraw.release();
@@ -364,7 +367,7 @@ dmb_status dmb_matvec(dmb_ctx *c, const double *x, double *y, int64_t nrhs) {
     DMB_REQUIRE(dmb::operator_ready(c), DMB_ERR_STATE, "no assembled impedance matrix");
     DMB_REQUIRE(x && y && nrhs >= 1, DMB_ERR_ARGUMENT, "bad matvec arguments");
     size_t bytes = sizeof(double2) * c->n * nrhs;
-    DevBuf bx, by;
+    DevBuf &bx = c->d_io[0], &by = c->d_io[1];
     bx.ensure(bytes);
     by.ensure(bytes);
     DMB_CUDA(cudaMemcpyAsync(bx.p, x, bytes, cudaMemcpyHostToDevice, c->stream));
@@ -376,8 +379,7 @@ dmb_status dmb_matvec(dmb_ctx *c, const double *x, double *y, int64_t nrhs) {
     } else {
       dmb::matvec_dev(c, bx.as<double2>(), by.as<double2>(), nrhs);
     }
-    DMB_CUDA(cudaMemcpyAsync(y, by.p, bytes, cudaMemcpyDeviceToHost, c->stream));
-    DMB_CUDA(cudaStreamSynchronize(c->stream));
+    dmb::copy_out(c, y, by.p, (int64_t)(bytes / sizeof(double2)));
   });
 }
 
@@ -389,13 +391,12 @@ dmb_status dmb_matvec_free(dmb_ctx *c, const double *x, double *y) {
   return guarded(c, [&] {
     DMB_REQUIRE(x && y, DMB_ERR_ARGUMENT, "bad matvec arguments");
     size_t bytes = sizeof(double2) * c->n;
-    DevBuf bx, by;
+    DevBuf &bx = c->d_io[0], &by = c->d_io[1];
     bx.ensure(bytes);
     by.ensure(bytes);
     DMB_CUDA(cudaMemcpyAsync(bx.p, x, bytes, cudaMemcpyHostToDevice, c->stream));
     dmb::matvec_free_dev(c, bx.as<double>(), by.as<double>());
-    DMB_CUDA(cudaMemcpyAsync(y, by.p, bytes, cudaMemcpyDeviceToHost, c->stream));
-    DMB_CUDA(cudaStreamSynchronize(c->stream));
+    dmb::copy_out(c, y, by.p, (int64_t)(bytes / sizeof(double2)));
   });
 }
 
@@ -418,12 +419,11 @@ dmb_status dmb_nf_apply(dmb_ctx *c, const double *x, double *y, int64_t nrhs) {
     DMB_REQUIRE(c->pc_valid, DMB_ERR_STATE, "no near-field preconditioner built");
     DMB_REQUIRE(x && y && nrhs >= 1, DMB_ERR_ARGUMENT, "bad apply arguments");
     size_t bytes = sizeof(double2) * c->n * nrhs;
-    DevBuf bx;
+    DevBuf &bx = c->d_io[0];
     bx.ensure(bytes);
     DMB_CUDA(cudaMemcpyAsync(bx.p, x, bytes, cudaMemcpyHostToDevice, c->stream));
     dmb::pc_apply_dev(c, bx.as<double>(), nrhs);
-    DMB_CUDA(cudaMemcpyAsync(y, bx.p, bytes, cudaMemcpyDeviceToHost, c->stream));
-    DMB_CUDA(cudaStreamSynchronize(c->stream));
+    dmb::copy_out(c, y, bx.p, (int64_t)(bytes / sizeof(double2)));
     DMB_REQUIRE((dmb::read_err_word(c) & 4u) == 0, DMB_ERR_TIMEOUT, "triangular solve wait expired");
   });
 }
@@ -495,11 +495,10 @@ dmb_status dmb_rhs_dipoles(dmb_ctx *c, int64_t R, const double *positions, const
                   "dipole frequency must be finite and positive");
     }
     const size_t bytes = sizeof(double2) * c->n * R;
-    DevBuf bv;
+    DevBuf &bv = c->d_io[0];
     bv.ensure(bytes);
     dmb::rhs_dipoles_dev(c, R, positions, moments, magnetic, frequencies, quad_order, bv.as<double>());
-    DMB_CUDA(cudaMemcpyAsync(V_out, bv.p, bytes, cudaMemcpyDeviceToHost, c->stream));
-    DMB_CUDA(cudaStreamSynchronize(c->stream));
+    dmb::copy_out(c, V_out, bv.p, (int64_t)(bytes / sizeof(double2)));
   });
 }
 
@@ -528,12 +527,11 @@ dmb_status dmb_rhs_pattern_feed(dmb_ctx *c, int ntheta, const double *theta, int
     DMB_REQUIRE(std::isfinite(frequency) && frequency > 0, DMB_ERR_ARGUMENT,
                 "Pattern feed frequency must be finite and positive.");
     const size_t bytes = sizeof(double2) * c->n;
-    DevBuf bv;
+    DevBuf &bv = c->d_io[0];
     bv.ensure(bytes);
     dmb::rhs_pattern_dev(c, ntheta, theta, nphi, phi, Ftheta, Fphi, frequency, phase_center,
                          conj_convention ? 1 : 0, quad_order, bv.as<double>());
-    DMB_CUDA(cudaMemcpyAsync(V_out, bv.p, bytes, cudaMemcpyDeviceToHost, c->stream));
-    DMB_CUDA(cudaStreamSynchronize(c->stream));
+    dmb::copy_out(c, V_out, bv.p, (int64_t)(bytes / sizeof(double2)));
   });
 }
 
@@ -551,7 +549,7 @@ dmb_status dmb_gradient_impedance(dmb_ctx *c, int64_t R, const double *I, const 
     check_finite(lambda, 2 * c->n * R, "lambda must contain only finite values");
     if (P == 0) return;
     const size_t vb = sizeof(double2) * c->n * R;
-    DevBuf bi, bl, bg;
+    DevBuf &bi = c->d_io[0], &bl = c->d_io[1], &bg = c->d_io[2];
     bi.ensure(vb);
     bl.ensure(vb);
     bg.ensure(sizeof(double) * P * R);
@@ -582,11 +580,10 @@ dmb_status dmb_rhs_plane_waves(dmb_ctx *c, const double *kvecs, const double *E0
       DMB_REQUIRE(dt <= 1e-10, DMB_ERR_ARGUMENT, "plane-wave polarization must be transverse to k_vec");
     }
     size_t bytes = sizeof(double2) * c->n * R;
-    DevBuf bv;
+    DevBuf &bv = c->d_io[0];
     bv.ensure(bytes);
     dmb::rhs_plane_waves_dev(c, kvecs, E0s, pols, R, quad_order, bv.as<double>());
-    DMB_CUDA(cudaMemcpyAsync(V_out, bv.p, bytes, cudaMemcpyDeviceToHost, c->stream));
-    DMB_CUDA(cudaStreamSynchronize(c->stream));
+    dmb::copy_out(c, V_out, bv.p, (int64_t)(bytes / sizeof(double2)));
   });
 }
 
@@ -603,14 +600,13 @@ dmb_status dmb_gmres(dmb_ctx *c, const double *rhs, double *x, int64_t nrhs, dou
     DMB_REQUIRE(dmb::operator_ready(c), DMB_ERR_STATE, "no assembled impedance matrix");
     check_finite(rhs, 2 * c->n * nrhs, "right-hand side");
     size_t bytes = sizeof(double2) * c->n * nrhs;
-    DevBuf bb, bx;
+    DevBuf &bb = c->d_io[0], &bx = c->d_io[1];
     bb.ensure(bytes);
     bx.ensure(bytes);
     DMB_CUDA(cudaMemcpyAsync(bb.p, rhs, bytes, cudaMemcpyHostToDevice, c->stream));
     dmb::gmres_dev(c, bb.as<double>(), bx.as<double>(), nrhs, tol, maxiter, precond_kind,
                    precond_side, &st);
-    DMB_CUDA(cudaMemcpyAsync(x, bx.p, bytes, cudaMemcpyDeviceToHost, c->stream));
-    DMB_CUDA(cudaStreamSynchronize(c->stream));
+    dmb::copy_out(c, x, bx.p, (int64_t)(bytes / sizeof(double2)));
     if (check_convergence && !st.solved)
       throw DmbError{DMB_ERR_NOT_CONVERGED,
                      "forward GMRES did not converge consistently: niter=" + std::to_string(st.niter) +
@@ -637,7 +633,7 @@ dmb_status dmb_gmres_adjoint(dmb_ctx *c, const double *rhs, double *x, int64_t n
     check_finite(rhs, 2 * c->n * nrhs, "right-hand side");
     const int64_t cnt = c->n * nrhs;
     size_t bytes = sizeof(double2) * cnt;
-    DevBuf bb, bx;
+    DevBuf &bb = c->d_io[0], &bx = c->d_io[1];
     bb.ensure(bytes);
     bx.ensure(bytes);
     DMB_CUDA(cudaMemcpyAsync(bb.p, rhs, bytes, cudaMemcpyHostToDevice, c->stream));
@@ -653,8 +649,7 @@ dmb_status dmb_gmres_adjoint(dmb_ctx *c, const double *rhs, double *x, int64_t n
     } tr(c);
     dmb::gmres_dev(c, bb.as<double>(), bx.as<double>(), nrhs, tol, maxiter, precond_kind, precond_side, &st);
     dmb::conj_dev(c, bx.as<double2>(), cnt);
-    DMB_CUDA(cudaMemcpyAsync(x, bx.p, bytes, cudaMemcpyDeviceToHost, c->stream));
-    DMB_CUDA(cudaStreamSynchronize(c->stream));
+    dmb::copy_out(c, x, bx.p, (int64_t)(bytes / sizeof(double2)));
     if (check_convergence && !st.solved)
       throw DmbError{DMB_ERR_NOT_CONVERGED,
                      "adjoint GMRES did not converge consistently: niter=" + std::to_string(st.niter) +
@@ -672,14 +667,13 @@ dmb_status dmb_solve_direct(dmb_ctx *c, const double *rhs, double *x, int64_t nr
     DMB_REQUIRE(c->z_valid && c->op_kind == 0, DMB_ERR_STATE, "no assembled impedance matrix");
     check_finite(rhs, 2 * c->n * nrhs, "right-hand side");
     size_t bytes = sizeof(double2) * c->n * nrhs;
-    DevBuf bb, bx;
+    DevBuf &bb = c->d_io[0], &bx = c->d_io[1];
     bb.ensure(bytes);
     bx.ensure(bytes);
     DMB_CUDA(cudaMemcpyAsync(bb.p, rhs, bytes, cudaMemcpyHostToDevice, c->stream));
     double berr = 0;
     dmb::solve_direct_dev(c, bb.as<double>(), bx.as<double>(), nrhs, &berr);
-    DMB_CUDA(cudaMemcpyAsync(x, bx.p, bytes, cudaMemcpyDeviceToHost, c->stream));
-    DMB_CUDA(cudaStreamSynchronize(c->stream));
+    dmb::copy_out(c, x, bx.p, (int64_t)(bytes / sizeof(double2)));
     if (backward_error_out) *backward_error_out = berr;
   });
 }
@@ -821,9 +815,7 @@ dmb_status dmb_solve_resident_many(dmb_ctx *c, const dmb_solve_params *p, int64_
 dmb_status dmb_copy_solution(dmb_ctx *c, double *I_out) {
   return guarded(c, [&] {
     DMB_REQUIRE(I_out && c->d_sol.p && c->sol_r > 0, DMB_ERR_STATE, "no resident solution");
-    DMB_CUDA(cudaMemcpyAsync(I_out, c->d_sol.p, sizeof(double2) * c->n * c->sol_r, cudaMemcpyDeviceToHost,
-                             c->stream));
-    DMB_CUDA(cudaStreamSynchronize(c->stream));
+    dmb::copy_out(c, I_out, c->d_sol.p, c->n * c->sol_r);
   });
 }
 
@@ -874,13 +866,12 @@ dmb_status dmb_farfield(dmb_ctx *c, const double *rhat, int64_t NO, double k, do
     check_finite(rhat, 3 * NO, "far-field directions");
     check_finite(I, 2 * c->n * nrhs, "current coefficients");
     size_t ib = sizeof(double2) * c->n * nrhs, eb = sizeof(double2) * 3 * NO * nrhs;
-    DevBuf bi, be;
+    DevBuf &bi = c->d_io[0], &be = c->d_io[1];
     bi.ensure(ib);
     be.ensure(eb);
     DMB_CUDA(cudaMemcpyAsync(bi.p, I, ib, cudaMemcpyHostToDevice, c->stream));
     dmb::farfield_dev(c, rhat, NO, k, eta0, quad_order, bi.as<double>(), nrhs, be.as<double>());
-    DMB_CUDA(cudaMemcpyAsync(E_out, be.p, eb, cudaMemcpyDeviceToHost, c->stream));
-    DMB_CUDA(cudaStreamSynchronize(c->stream));
+    dmb::copy_out(c, E_out, be.p, (int64_t)(eb / sizeof(double2)));
   });
 }
 

@@ -1065,7 +1065,7 @@ template <class T> void upload(dmb_ctx *c, DevBuf &b, const std::vector<T> &v) {
 // dense fill of the listed blocks
 void fill_dense(dmb_ctx *c, const std::vector<int> &ids) {
   if (ids.empty()) return;
-  DevBuf d_ids;
+  DevBuf &d_ids = c->aca.d_ids;
   upload(c, d_ids, ids);
   AcaGeo g = make_geo(c);
   AcaState &A = c->aca;
@@ -1140,7 +1140,7 @@ void aca_build(dmb_ctx *c, double k, double eta0, int quad_order, int leaf_size,
   DMB_REQUIRE(std::isfinite(inv_k2) && std::isfinite(k * eta0) && k * eta0 != 0.0, DMB_ERR_OVERFLOW,
               "EFIE prefactors are not representable");
   AcaState &A = c->aca;
-  A.release();
+  A.valid = false;  // the buffers stay for the new operator
   c->op_kind = 0;
   prepare_operator(c, k, eta0, quad_order);  // triangle cache + near records for this k
   const int64_t N = c->n;
@@ -1227,7 +1227,8 @@ void aca_build(dmb_ctx *c, double k, double eta0, int quad_order, int leaf_size,
       fo += d.m + d.n;
       so += (int64_t)ACA_SCR * d.rmax;
     }
-    DevBuf d_ids, d_foff, d_soff, d_flags, d_scr, d_rank, d_status, d_conv;
+    DevBuf &d_ids = A.d_ids, &d_foff = A.d_foff, &d_soff = A.d_soff, &d_flags = A.d_flags, &d_scr = A.d_scr,
+           &d_rank = A.d_rank, &d_status = A.d_status, &d_conv = A.d_conv;
     upload(c, d_ids, order);
     upload(c, d_foff, foff);
     upload(c, d_soff, soff);
@@ -1443,7 +1444,7 @@ void aca_nf_build(dmb_ctx *c, int kind, int precision) {
     // admissible against itself); evaluate them directly
     std::vector<int> mn(2 * N);
     for (int64_t i = 0; i < N; i++) mn[2 * i] = mn[2 * i + 1] = (int)i;
-    DevBuf d_mn, d_diag, tmp;
+    ScratchBuf d_mn, d_diag, tmp;
     upload(c, d_mn, mn);
     d_diag.ensure(sizeof(double2) * N);
     tmp.ensure(16);
@@ -1473,7 +1474,7 @@ void aca_nf_build(dmb_ctx *c, int kind, int precision) {
   const size_t esz = f64 ? sizeof(double2) : sizeof(float2);
   c->d_F.ensure(esz * N * N);
   DMB_CUDA(cudaMemsetAsync(c->d_F.p, 0, esz * N * N, c->stream));
-  DevBuf d_ids;
+  DevBuf &d_ids = A.d_ids;
   upload(c, d_ids, dense);
   if (!dense.empty()) {
     if (f64)
@@ -1506,7 +1507,7 @@ void aca_entries(dmb_ctx *c, const int64_t *m, const int64_t *n, int64_t count, 
     mn[2 * e] = (int)(m[e] - 1);
     mn[2 * e + 1] = (int)(n[e] - 1);
   }
-  DevBuf d_mn, d_out;
+  DevBuf &d_mn = c->d_tmp[0], &d_out = c->d_tmp[1];
   upload(c, d_mn, mn);
   d_out.ensure(sizeof(double2) * std::max<int64_t>(count, 1));
   AcaGeo g = make_geo(c);
@@ -1539,7 +1540,7 @@ int aca_lowrank_one(dmb_ctx *c, double k, double eta0, int quad_order, const std
   std::vector<AcaBlockDesc> blk = {d};
   std::vector<int> ids = {0};
   std::vector<int64_t> foff = {0}, soff = {0};
-  DevBuf d_idx, d_blk, d_ids, d_foff, d_soff, d_arena, d_flags, d_scr, d_out;
+  ScratchBuf d_idx, d_blk, d_ids, d_foff, d_soff, d_arena, d_flags, d_scr, d_out;
   upload(c, d_idx, idx);
   upload(c, d_blk, blk);
   upload(c, d_ids, ids);
@@ -1675,7 +1676,7 @@ dmb_status dmb_aca_matvec(dmb_ctx *c, const double *x, double *y, int64_t nrhs, 
     for (int64_t i = 0; i < 2 * c->aca.n * nrhs; i++)
       DMB_REQUIRE(std::isfinite(x[i]), DMB_ERR_ARGUMENT, "x must contain only finite values");
     const size_t bytes = sizeof(double2) * c->aca.n * nrhs;
-    DevBuf bx, by;
+    DevBuf &bx = c->d_io[0], &by = c->d_io[1];
     bx.ensure(bytes);
     by.ensure(bytes);
     DMB_CUDA(cudaMemcpyAsync(bx.p, x, bytes, cudaMemcpyHostToDevice, c->stream));

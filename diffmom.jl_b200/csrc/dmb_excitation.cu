@@ -777,7 +777,7 @@ void rhs_dipoles_dev(dmb_ctx *c, int64_t R, const double *pos, const double *mom
                      const double *freqs, int quad_order, double *V_dev) {
   double t0 = now_ms();
   ensure_cache(c, quad_order);
-  DevBuf bp, bm, bt, bf;
+  DevBuf &bp = c->d_tmp[0], &bm = c->d_tmp[1], &bt = c->d_tmp[2], &bf = c->d_tmp[3];
   bp.ensure(24 * R);
   bm.ensure(48 * R);
   bt.ensure(4 * R);
@@ -797,7 +797,7 @@ void rhs_pattern_dev(dmb_ctx *c, int nth, const double *theta, int nph, const do
                      const double *Fp, double freq, const double *pc, int conj_conv, int quad_order, double *V_dev) {
   double t0 = now_ms();
   ensure_cache(c, quad_order);
-  DevBuf bth, bph, bft, bfp;
+  DevBuf &bth = c->d_tmp[0], &bph = c->d_tmp[1], &bft = c->d_tmp[2], &bfp = c->d_tmp[3];
   const size_t nf = (size_t)nth * nph;
   bth.ensure(8 * nth);
   bph.ensure(8 * nph);

@@ -2140,7 +2140,7 @@ void nf_build(dmb_ctx *c, double cutoff, int kind) {
   const bool f64 = c->z_prec == DMB_PREC_FP64;
   c->pc_valid = false;
   if (kind == DMB_PRECOND_NF_DIAG) {
-    DevBuf tmp;
+    DevBuf &tmp = c->d_tmp[0];
     tmp.ensure(16);
     DMB_CUDA(cudaMemsetAsync(tmp.p, 0, 16, c->stream));
     c->d_dinv.ensure(sizeof(double2) * N);

@@ -460,7 +460,7 @@ void far_panels(dmb_ctx *c, int T, bool f64) {
   }
   int pbytes = 0;
   far_dispatch(c->nq, T, f64, [&](auto NQ, auto TT, auto FV) { pbytes = panel_bytes_t<decltype(NQ)::value, decltype(TT)::value, decltype(FV)::value>(); });
-  DevBuf lists;
+  ScratchBuf lists;
   lists.ensure(tile_tri.size() * 4);
   DMB_CUDA(cudaMemcpyAsync(lists.p, tile_tri.data(), tile_tri.size() * 4, cudaMemcpyHostToDevice, c->stream));
   st.d_cnt.ensure(cnt.size() * 4);

@@ -501,6 +501,13 @@ void gmres_dev(dmb_ctx *c, const double *b_dev, double *x_dev, int64_t R, double
         for (int jj = j0; jj < j0 + nb; jj++) iteration(jj);
       };
       if (!(graphs_ok && c->gmres_graphs)) return eager();
+      // a device allocation anywhere ends the life of all captured iterations
+      if (c->gm_graph_epoch != g_dev_alloc_epoch.load()) {
+        for (auto &kv : c->gm_graphs)
+          if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
+        c->gm_graphs.clear();
+        c->gm_graph_epoch = g_dev_alloc_epoch.load();
+      }
       const std::vector<int64_t> key = {j0, nb, N, R, kcap, vstride, precond_kind, side, flex, c->pc_kind,
                                         c->z_prec, (int64_t)(uintptr_t)V, (int64_t)(uintptr_t)Zv,
                                         (int64_t)(uintptr_t)w, (int64_t)(uintptr_t)tmp, (int64_t)(uintptr_t)H,

@@ -77,6 +77,14 @@ struct DevBuf {
   }
 };
 
+// a buffer that lives as long as its function
+struct ScratchBuf : DevBuf {
+  ScratchBuf() = default;
+  ScratchBuf(const ScratchBuf &) = delete;
+  ScratchBuf &operator=(const ScratchBuf &) = delete;
+  ~ScratchBuf() { release(); }
+};
+
 // ---------------------------------------------------------------------------
 // per-triangle cache (device, FP64).  Quadrature points are stored both in
 // global coordinates (FP64 path, as the reference's cache) and relative to the
@@ -133,13 +141,14 @@ struct AcaState {
   DevBuf d_leaf;                          // leaf node ranges (first, count)
   DevBuf d_zoff_r, d_zoff_c, d_z;         // per-block partial products (row / column side)
   DevBuf d_row_zbase, d_col_zbase;        // per leaf item: partial offset minus the block's first row / column
+  DevBuf d_ids, d_foff, d_soff, d_flags, d_scr, d_status, d_conv;  // the build's workspace
   int64_t n_leaves = 0, n_lr = 0, t_total = 0;
   double k = 0, eta0 = 0;
   int quad_order = 3;
   void release() {
     DevBuf *b[] = {&d_perm, &d_blocks, &d_arena, &d_rank, &d_tbuf_off, &d_t, &d_xp, &d_lr_list,
                    &d_row_off, &d_col_off, &d_leaf, &d_zoff_r, &d_zoff_c, &d_z,
-                   &d_row_zbase, &d_col_zbase};
+                   &d_row_zbase, &d_col_zbase, &d_ids, &d_foff, &d_soff, &d_flags, &d_scr, &d_status, &d_conv};
     for (DevBuf *x : b) x->release();
     valid = false;
   }
@@ -173,6 +182,8 @@ struct Oz64State {
   DevBuf planes[3], scale[3], res[3];
   bool attr = false;
 };
+
+struct HostCopy;
 
 struct dmb_ctx {
   int device = 0;
@@ -257,6 +268,9 @@ struct dmb_ctx {
 
   // resident solution of dmb_solve_resident / dmb_solve_resident_many
   DevBuf d_rhs, d_sol, d_mono;
+  DevBuf d_io[3];     // device copies of a call's host arrays
+  DevBuf d_tmp[4];    // workspace of a call's stages (nothing is kept in it between them)
+  HostCopy *hostcopy = nullptr;  // chunks of large copies to the host (dmb_hostcopy.cu)
   DevBuf d_far;       // far-field workspace
   DevBuf d_mf;        // matrix-free product workspace
   int64_t sol_r = 0;
@@ -284,6 +298,7 @@ struct dmb_ctx {
     bool seen = false;
   };
   std::map<std::vector<int64_t>, GraphEntry> gm_graphs;
+  uint64_t gm_graph_epoch = 0;   // device allocations when gm_graphs' entries were made
   int precond_tf32_terms = 3;    // TF32 products of the complex64 factor updates and packed sweeps (3 or 1)
   // those operands split into BF16 pieces (kind::f16 MMA) instead of TF32:
   // 1 always, 0 never, -1 (default) inside the resident solves only
@@ -414,6 +429,8 @@ void tune_end(dmb_ctx *c, TuneMark &mk);
 std::string tune_report();
 void assemble(dmb_ctx *c, double k, double eta0, int quad_order, int precision);
 void copy_z_out(dmb_ctx *c, double *Z_out);
+void copy_out(dmb_ctx *c, void *dst, const void *src, int64_t count, bool widen = false);
+void hostcopy_release(dmb_ctx *c);
 void z_entries(dmb_ctx *c, const int64_t *m, const int64_t *n, int64_t count, double *out);
 void apply_impedance(dmb_ctx *c, const double *zs);
 // FP64 complex GEMMs on the FP64 pipe (dmb_zgemm64.cu): Y = Z X (column-major

@@ -205,11 +205,6 @@ __global__ void k_conj(int64_t count, double2 *__restrict__ x) {
   if (i < count) x[i].y = -x[i].y;
 }
 
-__global__ void k_f2_to_d2(int64_t count, const float2 *__restrict__ a, double2 *__restrict__ b) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < count) b[i] = make_double2(a[i].x, a[i].y);
-}
-
 template <class ZC>
 __global__ void k_entries(int64_t count, int64_t N, const int64_t *__restrict__ mn, const ZC *__restrict__ Z,
                           double2 *__restrict__ out) {
@@ -288,19 +283,7 @@ unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 namespace dmb {
 
 void copy_z_out(dmb_ctx *c, double *Z_out) {
-  const int64_t N = c->n;
-  size_t bytes = sizeof(double2) * N * N;
-  if (c->z_prec == DMB_PREC_FP64) {
-    DMB_CUDA(cudaMemcpyAsync(Z_out, c->d_Z.p, bytes, cudaMemcpyDeviceToHost, c->stream));
-  } else {
-    DevBuf tmp;
-    tmp.ensure(bytes);
-    DMB_LAUNCH(c, k_f2_to_d2, blocks_for(N * N, 256), 256, 0, N * N, c->d_Z.as<float2>(),
-               tmp.as<double2>());
-    DMB_CUDA(cudaMemcpyAsync(Z_out, tmp.p, bytes, cudaMemcpyDeviceToHost, c->stream));
-    DMB_CUDA(cudaStreamSynchronize(c->stream));
-  }
-  DMB_CUDA(cudaStreamSynchronize(c->stream));
+  copy_out(c, Z_out, c->d_Z.p, c->n * c->n, c->z_prec != DMB_PREC_FP64);
 }
 
 void z_entries(dmb_ctx *c, const int64_t *m, const int64_t *n, int64_t count, double *out) {
@@ -310,7 +293,7 @@ void z_entries(dmb_ctx *c, const int64_t *m, const int64_t *n, int64_t count, do
     mn[2 * i] = m[i];
     mn[2 * i + 1] = n[i];
   }
-  DevBuf dmn, dout;
+  DevBuf &dmn = c->d_tmp[0], &dout = c->d_tmp[1];
   dmn.ensure(mn.size() * 8);
   dout.ensure(sizeof(double2) * count);
   DMB_CUDA(cudaMemcpyAsync(dmn.p, mn.data(), mn.size() * 8, cudaMemcpyHostToDevice, c->stream));
@@ -320,12 +303,11 @@ void z_entries(dmb_ctx *c, const int64_t *m, const int64_t *n, int64_t count, do
   else
     DMB_LAUNCH(c, k_entries<float2>, blocks_for(count, 256), 256, 0, count, c->n, dmn.as<int64_t>(),
                c->d_Z.as<float2>(), dout.as<double2>());
-  DMB_CUDA(cudaMemcpyAsync(out, dout.p, sizeof(double2) * count, cudaMemcpyDeviceToHost, c->stream));
-  DMB_CUDA(cudaStreamSynchronize(c->stream));
+  copy_out(c, out, dout.p, count);
 }
 
 void apply_impedance(dmb_ctx *c, const double *zs) {
-  DevBuf dz;
+  DevBuf &dz = c->d_tmp[0];
   dz.ensure(sizeof(double2) * c->nt);
   DMB_CUDA(cudaMemcpyAsync(dz.p, zs, sizeof(double2) * c->nt, cudaMemcpyHostToDevice, c->stream));
   const TriCache *tc = c->d_tcache.as<TriCache>();
@@ -402,7 +384,7 @@ void gradient_impedance_dev(dmb_ctx *c, int64_t R, const double2 *I_dev, const d
   for (int64_t p = 0; p < P; p++) off[p + 1] += off[p];
   std::vector<int> pos(off.begin(), off.end() - 1);
   for (int64_t t = 0; t < c->nt; t++) tri[pos[tri_patch[t]]++] = (int)t;
-  DevBuf boff, btri;
+  DevBuf &boff = c->d_tmp[0], &btri = c->d_tmp[1];
   boff.ensure(sizeof(int) * (P + 1));
   btri.ensure(sizeof(int) * std::max<int64_t>(1, c->nt));
   DMB_CUDA(cudaMemcpyAsync(boff.p, off.data(), sizeof(int) * (P + 1), cudaMemcpyHostToDevice, c->stream));
@@ -483,7 +465,7 @@ void solve_direct_dev(dmb_ctx *c, const double *b_dev, double *x_dev, int64_t nr
   double t0 = now_ms();
   nf_build(c, INFINITY, DMB_PRECOND_NF_LU);
   const int64_t N = c->n, cnt = N * nrhs;
-  DevBuf r, z;
+  DevBuf &r = c->d_tmp[0], &z = c->d_tmp[1];
   r.ensure(sizeof(double2) * cnt);
   z.ensure(sizeof(double2) * cnt);
   const double2 *b = (const double2 *)b_dev;

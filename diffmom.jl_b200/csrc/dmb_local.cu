@@ -1086,7 +1086,7 @@ double train_epochs(dmb_ctx *c, int epochs, int batch, double lr, uint64_t seed)
 void net_loss_grad(dmb_ctx *c, const float *feat, const float *tgt, const float *wgt, const int *cnt,
                    int64_t nrows, float *grad, float *loss) {
   ensure_net(c);
-  DevBuf f, t, s, k, part, lr, g, lv;
+  ScratchBuf f, t, s, k, part, lr, g, lv;
   f.ensure(sizeof(float) * nrows * KS * NF);
   t.ensure(sizeof(float) * nrows * KS * 2);
   s.ensure(sizeof(float) * nrows * KS);

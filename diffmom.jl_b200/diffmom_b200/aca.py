@@ -280,18 +280,32 @@ class ACAOperator:
         device.ctx.call("dmb_aca_blocks", nat.lptr(B))
         self._blocks = B[:info.n_dense + info.n_lowrank]
         self._cache = {}
-        self.dense_blocks, self.lowrank_blocks = [], []
-        for i, b in enumerate(self._blocks):
-            rr, cr = range(int(b[1]), int(b[2]) + 1), range(int(b[3]), int(b[4]) + 1)
-            if b[0] == 0:
-                self.dense_blocks.append(DenseBlock(rr, cr, self, i, bool(b[6])))
-            else:
-                self.lowrank_blocks.append(LowRankBlock(rr, cr, int(b[5]), self, i))
+        self._lists = None  # (dense, low-rank) block objects, made when asked for
         perm = np.empty(self.N, dtype=np.int64)
         device.ctx.call("dmb_aca_tree", nat.lptr(perm), None)
         iperm = np.empty_like(perm)
         iperm[perm - 1] = np.arange(1, self.N + 1)
         self.perm, self.iperm = perm, iperm
+
+    def _block_lists(self):
+        if self._lists is None:
+            dense, lowrank = [], []
+            for i, b in enumerate(self._blocks):
+                rr, cr = range(int(b[1]), int(b[2]) + 1), range(int(b[3]), int(b[4]) + 1)
+                if b[0] == 0:
+                    dense.append(DenseBlock(rr, cr, self, i, bool(b[6])))
+                else:
+                    lowrank.append(LowRankBlock(rr, cr, int(b[5]), self, i))
+            self._lists = dense, lowrank
+        return self._lists
+
+    @property
+    def dense_blocks(self):
+        return self._block_lists()[0]
+
+    @property
+    def lowrank_blocks(self):
+        return self._block_lists()[1]
 
     def _check_current(self):
         if getattr(self.device, "_aca_current", None) is not self:
