@@ -386,7 +386,10 @@ void make_plan(const double *ctr, int64_t n, int leaf_size, double eta, int64_t 
 // device: EFIE entries on the fly
 // ---------------------------------------------------------------------------
 struct AcaGeo {
-  const TriCache *tc;
+  const double *pts;  // quadrature data of the basis functions at np positions (k_aca_points)
+  const int *ptri;    // their triangles, [2][np]
+  const int *ipos;    // basis function -> position
+  int64_t np;
   const int *rslot;
   const int *aoff, *anb;
   const int2 *near_mn;
@@ -403,133 +406,184 @@ __device__ __forceinline__ bool aca_tri_adjacent(const int *__restrict__ off, co
   return false;
 }
 
-// Element (i, j) of the far triangle-pair block of (A, B), A the triangle of
-// the lower slot index: the moments and the contraction are written as in the
-// dense assembly's far-pair kernel, so both give the same value.
+// Quadrature data of the basis functions ids[0 .. np) on their two triangles:
+// per point the position, the weighted basis value w s (r - p) and the weighted
+// divergence w dv, then the triangle's centroid and the largest distance of a
+// vertex from it (times 1 + 1e-9); field by field over the
+// positions, pts[(side F + field) np + position].  With the ids in tree order a
+// block's rows and columns are runs of positions, and the lanes of a warp read
+// whole lines (the per-triangle cache scatters a function over 1.1 KB records).
+template <int NQ> constexpr int aca_fields() { return 7 * NQ + 4; }
+
 template <int NQ>
-__device__ double2 far_slot_value(const TriCache &A, const TriCache &B, int i, int j, double k, double inv_k2) {
-  double m0r = 0, m0i = 0, mar[3] = {0, 0, 0}, mai[3] = {0, 0, 0}, mbr[3] = {0, 0, 0}, mbi[3] = {0, 0, 0},
-         mabr = 0, mabi = 0;
-  // same operations in the same order; the points of A are read where they
-  // are used (cached) instead of held in registers
-#pragma unroll 1
-  for (int b = 0; b < NQ; b++) {
-    const double qb0 = B.qp[b][0], qb1 = B.qp[b][1], qb2 = B.qp[b][2];
-    const double lb0 = B.ql[b][0], lb1 = B.ql[b][1], lb2 = B.ql[b][2];
-    const double wb = B.w2a[b];
-#pragma unroll 1
-    for (int a = 0; a < NQ; a++) {
-      const double la0 = A.ql[a][0], la1 = A.ql[a][1], la2 = A.ql[a][2];
-      double dx = A.qp[a][0] - qb0, dy = A.qp[a][1] - qb1, dz = A.qp[a][2] - qb2;
-      double R = sqrt(dx * dx + dy * dy + dz * dz);
-      double sn, cs;
-      sincos(k * R, &sn, &cs);
-      double g = (DMB_INV_FOUR_PI / R) * (A.w2a[a] * wb);
-      double gr = cs * g, gi = -sn * g;
-      m0r += gr;
-      m0i += gi;
-      mar[0] = fma(gr, la0, mar[0]); mai[0] = fma(gi, la0, mai[0]);
-      mar[1] = fma(gr, la1, mar[1]); mai[1] = fma(gi, la1, mai[1]);
-      mar[2] = fma(gr, la2, mar[2]); mai[2] = fma(gi, la2, mai[2]);
-      mbr[0] = fma(gr, lb0, mbr[0]); mbi[0] = fma(gi, lb0, mbi[0]);
-      mbr[1] = fma(gr, lb1, mbr[1]); mbi[1] = fma(gi, lb1, mbi[1]);
-      mbr[2] = fma(gr, lb2, mbr[2]); mbi[2] = fma(gi, lb2, mbi[2]);
-      double dd = la0 * lb0 + la1 * lb1 + la2 * lb2;
-      mabr = fma(gr, dd, mabr);
-      mabi = fma(gi, dd, mabi);
+__global__ void k_aca_points(int64_t np, const int *__restrict__ ids, const TriCache *__restrict__ tc,
+                             const int *__restrict__ rslot, double *__restrict__ pts, int *__restrict__ ptri,
+                             int *__restrict__ ipos) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= 2 * np) return;
+  const int64_t side = e / np, pos = e % np;
+  const int sl = rslot[2 * (int64_t)ids[pos] + side];
+  const TriCache &T = tc[sl / 3];
+  const int i = sl % 3;
+  double *o = pts + side * aca_fields<NQ>() * np + pos;
+  for (int q = 0; q < NQ; q++) {
+    for (int c = 0; c < 3; c++) {
+      o[(7 * q + c) * np] = T.qp[q][c];
+      o[(7 * q + 3 + c) * np] = T.w2a[q] * T.s[i] * (T.qp[q][c] - T.p[i][c]);
     }
+    o[(7 * q + 6) * np] = T.w2a[q] * T.dv[i];
   }
-  double si = A.s[i], dvi = A.dv[i];
-  double pi0 = A.pl[i][0], pi1 = A.pl[i][1], pi2 = A.pl[i][2];
-  double mbpr = mbr[0] * pi0 + mbr[1] * pi1 + mbr[2] * pi2;
-  double mbpi = mbi[0] * pi0 + mbi[1] * pi1 + mbi[2] * pi2;
-  double sj = B.s[j], dvj = B.dv[j];
-  double pj0 = B.pl[j][0], pj1 = B.pl[j][1], pj2 = B.pl[j][2];
-  double mapr = mar[0] * pj0 + mar[1] * pj1 + mar[2] * pj2;
-  double mapi = mai[0] * pj0 + mai[1] * pj1 + mai[2] * pj2;
-  double pp = pi0 * pj0 + pi1 * pj1 + pi2 * pj2;
-  double ss = si * sj, sc = dvi * dvj * inv_k2;
-  double vr = ss * (mabr - mapr - mbpr + pp * m0r) - sc * m0r;
-  double vi = ss * (mabi - mapi - mbpi + pp * m0i) - sc * m0i;
-  return make_double2(vr, vi);
+  double r2 = 0;
+  for (int v = 0; v < 3; v++) {
+    const double x = T.p[v][0] - T.cen[0], y = T.p[v][1] - T.cen[1], z = T.p[v][2] - T.cen[2];
+    r2 = fmax(r2, x * x + y * y + z * z);
+  }
+  for (int c = 0; c < 3; c++) o[(7 * NQ + c) * np] = T.cen[c];
+  o[(7 * NQ + 3) * np] = sqrt(r2) * (1.0 + 1e-9);
+  ptri[side * np + pos] = sl / 3;
+  if (ipos && side == 0) ipos[ids[pos]] = (int)pos;
 }
 
-// Z[m][n] (0-based) in the dense assembly's order of operations: the four
-// slot-pair values summed (a over m's slots, b over n's), times -i omega mu0,
-// plus the entry's near records summed in their fixed order
+// The function that a row or column of entries shares, in shared memory: per
+// side and point eight doubles (position, basis value, divergence / k^2, one
+// unused), then the centroid
+template <int NQ> constexpr int aca_fixed_len() { return 8 * NQ + 4; }
 template <int NQ>
-__device__ double2 aca_entry(const AcaGeo &g, int m, int n) {
-  const int sm[2] = {g.rslot[2 * m], g.rslot[2 * m + 1]};
-  const int sn[2] = {g.rslot[2 * n], g.rslot[2 * n + 1]};
+__device__ void aca_load_fixed(const AcaGeo &g, int64_t pos, double *fx, int t0, int nt) {
+  constexpr int F = aca_fields<NQ>();
+  for (int e = t0; e < 2 * F; e += nt) {
+    const int side = e / F, f = e % F;
+    double v = g.pts[(int64_t)e * g.np + pos];
+    if (f < 7 * NQ && f % 7 == 6) v *= g.inv_k2;
+    fx[side * aca_fixed_len<NQ>() + (f < 7 * NQ ? 8 * (f / 7) + f % 7 : 8 * NQ + f - 7 * NQ)] = v;
+  }
+}
+
+// The singular part of entry (m, n), whose triangles are near each other: the
+// sum of its records (binary search of the entry list)
+__device__ double2 aca_near_part(const AcaGeo &g, int m, int n) {
+  const int a = m <= n ? m : n, b = m <= n ? n : m;
+  int64_t lo = 0, hi = g.n_near;
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) >> 1;
+    const int2 e = g.near_mn[mid];
+    if (e.x < a || (e.x == a && e.y < b))
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  double nr = 0, ni = 0;
+  if (lo < g.n_near && g.near_mn[lo].x == a && g.near_mn[lo].y == b)
+    for (int64_t r = g.near_off[lo]; r < g.near_off[lo + 1]; r++) {
+      nr += g.near_val[r].x;
+      ni += g.near_val[r].y;
+    }
+  return make_double2(g.omega_mu0 * ni, -g.omega_mu0 * nr);
+}
+
+// Z of the shared function m (fx, at position mpos) and the function n at
+// position npos: per pair of points one Green value times (f_m . f_n - div_m
+// div_n / k^2) -- an entry needs one slot pair of a triangle pair, so its sum is
+// formed directly, without the moments of the whole 3 x 3 block -- with the
+// phase of the centroid distance taken once per triangle pair (phase_exp).
+// Bound by the FP64 pipe: about 60 operations a point pair (150 with a square
+// root, a sincos and a division each, and the eight moments).  A call of its
+// own: inlined twice, the low-rank kernel spills in the inner loop.  Measured,
+// three points: 3.68 million dense entries in 0.82 ms (1.45 ms in the form of
+// the dense assembly; 2.66 ms with the quadrature data function by function,
+// whose loads are not coalesced).
+template <int NQ>
+__device__ __noinline__ double2 aca_entry(const AcaGeo &g, const double *fx, int64_t mpos, int m, int64_t npos,
+                                             int n) {
+  constexpr int F = aca_fields<NQ>(), L = aca_fixed_len<NQ>();
   double re = 0, im = 0;
   bool near = false;
-  // the four slot pairs one after another (unrolled, their quadrature loops
-  // would hold four sets of moments in registers)
 #pragma unroll 1
-  for (int a = 0; a < 2; a++)
-#pragma unroll 1
-    for (int b = 0; b < 2; b++) {
-      const int x = sm[a], y = sn[b];
-      const int lo = x <= y ? x : y, hi = x <= y ? y : x;
-      const int ta = lo / 3, tb = hi / 3;
-      double2 v = make_double2(0.0, 0.0);
-      if (ta == tb || aca_tri_adjacent(g.aoff, g.anb, ta, tb))
-        near = true;
-      else
-        v = far_slot_value<NQ>(g.tc[ta], g.tc[tb], lo - 3 * ta, hi - 3 * tb, g.k, g.inv_k2);
-      re += v.x;
-      im += v.y;
-    }
-  double2 z = make_double2(g.omega_mu0 * im, -g.omega_mu0 * re);
-  if (near && g.n_near > 0) {
-    const int a = m <= n ? m : n, b = m <= n ? n : m;
-    int64_t lo = 0, hi = g.n_near;
-    while (lo < hi) {
-      const int64_t mid = (lo + hi) >> 1;
-      const int2 e = g.near_mn[mid];
-      if (e.x < a || (e.x == a && e.y < b))
-        lo = mid + 1;
-      else
-        hi = mid;
-    }
-    if (lo < g.n_near && g.near_mn[lo].x == a && g.near_mn[lo].y == b) {
-      double nr = 0, ni = 0;
-      for (int64_t r = g.near_off[lo]; r < g.near_off[lo + 1]; r++) {
-        nr += g.near_val[r].x;
-        ni += g.near_val[r].y;
+  for (int b = 0; b < 2; b++) {
+    const double *v = g.pts + (int64_t)b * F * g.np + npos;
+    double Rc[2], s0[2], c0[2];
+    bool far[2];
+    const double *vc = v + 7 * NQ * g.np;
+#pragma unroll
+    for (int a = 0; a < 2; a++) {
+      const double *u = fx + a * L + 8 * NQ;
+      const double cx = u[0] - vc[0], cy = u[1] - vc[g.np], cz = u[2] - vc[2 * g.np];
+      Rc[a] = sqrt(cx * cx + cy * cy + cz * cz);
+      far[a] = true;
+      // triangles that share an edge are within their radii of each other:
+      // the neighbour lists are read for those few
+      if (!(Rc[a] > u[3] + vc[3 * g.np])) {
+        const int ta = g.ptri[a * g.np + mpos], tb = g.ptri[b * g.np + npos];
+        if (ta == tb || aca_tri_adjacent(g.aoff, g.anb, ta, tb)) {
+          far[a] = false;
+          near = true;
+        }
       }
-      z = cadd(z, make_double2(g.omega_mu0 * ni, -g.omega_mu0 * nr));
+      sincos(g.k * Rc[a], &s0[a], &c0[a]);
+    }
+#pragma unroll 1
+    for (int q = 0; q < NQ; q++, v += 7 * g.np) {
+      double y[7];
+#pragma unroll
+      for (int f = 0; f < 7; f++) y[f] = v[f * g.np];
+#pragma unroll
+      for (int a = 0; a < 2; a++) {
+        if (!far[a]) continue;
+#pragma unroll
+        for (int p = 0; p < NQ; p++) {
+          const double *u = fx + a * L + 8 * p;
+          const double dx = u[0] - y[0], dy = u[1] - y[1], dz = u[2] - y[2];
+          const double R2 = dx * dx + dy * dy + dz * dz, rinv = rsqrt(R2);
+          double sn, cs;
+          phase_exp(g.k, R2 * rinv, Rc[a], s0[a], c0[a], sn, cs);
+          const double w = rinv * (u[3] * y[3] + u[4] * y[4] + u[5] * y[5] - u[6] * y[6]);
+          re = fma(cs, w, re);
+          im = fma(-sn, w, im);
+        }
+      }
     }
   }
+  re *= DMB_INV_FOUR_PI;
+  im *= DMB_INV_FOUR_PI;
+  double2 z = make_double2(g.omega_mu0 * im, -g.omega_mu0 * re);
+  if (near && g.n_near > 0) z = cadd(z, aca_near_part(g, m, n));
   return z;
 }
 
 // ---------------------------------------------------------------------------
 // device: block fill and ACA
 // ---------------------------------------------------------------------------
+// one CTA per block, column by column
 template <int NQ>
-__global__ void __launch_bounds__(256) k_aca_dense(AcaGeo g, const AcaBlockDesc *__restrict__ blocks,
+__global__ void __launch_bounds__(128) k_aca_dense(AcaGeo g, const AcaBlockDesc *__restrict__ blocks,
                                                    const int *__restrict__ ids, const int *__restrict__ perm,
                                                    double2 *__restrict__ arena) {
+  constexpr int NC = 16;  // columns at a time: few idle threads in the last round
+  __shared__ double fx[NC][2 * aca_fixed_len<NQ>()];
   const AcaBlockDesc bd = blocks[ids[blockIdx.x]];
   double2 *D = arena + bd.off_a;
-  const int64_t cnt = (int64_t)bd.m * bd.n;
-  for (int64_t e = threadIdx.x; e < cnt; e += blockDim.x) {
-    const int ii = (int)(e % bd.m), jj = (int)(e / bd.m);
-    D[e] = aca_entry<NQ>(g, perm[bd.r0 + ii], perm[bd.c0 + jj]);
+  for (int j0 = 0; j0 < bd.n; j0 += NC) {
+    const int nj = min(NC, bd.n - j0);
+    __syncthreads();
+    for (int q = 0; q < nj; q++) aca_load_fixed<NQ>(g, bd.c0 + j0 + q, fx[q], threadIdx.x, 128);
+    __syncthreads();
+    for (int e = threadIdx.x; e < nj * bd.m; e += 128) {
+      const int ii = e % bd.m, q = e / bd.m, jj = j0 + q;
+      D[ii + (int64_t)jj * bd.m] = aca_entry<NQ>(g, fx[q], bd.c0 + jj, perm[bd.c0 + jj], bd.r0 + ii, perm[bd.r0 + ii]);
+    }
   }
 }
 
-__global__ void k_aca_entries(AcaGeo g, int nq, int64_t count, const int *__restrict__ mn, double2 *__restrict__ out) {
-  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// single entries (efie_entry of an operator, its diagonal), a thread each
+template <int NQ>
+__global__ void __launch_bounds__(32) k_aca_entries(AcaGeo g, int64_t count, const int *__restrict__ mn,
+                                                    double2 *__restrict__ out) {
+  __shared__ double fx[32][2 * aca_fixed_len<NQ>() + 1];
+  const int64_t e = (int64_t)blockIdx.x * 32 + threadIdx.x;
   if (e >= count) return;
-  const int m = mn[2 * e], n = mn[2 * e + 1];
-  double2 v;
-  if (nq == 1) v = aca_entry<1>(g, m, n);
-  else if (nq == 3) v = aca_entry<3>(g, m, n);
-  else if (nq == 4) v = aca_entry<4>(g, m, n);
-  else v = aca_entry<7>(g, m, n);
-  out[e] = v;
+  const int m = mn[2 * e], n = mn[2 * e + 1], pm = g.ipos[m];
+  aca_load_fixed<NQ>(g, pm, fx[threadIdx.x], 0, 1);
+  out[e] = aca_entry<NQ>(g, fx[threadIdx.x], pm, m, g.ipos[n], n);
 }
 
 // scaled magnitude (fraction in [0.5, 1), binary exponent) of
@@ -629,16 +683,31 @@ __device__ double block_max(double v, double *sh) {
   return s;
 }
 
+// c > 0 becomes the power of two next above it (within the normal range); its
+// reciprocal is returned
+__device__ double pow2_scale(double &c) {
+  int e;
+  frexp(c, &e);
+  e = min(max(e, -1022), 1022);
+  c = ldexp(1.0, e);
+  return ldexp(1.0, -e);
+}
+
 // per-rank scratch of one low-rank block: 10 doubles per rank
-constexpr int ACA_SCR = 10;  // su, nu, sv, nv, term f, term e, <U_p,u> re/im, <V_p,v> re/im
+constexpr int ACA_SCR = 10;  // 1 / su, nu, 1 / sv, nv, term f, term e, <U_p,u> re/im, <V_p,v> re/im
 
 // One CTA per admissible block: aca_lowrank (src/fast/ACA.jl:351-554).
 // status: 0 ok, 1 non-finite update (the block becomes dense), 2 zero-norm
 // update; conv: 1 converged, 0 stopped otherwise.
 // NT threads per CTA: the launcher buckets the blocks by size (small blocks
-// on narrow CTAs, the few large ones on wide CTAs).
+// on narrow CTAs, the few large ones on wide CTAs).  Bound by the latency of a
+// step (entries, pivot search, inner products, estimate), a CTA's steps being
+// one after another; about half of it is the entries' arithmetic.  Measured:
+// 5,844 blocks, 33 million entries of a 10,680-function plate in 18 ms (34 ms
+// with entries in the form of the dense assembly, the scales of the inner
+// products divided out element by element and the estimate on one thread).
 template <int NQ, int NT>
-__global__ void __launch_bounds__(NT) k_aca_lowrank(AcaGeo g, const AcaBlockDesc *__restrict__ blocks,
+__global__ void __launch_bounds__(NT, 512 / NT) k_aca_lowrank(AcaGeo g, const AcaBlockDesc *__restrict__ blocks,
                                                     const int *__restrict__ ids, const int *__restrict__ perm,
                                                     double2 *__restrict__ arena, const int64_t *__restrict__ foff,
                                                     unsigned char *__restrict__ flags,
@@ -650,6 +719,9 @@ __global__ void __launch_bounds__(NT) k_aca_lowrank(AcaGeo g, const AcaBlockDesc
   __shared__ double sh[96];
   __shared__ int s_pc, s_stop, s_conv;
   __shared__ double2 s_pivot;
+  __shared__ double fx[2 * aca_fixed_len<NQ>()];
+  constexpr int SR = 64;  // factors of the pivot row / column kept in shared memory
+  __shared__ double2 s_piv_f[SR];
   const int bi = ids[blockIdx.x];
   const AcaBlockDesc bd = blocks[bi];
   const int m = bd.m, n = bd.n, rmax = bd.rmax;
@@ -660,21 +732,24 @@ __global__ void __launch_bounds__(NT) k_aca_lowrank(AcaGeo g, const AcaBlockDesc
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
   int prow = 0, rank = 0, status = 0;
   bool converged = false;
-  // Frobenius estimate in units of the largest rank-one term (thread 0)
+  // Frobenius estimate in units of the largest rank-one term (warp 0)
   Mag fscale{0.0, 0};
   double fsq = 0.0;
   for (int k = 0; k < rmax; k++) {
     double2 *Uk = U + (int64_t)k * m, *Vk = V + (int64_t)k * n;
     // residual row at prow -> Vk (not yet conjugated); arg-max over unused columns
     const int ri = rows[prow];
+    aca_load_fixed<NQ>(g, bd.r0 + prow, fx, tid, nt);
+    const int ks = min(k, SR);
+    for (int p = tid; p < ks; p += nt) s_piv_f[p] = U[prow + (int64_t)p * m];
+    __syncthreads();
     double best = 0.0;
     int bidx = -1;
     for (int jj = tid; jj < n; jj += nt) {
-      double2 v = aca_entry<NQ>(g, ri, cols[jj]);
-      for (int p = 0; p < k; p++) {
-        const double2 u = U[prow + (int64_t)p * m], w = V[jj + (int64_t)p * n];
-        v = csub(v, cmul(u, cconj(w)));
-      }
+      double2 v = aca_entry<NQ>(g, fx, bd.r0 + prow, ri, bd.c0 + jj, cols[jj]);
+#pragma unroll 8
+      for (int p = 0; p < ks; p++) v = csub(v, cmul(s_piv_f[p], cconj(V[jj + (int64_t)p * n])));
+      for (int p = ks; p < k; p++) v = csub(v, cmul(U[prow + (int64_t)p * m], cconj(V[jj + (int64_t)p * n])));
       Vk[jj] = v;
       const double av = hypot(v.x, v.y);
       if (av > best && !ucol[jj]) {
@@ -716,12 +791,14 @@ __global__ void __launch_bounds__(NT) k_aca_lowrank(AcaGeo g, const AcaBlockDesc
     const double2 piv = s_pivot;
     // residual column at pc -> Uk = col / pivot
     const int cj = cols[pc];
+    aca_load_fixed<NQ>(g, bd.c0 + pc, fx, tid, nt);
+    for (int p = tid; p < ks; p += nt) s_piv_f[p] = cconj(V[pc + (int64_t)p * n]);
+    __syncthreads();
     for (int ii = tid; ii < m; ii += nt) {
-      double2 u = aca_entry<NQ>(g, rows[ii], cj);
-      for (int p = 0; p < k; p++) {
-        const double2 a = U[ii + (int64_t)p * m], w = V[pc + (int64_t)p * n];
-        u = csub(u, cmul(a, cconj(w)));
-      }
+      double2 u = aca_entry<NQ>(g, fx, bd.c0 + pc, cj, bd.r0 + ii, rows[ii]);
+#pragma unroll 8
+      for (int p = 0; p < ks; p++) u = csub(u, cmul(U[ii + (int64_t)p * m], s_piv_f[p]));
+      for (int p = ks; p < k; p++) u = csub(u, cmul(U[ii + (int64_t)p * m], cconj(V[pc + (int64_t)p * n])));
       Uk[ii] = cdiv(u, piv);
     }
     __syncthreads();
@@ -749,66 +826,74 @@ __global__ void __launch_bounds__(NT) k_aca_lowrank(AcaGeo g, const AcaBlockDesc
       status = 2;
       break;
     }
+    // scaled by powers of two: the quotients of the sums below are exact
+    // products (divided by the maxima themselves, eight FP64 divisions per
+    // element and earlier rank were the larger part of a step)
+    const double icu = pow2_scale(cu), icv = pow2_scale(cv);
     double su = 0, sv2 = 0;
     for (int ii = tid; ii < m; ii += nt) {
-      const double xr = Uk[ii].x / cu, xi = Uk[ii].y / cu;
+      const double xr = Uk[ii].x * icu, xi = Uk[ii].y * icu;
       su = fma(xr, xr, su);
       su = fma(xi, xi, su);
     }
     for (int jj = tid; jj < n; jj += nt) {
-      const double xr = Vk[jj].x / cv, xi = Vk[jj].y / cv;
+      const double xr = Vk[jj].x * icv, xi = Vk[jj].y * icv;
       sv2 = fma(xr, xr, sv2);
       sv2 = fma(xi, xi, sv2);
     }
     block_sum2(su, sv2, sh);
-    // normalised inner products with the earlier factors: warp w takes the
-    // ranks p = w, w + 8, ...
-    for (int p = warp; p < k; p += nw) {
-      const double2 *Up = U + (int64_t)p * m, *Vp = V + (int64_t)p * n;
-      const double cup = S[p * ACA_SCR + 0], cvp = S[p * ACA_SCR + 2];
-      double ur = 0, ui = 0, vr = 0, vi = 0;
-      for (int ii = lane; ii < m; ii += 32) {
-        const double lr = Up[ii].x / cup, li = Up[ii].y / cup, rr = Uk[ii].x / cu, ri2 = Uk[ii].y / cu;
-        ur = fma(lr, rr, ur);
-        ur = fma(li, ri2, ur);
-        ui = fma(lr, ri2, ui);
-        ui = fma(-li, rr, ui);
+    // normalised inner products with the earlier factors: a warp takes PB ranks
+    // at a time, their loads and sums side by side
+    constexpr int PB = 4;
+    for (int p0 = warp * PB; p0 < k; p0 += nw * PB) {
+      double2 d[2][PB];
+#pragma unroll
+      for (int h = 0; h < 2; h++) {  // u, v
+        const int len = h ? n : m;
+        const double2 *Fk = h ? Vk : Uk, *Fp = (h ? V : U) + (int64_t)p0 * len;
+        const double ik = h ? icv : icu;
+        double2 s[PB];
+        double ip[PB];
+#pragma unroll
+        for (int q = 0; q < PB; q++) {
+          s[q] = make_double2(0.0, 0.0);
+          ip[q] = p0 + q < k ? S[(p0 + q) * ACA_SCR + 2 * h] : 0.0;
+        }
+        for (int ii = lane; ii < len; ii += 32) {
+          const double rr = Fk[ii].x * ik, ri = Fk[ii].y * ik;
+#pragma unroll
+          for (int q = 0; q < PB; q++) {
+            const double2 f = p0 + q < k ? Fp[(int64_t)q * len + ii] : make_double2(0.0, 0.0);
+            const double lr = f.x * ip[q], li = f.y * ip[q];
+            s[q].x = fma(lr, rr, fma(li, ri, s[q].x));
+            s[q].y = fma(lr, ri, fma(-li, rr, s[q].y));
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < PB; q++) d[h][q] = s[q];
       }
-      for (int jj = lane; jj < n; jj += 32) {
-        const double lr = Vp[jj].x / cvp, li = Vp[jj].y / cvp, rr = Vk[jj].x / cv, ri2 = Vk[jj].y / cv;
-        vr = fma(lr, rr, vr);
-        vr = fma(li, ri2, vr);
-        vi = fma(lr, ri2, vi);
-        vi = fma(-li, rr, vi);
-      }
-      ur = warp_sum(ur);
-      ui = warp_sum(ui);
-      vr = warp_sum(vr);
-      vi = warp_sum(vi);
-      if (lane == 0) {
-        S[p * ACA_SCR + 6] = ur;
-        S[p * ACA_SCR + 7] = ui;
-        S[p * ACA_SCR + 8] = vr;
-        S[p * ACA_SCR + 9] = vi;
-      }
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int q = 0; q < PB; q++) d[h][q] = warp_sum2(d[h][q]);
+#pragma unroll
+      for (int q = 0; q < PB; q++)
+        if (lane == q && p0 + q < k) {
+          double *Sp = S + (p0 + q) * ACA_SCR;
+          Sp[6] = d[0][q].x;
+          Sp[7] = d[0][q].y;
+          Sp[8] = d[1][q].x;
+          Sp[9] = d[1][q].y;
+        }
     }
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0) {  // the Frobenius estimate, an earlier rank per lane
       const double nu = sqrt(su), nv = sqrt(sv2);
       Mag mu = mag_make(cu), mvv = mag_make(cv);
       Mag mun = mag_make(mu.f * nu), mvn = mag_make(mvv.f * nv);
       mun.e += mu.e;
       mvn.e += mvv.e;
       const Mag term = mag_mul(mun, mvn);
-      double *Sk = S + k * ACA_SCR;
-      Sk[0] = cu;
-      Sk[1] = nu;
-      Sk[2] = cv;
-      Sk[3] = nv;
-      Sk[4] = term.f;
-      Sk[5] = (double)term.e;
-      urow[prow] = 1;
-      ucol[pc] = 1;
       if (k == 0) {
         fscale = term;
       } else if (mag_less(fscale, term)) {
@@ -818,7 +903,7 @@ __global__ void __launch_bounds__(NT) k_aca_lowrank(AcaGeo g, const AcaBlockDesc
       }
       const double tr = mag_ratio(term, fscale);
       double cross = 0.0;
-      for (int p = 0; p < k; p++) {
+      for (int p = lane; p < k; p += 32) {
         const double *Sp = S + p * ACA_SCR;
         const Mag tp{Sp[4], (int)Sp[5]};
         const double pr = mag_ratio(tp, fscale);
@@ -826,9 +911,20 @@ __global__ void __launch_bounds__(NT) k_aca_lowrank(AcaGeo g, const AcaBlockDesc
         const double2 uc = make_double2(Sp[6] / un, Sp[7] / un), vc = make_double2(Sp[8] / vn, Sp[9] / vn);
         cross += 2.0 * pr * tr * (uc.x * vc.x + uc.y * vc.y);  // Re(uc conj(vc))
       }
-      fsq += tr * tr + cross;
+      fsq += tr * tr + warp_sum(cross);
       fsq = fmax(fsq, 0.0);
-      s_conv = tr < tol * sqrt(fsq) ? 1 : 0;
+      if (lane == 0) {
+        double *Sk = S + k * ACA_SCR;
+        Sk[0] = icu;
+        Sk[1] = nu;
+        Sk[2] = icv;
+        Sk[3] = nv;
+        Sk[4] = term.f;
+        Sk[5] = (double)term.e;
+        urow[prow] = 1;
+        ucol[pc] = 1;
+        s_conv = tr < tol * sqrt(fsq) ? 1 : 0;
+      }
     }
     __syncthreads();
     rank = k + 1;
@@ -1033,9 +1129,29 @@ __global__ void k_aca_diag_inv(int64_t N, const double2 *__restrict__ d, const d
   dinv[i] = cdiv(make_double2(1, 0), z);
 }
 
-AcaGeo make_geo(dmb_ctx *c) {
+#define ACA_NQ_DISPATCH(NQV, CALL)                  \
+  switch (NQV) {                                    \
+    case 1: { constexpr int NQ = 1; CALL; } break;  \
+    case 3: { constexpr int NQ = 3; CALL; } break;  \
+    case 4: { constexpr int NQ = 4; CALL; } break;  \
+    default: { constexpr int NQ = 7; CALL; } break; \
+  }
+
+// the entries' geometry over the positions of `ids` (device, np of them), whose
+// points go to the buffers given; ipos may be null
+AcaGeo make_geo(dmb_ctx *c, int64_t np, const int *ids, DevBuf &pts, DevBuf &ptri, int *ipos) {
   AcaGeo g;
-  g.tc = c->d_tcache.as<TriCache>();
+  ACA_NQ_DISPATCH(c->nq, {
+    pts.ensure(sizeof(double) * 2 * std::max<int64_t>(np, 1) * aca_fields<NQ>());
+    ptri.ensure(sizeof(int) * 2 * std::max<int64_t>(np, 1));
+    if (np > 0)
+      DMB_LAUNCH(c, k_aca_points<NQ>, blocks_for(2 * np, 128), 128, 0, np, ids, c->d_tcache.as<TriCache>(),
+                 c->d_rwg_slot.as<int>(), pts.as<double>(), ptri.as<int>(), ipos);
+  });
+  g.pts = pts.as<double>();
+  g.ptri = ptri.as<int>();
+  g.ipos = ipos;
+  g.np = np;
   g.rslot = c->d_rwg_slot.as<int>();
   g.aoff = c->d_adj_off.as<int>();
   g.anb = c->d_adj_nb.as<int>();
@@ -1048,19 +1164,17 @@ AcaGeo make_geo(dmb_ctx *c) {
   g.omega_mu0 = c->aca.k * c->aca.eta0;
   return g;
 }
+// ... of the context's operator, in tree order
+AcaGeo make_geo(dmb_ctx *c) {
+  AcaState &A = c->aca;
+  A.d_ipos.ensure(sizeof(int) * std::max<int64_t>(A.n, 1));
+  return make_geo(c, A.n, A.d_perm.as<int>(), A.d_pts, A.d_ptri, A.d_ipos.as<int>());
+}
 
 template <class T> void upload(dmb_ctx *c, DevBuf &b, const std::vector<T> &v) {
   b.ensure(std::max<size_t>(16, v.size() * sizeof(T)));
   if (!v.empty()) DMB_CUDA(cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream));
 }
-
-#define ACA_NQ_DISPATCH(NQV, CALL)                  \
-  switch (NQV) {                                    \
-    case 1: { constexpr int NQ = 1; CALL; } break;  \
-    case 3: { constexpr int NQ = 3; CALL; } break;  \
-    case 4: { constexpr int NQ = 4; CALL; } break;  \
-    default: { constexpr int NQ = 7; CALL; } break; \
-  }
 
 // dense fill of the listed blocks
 void fill_dense(dmb_ctx *c, const std::vector<int> &ids) {
@@ -1069,7 +1183,7 @@ void fill_dense(dmb_ctx *c, const std::vector<int> &ids) {
   upload(c, d_ids, ids);
   AcaGeo g = make_geo(c);
   AcaState &A = c->aca;
-  ACA_NQ_DISPATCH(c->nq, DMB_LAUNCH(c, k_aca_dense<NQ>, (unsigned)ids.size(), 256, 0, g,
+  ACA_NQ_DISPATCH(c->nq, DMB_LAUNCH(c, k_aca_dense<NQ>, (unsigned)ids.size(), 128, 0, g,
                                     A.d_blocks.as<AcaBlockDesc>(), d_ids.as<int>(), A.d_perm.as<int>(),
                                     A.d_arena.as<double2>()));
   DMB_CUDA(cudaStreamSynchronize(c->stream));
@@ -1450,7 +1564,8 @@ void aca_nf_build(dmb_ctx *c, int kind, int precision) {
     tmp.ensure(16);
     DMB_CUDA(cudaMemsetAsync(tmp.p, 0, 16, c->stream));
     AcaGeo g = make_geo(c);
-    DMB_LAUNCH(c, k_aca_entries, blocks_for(N, 128), 128, 0, g, c->nq, N, d_mn.as<int>(), d_diag.as<double2>());
+    ACA_NQ_DISPATCH(c->nq, DMB_LAUNCH(c, k_aca_entries<NQ>, blocks_for(N, 32), 32, 0, g, N, d_mn.as<int>(),
+                                      d_diag.as<double2>()));
     c->d_dinv.ensure(sizeof(double2) * N);
     unsigned *bad = (unsigned *)(tmp.as<double>() + 1);
     DMB_LAUNCH(c, k_aca_diag_max, 1, 1024, 0, N, d_diag.as<double2>(), tmp.as<double>(), bad);
@@ -1512,8 +1627,8 @@ void aca_entries(dmb_ctx *c, const int64_t *m, const int64_t *n, int64_t count, 
   d_out.ensure(sizeof(double2) * std::max<int64_t>(count, 1));
   AcaGeo g = make_geo(c);
   if (count > 0)
-    DMB_LAUNCH(c, k_aca_entries, blocks_for(count, 128), 128, 0, g, c->nq, count, d_mn.as<int>(),
-               d_out.as<double2>());
+    ACA_NQ_DISPATCH(c->nq, DMB_LAUNCH(c, k_aca_entries<NQ>, blocks_for(count, 32), 32, 0, g, count,
+                                      d_mn.as<int>(), d_out.as<double2>()));
   DMB_CUDA(cudaMemcpyAsync(out, d_out.p, sizeof(double2) * count, cudaMemcpyDeviceToHost, c->stream));
   DMB_CUDA(cudaStreamSynchronize(c->stream));
 }
@@ -1552,7 +1667,8 @@ int aca_lowrank_one(dmb_ctx *c, double k, double eta0, int quad_order, const std
   d_scr.ensure(sizeof(double) * std::max(2, ACA_SCR * rmax));
   d_out.ensure(sizeof(int) * 3);
   DMB_CUDA(cudaMemsetAsync(d_out.p, 0, sizeof(int) * 3, c->stream));
-  AcaGeo g = make_geo(c);
+  ScratchBuf d_pts, d_ptri;
+  AcaGeo g = make_geo(c, m + n, d_idx.as<int>(), d_pts, d_ptri, nullptr);
   g.k = k;
   g.inv_k2 = 1.0 / (k * k);
   g.omega_mu0 = k * eta0;

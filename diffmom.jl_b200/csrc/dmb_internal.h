@@ -142,13 +142,15 @@ struct AcaState {
   DevBuf d_zoff_r, d_zoff_c, d_z;         // per-block partial products (row / column side)
   DevBuf d_row_zbase, d_col_zbase;        // per leaf item: partial offset minus the block's first row / column
   DevBuf d_ids, d_foff, d_soff, d_flags, d_scr, d_status, d_conv;  // the build's workspace
+  DevBuf d_pts, d_ptri, d_ipos;           // quadrature data of the basis functions in tree order
   int64_t n_leaves = 0, n_lr = 0, t_total = 0;
   double k = 0, eta0 = 0;
   int quad_order = 3;
   void release() {
     DevBuf *b[] = {&d_perm, &d_blocks, &d_arena, &d_rank, &d_tbuf_off, &d_t, &d_xp, &d_lr_list,
                    &d_row_off, &d_col_off, &d_leaf, &d_zoff_r, &d_zoff_c, &d_z,
-                   &d_row_zbase, &d_col_zbase, &d_ids, &d_foff, &d_soff, &d_flags, &d_scr, &d_status, &d_conv};
+                   &d_row_zbase, &d_col_zbase, &d_ids, &d_foff, &d_soff, &d_flags, &d_scr, &d_status, &d_conv,
+                   &d_pts, &d_ptri, &d_ipos};
     for (DevBuf *x : b) x->release();
     valid = false;
   }
