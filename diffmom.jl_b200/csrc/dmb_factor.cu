@@ -8,10 +8,8 @@
 //     symmetric), so it is factored as L D L^T -- unit lower L, diagonal D, no
 //     pivoting -- which has the same inverse as the reference's UMFPACK LU up to
 //     rounding, at half the flops.  Right-looking, panel width NB = 64:
-//       k_ldlt_mid64   complex128: a 256-wide panel (four diagonal blocks, their
-//                      panel rows and the updates between them) in one launch;
-//       k_ldlt_first, k_ldlt_step  complex64: one launch per 64 columns (strip
-//                      update, next diagonal block, its panel rows);
+//       k_ldlt_mid     a 256-wide panel (four diagonal blocks, their panel rows
+//                      and the updates between them) in one launch;
 //     and updates A22 -= (L21 D1) L21^T after every 256 and 1,024 columns
 //     (complex128: int8 residue products, dmb_oz64.cu, or the FP64 pipe;
 //     complex64: the tensor-core kernels of dmb_tc.cu or FP32 units).
@@ -170,72 +168,6 @@ __device__ __forceinline__ double2 pivot_inverse(double2 d) {
 }
 __device__ __forceinline__ float2 cneg(float2 a) { return make_float2(-a.x, -a.y); }
 __device__ __forceinline__ double2 cneg(double2 a) { return make_double2(-a.x, -a.y); }
-__device__ __forceinline__ float2 csel(bool p, float2 a, float2 b) { return make_float2(p ? a.x : b.x, p ? a.y : b.y); }
-
-// Elimination of the 16 x 16 diagonal sub-block at s0 by one warp, all in
-// registers: lane (ih = lane >> 4, c = lane & 15) holds rows i = ih + 2 m
-// (m = 0..7) of column c.  The block is kept in full (both triangles: it is
-// complex symmetric and every update keeps it so), which puts each value a
-// pivot step needs -- the pivot, A[k][c] = A[c][k], X[k][c] and A[i][k] -- in
-// a register whose index is known at compile time on a lane known per lane,
-// so one shuffle fetches it; no shared memory, no warp barriers.  The updates
-// are selects, not branches (the lane conditions differ within the warp).  On
-// return the lower triangle holds L (strict) and D, X the unit-lower inverse.
-// 1/d = conj(d) / |d|^2 with |d|^2 inverted by rcp_nr; a pivot whose |d|^2 is
-// zero, non-finite or outside the FP32 normal range (|d| below ~1e-19 or above
-// ~1e19) is a breakdown (false, uniform over the warp, decided after the 16
-// steps).
-__device__ __forceinline__ bool elim16_warp(float2 (*A)[65], float2 (*Xs)[17], int s0, int lane, float2 *, float2 *) {
-  const unsigned FULL = 0xffffffffu;
-  const int c = lane & 15, ih = lane >> 4;
-  float2 a[8], x[8];
-#pragma unroll
-  for (int m = 0; m < 8; m++) {
-    const int i = ih + 2 * m;
-    a[m] = (c <= i) ? A[s0 + i][s0 + c] : A[s0 + c][s0 + i];
-    x[m] = (i == c) ? make_float2(1.f, 0.f) : make_float2(0.f, 0.f);
-  }
-  bool ok = true;
-#pragma unroll
-  for (int k = 0; k < 16; k++) {
-    const int kl = (k & 1) << 4, km = k >> 1;
-    float2 d, akc, xk, aik[8];
-    d.x = __shfl_sync(FULL, a[km].x, kl | k);
-    d.y = __shfl_sync(FULL, a[km].y, kl | k);
-    akc.x = __shfl_sync(FULL, a[km].x, kl | c);
-    akc.y = __shfl_sync(FULL, a[km].y, kl | c);
-    xk.x = __shfl_sync(FULL, x[km].x, kl | c);
-    xk.y = __shfl_sync(FULL, x[km].y, kl | c);
-#pragma unroll
-    for (int m = 0; m < 8; m++) {
-      aik[m].x = __shfl_sync(FULL, a[m].x, (ih << 4) | k);
-      aik[m].y = __shfl_sync(FULL, a[m].y, (ih << 4) | k);
-    }
-    const float d2 = fmaf(d.x, d.x, d.y * d.y);
-    ok = ok && (d2 >= 1.17549435e-38f) && (d2 <= 3.40282347e38f);
-    const float rd = rcp_nr(d2);
-    const float2 inv_d = make_float2(d.x * rd, -d.y * rd);
-    const float2 lc = cmul(akc, inv_d);
-#pragma unroll
-    for (int m = 0; m < 8; m++) {
-      const int i = ih + 2 * m;
-      const bool below = i > k;
-      const float2 lik = cmul(aik[m], inv_d);
-      const float2 upd = csub(a[m], cmul(aik[m], lc));
-      a[m] = csel(below && c > k, upd, csel(below && c == k, lik, a[m]));
-      x[m] = csel(below, csub(x[m], cmul(lik, xk)), x[m]);
-    }
-  }
-  if (!__all_sync(FULL, ok)) return false;
-#pragma unroll
-  for (int m = 0; m < 8; m++) {
-    const int i = ih + 2 * m;
-    if (c <= i) A[s0 + i][s0 + c] = a[m];
-    Xs[i][c] = x[m];
-  }
-  return true;
-}
-
 
 // The plain form for complex128 blocks with a pivot outside the range of the
 // fast one below: entry by entry in shared memory, pivots divided by Smith's
@@ -270,66 +202,103 @@ __device__ __noinline__ bool elim16_any(double2 (*A)[68], double2 (*Xs)[17], int
   return true;
 }
 
-// The same for complex128 blocks (lanes and rows as above).  A double takes
-// two shuffles, so column k and row k of X go through shared memory (buf: 48
-// values).  Bound by the latency of the chain pivot -> reciprocal -> next
-// pivot, so that chain is kept to itself: every lane forms the next pivot
-// a_{k+1,k+1} - a_{k+1,k}^2 / d from the column of this step and inverts it
-// while the block's updates and their exchange run.  The L entry of column k
-// and the update of the columns right of it are one multiply-add with a
-// per-lane factor.  dinv receives the reciprocal pivots.
-__device__ __forceinline__ bool elim16_warp(double2 (*A)[68], double2 (*Xs)[17], int s0, int lane, double2 *buf,
-                                            double2 *dinv) {
-  const unsigned FULL = 0xffffffffu;
-  const int c = lane & 15, ih = lane >> 4;
-  double2 *colb = buf, *rowb = buf + 16, *diag = buf + 32;
-  double2 a[8], x[8];
+// two values at an address that is a multiple of their size
+__device__ __forceinline__ void load_pair(const double2 *p, double2 &a, double2 &b) {
+  a = p[0];
+  b = p[1];
+}
+__device__ __forceinline__ void load_pair(const float2 *p, float2 &a, float2 &b) {
+  const float4 v = *reinterpret_cast<const float4 *>(p);
+  a = make_float2(v.x, v.y);
+  b = make_float2(v.z, v.w);
+}
+__device__ __forceinline__ void store_pair(double2 *p, double2 a, double2 b) {
+  p[0] = a;
+  p[1] = b;
+}
+__device__ __forceinline__ void store_pair(float2 *p, float2 a, float2 b) {
+  *reinterpret_cast<float4 *>(p) = make_float4(a.x, a.y, b.x, b.y);
+}
+
+// Elimination of the 16 x 16 diagonal sub-block at s0 by one warp, the values
+// in registers: lane c < 16 holds column c of the upper triangle (the block is
+// complex symmetric), lane 16 + c column c of the unit-lower inverse X.  Row k,
+// which by symmetry is also the column of multipliers, goes to all lanes through
+// shared memory, two rows at a time (buf: two pairs of 32 values in turn); then
+// every lane takes the same steps, t = a_k / d, a_i -= a_ki t for i > k, without
+// a select or a branch: entries below the diagonal are garbage that nobody
+// reads, and the rows of X are subject to the same operations.  Unrolled, so that the registers
+// are named at compile time.  Bound by the chain rows -> two reciprocals ->
+// update -> next rows of a single warp: 5,300 cycles a block (complex128 7,900)
+// against 30,000 with a lane holding eight entries of a column, whose selects
+// and predicated exchange stores came to 1,900 cycles a pivot, and 10,400 with
+// one row an exchange.  On return the lower triangle holds L (strict) and
+// D, Xs the unit-lower inverse, dinv the reciprocal pivots.  Complex64: a pivot
+// whose |d|^2 is zero, non-finite or outside the FP32 normal range (|d| below
+// ~1e-19 or above ~1e19) is a breakdown; complex128 ones outside the fast range
+// go to elim16_any.
+template <class C, int LD>
+__device__ __forceinline__ bool elim16_warp(C (*A)[LD], C (*Xs)[17], int s0, int lane, C *buf, C *dinv) {
+  constexpr bool f64 = sizeof(C) == 16;
+  const int c = lane & 15;
+  const bool isx = lane >= 16;
+  C a[16];
 #pragma unroll
-  for (int m = 0; m < 8; m++) {
-    const int i = ih + 2 * m;
-    a[m] = (c <= i) ? A[s0 + i][s0 + c] : A[s0 + c][s0 + i];
-    x[m] = (i == c) ? make_double2(1.0, 0.0) : make_double2(0.0, 0.0);
-    if (c == 0) colb[i] = a[m];
-    if (c == 1 && i == 1) diag[0] = a[m];
+  for (int i = 0; i < 16; i++) {
+    const C v = A[s0 + c][s0 + (i <= c ? i : 0)];
+    a[i] = isx ? (i == c ? cone<C>() : czero<C>()) : i <= c ? v : czero<C>();
   }
-  if (ih == 0) rowb[c] = x[0];
-  __syncwarp();
   bool ok = true;
-  double2 d = colb[0];
-#pragma unroll 2
-  for (int k = 0; k < 16; k++) {
-    const double d2 = fma(d.x, d.x, d.y * d.y);
-    ok = ok && d2 > 1e-290 && d2 < 1e290;
-    const double rd = rcp_nr(d2);
-    const double2 inv_d = make_double2(d.x * rd, -d.y * rd);
-    const double2 akc = colb[c], xk = rowb[c], an = colb[min(k + 1, 15)], dn = diag[0];
-    double2 aik[8];
-#pragma unroll
-    for (int m = 0; m < 8; m++) aik[m] = colb[ih + 2 * m];
-    __syncwarp();
-    d = csub(dn, cmul(cmul(an, an), inv_d));
-    if (lane == 0) dinv[k] = inv_d;
-    const double2 f = c > k ? cneg(cmul(akc, inv_d)) : inv_d, xf = cneg(cmul(inv_d, xk));
-#pragma unroll
-    for (int m = 0; m < 8; m++) {
-      const int i = ih + 2 * m;
-      double2 u = c > k ? a[m] : make_double2(0.0, 0.0), v = x[m];
-      cfma(u, aik[m], f);
-      cfma(v, aik[m], xf);
-      if (i > k && c >= k) a[m] = u;
-      if (i > k) x[m] = v;
-      if (c == k + 1) colb[i] = a[m];
-      if (i == k + 1) rowb[c] = x[m];
-      if (i == k + 2 && c == k + 2) diag[0] = a[m];
+  auto invert = [&](C d) {
+    if constexpr (f64) {
+      const double d2 = fma(d.x, d.x, d.y * d.y);
+      ok = ok && d2 > 1e-290 && d2 < 1e290;
+      const double rd = rcp_nr(d2);
+      return make_double2(d.x * rd, -d.y * rd);
+    } else {
+      const float d2 = fmaf(d.x, d.x, d.y * d.y);
+      ok = ok && d2 >= 1.17549435e-38f && d2 <= 3.40282347e38f;
+      const float rd = rcp_nr(d2);
+      return make_float2(d.x * rd, -d.y * rd);
     }
-    __syncwarp();
-  }
-  if (!__all_sync(FULL, ok)) return elim16_any(A, Xs, s0, lane, dinv);
+  };
 #pragma unroll
-  for (int m = 0; m < 8; m++) {
-    const int i = ih + 2 * m;
-    if (c <= i) A[s0 + i][s0 + c] = a[m];
-    Xs[i][c] = x[m];
+  for (int k = 0; k < 16; k += 2) {
+    C *row = buf + 64 * ((k >> 1) & 1);
+    store_pair(row + 2 * lane, a[k], a[k + 1]);
+    __syncwarp();
+    // r_i = row[2 i], s_i = row[2 i + 1]: rows k and k + 1 before this step
+    C d0, r1, d1;
+    d0 = row[2 * k];
+    load_pair(row + 2 * k + 2, r1, d1);
+    const C inv0 = invert(d0), l = cmul(r1, inv0);
+    cfma(d1, cneg(r1), l);
+    const C inv1 = invert(d1);
+    if (lane == 0) {
+      dinv[k] = inv0;
+      dinv[k + 1] = inv1;
+    }
+    C t0 = cneg(cmul(a[k], inv0));
+    cfma(a[k + 1], r1, t0);
+    const C t1 = cneg(cmul(a[k + 1], inv1));
+    cfma(t0, cneg(l), t1);  // r_i t0 + (s_i - l r_i) t1 = r_i (t0 - l t1) + s_i t1
+#pragma unroll
+    for (int i = k + 2; i < 16; i++) {
+      C r, s;
+      load_pair(row + 2 * i, r, s);
+      cfma(a[i], r, t0);
+      cfma(a[i], s, t1);
+    }
+  }
+  if (!__all_sync(0xffffffffu, ok)) {
+    if constexpr (f64) return elim16_any(A, Xs, s0, lane, dinv);
+    return false;
+  }
+  __syncwarp();  // dinv
+#pragma unroll
+  for (int i = 0; i < 16; i++) {
+    if (isx) Xs[i][c] = a[i];
+    else if (i <= c) A[s0 + c][s0 + i] = i < c ? cmul(a[i], dinv[i]) : a[i];
   }
   return true;
 }
@@ -355,7 +324,7 @@ __device__ __forceinline__ void zmma(double (&cr)[2], double (&ci)[2], double2 a
 // fragments (8 rows x 4 columns of 16 bytes without bank conflicts).
 template <class C> struct DiagSmem {
   static constexpr int LD = sizeof(C) == 16 ? 68 : 65;
-  static constexpr size_t bytes = sizeof(C) * (2 * 64 * LD + 64 * 17 + 4 * 16 * 17 + 16) + 16;
+  static constexpr size_t bytes = sizeof(C) * (2 * 64 * LD + 64 * 17 + 4 * 16 * 17 + 32) + 16;
   C (*A)[LD];
   C (*Wp)[17];
   C (*Xd)[16][17];
@@ -369,118 +338,25 @@ template <class C> struct DiagSmem {
     Xd = reinterpret_cast<C(*)[16][17]>(p + 64 * LD + 64 * 17);
     LI = reinterpret_cast<C(*)[LD]>(p + 64 * LD + 64 * 17 + 4 * 16 * 17);
     dinv = p + 2 * 64 * LD + 64 * 17 + 4 * 16 * 17;
-    bad = reinterpret_cast<int *>(dinv + 16);
+    bad = reinterpret_cast<int *>(dinv + 32);
   }
 };
 
-// Blocked factorisation of a 64 x 64 diagonal tile: four 16-wide sub-panels;
-// warp 0 eliminates the 16 x 16 diagonal sub-block in registers (elim16_warp,
-// which also forms its unit-lower inverse), then the CTA computes the sub-panel
-// below it and the trailing update (complex64: up to three rows, four columns
-// per thread; complex128: 8 x 8 tiles of matrix instructions per warp).  The
-// 64 x 64 inverse is assembled from the four 16 x 16 inverses by recursive
-// doubling (16-wide pairs, then the 32-wide halves), each phase a small product
-// with several independent sums per thread.  Rows and columns at or beyond b
-// are padded with the identity (D = 1, L = 0).
-constexpr size_t DIAG_BLOCKED_SMEM = DiagSmem<float2>::bytes;
-
-// The diagonal tile as the blocked factorisation expects it in shared memory:
-// lower triangle of F at (j, j), zeros above, identity padding beyond b.
-__device__ __forceinline__ void diag_tile_load(int64_t N, int64_t j, int b, const float2 *__restrict__ F,
-                                               float2 (*A)[65]) {
-  const int t = threadIdx.x;
-  float2 v[16];
-#pragma unroll
-  for (int m = 0; m < 16; m++) {
-    const int e = t + 256 * m, i = e >> 6, c = e & 63;
-    v[m] = make_float2(0.f, 0.f);
-    if (i < b && c < b) {
-      if (c <= i) v[m] = __ldcg(F + (j + i) * N + j + c);
-    } else if (i == c) {
-      v[m] = make_float2(1.f, 0.f);
-    }
-  }
-#pragma unroll
-  for (int m = 0; m < 16; m++) {
-    const int e = t + 256 * m;
-    A[e >> 6][e & 63] = v[m];
-  }
-}
-
-// The panel step's update of the next diagonal tile, applied to the tile in
-// shared memory: A[r][c] -= sum_{k<K} W[j + r][woff + k] F[j + c][jcol + k]
-// for c <= r < b (the same products and order as ldlt_tile_update).  The K
-// chunks of 16 are staged in two buffers (the space of the inverse, unused
-// until the end of the factorisation), the next chunk's loads in flight while
-// the current one is multiplied.
-__device__ __forceinline__ void diag_tile_update_smem(int64_t N, int64_t j, int b, int64_t jcol, int K,
-                                                      const float2 *__restrict__ F, const float2 *__restrict__ W,
-                                                      int wstride, int woff, float2 (*A)[65],
-                                                      float2 (*St)[16][65]) {
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  float2 acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int jj = 0; jj < 4; jj++) acc[i][jj] = make_float2(0.f, 0.f);
-  const int nch = (K + 15) / 16;
-  float2 rw[4], rl[4];
-  auto fetch = [&](int k0) {
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int e = threadIdx.x + 256 * q, kk = e & 15, rr = e >> 4;
-      const bool ok = rr < b && k0 + kk < K;
-      rw[q] = ok ? __ldcg(W + (j + rr) * wstride + woff + k0 + kk) : make_float2(0.f, 0.f);
-      rl[q] = ok ? __ldcg(F + (j + rr) * N + jcol + k0 + kk) : make_float2(0.f, 0.f);
-    }
-  };
-  auto stage = [&](int buf) {
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int e = threadIdx.x + 256 * q, kk = e & 15, rr = e >> 4;
-      St[2 * buf][kk][rr] = rw[q];
-      St[2 * buf + 1][kk][rr] = rl[q];
-    }
-  };
-  fetch(0);
-  stage(0);
-  __syncthreads();
-  for (int c = 0; c < nch; c++) {
-    if (c + 1 < nch) fetch(16 * (c + 1));
-    const int buf = c & 1;
-#pragma unroll
-    for (int kk = 0; kk < 16; kk++) {
-      float2 a[4], l[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) a[i] = St[2 * buf][kk][ty + 16 * i];
-#pragma unroll
-      for (int jj = 0; jj < 4; jj++) l[jj] = St[2 * buf + 1][kk][tx + 16 * jj];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int jj = 0; jj < 4; jj++) cfma(acc[i][jj], a[i], l[jj]);
-    }
-    if (c + 1 < nch) stage(buf ^ 1);
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int jj = 0; jj < 4; jj++) {
-      const int r = ty + 16 * i, cc = tx + 16 * jj;
-      if (r < b && cc <= r) A[r][cc] = csub(A[r][cc], acc[i][jj]);
-    }
-  __syncthreads();
-}
-
+// Blocked factorisation of a 64 x 64 diagonal tile: four 16-wide sub-panels.
+// Warp 0 eliminates the 16 x 16 diagonal sub-block in registers (elim16_warp,
+// which also forms its unit-lower inverse X), the CTA forms W = A21 X^T below
+// it, and warp 0 updates the next diagonal sub-block and goes on with it while
+// the other warps store L21 = W D^-1 and update the rest; the products are
+// 8 x 8 tiles of FP64 matrix instructions for both types (complex64 on FP32 units
+// took twice as long).  Rows and columns at or beyond b are padded with the
+// identity (D = 1, L = 0).
 // Phase 1 of the blocked factorisation: L and D of the diagonal tile (in
-// shared memory, written back to F) and the unit-lower inverses Xd of its
-// four 16 x 16 diagonal blocks.  loaded: the tile is already in shared memory
-// (diag_tile_load, possibly updated by diag_tile_update_smem).  Returns false
+// shared memory: lower triangle, identity padding; written back to F) and the
+// unit-lower inverses Xd of its four 16 x 16 diagonal blocks.  Returns false
 // after a breakdown (uniform).
 template <class C>
 __device__ bool ldlt_diag_phase1(int64_t N, int64_t j, int b, C *__restrict__ F, unsigned *__restrict__ err,
-                                 unsigned char *smem, bool loaded) {
+                                 unsigned char *smem) {
   DiagSmem<C> sm(smem);
   auto A = sm.A;
   auto Wp = sm.Wp;
@@ -488,131 +364,66 @@ __device__ bool ldlt_diag_phase1(int64_t N, int64_t j, int b, C *__restrict__ F,
   C *dinv = sm.dinv;
   volatile int *bad = sm.bad;
   const int t = threadIdx.x;  // 256 threads
-  if (!loaded) {
-    C v[16];
-#pragma unroll
-    for (int m = 0; m < 16; m++) {
-      const int e = t + 256 * m, i = e >> 6, c = e & 63;
-      v[m] = czero<C>();
-      if (i < b && c < b) {
-        if (c <= i) v[m] = F[(j + i) * N + j + c];
-      } else if (i == c) {
-        v[m] = cone<C>();
-      }
-    }
-#pragma unroll
-    for (int m = 0; m < 16; m++) {
-      const int e = t + 256 * m;
-      A[e >> 6][e & 63] = v[m];
-    }
-  }
   if (t == 0) *bad = 0;
   __syncthreads();
-  for (int s = 0; s < 4; s++) {
+  const int warp = t >> 5, l4 = t & 3, l8 = (t & 31) >> 2;
+  for (int s = 0;; s++) {
     const int s0 = 16 * s;
-    if (t < 32) {
-      if (!elim16_warp(A, Xd[s], s0, t, &Wp[0][0], dinv)) {  // uniform over the warp
-        if (t == 0) {
-          atomicOr(err, 2u);
-          *bad = 1;
+    if (s > 0) {
+      // the step below sub-panel s - 1, whose W has nr rows from s0
+      const int nr = 64 - s0, nt = nr / 8 * (nr / 8 + 1) / 2;
+      const C *dv = dinv + 16 * ((s - 1) & 1);
+      // tile q of the lower tiles of A22 (row by row) -= W (W D^-1)^T
+      auto update = [&](int q) {
+        int ti = 0, tj = q;
+        while (tj > ti) tj -= ++ti;
+        const int r = s0 + 8 * ti, cc = s0 + 8 * tj;
+        double ur[2] = {0.0, 0.0}, ui[2] = {0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < 16; k += 4)
+          zmma(ur, ui, to_d2(Wp[r + l8][k + l4]), to_d2(cmul(Wp[cc + l8][k + l4], dv[k + l4])));
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          C &v = A[r + l8][cc + 2 * l4 + u];
+          store_c(&v, csub(to_d2(v), make_double2(ur[u], ui[u])));
         }
+      };
+      if (warp != 0)
+        for (int e = t - 32; e < nr * 16; e += 224) {
+          const int r = s0 + (e >> 4), c = e & 15;
+          const C l = cmul(Wp[r][c], dv[c]);
+          A[r][s0 - 16 + c] = l;
+          if (r < b && s0 - 16 + c < b) F[(j + r) * N + j + s0 - 16 + c] = l;
+        }
+#pragma unroll 1
+      for (int q = warp == 0 ? 0 : 2 + warp; q < (warp == 0 ? 3 : nt); q += warp == 0 ? 1 : 7) update(q);
+    }
+    if (warp == 0) {
+      __syncwarp();
+      // its exchange rows in Wp are above those of W
+      if (!elim16_warp(A, Xd[s], s0, t, &Wp[0][0], dinv + 16 * (s & 1)) && t == 0) {
+        atomicOr(err, 2u);
+        *bad = 1;
       }
     }
     __syncthreads();
     if (*bad) return false;  // uniform
     if (s == 3) break;
-    const int nr = 48 - s0;
-    if constexpr (sizeof(C) == 16) {
-      // FP64 matrix instructions on 8 x 8 tiles: W = A21 X^T (12, 8 or 4
-      // tiles), L21 = W / D, then the lower tiles of A22 -= W L21^T (21, 10
-      // or 3); a warp takes every eighth tile
-      const int warp = t >> 5, l4 = t & 3, l8 = (t & 31) >> 2, n8 = nr / 8;
-      for (int q = warp; q < 2 * n8; q += 8) {
-        const int r = s0 + 16 + 8 * (q >> 1), cj = 8 * (q & 1);
-        double wr[2] = {0.0, 0.0}, wi[2] = {0.0, 0.0};
+    // W = A21 X^T: 12, 8 or 4 tiles, a warp takes every eighth
+    for (int q = warp; q < 2 * (6 - 2 * s); q += 8) {
+      const int r = s0 + 16 + 8 * (q >> 1), cj = 8 * (q & 1);
+      double wr[2] = {0.0, 0.0}, wi[2] = {0.0, 0.0};
 #pragma unroll
-        for (int k = 0; k < 16; k += 4)
-          if (k < cj + 8) zmma(wr, wi, A[r + l8][s0 + k + l4], Xd[s][cj + l8][k + l4]);
+      for (int k = 0; k < 16; k += 4)
+        if (k < cj + 8) zmma(wr, wi, to_d2(A[r + l8][s0 + k + l4]), to_d2(Xd[s][cj + l8][k + l4]));
 #pragma unroll
-        for (int u = 0; u < 2; u++) Wp[r + l8][cj + 2 * l4 + u] = make_double2(wr[u], wi[u]);
-      }
-      __syncthreads();
-      for (int e = t; e < nr * 16; e += blockDim.x) {
-        const int r = s0 + 16 + (e >> 4), c = e & 15;
-        A[r][s0 + c] = cmul(Wp[r][c], dinv[c]);
-      }
-      __syncthreads();
-      for (int q = warp; q < n8 * (n8 + 1) / 2; q += 8) {
-        int ti = 0, tj = q;
-        while (tj > ti) tj -= ++ti;  // tile (ti, tj), row by row of the lower triangle
-        const int r = s0 + 16 + 8 * ti, cc = s0 + 16 + 8 * tj;
-        double ur[2] = {0.0, 0.0}, ui[2] = {0.0, 0.0};
-#pragma unroll
-        for (int k = 0; k < 16; k += 4) zmma(ur, ui, Wp[r + l8][k + l4], A[cc + l8][s0 + k + l4]);
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-          C &v = A[r + l8][cc + 2 * l4 + u];
-          v = csub(v, make_double2(ur[u], ui[u]));
-        }
-      }
-      __syncthreads();
-      continue;
-    }
-    // 1 / D of the 16 pivots; sub-panel W = A21 X^T with up to three outputs
-    // per thread accumulated together
-    if (t < 16) {
-      dinv[t] = pivot_inverse(A[s0 + t][s0 + t]);
-    }
-    {
-      C acc[3];
-      int rr[3];
-      const int c = t & 15;
-#pragma unroll
-      for (int u = 0; u < 3; u++) {
-        acc[u] = czero<C>();
-        rr[u] = s0 + 16 + (t >> 4) + 16 * u;
-      }
-#pragma unroll
-      for (int k = 0; k < 16; k++) {
-        if (k <= c) {
-          const C xk = Xd[s][c][k];
-#pragma unroll
-          for (int u = 0; u < 3; u++)
-            if (rr[u] < 64) cfma(acc[u], A[rr[u]][s0 + k], xk);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 3; u++)
-        if (rr[u] < 64) Wp[rr[u]][c] = acc[u];
+      for (int u = 0; u < 2; u++) store_c(&Wp[r + l8][cj + 2 * l4 + u], make_double2(wr[u], wi[u]));
     }
     __syncthreads();
-    for (int e = t; e < nr * 16; e += blockDim.x) {
-      const int r = s0 + 16 + (e >> 4), c = e & 15;
-      A[r][s0 + c] = cmul(Wp[r][c], dinv[c]);
-    }
-    __syncthreads();
-    // trailing update A22 -= W L21^T on the lower part: thread -> (row, 4 columns)
-    {
-      const int ncq = (nr + 3) / 4;  // column quads
-      for (int e = t; e < nr * ncq; e += blockDim.x) {
-        const int i = s0 + 16 + e / ncq, j0 = s0 + 16 + 4 * (e % ncq);
-        if (j0 > i) continue;
-        C acc[4] = {czero<C>(), czero<C>(), czero<C>(), czero<C>()};
-#pragma unroll
-        for (int k = 0; k < 16; k++) {
-          const C w = Wp[i][k];
-#pragma unroll
-          for (int q = 0; q < 4; q++) cfma(acc[q], w, A[min(j0 + q, 63)][s0 + k]);
-        }
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-          if (j0 + q <= i) A[i][j0 + q] = csub(A[i][j0 + q], acc[q]);
-      }
-    }
-    __syncthreads();
-    }
-  for (int e = t; e < 64 * 64; e += blockDim.x) {
-    const int i = e >> 6, c = e & 63;
+  }
+  // the diagonal 16 x 16 blocks
+  for (int e = t; e < 4 * 256; e += blockDim.x) {
+    const int i = 16 * (e >> 8) + ((e >> 4) & 15), c = 16 * (e >> 8) + (e & 15);
     if (i < b && c <= i) F[(j + i) * N + j + c] = A[i][c];
   }
   return true;
@@ -622,7 +433,7 @@ __device__ bool ldlt_diag_phase1(int64_t N, int64_t j, int b, C *__restrict__ F,
 // by recursive doubling from the four 16 x 16 inverses of phase 1, and its
 // store to Linv.
 template <class C>
-__device__ void ldlt_diag_phase2(C *__restrict__ Linv, unsigned char *smem, bool skip_diag_blocks = false) {
+__device__ void ldlt_diag_phase2(C *__restrict__ Linv, unsigned char *smem) {
   DiagSmem<C> sm(smem);
   auto A = sm.A;
   auto Wp = sm.Wp;
@@ -704,94 +515,10 @@ __device__ void ldlt_diag_phase2(C *__restrict__ Linv, unsigned char *smem, bool
     for (int q = 0; q < 4; q++) LI[32 + r0 + 8 * q][c] = cneg(p[q]);
   }
   __syncthreads();
-  // (skip_diag_blocks: the 16 x 16 diagonal blocks were stored already)
+  // (the 16 x 16 diagonal blocks were stored already)
   for (int e = t; e < 64 * 64; e += blockDim.x)
-    if (!skip_diag_blocks || (e >> 10) != ((e & 63) >> 4)) Linv[e] = LI[e >> 6][e & 63];
+    if ((e >> 10) != ((e & 63) >> 4)) Linv[e] = LI[e >> 6][e & 63];
   __syncthreads();
-}
-
-// Panel rows of the fused step by blocked forward substitution, W L11^T =
-// A21 in four 16-column blocks: T_J = A21_J - sum_{K<J} W_K L_JK^T, then
-// W_J = T_J X_J^T with X_J the inverse of L_JJ (the diagonal 16 x 16 blocks
-// of the tile's inverse, published with L and D before the rest of the
-// inverse exists).  A21 is already in As (ldlt_strip_update_smem); T and W
-// overwrite it in place.  L21 = W D^-1 to F, W to the panel buffer.
-__device__ __forceinline__ void ldlt_panel_rows_blk(int64_t N, int64_t j, int b, int64_t r0,
-                                                    float2 *__restrict__ F, const float2 *__restrict__ Linv,
-                                                    float2 *__restrict__ W, int wstride, int woff,
-                                                    unsigned char *smem_raw) {
-  float2(*As)[NB + 1] = reinterpret_cast<float2(*)[NB + 1]>(smem_raw);
-  float2(*Lb)[NB + 1] = reinterpret_cast<float2(*)[NB + 1]>(smem_raw + sizeof(float2) * NB * (NB + 1));
-  float2 *dinv = reinterpret_cast<float2 *>(smem_raw + 2 * sizeof(float2) * NB * (NB + 1));
-  float2(*X)[16][17] = reinterpret_cast<float2(*)[16][17]>(smem_raw + 2 * sizeof(float2) * NB * (NB + 1) +
-                                                          sizeof(float2) * NB);
-  {
-    float2 v[16], xv[4];
-#pragma unroll
-    for (int m = 0; m < 16; m++) {
-      const int e = threadIdx.x + 256 * m, c = e >> 6, k = e & 63;
-      v[m] = (c < b && k <= c) ? __ldcg(F + (j + c) * N + j + k) : make_float2(0.f, 0.f);
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int e = threadIdx.x + 256 * q, J = e >> 8, i = (e >> 4) & 15, c = e & 15;
-      xv[q] = __ldcg(Linv + (16 * J + i) * NB + 16 * J + c);
-    }
-#pragma unroll
-    for (int m = 0; m < 16; m++) {
-      const int e = threadIdx.x + 256 * m;
-      Lb[e >> 6][e & 63] = v[m];
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int e = threadIdx.x + 256 * q;
-      X[e >> 8][(e >> 4) & 15][e & 15] = xv[q];
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < b) dinv[threadIdx.x] = cdiv(make_float2(1.f, 0.f), Lb[threadIdx.x][threadIdx.x]);
-  const int c = threadIdx.x & 15, rq = threadIdx.x >> 4;  // rows rq + 16 q
-  for (int J = 0; J < 4; J++) {
-    if (16 * J >= b) break;  // uniform
-    float2 tq[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) tq[q] = As[rq + 16 * q][16 * J + c];
-    for (int k = 0; k < 16 * J; k++) {
-      const float2 l = Lb[16 * J + c][k];
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const float2 w = As[rq + 16 * q][k];
-        tq[q].x -= w.x * l.x - w.y * l.y;
-        tq[q].y -= w.x * l.y + w.y * l.x;
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 4; q++) As[rq + 16 * q][16 * J + c] = tq[q];
-    __syncthreads();
-    float2 wq[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
-    for (int k = 0; k < 16; k++) {
-      if (k <= c) {
-        const float2 x = X[J][c][k];
-#pragma unroll
-        for (int q = 0; q < 4; q++) cfma(wq[q], As[rq + 16 * q][16 * J + k], x);
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 4; q++) As[rq + 16 * q][16 * J + c] = wq[q];
-    __syncthreads();
-  }
-  for (int e = threadIdx.x; e < 64 * 64; e += 256) {
-    const int r = e >> 6, cc = e & 63;
-    const int64_t gr = r0 + r;
-    if (gr < N && cc < b) {
-      const float2 w = As[r][cc];
-      W[gr * wstride + woff + cc] = w;
-      F[gr * N + j + cc] = cmul(w, dinv[cc]);
-    }
-  }
 }
 
 // F[r][c] -= sum_{k<K} W[r][woff+k] F[c][jcol+k] on the 64 x 64 tile at
@@ -841,58 +568,6 @@ __device__ __forceinline__ void ldlt_tile_update(int64_t N, int64_t r0, int64_t 
     }
 }
 
-// The panel step's strip update of a column-0 tile (rows r0.., the next
-// panel's columns c0.. = its diagonal block's), kept in shared memory as the
-// A21 tile of the panel rows that follow (As: its first b columns, zeros
-// beyond): the same products as ldlt_tile_update, without the round trip
-// through F.  Ws / Ls staging past the panel's As / Li / dg space.
-template <class C>
-__device__ __forceinline__ void ldlt_strip_update_smem(int64_t N, int64_t r0, int64_t c0, int b, int64_t jcol,
-                                                       int K, const C *__restrict__ F, const C *__restrict__ W,
-                                                       int wstride, int woff, unsigned char *smem_raw) {
-  C(*As)[NB + 1] = reinterpret_cast<C(*)[NB + 1]>(smem_raw);
-  C(*Ws)[65] = reinterpret_cast<C(*)[65]>(smem_raw + 2 * sizeof(C) * NB * (NB + 1) + sizeof(C) * NB);
-  C(*Ls)[65] = reinterpret_cast<C(*)[65]>(smem_raw + 2 * sizeof(C) * NB * (NB + 1) + sizeof(C) * NB +
-                                          sizeof(C) * 16 * 65);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  C acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int jj = 0; jj < 4; jj++) acc[i][jj] = czero<C>();
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-      int kk = e & 15, rr = e >> 4;
-      int64_t r = r0 + rr;
-      bool kin = k0 + kk < K;
-      Ws[kk][rr] = (r < N && kin) ? __ldcg(W + r * wstride + woff + k0 + kk) : czero<C>();
-      Ls[kk][rr] = (rr < b && kin) ? __ldcg(F + (c0 + rr) * N + jcol + k0 + kk) : czero<C>();
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < 16; kk++) {
-      C a[4], l[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) a[i] = Ws[kk][ty + 16 * i];
-#pragma unroll
-      for (int jj = 0; jj < 4; jj++) l[jj] = Ls[kk][tx + 16 * jj];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int jj = 0; jj < 4; jj++) cfma(acc[i][jj], a[i], l[jj]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int jj = 0; jj < 4; jj++) {
-      const int rr = ty + 16 * i, k = tx + 16 * jj;
-      const int64_t r = r0 + rr;
-      As[rr][k] = (r < N && k < b) ? csub(__ldcg(F + r * N + c0 + k), acc[i][jj]) : czero<C>();
-    }
-}
-
 // Trailing update of a complex64 factor on FP32 units (grid.x row tiles, grid.y
 // column tiles from r_lo; tiles entirely above the diagonal exit at once).
 template <class C>
@@ -906,153 +581,10 @@ __global__ void __launch_bounds__(256) k_ldlt_update(int64_t N, int64_t r_lo, in
   ldlt_tile_update<C>(N, r0, c0, c_hi, jcol, K, F, W, wstride, woff, Ws, Ls);
 }
 
-// One panel step inside a 256-wide middle panel (complex64), fused: strip update of the
-// columns [r_lo, c_hi) by the panel at jcol; the CTA holding ticket 0 updates
-// the next diagonal block (tile (0, 0)), factors it and publishes its inverse
-// (sync[1]); every other CTA of column tile 0 then runs the next panel on its
-// own rows (W at woff_next, L21 = W D^-1).  Tickets are drawn in launch order,
-// so the CTA that the others wait for is already running; the wait is bounded
-// (error bit 4 on expiry).
-__global__ void __launch_bounds__(256) k_ldlt_step(int64_t N, int64_t r_lo, int64_t c_hi, int64_t jcol, int K,
-                                                   float2 *__restrict__ F, float2 *__restrict__ W, int wstride, int woff,
-                                                   int woff_next, int nb_next, float2 *__restrict__ Linv_next,
-                                                   unsigned *__restrict__ sync, unsigned *__restrict__ err) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ unsigned s_ticket;
-  __shared__ int s_ok;
-  if (threadIdx.x == 0) s_ticket = atomicAdd(&sync[0], 1u);
-  __syncthreads();
-  const unsigned t = s_ticket;
-  const int nct = (int)((c_hi - r_lo + 63) / 64);
-  const int64_t rt = t / nct;
-  const int ct = (int)(t % nct);
-  const int64_t r0 = r_lo + rt * 64, c0 = r_lo + (int64_t)ct * 64;
-  if (r0 >= N || c0 > r0 + 63) return;
-  float2(*Ws)[65] = reinterpret_cast<float2(*)[65]>(smem_raw);
-  float2(*Ls)[65] = reinterpret_cast<float2(*)[65]>(smem_raw + sizeof(float2) * 16 * 65);
-  if (t == 0) {
-    // the next diagonal tile: loaded once, updated and factored in shared
-    // memory (complex64); the update's K chunks are staged in the space of
-    // the tile's inverse
-    float2(*A)[65] = reinterpret_cast<float2(*)[65]>(smem_raw);
-    float2(*St)[16][65] =
-        reinterpret_cast<float2(*)[16][65]>(smem_raw + sizeof(float2) * (64 * 65 + 64 * 17 + 4 * 16 * 17));
-    diag_tile_load(N, r_lo, nb_next, F, A);
-    diag_tile_update_smem(N, r_lo, nb_next, jcol, K, F, W, wstride, woff, A, St);
-    // L, D and the 16 x 16 diagonal blocks of the inverse are published
-    // first (the panel rows need only them); the rest of the tile's
-    // inverse, for the solves, is formed while the panel rows run
-    const bool ok = ldlt_diag_phase1(N, r_lo, nb_next, F, err, smem_raw, true);
-    if (ok) {
-      float2(*Xd)[16][17] = reinterpret_cast<float2(*)[16][17]>(smem_raw + sizeof(float2) * (64 * 65 + 64 * 17));
-      for (int e = threadIdx.x; e < 4 * 256; e += 256) {
-        const int s = e >> 8, i = (e >> 4) & 15, c = e & 15;
-        Linv_next[(16 * s + i) * NB + 16 * s + c] = Xd[s][i][c];
-      }
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) atomicExch(&sync[1], 1u);
-    if (ok) ldlt_diag_phase2(Linv_next, smem_raw, true);
-    return;
-  }
-  if (ct != 0) {
-    ldlt_tile_update<float2>(N, r0, c0, c_hi, jcol, K, F, W, wstride, woff, Ws, Ls);
-    return;
-  }
-  // column 0: the strip tile is the next panel's A21 tile; it stays in
-  // shared memory for the panel rows after the diagonal block is published
-  ldlt_strip_update_smem<float2>(N, r0, c0, nb_next, jcol, K, F, W, wstride, woff, smem_raw);
-  if (threadIdx.x == 0) {
-    long long it = 0;
-    int ok = 1;
-    while (*((volatile unsigned *)&sync[1]) == 0u) {
-      if (++it > SPIN_LIMIT) {
-        atomicOr(err, 4u);
-        ok = 0;
-        break;
-      }
-      __nanosleep(64);
-    }
-    __threadfence();
-    s_ok = ok;
-  }
-  __syncthreads();
-  if (!s_ok) return;
-  ldlt_panel_rows_blk(N, r_lo, nb_next, r0, F, Linv_next, W, wstride, woff_next, smem_raw);
-}
-
-// The first 64-wide block of a middle panel (complex64), one launch: the
-// CTA holding ticket 0 factors the diagonal tile at j (phase 1), publishes
-// L, D and the 16 x 16 inverse blocks, then forms the rest of the inverse
-// (phase 2); every other CTA loads its 64 rows of the block column, waits for
-// the publication (bounded, error bit 4 on expiry) and runs its panel rows
-// by blocked forward substitution.
-__global__ void __launch_bounds__(256) k_ldlt_first(int64_t N, int64_t j, int b, float2 *__restrict__ F,
-                                                    float2 *__restrict__ Linv, float2 *__restrict__ W, int wstride,
-                                                    int woff, unsigned *__restrict__ sync,
-                                                    unsigned *__restrict__ err) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ unsigned s_ticket;
-  __shared__ int s_ok;
-  if (threadIdx.x == 0) s_ticket = atomicAdd(&sync[0], 1u);
-  __syncthreads();
-  const unsigned t = s_ticket;
-  if (t == 0) {
-    const bool ok = ldlt_diag_phase1(N, j, b, F, err, smem_raw, false);
-    if (ok) {
-      float2(*Xd)[16][17] = reinterpret_cast<float2(*)[16][17]>(smem_raw + sizeof(float2) * (64 * 65 + 64 * 17));
-      for (int e = threadIdx.x; e < 4 * 256; e += 256) {
-        const int s = e >> 8, i = (e >> 4) & 15, c = e & 15;
-        Linv[(16 * s + i) * NB + 16 * s + c] = Xd[s][i][c];
-      }
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) atomicExch(&sync[1], 1u);
-    if (ok) ldlt_diag_phase2(Linv, smem_raw, true);
-    return;
-  }
-  const int64_t r0 = j + b + (int64_t)(t - 1) * NB;
-  if (r0 >= N) return;
-  {
-    float2(*As)[NB + 1] = reinterpret_cast<float2(*)[NB + 1]>(smem_raw);
-    float2 va[16];
-#pragma unroll
-    for (int m = 0; m < 16; m++) {
-      const int e = threadIdx.x + 256 * m, rr = e >> 6, k = e & 63;
-      const int64_t r = r0 + rr;
-      va[m] = (r < N && k < b) ? __ldcg(F + r * N + j + k) : make_float2(0.f, 0.f);
-    }
-#pragma unroll
-    for (int m = 0; m < 16; m++) {
-      const int e = threadIdx.x + 256 * m;
-      As[e >> 6][e & 63] = va[m];
-    }
-  }
-  if (threadIdx.x == 0) {
-    long long it = 0;
-    int ok = 1;
-    while (*((volatile unsigned *)&sync[1]) == 0u) {
-      if (++it > SPIN_LIMIT) {
-        atomicOr(err, 4u);
-        ok = 0;
-        break;
-      }
-      __nanosleep(64);
-    }
-    __threadfence();
-    s_ok = ok;
-  }
-  __syncthreads();
-  if (!s_ok) return;
-  ldlt_panel_rows_blk(N, j, b, r0, F, Linv, W, wstride, woff, smem_raw);
-}
-
 // ---------------------------------------------------------------------------
-// A 256-wide middle panel of a complex128 factor in one launch, driven by data
-// flow.  The CTA that draws ticket r owns the 64-row tile r (rows J + 64 r ..)
-// of the panel's four 64-wide block columns s:
+// A 256-wide middle panel in one launch, driven by data flow.  The CTA that
+// draws ticket r owns the 64-row tile r (rows J + 64 r ..) of the panel's four
+// 64-wide block columns s:
 //   * r > s: T = A_rs - sum_{q<s} W_rq L_sq^T as soon as tile s has published
 //     its L_sq; then, once tile s has published its factored diagonal block,
 //     W_rs L_ss^T = T by forward substitution with the inverses of the 16 x 16
@@ -1064,12 +596,16 @@ __global__ void __launch_bounds__(256) k_ldlt_first(int64_t N, int64_t j, int b,
 // one 64 x 64 x 64 update on a single SM; everything else runs while others
 // wait.  Tickets are drawn in launch order and a CTA waits only for tiles 0-3,
 // which started before it; the waits are bounded (error bit 4).
-// The products are FP64 matrix instructions (mma.sync m8n8k4, full FP64
-// multiply-adds; 37.0 TFLOP/s measured against 33.1 for FMA), which leave the
-// shared-memory pipe idle enough to sit at the FP64 rate with eight warps.
-// Measured: 220 us a panel of 7,680 rows; before, a launch with the 64-column
-// strip update and the next diagonal block (105-130 us) and one with its panel
-// rows (17-28 us) per 64 columns.
+// The complex128 products are FP64 matrix instructions (mma.sync m8n8k4, full
+// FP64 multiply-adds; 37.0 TFLOP/s measured against 33.1 for FMA), which leave
+// the shared-memory pipe idle enough to sit at the FP64 rate with eight warps;
+// the complex64 ones FP32 FMAs.
+// Measured, complex128: 160 us a panel of 1,825 rows (200 us with the block
+// elimination on selects and two barriers a pivot; before, a launch with the
+// 64-column strip update and the next diagonal block, 105-130 us, and one with
+// its panel rows, 17-28 us, per 64 columns).  complex64: 184 us a panel on average
+// over a matrix of 4,693 rows with the updates beside it (220 us with the former
+// elimination and trailing updates on FP32 units; as much in launches per 64 columns).
 // ---------------------------------------------------------------------------
 // spin until *flag is set (one thread); false on expiry
 __device__ __forceinline__ bool wait_word(volatile unsigned *flag, unsigned *err) {
@@ -1087,22 +623,223 @@ __device__ __forceinline__ bool wait_word(volatile unsigned *flag, unsigned *err
 
 constexpr int MID_WORDS = 24;  // per middle panel: ticket, diagonal flags [4], row flags [4][4]
 
-__global__ void __launch_bounds__(256, 1) k_ldlt_mid64(int64_t N, int64_t J, int w, double2 *__restrict__ F,
-                                                       double2 *__restrict__ Linv, double2 *__restrict__ W,
-                                                       int wstride, unsigned *sync, unsigned *err) {
+// The CTA's share-out of a 64 x 64 product acc += A B^T (A, B rows in shared
+// memory, K = 64).  complex128: a warp has 2 x 4 8 x 8 matrix-instruction tiles
+// (rows 16 (warp / 2), columns 32 (warp % 2)); complex64: a thread has rows ty +
+// 16 i, columns tx + 16 j on FP32 FMAs.  LOWER: only the lower triangle is
+// wanted -- complex64 skips the blocks j > i, complex128 deals the 36 lower
+// tiles out as warp v < 4: row tile 7 - v, columns 0-4; warp 4 + v: the rest of
+// that row tile and row tile v (nine tiles per SM quarter).
+template <class C, bool LOWER> struct MidAcc;
+
+template <bool LOWER> struct MidAcc<double2, LOWER> {
+  static constexpr int NT = LOWER ? 5 : 8;
+  double re[NT][2], im[NT][2];
+  int l4, l8, ti[NT], tj[NT], nt;
+  __device__ MidAcc() {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    l4 = lane & 3;
+    l8 = lane >> 2;
+    nt = LOWER && warp >= 4 ? 4 : NT;
+#pragma unroll
+    for (int x = 0; x < NT; x++) {
+      re[x][0] = re[x][1] = im[x][0] = im[x][1] = 0.0;
+      const int v = warp & 3;
+      if (!LOWER) {
+        ti[x] = 2 * (warp >> 1) + x / 4;
+        tj[x] = 4 * (warp & 1) + x % 4;
+      } else if (warp < 4) {
+        ti[x] = 7 - v;
+        tj[x] = x;
+      } else {
+        ti[x] = x < 3 - v ? 7 - v : v;
+        tj[x] = x < 3 - v ? 5 + x : x - (3 - v);
+      }
+    }
+  }
+  template <int LD> __device__ void mul(const double2 (*A)[LD], const double2 (*B)[LD]) {
+    if constexpr (LOWER) {
+#pragma unroll 4
+      for (int k = 0; k < 64; k += 4)
+#pragma unroll
+        for (int x = 0; x < NT; x++)
+          if (x < nt) zmma(re[x], im[x], A[8 * ti[x] + l8][k + l4], B[8 * tj[x] + l8][k + l4]);
+    } else {
+#pragma unroll 4
+      for (int k = 0; k < 64; k += 4) {
+        double2 a[2], b[4];
+#pragma unroll
+        for (int i = 0; i < 2; i++) a[i] = A[8 * ti[4 * i] + l8][k + l4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) b[j] = B[8 * tj[j] + l8][k + l4];
+#pragma unroll
+        for (int x = 0; x < 8; x++) zmma(re[x], im[x], a[x / 4], b[x % 4]);
+      }
+    }
+  }
+  // g(row, column, index) for every element; get / set by index
+  template <class G> __device__ void each(G g) {
+#pragma unroll
+    for (int x = 0; x < NT; x++)
+      if (x < nt) {
+#pragma unroll
+        for (int u = 0; u < 2; u++) g(8 * ti[x] + l8, 8 * tj[x] + 2 * l4 + u, 2 * x + u);
+      }
+  }
+  __device__ double2 get(int e) const { return make_double2(re[e >> 1][e & 1], im[e >> 1][e & 1]); }
+  __device__ void set(int e, double2 v) {
+    re[e >> 1][e & 1] = v.x;
+    im[e >> 1][e & 1] = v.y;
+  }
+};
+
+template <bool LOWER> struct MidAcc<float2, LOWER> {
+  float2 acc[4][4];
+  int tx, ty;
+  __device__ MidAcc() {
+    tx = threadIdx.x & 15;
+    ty = threadIdx.x >> 4;
+#pragma unroll
+    for (int e = 0; e < 16; e++) acc[e >> 2][e & 3] = make_float2(0.f, 0.f);
+  }
+  template <int LD> __device__ void mul(const float2 (*A)[LD], const float2 (*B)[LD]) {
+#pragma unroll 8
+    for (int k = 0; k < 64; k++) {
+      float2 a[4], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) a[i] = A[ty + 16 * i][k];
+#pragma unroll
+      for (int j = 0; j < 4; j++) b[j] = B[tx + 16 * j][k];
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          if (!LOWER || j <= i) cfma(acc[i][j], a[i], b[j]);
+    }
+  }
+  template <class G> __device__ void each(G g) {
+#pragma unroll
+    for (int e = 0; e < 16; e++)
+      if (!LOWER || (e & 3) <= (e >> 2)) g(ty + 16 * (e >> 2), tx + 16 * (e & 3), e);
+  }
+  __device__ float2 get(int e) const { return acc[e >> 2][e & 3]; }
+  __device__ void set(int e, float2 v) { acc[e >> 2][e & 3] = v; }
+};
+
+// W L^T = T in place for the 8 rows Tw of a warp, 16 columns q at a time: T_q -=
+// sum_{k < 16 q} W_k L_qk^T, W_q = T_q X_q^T (L: the diagonal tile, X: the
+// inverses of its 16 x 16 diagonal blocks); columns at or beyond b are skipped
+template <int LD>
+__device__ __forceinline__ void mid_substitute(double2 (*Tw)[LD], const double2 (*L)[LD], const double2 (*X)[16][17],
+                                               int b) {
+  const int lane = threadIdx.x & 31, l4 = lane & 3, l8 = lane >> 2;
+#pragma unroll 1
+  for (int q = 0; q < 4; q++) {
+    if (16 * q >= b) break;  // uniform
+    double tr[2][2], ti[2][2];
+    if (q > 0) {
+#pragma unroll
+      for (int n = 0; n < 2; n++)
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const double2 v = Tw[l8][16 * q + 8 * n + 2 * l4 + u];
+          tr[n][u] = v.x;
+          ti[n][u] = v.y;
+        }
+      for (int k = 0; k < 16 * q; k += 4) {
+        const double2 a = cneg(Tw[l8][k + l4]);
+#pragma unroll
+        for (int n = 0; n < 2; n++) zmma(tr[n], ti[n], a, L[16 * q + 8 * n + l8][k + l4]);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int n = 0; n < 2; n++)
+#pragma unroll
+        for (int u = 0; u < 2; u++) Tw[l8][16 * q + 8 * n + 2 * l4 + u] = make_double2(tr[n][u], ti[n][u]);
+      __syncwarp();
+    }
+#pragma unroll
+    for (int n = 0; n < 2; n++) tr[n][0] = tr[n][1] = ti[n][0] = ti[n][1] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 16; k += 4) {
+      const double2 a = Tw[l8][16 * q + k + l4];
+#pragma unroll
+      for (int n = 0; n < 2; n++)
+        if (k < 8 * n + 8) zmma(tr[n], ti[n], a, X[q][8 * n + l8][k + l4]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int n = 0; n < 2; n++)
+#pragma unroll
+      for (int u = 0; u < 2; u++) Tw[l8][16 * q + 8 * n + 2 * l4 + u] = make_double2(tr[n][u], ti[n][u]);
+    __syncwarp();
+  }
+}
+// complex64: a lane has 2 rows x 2 columns of a step's 8 x 16
+template <int LD>
+__device__ __forceinline__ void mid_substitute(float2 (*Tw)[LD], const float2 (*L)[LD], const float2 (*X)[16][17],
+                                               int b) {
+  const int lane = threadIdx.x & 31, r = 2 * (lane >> 3), c = 2 * (lane & 7);
+#pragma unroll 1
+  for (int q = 0; q < 4; q++) {
+    if (16 * q >= b) break;  // uniform
+    float2 t[2][2];
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+      for (int v = 0; v < 2; v++) t[u][v] = Tw[r + u][16 * q + c + v];
+#pragma unroll 8
+    for (int k = 0; k < 16 * q; k++) {
+      const float2 w0 = cneg(Tw[r][k]), w1 = cneg(Tw[r + 1][k]), l0 = L[16 * q + c][k], l1 = L[16 * q + c + 1][k];
+      cfma(t[0][0], w0, l0);
+      cfma(t[0][1], w0, l1);
+      cfma(t[1][0], w1, l0);
+      cfma(t[1][1], w1, l1);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+      for (int v = 0; v < 2; v++) {
+        Tw[r + u][16 * q + c + v] = t[u][v];
+        t[u][v] = make_float2(0.f, 0.f);
+      }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 16; k++) {  // X is lower triangular with zeros above
+      const float2 w0 = Tw[r][16 * q + k], w1 = Tw[r + 1][16 * q + k], x0 = X[q][c][k], x1 = X[q][c + 1][k];
+      cfma(t[0][0], w0, x0);
+      cfma(t[0][1], w0, x1);
+      cfma(t[1][0], w1, x0);
+      cfma(t[1][1], w1, x1);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+      for (int v = 0; v < 2; v++) Tw[r + u][16 * q + c + v] = t[u][v];
+    __syncwarp();
+  }
+}
+
+template <class C>
+__global__ void __launch_bounds__(256, sizeof(C) == 16 ? 1 : 2) k_ldlt_mid(int64_t N, int64_t J, int w, C *__restrict__ F,
+                                                                           C *__restrict__ Linv, C *__restrict__ W,
+                                                                           int wstride, unsigned *sync,
+                                                                           unsigned *err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned s_ticket;
   __shared__ int s_ok;
-  constexpr int LD = DiagSmem<double2>::LD;
-  DiagSmem<double2> sm(smem_raw);
-  double2(*As)[LD] = sm.A;
-  double2(*Ls)[LD] = sm.LI;
-  double2 *dinv = &sm.Wp[0][0];  // 64 reciprocal pivots
+  constexpr int LD = DiagSmem<C>::LD;
+  DiagSmem<C> sm(smem_raw);
+  C(*As)[LD] = sm.A;
+  C(*Ls)[LD] = sm.LI;
+  C *dinv = &sm.Wp[0][0];  // 64 reciprocal pivots
   unsigned *diag_flag = sync + 1, *row_flag = sync + 5;
   if (threadIdx.x == 0) s_ticket = atomicAdd(sync, 1u);
   __syncthreads();
   const int rt = (int)s_ticket;
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, l4 = lane & 3, l8 = lane >> 2;
+  const int t = threadIdx.x, warp = t >> 5;
   const int nsb = (w + 63) / 64;
   const int64_t r0 = J + 64 * (int64_t)rt;
   const int nr = (int)min((int64_t)64, N - r0);
@@ -1120,12 +857,12 @@ __global__ void __launch_bounds__(256, 1) k_ldlt_mid64(int64_t N, int64_t J, int
     if (t == 0) atomicExch(flag, 1u);
   };
   // T[64][LD] <- G rows (row r at G + r ld), zero outside nrow x ncol
-  auto stage = [&](double2(*T)[LD], const double2 *G, int64_t ld, int nrow, int ncol) {
-    double2 v[16];
+  auto stage = [&](C(*T)[LD], const C *G, int64_t ld, int nrow, int ncol) {
+    C v[16];
 #pragma unroll
     for (int m = 0; m < 16; m++) {
       const int e = t + 256 * m, i = e >> 6, c = e & 63;
-      v[m] = (i < nrow && c < ncol) ? __ldcg(G + i * ld + c) : make_double2(0.0, 0.0);
+      v[m] = (i < nrow && c < ncol) ? __ldcg(G + i * ld + c) : czero<C>();
     }
 #pragma unroll
     for (int m = 0; m < 16; m++) {
@@ -1133,8 +870,6 @@ __global__ void __launch_bounds__(256, 1) k_ldlt_mid64(int64_t N, int64_t J, int
       T[e >> 6][e & 63] = v[m];
     }
   };
-  // rows 16 (warp / 2) .., columns 32 (warp % 2) .. of a 64 x 64 product
-  const int wr = 16 * (warp >> 1), wc = 32 * (warp & 1);
   for (int s = 0; s < nsb && s <= rt; s++) {
     const int64_t jc = J + 64 * s;
     const int b = (int)min((int64_t)64, J + w - jc);
@@ -1146,59 +881,36 @@ __global__ void __launch_bounds__(256, 1) k_ldlt_mid64(int64_t N, int64_t J, int
       }
       for (int e = t; e < 64 * 64; e += 256) {  // lower part, identity beyond b
         const int i = e >> 6, c = e & 63;
-        if (i >= b || c >= b) As[i][c] = make_double2(i == c ? 1.0 : 0.0, 0.0);
-        else if (c > i) As[i][c] = make_double2(0.0, 0.0);
+        if (i >= b || c >= b) As[i][c] = i == c ? cone<C>() : czero<C>();
+        else if (c > i) As[i][c] = czero<C>();
       }
-      double2 *Lb = Linv + (jc / 64) * 4096;
-      const bool ok = ldlt_diag_phase1(N, jc, b, F, err, smem_raw, true);
+      C *Lb = Linv + (jc / 64) * 4096;
+      const bool ok = ldlt_diag_phase1<C>(N, jc, b, F, err, smem_raw);
       if (ok)
         for (int e = t; e < 4 * 256; e += 256) {
           const int q = e >> 8, i = (e >> 4) & 15, c = e & 15;
           Lb[(16 * q + i) * 64 + 16 * q + c] = sm.Xd[q][i][c];
         }
       publish(diag_flag + s);
-      if (ok) ldlt_diag_phase2(Lb, smem_raw, true);
+      if (ok) ldlt_diag_phase2<C>(Lb, smem_raw);
       return;
     }
     // acc = -A_rs + sum_q W_rq L_sq^T
-    double cr[2][4][2], ci[2][4][2];
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-          const int rr = wr + 8 * i + l8, cc = wc + 8 * j + 2 * l4 + u;
-          const double2 v = (rr < nr && cc < b) ? __ldcg(F + (r0 + rr) * N + jc + cc) : make_double2(0.0, 0.0);
-          cr[i][j][u] = -v.x;
-          ci[i][j][u] = -v.y;
-        }
-    for (int q = 0; q < s; q++) {
-      if (!wait(row_flag + 4 * s + q)) return;
-      stage(As, W + r0 * wstride + 64 * q, wstride, nr, 64);
-      stage(Ls, F + jc * N + J + 64 * q, N, b, 64);
-      __syncthreads();
-#pragma unroll 4
-      for (int k = 0; k < 64; k += 4) {
-        double2 a[2], l[4];
-#pragma unroll
-        for (int i = 0; i < 2; i++) a[i] = As[wr + 8 * i + l8][k + l4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) l[j] = Ls[wc + 8 * j + l8][k + l4];
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-          for (int j = 0; j < 4; j++) zmma(cr[i][j], ci[i][j], a[i], l[j]);
+    {
+      MidAcc<C, false> acc;
+      acc.each([&](int i, int c, int e) {
+        acc.set(e, (i < nr && c < b) ? cneg(__ldcg(F + (r0 + i) * N + jc + c)) : czero<C>());
+      });
+      for (int q = 0; q < s; q++) {
+        if (!wait(row_flag + 4 * s + q)) return;
+        stage(As, W + r0 * wstride + 64 * q, wstride, nr, 64);
+        stage(Ls, F + jc * N + J + 64 * q, N, b, 64);
+        __syncthreads();
+        acc.mul(As, Ls);
+        __syncthreads();
       }
-      __syncthreads();
+      acc.each([&](int i, int c, int e) { As[i][c] = cneg(acc.get(e)); });
     }
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-#pragma unroll
-        for (int u = 0; u < 2; u++)
-          As[wr + 8 * i + l8][wc + 8 * j + 2 * l4 + u] = make_double2(-cr[i][j][u], -ci[i][j][u]);
     if (!wait(diag_flag + s)) return;
     stage(Ls, F + jc * N + jc, N, b, b);
 #pragma unroll
@@ -1208,58 +920,15 @@ __global__ void __launch_bounds__(256, 1) k_ldlt_mid64(int64_t N, int64_t J, int
     }
     __syncthreads();
     if (t < b) dinv[t] = pivot_inverse(Ls[t][t]);
-    // W_rs: 8 rows per warp, 16 columns at a time
-    double2(*Tw)[LD] = As + 8 * warp;
-#pragma unroll 1
-    for (int q = 0; q < 4; q++) {
-      if (16 * q >= b) break;  // uniform
-      double tr[2][2], ti[2][2];
-      if (q > 0) {
-#pragma unroll
-        for (int n = 0; n < 2; n++)
-#pragma unroll
-          for (int u = 0; u < 2; u++) {
-            const double2 v = Tw[l8][16 * q + 8 * n + 2 * l4 + u];
-            tr[n][u] = v.x;
-            ti[n][u] = v.y;
-          }
-        for (int k = 0; k < 16 * q; k += 4) {
-          const double2 a = cneg(Tw[l8][k + l4]);
-#pragma unroll
-          for (int n = 0; n < 2; n++) zmma(tr[n], ti[n], a, Ls[16 * q + 8 * n + l8][k + l4]);
-        }
-        __syncwarp();
-#pragma unroll
-        for (int n = 0; n < 2; n++)
-#pragma unroll
-          for (int u = 0; u < 2; u++)
-            Tw[l8][16 * q + 8 * n + 2 * l4 + u] = make_double2(tr[n][u], ti[n][u]);
-        __syncwarp();
-      }
-#pragma unroll
-      for (int n = 0; n < 2; n++) tr[n][0] = tr[n][1] = ti[n][0] = ti[n][1] = 0.0;
-#pragma unroll
-      for (int k = 0; k < 16; k += 4) {
-        const double2 a = Tw[l8][16 * q + k + l4];
-#pragma unroll
-        for (int n = 0; n < 2; n++)
-          if (k < 8 * n + 8) zmma(tr[n], ti[n], a, sm.Xd[q][8 * n + l8][k + l4]);
-      }
-      __syncwarp();
-#pragma unroll
-      for (int n = 0; n < 2; n++)
-#pragma unroll
-        for (int u = 0; u < 2; u++) Tw[l8][16 * q + 8 * n + 2 * l4 + u] = make_double2(tr[n][u], ti[n][u]);
-      __syncwarp();
-    }
+    mid_substitute(As + 8 * warp, Ls, sm.Xd, b);  // W_rs, 8 rows per warp
     __syncthreads();
     const bool below = rt < nsb;   // tiles of the panel's diagonal part keep L_rs for their own update
     const bool last = rt == s + 1;  // the factorisation of this tile comes next
 #pragma unroll 4
     for (int m = 0; m < 16; m++) {
       const int e = t + 256 * m, i = e >> 6, c = e & 63;
-      const double2 v = c < b ? As[i][c] : make_double2(0.0, 0.0);
-      const double2 l = c < b ? cmul(v, dinv[c]) : make_double2(0.0, 0.0);
+      const C v = c < b ? As[i][c] : czero<C>();
+      const C l = c < b ? cmul(v, dinv[c]) : czero<C>();
       if (i < nr && c < b) {
         W[(r0 + i) * wstride + 64 * s + c] = v;
         F[(r0 + i) * N + jc + c] = l;
@@ -1272,53 +941,22 @@ __global__ void __launch_bounds__(256, 1) k_ldlt_mid64(int64_t N, int64_t J, int
     }
     if (last) __syncthreads();  // published after the update, when the stores have drained
     else publish(row_flag + 4 * rt + s);
-    // the own diagonal tile -= W_rs L_rs^T, 36 lower 8 x 8 tiles: warp v < 4
-    // takes row tile 7 - v, columns 0-4, warp 4 + v the rest of that row tile
-    // and row tile v (nine tiles per SM quarter)
-    {
-      const int v = warp & 3;
-      const int nt = warp < 4 ? 5 : 4;
-      double ur[5][2], ui[5][2];
-      int ti[5], tj[5];
-      double2 fd[5][2];
-#pragma unroll
-      for (int x = 0; x < 5; x++) {
-        ur[x][0] = ur[x][1] = ui[x][0] = ui[x][1] = 0.0;
-        if (warp < 4) {
-          ti[x] = 7 - v;
-          tj[x] = x;
-        } else {
-          ti[x] = x < 3 - v ? 7 - v : v;
-          tj[x] = x < 3 - v ? 5 + x : x - (3 - v);
-        }
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-          const int i = 8 * ti[x] + l8, c = 8 * tj[x] + 2 * l4 + u;
-          fd[x][u] = (x < nt && i < nr && c <= i) ? __ldcg(F + (r0 + i) * N + r0 + c) : make_double2(0.0, 0.0);
-        }
-      }
-#pragma unroll 4
-      for (int k = 0; k < 64; k += 4) {
-#pragma unroll
-        for (int x = 0; x < 5; x++)
-          if (x < nt) zmma(ur[x], ui[x], As[8 * ti[x] + l8][k + l4], Ls[8 * tj[x] + l8][k + l4]);
-      }
-      if (last) publish(row_flag + 4 * rt + s);
-      else __syncthreads();
-#pragma unroll
-      for (int x = 0; x < 5; x++) {
-        if (x >= nt) continue;
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-          const int i = 8 * ti[x] + l8, c = 8 * tj[x] + 2 * l4 + u;
-          if (i >= nr || c > i) continue;
-          const double2 d = csub(fd[x][u], make_double2(ur[x][u], ui[x][u]));
-          if (last) As[i][c] = d;
-          else __stcg(F + (r0 + i) * N + r0 + c, d);
-        }
-      }
-      __syncthreads();
-    }
+    // the own diagonal tile -= W_rs L_rs^T
+    MidAcc<C, true> acc;
+    C fd[sizeof(C) == 16 ? 10 : 16];  // the tile's own elements, by the accumulator's index
+    acc.each([&](int i, int c, int e) {
+      fd[e] = (i < nr && c <= i) ? __ldcg(F + (r0 + i) * N + r0 + c) : czero<C>();
+    });
+    acc.mul(As, Ls);
+    if (last) publish(row_flag + 4 * rt + s);
+    else __syncthreads();
+    acc.each([&](int i, int c, int e) {
+      if (i >= nr || c > i) return;
+      const C d = csub(fd[e], acc.get(e));
+      if (last) As[i][c] = d;
+      else __stcg(F + (r0 + i) * N + r0 + c, d);
+    });
+    __syncthreads();
   }
 }
 
@@ -1336,25 +974,15 @@ __global__ void k_scale_vec(int64_t N, int64_t R, const double2 *__restrict__ d,
   x[i] = cmul(x[i], d[i % N]);
 }
 
-// the complex64 panel steps: panel rows or the diagonal tile
-constexpr size_t STEP_SMEM = std::max(sizeof(float2) * (2 * NB * (NB + 1) + NB), DIAG_BLOCKED_SMEM);
-
 template <class C> void set_smem_attrs() {
   static bool done = false;
   if (done) return;
-  if constexpr (std::is_same<C, float2>::value) {
-    DMB_CUDA(cudaFuncSetAttribute(k_ldlt_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STEP_SMEM));
-    DMB_CUDA(cudaFuncSetAttribute(k_ldlt_first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STEP_SMEM));
-  } else {
-    DMB_CUDA(cudaFuncSetAttribute(k_ldlt_mid64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)DiagSmem<double2>::bytes));
-  }
+  DMB_CUDA(cudaFuncSetAttribute(k_ldlt_mid<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DiagSmem<C>::bytes));
   done = true;
 }
 
 // Three-level right-looking LDL^T.  Block columns of NBW = 1024 are factored
-// as 256-wide middle panels (complex128: one launch; complex64: one launch per
-// 64 columns).  After each middle panel the rest of the 1024-wide block column
+// as 256-wide middle panels (one launch each).  After each middle panel the rest of the 1024-wide block column
 // receives one K = 256 update, and after the block column the whole trailing
 // matrix receives one K = 1024 update -- on the tensor cores (complex64: split
 // operands, complex128: int8 residues).
@@ -1373,11 +1001,8 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
   const int nblk = (int)((N + NB - 1) / NB);
   c->d_W.ensure(sizeof(C) * N * NBW * 2);
   c->d_dinv.ensure(sizeof(C) * (size_t)nblk * NB * NB);  // Linv blocks
-  // err word, then two words (ticket, ready flag) per panel step
-  // (then two more per 64-block for the first block of each middle panel)
-  // (complex128: MID_WORDS per middle panel)
-  const size_t flag_words = 4 + (std::is_same<C, float2>::value ? 4 * (size_t)nblk
-                                                                : MID_WORDS * (size_t)((N + NBO - 1) / NBO));
+  // err word, then the tickets and flags of each middle panel
+  const size_t flag_words = 4 + MID_WORDS * (size_t)((N + NBO - 1) / NBO);
   c->d_flags.ensure(std::max<size_t>(64, 4 * flag_words));
   if (!c->stream2 || !c->stream3) {
     // the panel chain (context stream) first, then the lookahead updates,
@@ -1489,27 +1114,8 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
     const int64_t J2E = std::min<int64_t>(N, J2 + NBW);
     for (int64_t J = J2; J < J2E; J += NBO) {
       const int64_t JE = std::min<int64_t>(J2E, J + NBO);
-      if constexpr (std::is_same<C, double2>::value) {
-        DMB_LAUNCH(c, k_ldlt_mid64, blocks_for(N - J, NB), 256, DiagSmem<double2>::bytes, N, J, (int)(JE - J), F, Linv,
-                   Wb + (J - J2), NBW, step_sync + MID_WORDS * (J / NBO), err);
-      } else {
-        // the first block: factor and panel rows in one launch; then, per
-        // block, the strip update by the previous one, its diagonal tile and
-        // its panel rows
-        for (int64_t j = J; j < JE; j += NB) {
-          const int b = (int)std::min<int64_t>(NB, N - j);
-          C *Lblk = Linv + (j / NB) * NB * NB;
-          if (j == J) {
-            DMB_LAUNCH(c, k_ldlt_first, 1 + blocks_for(N - j - b, NB), 256, STEP_SMEM, N, j, b, F, Lblk, Wb, NBW,
-                       (int)(j - J2), step_sync + 2 * nblk + 2 * (j / NB), err);
-          } else {
-            const int64_t p = j - NB;  // the previous block
-            const dim3 g(blocks_for(N - j, 64), blocks_for(JE - j, 64));
-            DMB_LAUNCH(c, k_ldlt_step, g.x * g.y, 256, STEP_SMEM, N, j, JE, p, NB, F, Wb, NBW, (int)(p - J2),
-                       (int)(j - J2), b, Lblk, step_sync + 2 * (p / NB), err);
-          }
-        }
-      }
+      DMB_LAUNCH(c, k_ldlt_mid<C>, blocks_for(N - J, NB), 256, DiagSmem<C>::bytes, N, J, (int)(JE - J), F, Linv,
+                 Wb + (J - J2), NBW, step_sync + MID_WORDS * (J / NBO), err);
       update_block_column(JE, J2E, J, (int)(JE - J), Wb, (int)(J - J2));
     }
     update_trailing(J2E, J2, (int)(J2E - J2), Wb);
