@@ -1479,219 +1479,238 @@ void prepare_packed_factor(dmb_ctx *c, const float2 *F) {
 //   backward, o = last..0: a_o = y_o / D - L[>o, o]^T x, x_o = X_o^T a_o
 // with X_o the inverse of L's diagonal block.  A CTA owns 16 rows (forward) or
 // columns (backward) of a block: it streams its part of L block by block as the
-// blocks of y (x) are published, publishes its 16 values of a_o, and, once all
-// of a_o is there, its 16 values of X_o a_o.  The next block's part of L and
-// the part of X_o are loaded ahead of the waits, so a block costs two flag round
-// trips and two short on-chip sums; the stream of L runs beside that chain
-// over all SMs.  CTAs take their slices in ticket order and wait only on
-// earlier tickets; every wait is bounded (error bit 4).  All sums in a fixed
-// order.  Bound by the chain, about 6 us a block, up to N = 10,000 and by the
-// read of L above.  (Chains of 64-row blocks on one CTA each took 8 us a block:
-// 1.39 ms a sweep at N = 10,680, complex128.)
+// blocks of y (x) appear, publishes its 16 values of a_o, and, once all of a_o
+// is there, its 16 values of X_o a_o.  The values are their own flags: the
+// buffers are filled with a bit pattern that no published value has (SV_EMPTY),
+// and a thread that needs a value reads it until it is there.  The next block's
+// part of L is loaded ahead of that, the part of X_o at the start, so a block
+// costs two trips through L2 and two short sums; the stream of L runs beside
+// that chain over all SMs.  CTAs take their slices in ticket order and wait only
+// on earlier tickets; every wait is bounded (error bit 4).  All sums in a fixed
+// order.  Bound by the chain up to N = 10,000 and by the read of L above.
+// Measured, both sweeps: complex128 415 us at N = 10,680 (912 MB of L each), 56 us
+// at 1,825; complex64 177 us at 4,693.  With counters as flags (two
+// barriers, a fence and an atomic a hand-over): 640, 95 and 260 us.
 // ---------------------------------------------------------------------------
 constexpr int SV = 256;  // rows per block
 constexpr int SW = 16;   // rows per CTA
+constexpr int SV_LD = SV + 1;
+constexpr unsigned long long SV_EMPTY = ~0ull;  // a NaN; published NaNs are made to differ from it
 
-// wait until *cnt reaches want (thread 0); false on expiry or another CTA's
-__device__ __forceinline__ bool wait_count(volatile unsigned *cnt, unsigned want, unsigned *err, long long limit) {
-  long long it = 0;
-  while (*cnt < want) {
-    if (++it > limit) {
-      atomicOr(err, 4u);
-      return false;
-    }
-    if ((it & 15) == 0) {
-      if (*((volatile unsigned *)err) & 4u) return false;
-      if (it > 64) __nanosleep(20);
+__device__ __forceinline__ void sv_publish(double2 *p, double2 v) {
+  unsigned long long x = __double_as_longlong(v.x), y = __double_as_longlong(v.y);
+  if (x == SV_EMPTY) x = 0x7ff8000000000000ull;
+  if (y == SV_EMPTY) y = 0x7ff8000000000000ull;
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(x), "l"(y) : "memory");
+}
+
+// The n values at p into v[0..255] (zero beyond n), a thread each, as they are
+// published; for the whole CTA, false on expiry or another CTA's.  v is read
+// after, and written before, the next barrier.
+__device__ __forceinline__ bool sv_gather(const double2 *p, int n, double2 *v, int64_t ahead, unsigned *err,
+                                          long long limit) {
+  const int t = threadIdx.x;
+  bool ok = true;
+  unsigned long long x = 0, y = 0;
+  if (t < n) {
+    for (long long it = 0;;) {
+      asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "l"(p + t) : "memory");
+      if (x != SV_EMPTY && y != SV_EMPTY) break;
+      if (++it > limit) {
+        atomicOr(err, 4u);
+        ok = false;
+        break;
+      }
+      if ((it & 15) == 0 && (*((volatile unsigned *)err) & 4u)) {
+        ok = false;
+        break;
+      }
+      // blocks ahead of the chain leave L2 to it
+      if (ahead > 1) __nanosleep(ahead > 3 ? 500 : 100);
+      else if (it > 64) __nanosleep(20);
     }
   }
-  __threadfence();
-  return true;
+  v[t] = make_double2(__longlong_as_double((long long)x), __longlong_as_double((long long)y));
+  return __syncthreads_and(ok);
 }
 
-__device__ __forceinline__ unsigned sweep_slices(int64_t N, int64_t o) {  // CTAs of block o
-  return (unsigned)((min((int64_t)SV, N - o * SV) + SW - 1) / SW);
-}
-
-// Rows r, r + 1 of a warp against the 256 vector values v (lane + 32 j):
-// the matrix values m0, m1 are in registers already
-template <class MC>
-__device__ __forceinline__ void rows2_fma(const MC (&m0)[8], const MC (&m1)[8], const double2 *v, int n, int lane,
-                                          double2 &s0, double2 &s1) {
+// sums of a warp's two rows m (entries lane + 32 j) times v
+__device__ __forceinline__ void rows2_fma(const double2 *m, const double2 *v, int lane, double2 &s0, double2 &s1) {
 #pragma unroll
   for (int j = 0; j < 8; j++) {
-    const double2 y = lane + 32 * j < n ? __ldcg(v + lane + 32 * j) : make_double2(0.0, 0.0);
-    cfma(s0, to_d2(m0[j]), y);
-    cfma(s1, to_d2(m1[j]), y);
+    const double2 y = v[lane + 32 * j];
+    cfma(s0, m[lane + 32 * j], y);
+    cfma(s1, m[SV_LD + lane + 32 * j], y);
   }
 }
 
-// sum of the 16 row groups (threads t with equal t & 15) -> red[0][t & 15]'s
-// total on threads below 16
-__device__ __forceinline__ double2 cols_sum(double2 v, double2 (*red)[SW]) {
-  const int t = threadIdx.x;
-  v.x += __shfl_xor_sync(0xffffffffu, v.x, 16);
-  v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
-  __syncthreads();
-  if ((t & 31) < 16) red[t >> 5][t & 15] = v;
-  __syncthreads();
-  double2 s = make_double2(0.0, 0.0);
-  if (t < 16)
-#pragma unroll
-    for (int g = 0; g < 8; g++) s = cadd(s, red[g][t]);
-  return s;
+__global__ void k_sweep_clear(int64_t n, ulonglong2 *buf, int words, unsigned *err) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < n) buf[e] = make_ulonglong2(SV_EMPTY, SV_EMPTY);
+  if (e < words) err[e] = 0u;
 }
+
+struct SweepSmem {
+  double2 X[SW][SV_LD];  // the CTA's rows of the block inverse (its transpose)
+  double2 v[2][SV];      // blocks in turn
+  double2 red[8][SW];
+};
 
 template <class FC>
 __global__ void __launch_bounds__(256, 2) k_sweep_fwd(int64_t N, const FC *__restrict__ F,
-                                                      const double2 *__restrict__ X, double2 *x, double2 *abuf,
-                                                      unsigned *tickets, unsigned *acnt, unsigned *ycnt, unsigned *err,
+                                                      const double2 *__restrict__ X, const double2 *__restrict__ b,
+                                                      double2 *abuf, double2 *y, unsigned *tickets, unsigned *err,
                                                       long long limit) {
-  __shared__ double2 red[8][SW];
-  __shared__ int s_t, s_ok;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  SweepSmem &sm = *reinterpret_cast<SweepSmem *>(smem_raw);
+  constexpr bool AHEAD = sizeof(FC) == 8;  // room in registers for two blocks of L
+  __shared__ int s_t;
   const int rhs = blockIdx.y, t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const int64_t nblk = (N + SV - 1) / SV;
-  x += rhs * N;
+  b += rhs * N;
   abuf += rhs * N;
-  acnt += rhs * nblk;
-  ycnt += rhs * nblk;
+  y += rhs * N;
   if (t == 0) s_t = (int)atomicAdd(tickets + rhs, 1u);
   __syncthreads();
   const int64_t r0 = (int64_t)s_t * SW, o = r0 / SV, o0 = o * SV;
-  const int i = (int)((r0 - o0) / SW), nr = (int)min((int64_t)SW, N - r0);
-  auto wait = [&](unsigned *cnt, unsigned want) {
-    if (t == 0) s_ok = wait_count(cnt, want, err, limit) ? 1 : 0;
-    __syncthreads();
-    const bool ok = s_ok != 0;
-    __syncthreads();
-    return ok;
-  };
+  const int nr = (int)min((int64_t)SW, N - r0), w = (int)min((int64_t)SV, N - o0);
+  for (int e = t; e < SW * SV; e += 256) {  // the inverse is kept transposed
+    const int c = e & 15, k = e >> 4;
+    sm.X[c][k] = (c < nr && k <= r0 - o0 + c) ? X[(int64_t)k * N + r0 + c] : make_double2(0.0, 0.0);
+  }
   const int64_t ra = r0 + 2 * warp;  // this warp's rows ra, ra + 1
+  const double2 br = lane < 2 && 2 * warp + lane < nr ? b[ra + lane] : make_double2(0.0, 0.0);
   double2 s0 = make_double2(0.0, 0.0), s1 = s0;
-  for (int64_t p = 0; p < o; p++) {
-    FC m0[8], m1[8];
+  auto load = [&](FC(&m)[16], int64_t p) {
+    if (p >= o) return;
 #pragma unroll
     for (int j = 0; j < 8; j++) {
-      m0[j] = ra < N ? F[ra * N + p * SV + lane + 32 * j] : czero<FC>();
-      m1[j] = ra + 1 < N ? F[(ra + 1) * N + p * SV + lane + 32 * j] : czero<FC>();
+      m[j] = ra < N ? F[ra * N + p * SV + lane + 32 * j] : czero<FC>();
+      m[8 + j] = ra + 1 < N ? F[(ra + 1) * N + p * SV + lane + 32 * j] : czero<FC>();
     }
-    if (!wait(ycnt + p, SV / SW)) return;
-    rows2_fma(m0, m1, x + p * SV, SV, lane, s0, s1);
+  };
+  // block p of L, already loaded (complex64: the next one's loads on their way)
+  auto step = [&](FC(&m)[16], FC(&next)[16], int64_t p) {
+    if (AHEAD) load(next, p + 1);
+    else load(m, p);
+    if (!sv_gather(y + p * SV, SV, sm.v[p & 1], o - p, err, limit)) return false;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const double2 yv = sm.v[p & 1][lane + 32 * j];
+      cfma(s0, to_d2(m[j]), yv);
+      cfma(s1, to_d2(m[8 + j]), yv);
+    }
+    return true;
+  };
+  FC ma[16], mb[16];
+  if (AHEAD) load(ma, 0);
+  for (int64_t p = 0; p < o; p += 2) {
+    if (!step(ma, mb, p)) return;
+    if (p + 1 < o && !step(mb, ma, p + 1)) return;
   }
   s0 = warp_sum2(s0);
   s1 = warp_sum2(s1);
-  if (lane < 2 && 2 * warp + lane < nr)
-    __stcg(abuf + ra + lane, csub(x[ra + lane], lane == 0 ? s0 : s1));
-  // X_o: column r0 + c of the inverse's rows, k = g + 16 j <= row
-  const int c = t & 15, g = t >> 4;
-  double2 xv[16];
-#pragma unroll
-  for (int j = 0; j < 16; j++)
-    xv[j] = (j <= i && c < nr) ? X[(int64_t)(g + 16 * j) * N + r0 + c] : make_double2(0.0, 0.0);
-  __syncthreads();
-  if (t == 0) {
-    __threadfence();
-    atomicAdd(acnt + o, 1u);
-  }
-  if (!wait(acnt + o, sweep_slices(N, o))) return;
-  double2 v = make_double2(0.0, 0.0);
-#pragma unroll
-  for (int j = 0; j < 16; j++)
-    if (j <= i && g + 16 * j < N - o0) cfma(v, xv[j], __ldcg(abuf + o0 + g + 16 * j));
-  v = cols_sum(v, red);
-  if (t < nr) __stcg(x + r0 + t, v);
-  __syncthreads();
-  if (t == 0) {
-    __threadfence();
-    atomicAdd(ycnt + o, 1u);
-  }
+  if (lane < 2 && 2 * warp + lane < nr) sv_publish(abuf + ra + lane, csub(br, lane == 0 ? s0 : s1));
+  if (!sv_gather(abuf + o0, w, sm.v[o & 1], 0, err, limit)) return;
+  s0 = s1 = make_double2(0.0, 0.0);
+  rows2_fma(sm.X[2 * warp], sm.v[o & 1], lane, s0, s1);
+  s0 = warp_sum2(s0);
+  s1 = warp_sum2(s1);
+  if (lane < 2 && 2 * warp + lane < nr) sv_publish(y + ra + lane, lane == 0 ? s0 : s1);
 }
 
 template <class FC>
 __global__ void __launch_bounds__(256, 2) k_sweep_bwd(int64_t N, const FC *__restrict__ F,
-                                                      const double2 *__restrict__ X, double2 *x, double2 *abuf,
-                                                      unsigned *tickets, unsigned *acnt, unsigned *xcnt, unsigned *err,
-                                                      long long limit) {
-  __shared__ double2 red[8][SW];
-  __shared__ int s_t, s_ok;
+                                                      const double2 *__restrict__ X, const double2 *__restrict__ y,
+                                                      double2 *abuf, double2 *xbuf, double2 *x, unsigned *tickets,
+                                                      unsigned *err, long long limit) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  SweepSmem &sm = *reinterpret_cast<SweepSmem *>(smem_raw);
+  constexpr bool AHEAD = sizeof(FC) == 8;  // room in registers for two blocks of L
+  __shared__ int s_t;
   const int rhs = blockIdx.y, t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int64_t nblk = (N + SV - 1) / SV;
-  x += rhs * N;
+  y += rhs * N;
   abuf += rhs * N;
-  acnt += rhs * nblk;
-  xcnt += rhs * nblk;
+  xbuf += rhs * N;
+  x += rhs * N;
   if (t == 0) s_t = (int)atomicAdd(tickets + rhs, 1u);
   __syncthreads();
   const int64_t r0 = ((N + SW - 1) / SW - 1 - s_t) * SW, o = r0 / SV, o0 = o * SV;
   const int nr = (int)min((int64_t)SW, N - r0), w = (int)min((int64_t)SV, N - o0);
-  auto wait = [&](unsigned *cnt, unsigned want) {
-    if (t == 0) s_ok = wait_count(cnt, want, err, limit) ? 1 : 0;
-    __syncthreads();
-    const bool ok = s_ok != 0;
-    __syncthreads();
-    return ok;
-  };
+  for (int e = t; e < SW * SV; e += 256) {
+    const int c = e >> 8, k = e & 255;
+    sm.X[c][k] = (c < nr && k >= r0 - o0 + c && k < w) ? X[(r0 - o0 + c) * N + o0 + k] : make_double2(0.0, 0.0);
+  }
+  double2 yd = make_double2(0.0, 0.0);
+  if (t < nr) yd = cdiv(y[r0 + t], to_d2(F[(r0 + t) * N + r0 + t]));
   const int c = t & 15, g = t >> 4;  // column r0 + c, rows g + 16 j of a block
   double2 v = make_double2(0.0, 0.0);
-  for (int64_t p = nblk - 1; p > o; p--) {
+  auto load = [&](FC(&m)[16], int64_t p) {
+    if (p <= o) return;
     const int n = (int)min((int64_t)SV, N - p * SV);
-    FC m[16];
 #pragma unroll
     for (int j = 0; j < 16; j++)
       m[j] = (g + 16 * j < n && c < nr) ? F[(p * SV + g + 16 * j) * N + r0 + c] : czero<FC>();
-    if (!wait(xcnt + p, sweep_slices(N, p))) return;
+  };
+  auto step = [&](FC(&m)[16], FC(&next)[16], int64_t p) {
+    if (AHEAD) load(next, p - 1);
+    else load(m, p);
+    if (!sv_gather(xbuf + p * SV, (int)min((int64_t)SV, N - p * SV), sm.v[p & 1], p - o, err, limit)) return false;
 #pragma unroll
-    for (int j = 0; j < 16; j++)
-      if (g + 16 * j < n) cfma(v, to_d2(m[j]), __ldcg(x + p * SV + g + 16 * j));
+    for (int j = 0; j < 16; j++) cfma(v, to_d2(m[j]), sm.v[p & 1][g + 16 * j]);
+    return true;
+  };
+  FC ma[16], mb[16];
+  if (AHEAD) load(ma, nblk - 1);
+  for (int64_t p = nblk - 1; p > o; p -= 2) {
+    if (!step(ma, mb, p)) return;
+    if (p - 1 > o && !step(mb, ma, p - 1)) return;
   }
-  v = cols_sum(v, red);
-  if (t < nr) {
-    const int64_t r = r0 + t;
-    __stcg(abuf + r, csub(cdiv(x[r], to_d2(F[r * N + r])), v));
-  }
-  // X_o^T: outputs ra, ra + 1 of a warp, the inverse's columns of these rows
-  const int64_t ra = r0 + 2 * warp;
-  double2 m0[8], m1[8];
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    const int k = lane + 32 * j;
-    m0[j] = (ra < N && k < w) ? X[(ra - o0) * N + o0 + k] : make_double2(0.0, 0.0);
-    m1[j] = (ra + 1 < N && k < w) ? X[(ra + 1 - o0) * N + o0 + k] : make_double2(0.0, 0.0);
-  }
+  // sum of the 16 row groups
+  v.x += __shfl_xor_sync(0xffffffffu, v.x, 16);
+  v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
+  if (lane < 16) sm.red[warp][lane] = v;
   __syncthreads();
-  if (t == 0) {
-    __threadfence();
-    atomicAdd(acnt + o, 1u);
+  if (t < nr) {
+    double2 s = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int q = 0; q < 8; q++) s = cadd(s, sm.red[q][t]);
+    sv_publish(abuf + r0 + t, csub(yd, s));
   }
-  if (!wait(acnt + o, sweep_slices(N, o))) return;
+  if (!sv_gather(abuf + o0, w, sm.v[o & 1], 0, err, limit)) return;
   double2 s0 = make_double2(0.0, 0.0), s1 = s0;
-  rows2_fma(m0, m1, abuf + o0, w, lane, s0, s1);
+  rows2_fma(sm.X[2 * warp], sm.v[o & 1], lane, s0, s1);
   s0 = warp_sum2(s0);
   s1 = warp_sum2(s1);
-  if (lane < 2 && 2 * warp + lane < nr) __stcg(x + ra + lane, lane == 0 ? s0 : s1);
-  __syncthreads();
-  if (t == 0) {
-    __threadfence();
-    atomicAdd(xcnt + o, 1u);
+  if (lane < 2 && 2 * warp + lane < nr) {
+    const double2 r = lane == 0 ? s0 : s1;
+    sv_publish(xbuf + r0 + 2 * warp + lane, r);
+    x[r0 + 2 * warp + lane] = r;
   }
 }
 
 template <class C> void ldlt_solve(dmb_ctx *c, const C *F, double2 *x, int64_t R) {
-  const int64_t N = c->n, nblk = (N + SV - 1) / SV;
+  const int64_t N = c->n;
   prepare_block_inverses<SV, C, double2>(c, F, c->d_sv_inv, c->f_inv64);
   const double2 *X = c->d_sv_inv.as<double2>();
-  c->d_sv_acc.ensure(sizeof(double2) * 2 * N * R);
-  double2 *abuf = c->d_sv_acc.as<double2>();
-  // the error word, a ticket counter per column and sweep, four counters per
-  // block, column
-  const size_t words = 1 + 2 * R + 4 * R * nblk;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    DMB_CUDA(cudaFuncSetAttribute(k_sweep_fwd<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SweepSmem)));
+    DMB_CUDA(cudaFuncSetAttribute(k_sweep_bwd<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SweepSmem)));
+  });
+  // a and y of the forward sweep, a and x of the backward one, all empty
+  c->d_sv_acc.ensure(sizeof(double2) * 4 * N * R);
+  double2 *buf = c->d_sv_acc.as<double2>();
+  // the error word, a ticket counter per column and sweep
+  const size_t words = 1 + 2 * R;
   c->d_flags.ensure(std::max<size_t>(64, 4 * words));
-  unsigned *err = c->d_flags.as<unsigned>(), *tickets = err + 1, *cnt = tickets + 2 * R;
-  DMB_CUDA(cudaMemsetAsync(err, 0, 4 * words, c->stream));
+  unsigned *err = c->d_flags.as<unsigned>(), *tickets = err + 1;
+  DMB_LAUNCH(c, k_sweep_clear, blocks_for(4 * N * R, 256), 256, 0, 4 * N * R, reinterpret_cast<ulonglong2 *>(buf),
+             (int)words, err);
   const dim3 g((unsigned)((N + SW - 1) / SW), (unsigned)R);
-  DMB_LAUNCH(c, k_sweep_fwd<C>, g, 256, 0, N, F, X, x, abuf, tickets, cnt, cnt + R * nblk, err, c->spin_limit);
-  DMB_LAUNCH(c, k_sweep_bwd<C>, g, 256, 0, N, F, X, x, abuf + N * R, tickets + R, cnt + 2 * R * nblk,
-             cnt + 3 * R * nblk, err, c->spin_limit);
+  DMB_LAUNCH(c, k_sweep_fwd<C>, g, 256, sizeof(SweepSmem), N, F, X, x, buf, buf + N * R, tickets, err, c->spin_limit);
+  DMB_LAUNCH(c, k_sweep_bwd<C>, g, 256, sizeof(SweepSmem), N, F, X, buf + N * R, buf + 2 * N * R, buf + 3 * N * R, x,
+             tickets + R, err, c->spin_limit);
 }
 
 template <class C> void ldlt_solve_batched(dmb_ctx *c, const C *F, double2 *X, int64_t R) {

@@ -47,3 +47,20 @@ def test_new_factor_between_solves():
             assert st.niter <= 2
             assert np.linalg.norm(Z @ x - b) < 1e-9 * np.linalg.norm(b)
     dev.close()
+
+
+def test_nan_with_the_empty_pattern():
+    """A NaN of all ones in the right-hand side, the pattern of a value not yet
+    there, passes through as a NaN; the next solve is right."""
+    from diffmom_b200 import EFIEDevice, build_rwg, make_rect_plate
+    mesh = make_rect_plate(0.05, 0.05, 12, 12)
+    dev = EFIEDevice(mesh, build_rwg(mesh))
+    Z = dev.assemble(2 * math.pi / 0.1, precision="fp64", copy_out=True)
+    dev.build_nearfield(math.inf, "lu")
+    b = np.ones(dev.N, dtype=np.complex128)
+    bad = b.copy()
+    bad.view(np.uint64)[6:8] = 0xffffffffffffffff
+    assert np.isnan(dev.nf_apply(bad)).any()
+    x = dev.nf_apply(b)
+    dev.close()
+    assert np.linalg.norm(Z @ x - b) < dev.N * 2.0 ** -52 * np.linalg.norm(Z) * np.linalg.norm(x)
