@@ -303,21 +303,6 @@ __device__ __forceinline__ bool elim16_warp(C (*A)[LD], C (*Xs)[17], int s0, int
   return true;
 }
 
-// (cr, ci) += a b on an 8 x 8 tile by FP64 matrix instructions: a[row lane / 4]
-// [k lane % 4], b[k lane % 4][col lane / 4]; the accumulators hold columns
-// 2 (lane % 4) + {0, 1} of row lane / 4
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
-__device__ __forceinline__ void zmma(double (&cr)[2], double (&ci)[2], double2 a, double2 b) {
-  dmma(cr, a.x, b.x);
-  dmma(ci, a.x, b.y);
-  dmma(cr, -a.y, b.y);
-  dmma(ci, a.y, b.x);
-}
-
 // Shared memory of a diagonal tile's factorisation: the tile A, the sub-panel
 // Wp, the inverses Xd of its 16 x 16 diagonal blocks, its inverse LI.  The
 // leading dimension of complex128 tiles suits the FP64 matrix instruction's
