@@ -60,6 +60,7 @@ __global__ void __launch_bounds__(256) k_dots(int64_t N, int64_t vstride, const 
 // w(r) -= sum_{i < m} h_i V_i(r), h_i the sum of hp's S parts; the first CTA of
 // a system adds h to column m - 1 of its H; np (if not null): per CTA the
 // partial sum of |w|^2
+constexpr size_t GRAPHS_KEPT = 1024;    // captured iterations of a context
 constexpr int UPD_T = 64, UPD_H = 512;  // threads per CTA, coefficients per shared pass
 __global__ void __launch_bounds__(UPD_T) k_cgs_update(int64_t N, int m, int S, int64_t vstride,
                                                       const double2 *__restrict__ V, const double2 *__restrict__ hp,
@@ -331,6 +332,20 @@ void apply_operator(dmb_ctx *c, int precond_kind, int side, const double2 *v, do
 
 unsigned read_err_word(dmb_ctx *c);
 
+// What decides, beside sizes and buffer addresses, which kernels an iteration
+// launches and with which host-side arguments: the operator and its launch
+// sizes, the factor's type, and the options that the launches read.  Part of
+// the key of a captured iteration; everything else is read from device buffers
+// at replay.
+static void append_launch_state(const dmb_ctx *c, std::vector<int64_t> &key) {
+  const bool h = c->op_kind == 1;
+  key.insert(key.end(), {c->op_kind, c->aca_transposed, c->z_prec, c->pc_kind, c->pc_prec, (int64_t)c->spin_limit,
+                         c->use_tensor_cores, c->tc_min_rhs, c->precond_tf32_terms, c->pc_bf16(), c->int8_scheme,
+                         c->exact_krylov, h ? c->aca.n_lr : 0, h ? (int64_t)c->aca.blocks.size() : 0,
+                         h ? c->aca.n_leaves : 0});
+  for (int pin : c->tune_pin) key.push_back(pin);
+}
+
 void gmres_dev(dmb_ctx *c, const double *b_dev, double *x_dev, int64_t R, double tol, int maxiter,
                int precond_kind, int side, dmb_gmres_stats *out) {
   double t0 = now_ms();
@@ -501,18 +516,20 @@ void gmres_dev(dmb_ctx *c, const double *b_dev, double *x_dev, int64_t R, double
         for (int jj = j0; jj < j0 + nb; jj++) iteration(jj);
       };
       if (!(graphs_ok && c->gmres_graphs)) return eager();
-      // a device allocation anywhere ends the life of all captured iterations
-      if (c->gm_graph_epoch != g_dev_alloc_epoch.load()) {
+      // a device allocation anywhere ends the life of all captured iterations;
+      // so does their number (a few operators and shapes in turn stay below it)
+      if (c->gm_graph_epoch != g_dev_alloc_epoch.load() || c->gm_graphs.size() >= GRAPHS_KEPT) {
         for (auto &kv : c->gm_graphs)
           if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
         c->gm_graphs.clear();
         c->gm_graph_epoch = g_dev_alloc_epoch.load();
       }
-      const std::vector<int64_t> key = {j0, nb, N, R, kcap, vstride, precond_kind, side, flex, c->pc_kind,
-                                        c->z_prec, (int64_t)(uintptr_t)V, (int64_t)(uintptr_t)Zv,
-                                        (int64_t)(uintptr_t)w, (int64_t)(uintptr_t)tmp, (int64_t)(uintptr_t)H,
-                                        (int64_t)(uintptr_t)hb, (int64_t)(uintptr_t)g,
-                                        (int64_t)(uintptr_t)st, (int64_t)g_dev_alloc_epoch.load()};
+      std::vector<int64_t> key = {j0, nb, N, R, kcap, vstride, precond_kind, side, flex, prod_resid,
+                                  (int64_t)(uintptr_t)V, (int64_t)(uintptr_t)Zv, (int64_t)(uintptr_t)Wraw,
+                                  (int64_t)(uintptr_t)w, (int64_t)(uintptr_t)tmp, (int64_t)(uintptr_t)H,
+                                  (int64_t)(uintptr_t)hb, (int64_t)(uintptr_t)g, (int64_t)(uintptr_t)st,
+                                  (int64_t)g_dev_alloc_epoch.load()};
+      append_launch_state(c, key);
       dmb_ctx::GraphEntry &e = c->gm_graphs[key];
       if (e.exec) {
         DMB_CUDA(cudaGraphLaunch(e.exec, c->stream));

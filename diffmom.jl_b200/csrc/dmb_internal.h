@@ -284,8 +284,8 @@ struct dmb_ctx {
   int far_tile = 0;              // far-pair RWG tile width (FP64 16/32, FP32 32/64), 0 = autotuned
   bool exact_krylov = true;      // many-RHS Krylov product on the INT8 slices (FP64-accurate)
   // GMRES iterations between host checks replayed as captured CUDA graphs
-  // (few right-hand sides); key: iteration range, shape, buffer addresses and
-  // the allocation epoch
+  // (few right-hand sides); key: iteration range, shape, buffer addresses, the
+  // allocation epoch and what else decides the launches (append_launch_state)
   bool gmres_graphs = true;
   // GMRES tests convergence on ||b - Z x|| / ||b|| (FP64-accurate product):
   // a system whose recurrence estimate met the tolerance but whose true
