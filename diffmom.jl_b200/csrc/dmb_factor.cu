@@ -1827,7 +1827,12 @@ void nf_factor_resident(dmb_ctx *c, int kind, int precision) {
 // what applications of the factor keep per factor, made now: a captured
 // iteration replayed with a later factor does not make it
 void pc_prepare_dev(dmb_ctx *c, int64_t nrhs) {
-  if (c->pc_kind != DMB_PRECOND_NF_LU || nrhs >= 8) return;
+  if (c->pc_kind != DMB_PRECOND_NF_LU) return;
+  if (nrhs >= 8) {  // as ldlt_solve_batched chooses
+    if (c->pc_prec == DMB_PREC_MIXED && nrhs >= c->tc_min_rhs && tc_available(c))
+      prepare_packed_factor(c, c->d_F.as<float2>());
+    return;
+  }
   if (c->pc_prec == DMB_PREC_FP64)
     prepare_block_inverses<SV, double2, double2>(c, c->d_F.as<double2>(), c->d_sv_inv, c->f_inv64);
   else

@@ -337,11 +337,11 @@ unsigned read_err_word(dmb_ctx *c);
 // sizes, the factor's type, and the options that the launches read.  Part of
 // the key of a captured iteration; everything else is read from device buffers
 // at replay.
-static void append_launch_state(const dmb_ctx *c, std::vector<int64_t> &key) {
+static void append_launch_state(dmb_ctx *c, std::vector<int64_t> &key) {
   const bool h = c->op_kind == 1;
   key.insert(key.end(), {c->op_kind, c->aca_transposed, c->z_prec, c->pc_kind, c->pc_prec, (int64_t)c->spin_limit,
-                         c->use_tensor_cores, c->tc_min_rhs, c->precond_tf32_terms, c->pc_bf16(), c->int8_scheme,
-                         c->exact_krylov, h ? c->aca.n_lr : 0, h ? (int64_t)c->aca.blocks.size() : 0,
+                         c->use_tensor_cores, c->tc_min_rhs, c->precond_tf32_terms, c->pc_bf16(), tc_packed_format(c),
+                         c->int8_scheme, c->exact_krylov, h ? c->aca.n_lr : 0, h ? (int64_t)c->aca.blocks.size() : 0,
                          h ? c->aca.n_leaves : 0});
   for (int pin : c->tune_pin) key.push_back(pin);
 }
@@ -355,6 +355,7 @@ void gmres_dev(dmb_ctx *c, const double *b_dev, double *x_dev, int64_t R, double
   DMB_REQUIRE(precond_kind == DMB_PRECOND_NONE || precond_kind == c->pc_kind, DMB_ERR_STATE,
               "requested preconditioner kind differs from the one built");
   if (precond_kind == DMB_PRECOND_NF_LU) pc_prepare_dev(c, R);
+  if (matvec_op_inexact(c, R)) tc_zx_prepare(c);
   // basis capacity: maxiter vectors, bounded by a 40% share of free memory
   // (decided once per problem shape; repeated solves reuse the buffers); the
   // right-preconditioned form also keeps the preconditioned vectors

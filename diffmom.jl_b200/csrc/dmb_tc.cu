@@ -1052,23 +1052,33 @@ unsigned tc_error_word(dmb_ctx *c) {
   return e;
 }
 
-// Packed Z (re-packed whenever Z changes), Y = Z X for R right-hand sides
-// (X, Y complex128 column-major N x R) on the tensor cores.
-void tc_zx(dmb_ctx *c, const double2 *X, double2 *Y, int64_t R) {
+// format of the packed factor of the triangular sweeps (0 TF32, 1 BF16, -1 none)
+int tc_packed_format(dmb_ctx *c) { return tc_state(c).lp_fmt; }
+
+// Packed Z of tc_zx, made once per Z.  Solves call it before their iterations:
+// a captured product that is replayed with a later Z does not make it.
+void tc_zx_prepare(dmb_ctx *c) {
   DMB_REQUIRE(c->z_prec == DMB_PREC_MIXED, DMB_ERR_STATE, "tensor-core Z X needs the complex64 matrix");
+  TcState &st = tc_state(c);
+  const int64_t N = c->n, Kpad = round_up(N, 256), Mpad = round_up(N, 64), ld = 6 * Kpad;
+  if (st.zp_version == c->z_version && st.zp_n == N) return;
+  st.Zp.ensure(sizeof(float) * 2 * Mpad * ld);
+  dim3 g((unsigned)(Kpad / 32), (unsigned)(Mpad / 32));
+  DMB_LAUNCH(c, (k_pack_a<false, false, float2, float>), g, 256, 0, N, N, Kpad, c->d_Z.as<float2>(), N,
+             st.Zp.as<float>());
+  make_map(&st.mapZ, st.Zp.as<float>(), (uint64_t)(2 * Mpad), TC_BM, (uint64_t)ld);
+  st.zp_version = c->z_version;
+  st.zp_n = N;
+}
+
+// Y = Z X for R right-hand sides (X, Y complex128 column-major N x R) on the
+// tensor cores
+void tc_zx(dmb_ctx *c, const double2 *X, double2 *Y, int64_t R) {
+  tc_zx_prepare(c);
   TcState &st = tc_state(c);
   ensure_gemm(c, st);
   const int64_t N = c->n, Kpad = round_up(N, 256), Mpad = round_up(N, 64), Rpad = round_up(R, TC_BN);
   const int64_t ld = 6 * Kpad;
-  if (st.zp_version != c->z_version || st.zp_n != N) {
-    st.Zp.ensure(sizeof(float) * 2 * Mpad * ld);
-    dim3 g((unsigned)(Kpad / 32), (unsigned)(Mpad / 32));
-    DMB_LAUNCH(c, (k_pack_a<false, false, float2, float>), g, 256, 0, N, N, Kpad, c->d_Z.as<float2>(), N,
-               st.Zp.as<float>());
-    make_map(&st.mapZ, st.Zp.as<float>(), (uint64_t)(2 * Mpad), TC_BM, (uint64_t)ld);
-    st.zp_version = c->z_version;
-    st.zp_n = N;
-  }
   st.Xp.ensure(sizeof(float) * Rpad * ld);
   if (st.xp_key != Rpad || st.xp_n != N) {
     make_map(&st.mapX, st.Xp.as<float>(), (uint64_t)Rpad, TC_BN, (uint64_t)ld);

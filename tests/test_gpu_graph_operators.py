@@ -86,6 +86,22 @@ def test_hmatrix_plans():
     _alternating(states)
 
 
+@pytest.mark.parametrize("side", ["left", "right"])
+def test_packed_operands_follow_the_matrix(side):
+    """Tensor-core products and sweeps of a batch small enough to be captured
+    use operands packed once per matrix and once per factor."""
+    def states(dev, mesh, rwg):
+        dev.set_option("tc_min_rhs", 16)
+        for k in (K, 1.2 * K):
+            dev.assemble(k, precision="mixed")
+            P = dev.build_nearfield(math.inf, "lu")
+            for _ in range(3):  # captured while the packed operands are up to date
+                x, st = dev.gmres(_rhs(dev.N, 16), tol=1e-6, maxiter=30, preconditioner=P, precond_side=side)
+                assert st.solved and st.niter < 10
+                yield x
+    _alternating(states)
+
+
 def test_spin_limit_reaches_captured_sweeps():
     mesh, rwg = _plate(20, 23)
     dev = EFIEDevice(mesh, rwg)
