@@ -810,8 +810,8 @@ __device__ __forceinline__ void mid_substitute(float2 (*Tw)[LD], const float2 (*
 template <class C>
 __global__ void __launch_bounds__(256, sizeof(C) == 16 ? 1 : 2) k_ldlt_mid(int64_t N, int64_t J, int w, C *__restrict__ F,
                                                                            C *__restrict__ Linv, C *__restrict__ W,
-                                                                           int wstride, unsigned *sync,
-                                                                           unsigned *err) {
+                                                                           int wstride, double *__restrict__ bal,
+                                                                           unsigned *sync, unsigned *err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned s_ticket;
   __shared__ int s_ok;
@@ -877,6 +877,14 @@ __global__ void __launch_bounds__(256, sizeof(C) == 16 ? 1 : 2) k_ldlt_mid(int64
           Lb[(16 * q + i) * 64 + 16 * q + c] = sm.Xd[q][i][c];
         }
       publish(diag_flag + s);
+      // 2^-e and 2^e of the panel's columns, 4^e about |D|: what balances W and L
+      // for the int8 updates
+      if (bal && ok && t < b) {
+        int e;
+        frexp(fmax(fabs((double)As[t][t].x), fabs((double)As[t][t].y)), &e);
+        bal[jc + t] = ldexp(1.0, -(e >> 1));
+        bal[N + jc + t] = ldexp(1.0, e >> 1);
+      }
       if (ok) ldlt_diag_phase2<C>(Lb, smem_raw);
       return;
     }
@@ -1006,6 +1014,11 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
   unsigned *step_sync = err + 4;
   DMB_CUDA(cudaMemsetAsync(err, 0, 4 * flag_words, c->stream));
   const bool use_tc = std::is_same<C, float2>::value && dmb::tc_available(c);
+  double *bal = nullptr;  // column scales of the int8 updates
+  if (std::is_same<C, double2>::value && dmb::oz64_available(c, NBO)) {
+    c->oz64.bal.ensure(sizeof(double) * 2 * N);
+    bal = c->oz64.bal.as<double>();
+  }
   // trailing update F[r][cc] -= W[r][woff..woff+K) L[cc][jcol..jcol+K) on
   // rows >= r0, columns [r0, c_hi); slot: the packed-operand buffers of the
   // issuing stream (0 main, 1 stream2, 2 stream3)
@@ -1018,7 +1031,8 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
     } else if constexpr (std::is_same<C, double2>::value) {
       const double2 *Wk = (const double2 *)Wb + r0 * NBW + woff, *Lk = (const double2 *)F + r0 * N + jcol;
       if (dmb::oz64_available(c, K) && dmb::oz64_reserve(c, rest, c_hi - r0, K, slot))
-        dmb::oz64_lower_update(c, rest, c_hi - r0, K, Wk, NBW, Lk, N, (double2 *)F + r0 * N + r0, N, slot, err);
+        dmb::oz64_lower_update(c, rest, c_hi - r0, K, Wk, NBW, Lk, N, bal + jcol, bal + N + jcol,
+                               (double2 *)F + r0 * N + r0, N, slot, err);
       else
         // the FP64-pipe GEMM (128 x 64 tiles, lower triangle)
         dmb::zgemm64_lower_update(c, rest, c_hi - r0, K, Wk, NBW, Lk, N, (double2 *)F + r0 * N + r0, N);
@@ -1100,7 +1114,7 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
     for (int64_t J = J2; J < J2E; J += NBO) {
       const int64_t JE = std::min<int64_t>(J2E, J + NBO);
       DMB_LAUNCH(c, k_ldlt_mid<C>, blocks_for(N - J, NB), 256, DiagSmem<C>::bytes, N, J, (int)(JE - J), F, Linv,
-                 Wb + (J - J2), NBW, step_sync + MID_WORDS * (J / NBO), err);
+                 Wb + (J - J2), NBW, bal, step_sync + MID_WORDS * (J / NBO), err);
       update_block_column(JE, J2E, J, (int)(JE - J), Wb, (int)(J - J2));
     }
     update_trailing(J2E, J2, (int)(J2E - J2), Wb);

@@ -182,6 +182,7 @@ struct FarTileState {
 // the INT8 tensor cores (dmb_oz64.cu), one set per issuing stream.
 struct Oz64State {
   DevBuf planes[3], scale[3], res[3];
+  DevBuf bal;  // per factor column 2^-e (scales W) and 2^e (scales L)
   bool attr = false;
 };
 
@@ -450,7 +451,8 @@ void zgemm64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int64_t K, const dou
 bool oz64_available(dmb_ctx *c, int K);
 bool oz64_reserve(dmb_ctx *c, int64_t M, int64_t C, int K, int slot);
 void oz64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int K, const double2 *W, int64_t ldw, const double2 *L,
-                       int64_t ldl, double2 *F, int64_t ldf, int slot, unsigned *err);
+                       int64_t ldl, const double *balW, const double *balL, double2 *F, int64_t ldf, int slot,
+                       unsigned *err);
 void oz64_release(dmb_ctx *c);
 unsigned read_err_word(dmb_ctx *c);  // error word of the triangular solves (bit 2: a wait expired)
 void matvec_dev(dmb_ctx *c, const void *x, void *y, int64_t nrhs);  // device buffers, c128

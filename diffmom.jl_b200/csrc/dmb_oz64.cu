@@ -11,6 +11,15 @@
 // 96-bit fraction.  The only errors are the two roundings to 55 bits and one
 // rounding of the result; an FP64 sum of K products rounds K times.
 //
+// The roundings are relative to the largest element of a row, so the columns
+// are balanced first: column k of W = L D is scaled by 2^-e, column k of L by
+// 2^e, 4^e about |D_k| (exact).  Both rows are then rows of about L sqrt(|D|),
+// whose elements do not carry the scales of the basis functions of their
+// columns.  Without it an error grew with the spread of these scales: largest
+// |A - L D L^T| over the diagonal scales of a graded plate, 519 unknowns, scales
+// over 1.6e3: 2e-11, balanced 1e-13, FP64 sums 1e-13; over 3e6: 0.4, 3e-9 and 2e-9;
+// on plates and disks of even meshes 1e-15 to 3e-15 in all three.
+//
 // Why: B200 has no FP64 tcgen05 kind, and an FP64-pipe GEMM stops at 36.8
 // TFLOP/s (a complex MAC = 8 flops); 16 int8 products at the nominal int8
 // rate amount to 280.  Measured (trailing updates of a 7,680-unknown factor):
@@ -305,6 +314,7 @@ struct Mods64 {
 struct Operand64 {
   const double2 *S;   // rows x K, row-major
   int64_t ld, rows, padded;
+  const double *bal;  // scales of the K columns, powers of two
   double *scale;      // padded
   signed char *P;     // OZ_NMOD64 planes of 2 padded rows of K bytes
 };
@@ -334,7 +344,7 @@ __global__ void __launch_bounds__(64) k_oz64_planes(Operand64 A, Operand64 B, co
   for (int u = 0; u < 16; u++) {
     const int e = t + 64 * u;
     const int64_t rr = r0 + e / K;
-    st[e + (e >> 4)] = rr < O.rows ? O.S[rr * O.ld + e % K] : make_double2(0, 0);
+    st[e + (e >> 4)] = rr < O.rows ? cscale(O.S[rr * O.ld + e % K], O.bal[e % K]) : make_double2(0, 0);
   }
   __syncthreads();
   const double2 *my = st + 17 * t;
@@ -458,7 +468,8 @@ bool oz64_reserve(dmb_ctx *c, int64_t M, int64_t C, int K, int slot) {
 }
 
 void oz64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int K, const double2 *W, int64_t ldw, const double2 *L,
-                       int64_t ldl, double2 *F, int64_t ldf, int slot, unsigned *err) {
+                       int64_t ldl, const double *balW, const double *balL, double2 *F, int64_t ldf, int slot,
+                       unsigned *err) {
   Oz64State &st = c->oz64;
   if (!st.attr) {
     DMB_CUDA(cudaFuncSetAttribute(k_oz64_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, O6_SMEM));
@@ -474,7 +485,7 @@ void oz64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int K, const double2 *W
       if (ntiles == 0) continue;
       double *rs = st.scale[slot].as<double>(), *cs = rs + nmp;
       signed char *PA = st.planes[slot].as<signed char>(), *PB = PA + (size_t)OZ_NMOD64 * 2 * nmp * K;
-      const Operand64 A{W + m0 * ldw, ldw, nm, nmp, rs, PA}, B{L + c0 * ldl, ldl, nc, ncp, cs, PB};
+      const Operand64 A{W + m0 * ldw, ldw, nm, nmp, balW, rs, PA}, B{L + c0 * ldl, ldl, nc, ncp, balL, cs, PB};
       const unsigned g = (unsigned)((nmp + ncp) / (1024 / K));
       if (K == 1024)
         DMB_LAUNCH(c, k_oz64_planes<1024>, g, 64, 0, A, B, mods64());
@@ -497,6 +508,7 @@ void oz64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int K, const double2 *W
 void oz64_release(dmb_ctx *c) {
   for (int s = 0; s < 3; s++)
     for (DevBuf *b : {&c->oz64.planes[s], &c->oz64.scale[s], &c->oz64.res[s]}) b->release();
+  c->oz64.bal.release();
 }
 
 }  // namespace dmb

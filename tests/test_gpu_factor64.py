@@ -52,6 +52,39 @@ def test_int8_update_no_worse_than_fp64_pipe():
     assert e8 < 2 * e64
 
 
+def _graded_plate(power):
+    from diffmom_b200 import TriMesh, make_rect_plate
+    m = make_rect_plate(0.06, 0.06, 18, 20)
+    xyz = m.xyz.copy()
+    lo = xyz[:, 0].min()
+    xyz[:, 0] = lo + 0.06 * ((xyz[:, 0] - lo) / 0.06) ** power
+    return TriMesh(xyz, m.tri)
+
+
+@pytest.mark.parametrize("mesh", ["disk", "graded 4", "graded 7"])
+def test_int8_update_on_graded_meshes(mesh):
+    """Slivers and cells graded over decades: basis functions of scales up to
+    3e6 apart.  The residual is compared row by row with |Z| |x|, so that rows
+    of small scale count as the others do."""
+    from diffmom_b200 import EFIEDevice, build_rwg, make_circular_plate
+    mesh = make_circular_plate(0.05, 12, 48) if mesh == "disk" else _graded_plate(int(mesh.split()[1]))
+    dev = EFIEDevice(mesh, build_rwg(mesh))
+    Z = dev.assemble(K, copy_out=True)
+    rng = np.random.default_rng(3)
+    b = (rng.standard_normal(dev.N) + 1j * rng.standard_normal(dev.N)) * np.sqrt(np.abs(np.diag(Z)))
+    omega = {}
+    for tensor_cores in (1, 0):
+        dev.set_option("tensor_cores", tensor_cores)
+        dev.build_nearfield(math.inf, "lu")
+        x = dev.nf_apply(b)
+        r = Z.astype(np.clongdouble) @ x.astype(np.clongdouble) - b
+        omega[tensor_cores] = float(np.max(np.abs(r) / (np.abs(Z) @ np.abs(x))))
+    dev.close()
+    # both are rounding, seen through the growth of an elimination without
+    # pivoting: a factor of four covers the scatter of a largest row
+    assert omega[1] < 4 * omega[0], omega
+
+
 def test_pivots_outside_the_fast_range():
     """|pivot|^2 underflows; the factor does not (the matrix is scaled by a
     power of two, which changes no rounding of a sum)."""
