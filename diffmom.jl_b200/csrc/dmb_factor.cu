@@ -1478,14 +1478,16 @@ void prepare_packed_factor(dmb_ctx *c, const float2 *F) {
 //   backward, o = last..0: a_o = y_o / D - L[>o, o]^T x, x_o = X_o^T a_o
 // with X_o the inverse of L's diagonal block.  A CTA owns 16 rows (forward) or
 // columns (backward) of a block: it streams its part of L block by block as the
-// blocks of y (x) appear, publishes its 16 values of a_o, and, once all of a_o
-// is there, its 16 values of X_o a_o.  The values are their own flags: the
+// blocks of y (x) appear, publishes its 16 values of a_o, and, once the part of
+// a_o that its rows of X_o need is there, its 16 values of X_o a_o.  The values are their own flags: the
 // buffers are filled with a bit pattern that no published value has (SV_EMPTY),
 // and a thread that needs a value reads it until it is there.  The next block's
 // part of L is loaded ahead of that, the part of X_o at the start, so a block
 // costs two trips through L2 and two short sums; the stream of L runs beside
-// that chain over all SMs.  CTAs take their slices in ticket order and wait only
-// on earlier tickets; every wait is bounded (error bit 4).  All sums in a fixed
+// that chain over all SMs.  CTAs take their slices in ticket order (forward
+// sweep downwards, backward upwards) and wait only on earlier tickets -- of their
+// own block too, X_o being triangular -- so a sweep goes on however few of its
+// CTAs are resident; every wait is bounded (error bit 4).  All sums in a fixed
 // order.  Bound by the chain up to N = 10,000 and by the read of L above.
 // Measured, both sweeps: complex128 415 us at N = 10,680 (912 MB of L each), 56 us
 // at 1,825; complex64 177 us at 4,693.  With counters as flags (two
@@ -1503,15 +1505,15 @@ __device__ __forceinline__ void sv_publish(double2 *p, double2 v) {
   asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(x), "l"(y) : "memory");
 }
 
-// The n values at p into v[0..255] (zero beyond n), a thread each, as they are
-// published; for the whole CTA, false on expiry or another CTA's.  v is read
-// after, and written before, the next barrier.
-__device__ __forceinline__ bool sv_gather(const double2 *p, int n, double2 *v, int64_t ahead, unsigned *err,
+// The values lo to n - 1 at p into v[0..255] (zero elsewhere), a thread each, as
+// they are published; for the whole CTA, false on expiry or another CTA's.  v is
+// read after, and written before, the next barrier.
+__device__ __forceinline__ bool sv_gather(const double2 *p, int lo, int n, double2 *v, int64_t ahead, unsigned *err,
                                           long long limit) {
   const int t = threadIdx.x;
   bool ok = true;
   unsigned long long x = 0, y = 0;
-  if (t < n) {
+  if (t >= lo && t < n) {
     for (long long it = 0;;) {
       asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "l"(p + t) : "memory");
       if (x != SV_EMPTY && y != SV_EMPTY) break;
@@ -1571,7 +1573,7 @@ __global__ void __launch_bounds__(256, 2) k_sweep_fwd(int64_t N, const FC *__res
   if (t == 0) s_t = (int)atomicAdd(tickets + rhs, 1u);
   __syncthreads();
   const int64_t r0 = (int64_t)s_t * SW, o = r0 / SV, o0 = o * SV;
-  const int nr = (int)min((int64_t)SW, N - r0), w = (int)min((int64_t)SV, N - o0);
+  const int nr = (int)min((int64_t)SW, N - r0);
   for (int e = t; e < SW * SV; e += 256) {  // the inverse is kept transposed
     const int c = e & 15, k = e >> 4;
     sm.X[c][k] = (c < nr && k <= r0 - o0 + c) ? X[(int64_t)k * N + r0 + c] : make_double2(0.0, 0.0);
@@ -1591,7 +1593,7 @@ __global__ void __launch_bounds__(256, 2) k_sweep_fwd(int64_t N, const FC *__res
   auto step = [&](FC(&m)[16], FC(&next)[16], int64_t p) {
     if (AHEAD) load(next, p + 1);
     else load(m, p);
-    if (!sv_gather(y + p * SV, SV, sm.v[p & 1], o - p, err, limit)) return false;
+    if (!sv_gather(y + p * SV, 0, SV, sm.v[p & 1], o - p, err, limit)) return false;
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       const double2 yv = sm.v[p & 1][lane + 32 * j];
@@ -1609,7 +1611,8 @@ __global__ void __launch_bounds__(256, 2) k_sweep_fwd(int64_t N, const FC *__res
   s0 = warp_sum2(s0);
   s1 = warp_sum2(s1);
   if (lane < 2 && 2 * warp + lane < nr) sv_publish(abuf + ra + lane, csub(br, lane == 0 ? s0 : s1));
-  if (!sv_gather(abuf + o0, w, sm.v[o & 1], 0, err, limit)) return;
+  // X_o is lower triangular: the rows up to this CTA's, of earlier tickets
+  if (!sv_gather(abuf + o0, 0, (int)(r0 - o0) + nr, sm.v[o & 1], 0, err, limit)) return;
   s0 = s1 = make_double2(0.0, 0.0);
   rows2_fma(sm.X[2 * warp], sm.v[o & 1], lane, s0, s1);
   s0 = warp_sum2(s0);
@@ -1654,7 +1657,7 @@ __global__ void __launch_bounds__(256, 2) k_sweep_bwd(int64_t N, const FC *__res
   auto step = [&](FC(&m)[16], FC(&next)[16], int64_t p) {
     if (AHEAD) load(next, p - 1);
     else load(m, p);
-    if (!sv_gather(xbuf + p * SV, (int)min((int64_t)SV, N - p * SV), sm.v[p & 1], p - o, err, limit)) return false;
+    if (!sv_gather(xbuf + p * SV, 0, (int)min((int64_t)SV, N - p * SV), sm.v[p & 1], p - o, err, limit)) return false;
 #pragma unroll
     for (int j = 0; j < 16; j++) cfma(v, to_d2(m[j]), sm.v[p & 1][g + 16 * j]);
     return true;
@@ -1676,7 +1679,8 @@ __global__ void __launch_bounds__(256, 2) k_sweep_bwd(int64_t N, const FC *__res
     for (int q = 0; q < 8; q++) s = cadd(s, sm.red[q][t]);
     sv_publish(abuf + r0 + t, csub(yd, s));
   }
-  if (!sv_gather(abuf + o0, w, sm.v[o & 1], 0, err, limit)) return;
+  // X_o^T is upper triangular: the rows from this CTA's on, of earlier tickets
+  if (!sv_gather(abuf + o0, (int)(r0 - o0), w, sm.v[o & 1], 0, err, limit)) return;
   double2 s0 = make_double2(0.0, 0.0), s1 = s0;
   rows2_fma(sm.X[2 * warp], sm.v[o & 1], lane, s0, s1);
   s0 = warp_sum2(s0);

@@ -64,3 +64,24 @@ def test_nan_with_the_empty_pattern():
     x = dev.nf_apply(b)
     dev.close()
     assert np.linalg.norm(Z @ x - b) < dev.N * 2.0 ** -52 * np.linalg.norm(Z) * np.linalg.norm(x)
+
+
+def test_many_contexts_sweep_at_once():
+    """Twenty contexts of seven columns: more waiting CTAs than the GPU holds."""
+    from concurrent.futures import ThreadPoolExecutor
+    from diffmom_b200 import EFIEDevice, build_rwg, make_rect_plate
+    mesh = make_rect_plate(0.09, 0.1, 18, 20)
+    rwg = build_rwg(mesh)
+    rng = np.random.default_rng(2)
+    B = np.asfortranarray(rng.standard_normal((rwg.nedges, 7)) + 1j * rng.standard_normal((rwg.nedges, 7)))
+    devs = [EFIEDevice(mesh, rwg) for _ in range(20)]
+    for dev in devs:
+        dev.assemble(2 * math.pi / 0.1)
+        dev.build_nearfield(math.inf, "lu")
+    alone = devs[0].nf_apply(B)
+    with ThreadPoolExecutor(len(devs)) as pool:
+        for X in pool.map(lambda dev: [dev.nf_apply(B) for _ in range(10)], devs):
+            for x in X:
+                np.testing.assert_array_equal(x, alone)
+    for dev in devs:
+        dev.close()
