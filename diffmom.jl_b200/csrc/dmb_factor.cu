@@ -34,8 +34,7 @@ void tc_ldlt_update_c64(dmb_ctx *c, int64_t N, int64_t r0, int64_t c_hi, int64_t
 
 namespace {
 
-constexpr int NB = 64;                      // panel width == triangular-solve block
-constexpr long long SPIN_LIMIT = 20000000;  // ~2-4 s with nanosleep
+constexpr int NB = 64;  // panel width == triangular-solve block
 
 unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
@@ -592,14 +591,16 @@ __global__ void __launch_bounds__(256) k_ldlt_update(int64_t N, int64_t r_lo, in
 // over a matrix of 4,693 rows with the updates beside it (220 us with the former
 // elimination and trailing updates on FP32 units; as much in launches per 64 columns).
 // ---------------------------------------------------------------------------
-// spin until *flag is set (one thread); false on expiry
-__device__ __forceinline__ bool wait_word(volatile unsigned *flag, unsigned *err) {
+// spin until *flag is set (one thread); false on expiry, this wait's or another
+// CTA's (bit 4 of the error word)
+__device__ __forceinline__ bool wait_word(volatile unsigned *flag, unsigned *err, long long limit) {
   long long it = 0;
   while (*flag == 0u) {
-    if (++it > SPIN_LIMIT) {
+    if (++it > limit) {
       atomicOr(err, 4u);
       return false;
     }
+    if ((it & 15) == 0 && (*(volatile unsigned *)err & 4u)) return false;
     __nanosleep(32);
   }
   __threadfence();
@@ -811,7 +812,8 @@ template <class C>
 __global__ void __launch_bounds__(256, sizeof(C) == 16 ? 1 : 2) k_ldlt_mid(int64_t N, int64_t J, int w, C *__restrict__ F,
                                                                            C *__restrict__ Linv, C *__restrict__ W,
                                                                            int wstride, double *__restrict__ bal,
-                                                                           unsigned *sync, unsigned *err) {
+                                                                           unsigned *sync, unsigned *err,
+                                                                           long long limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned s_ticket;
   __shared__ int s_ok;
@@ -830,7 +832,7 @@ __global__ void __launch_bounds__(256, sizeof(C) == 16 ? 1 : 2) k_ldlt_mid(int64
   const int nr = (int)min((int64_t)64, N - r0);
   // wait for a flag, the whole CTA (uniform result)
   auto wait = [&](unsigned *flag) {
-    if (t == 0) s_ok = wait_word(flag, err) ? 1 : 0;
+    if (t == 0) s_ok = wait_word(flag, err, limit) ? 1 : 0;
     __syncthreads();
     const bool ok = s_ok != 0;
     __syncthreads();
@@ -1114,7 +1116,8 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
     for (int64_t J = J2; J < J2E; J += NBO) {
       const int64_t JE = std::min<int64_t>(J2E, J + NBO);
       DMB_LAUNCH(c, k_ldlt_mid<C>, blocks_for(N - J, NB), 256, DiagSmem<C>::bytes, N, J, (int)(JE - J), F, Linv,
-                 Wb + (J - J2), NBW, bal, step_sync + MID_WORDS * (J / NBO), err);
+                 Wb + (J - J2), NBW, bal, step_sync + MID_WORDS * (J / NBO), err,
+                 c->spin_limit);
       update_block_column(JE, J2E, J, (int)(JE - J), Wb, (int)(J - J2));
     }
     update_trailing(J2E, J2, (int)(J2E - J2), Wb);

@@ -292,7 +292,7 @@ struct dmb_ctx {
   // a system whose recurrence estimate met the tolerance but whose true
   // residual did not is refined by further cycles from its current iterate
   bool true_residual_check = true;
-  // polls of a triangular-solve chain wait before it gives up (DMB_ERR_TIMEOUT);
+  // polls of a panel's or a triangular sweep's wait before it gives up (DMB_ERR_TIMEOUT);
   // DMB_OPT_SPIN_LIMIT lowers it to exercise the timeout path
   long long spin_limit = 20000000;
   struct GraphEntry {

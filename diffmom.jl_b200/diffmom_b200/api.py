@@ -93,8 +93,9 @@ class EFIEDevice:
         "gmres_graphs" (0/1) for CUDA-graph replay of GMRES iterations,
         "true_residual" (1 = default: GMRES refines until ||b - Z x|| / ||b||
         meets the tolerance; 0: it stops where Krylov.gmres stops),
-        "spin_limit" (polls of a chained triangular-sweep wait before the call
-        fails with TimeoutError; negative restores the default),
+        "spin_limit" (polls of a wait in a factorisation panel or a triangular
+        sweep before the call fails with TimeoutError; negative restores the
+        default),
         "tune_tc_gemm" / "tune_tc_syrk" (0 = autotuned; k pins candidate k:
         256- or 128-wide sweep GEMM tiles or a persistent 256-wide grid;
         4-stage, 2-stage or persistent

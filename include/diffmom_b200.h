@@ -140,10 +140,11 @@ const char *dmb_version(void);
  * meets the tolerance.  0 stops exactly where Krylov.gmres stops (iteration
  * counts of the reference). */
 #define DMB_OPT_TRUE_RESIDUAL 8
-/* DMB_OPT_SPIN_LIMIT: polls a waiting CTA of the data-flow triangular sweeps
- * (one to seven right-hand sides) makes before it gives up; the call then fails with DMB_ERR_TIMEOUT and the context
- * stays usable.  A negative value restores the default (2e7 polls, seconds);
- * small values exercise the timeout path without any GPU fault. */
+/* DMB_OPT_SPIN_LIMIT: polls a waiting CTA makes before it gives up, in the
+ * panels of the LDL^T factorisation and in the data-flow triangular sweeps (one
+ * to seven right-hand sides); the call then fails with DMB_ERR_TIMEOUT and the
+ * context stays usable.  A negative value restores the default (2e7 polls,
+ * seconds); small values exercise the timeout path without any GPU fault. */
 #define DMB_OPT_SPIN_LIMIT 9
 /* DMB_OPT_TUNE_TC_GEMM / DMB_OPT_TUNE_TC_SYRK: pin a candidate of the online
  * autotuner (0, the default, lets it choose): the tile width of the

@@ -40,3 +40,22 @@ def test_chain_wait_expires_and_context_recovers():
     I, st = dev.gmres(v, tol=1e-8, maxiter=200, preconditioner=dev.preconditioner)
     assert st.solved and st.true_residual <= 1e-8
     dev.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_factorisation_wait_expires_and_context_recovers(precision):
+    """The tiles of a 256-wide panel wait for its diagonal tiles."""
+    m = make_rect_plate(0.1, 0.1, 20, 23)   # 1,337 RWG: six panels, two block columns
+    dev = EFIEDevice(m, build_rwg(m))
+    Z = dev.assemble(2 * math.pi / 0.1, precision=precision, copy_out=True)
+    dev.set_option("spin_limit", 0)
+    with pytest.raises(DeviceWaitTimeout):
+        dev.build_nearfield(math.inf, "lu")
+    dev.set_option("spin_limit", -1)
+    dev.build_nearfield(math.inf, "lu")
+    b = np.random.default_rng(3).standard_normal(dev.N) + 0j
+    x = dev.nf_apply(b)
+    dev.close()
+    # N-term sums of the factor's precision, twice (factor and sweeps)
+    eps = 2.0 ** -52 if precision == "fp64" else 2.0 ** -23
+    assert np.linalg.norm(Z @ x - b) < Z.shape[0] * eps * np.linalg.norm(Z) * np.linalg.norm(x)
