@@ -116,7 +116,8 @@ __global__ void __launch_bounds__(O6_THREADS, 1) k_oz64_gemm(const __grid_consta
   uint64_t *bar_ptr = reinterpret_cast<uint64_t *>(gbase + (sBar - base));
   volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(bar_ptr + 16);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(bar_ptr + 17);
-  const uint32_t full0 = sBar, empty0 = sBar + 8 * O6_STAGES, accf0 = sBar + 16 * O6_STAGES, acce0 = accf0 + 16;
+  const uint32_t full0 = sBar, empty0 = sBar + 8 * O6_STAGES, accf0 = sBar + 16 * O6_STAGES, acce0 = accf0 + 16,
+                 fin = acce0 + 16;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < O6_STAGES; s++) {
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(O6_THREADS, 1) k_oz64_gemm(const __grid_consta
       mbar_init(accf0 + 8 * b, 1);
       mbar_init(acce0 + 8 * b, O6_DRAIN);  // one arrival per drain warp
     }
+    mbar_init(fin, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -162,6 +164,9 @@ __global__ void __launch_bounds__(O6_THREADS, 1) k_oz64_gemm(const __grid_consta
           tma_load_2d(sB + s * O6_B_STAGE, &tmB, kc * OZ_BK, i * brow + OZ_BN * ct, full0 + 8 * s);
         }
       }
+      // given up: the last fill of each stage
+      for (long long f = t > O6_STAGES ? t - O6_STAGES : 0; !go && f < t; f++)
+        mbar_wait_in_flight(full0 + 8 * (int)(f % O6_STAGES), (uint32_t)(f / O6_STAGES) & 1u);
     }
   } else if (warp == O6_DRAIN + 1) {
     if (lane == 0) {
@@ -170,7 +175,10 @@ __global__ void __launch_bounds__(O6_THREADS, 1) k_oz64_gemm(const __grid_consta
       bool ok = true;
       for (int64_t u = blockIdx.x; ok && u < units; u += gridDim.x, g++) {
         // unit g accumulates in buffer g & 1, free once unit g - 2 drained
-        if (g >= 2 && !mbar_wait(acce0 + 8 * (g & 1), (uint32_t)((g >> 1) - 1) & 1u, err, abort_flag)) break;
+        if (g >= 2 && !mbar_wait(acce0 + 8 * (g & 1), (uint32_t)((g >> 1) - 1) & 1u, err, abort_flag)) {
+          ok = false;
+          break;
+        }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem_d + (uint32_t)((g & 1) * OZ_BN);
         for (int kc = 0; kc < kchunks; kc++, t++) {
@@ -187,6 +195,10 @@ __global__ void __launch_bounds__(O6_THREADS, 1) k_oz64_gemm(const __grid_consta
           umma_commit(empty0 + 8 * s);
         }
         if (ok) umma_commit(accf0 + 8 * (g & 1));
+      }
+      if (!ok) {  // given up: the products issued
+        umma_commit(fin);
+        mbar_wait_in_flight(fin, 0);
       }
     }
   } else {
