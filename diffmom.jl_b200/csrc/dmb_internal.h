@@ -10,6 +10,7 @@
 #include <string>
 #include <atomic>
 #include <map>
+#include <memory>
 #include <vector>
 
 #include "../../include/diffmom_b200.h"
@@ -273,7 +274,8 @@ struct dmb_ctx {
   DevBuf d_rhs, d_sol, d_mono;
   DevBuf d_io[3];     // device copies of a call's host arrays
   DevBuf d_tmp[4];    // workspace of a call's stages (nothing is kept in it between them)
-  HostCopy *hostcopy = nullptr;  // chunks of large copies to the host (dmb_hostcopy.cu)
+  std::shared_ptr<HostCopy> hostcopy;  // the device's chunks of large copies to the host (dmb_hostcopy.cu)
+  size_t copied = 0;                   // bytes of large results so far
   DevBuf d_far;       // far-field workspace
   DevBuf d_mf;        // matrix-free product workspace
   int64_t sol_r = 0;

@@ -54,3 +54,37 @@ def test_repeated_calls_keep_device_memory():
     # one pass takes over 100 MB of buffers: any of them allocated again would show
     assert free - torch.cuda.mem_get_info()[0] < 32 << 20
     dev.close()
+
+
+def test_contexts_share_the_chunks():
+    """Large results of many contexts, one after another and from several
+    threads at once: the chunks are the device's, so a context's first result
+    neither makes its own nor keeps device memory for them."""
+    from concurrent.futures import ThreadPoolExecutor
+    import torch
+    from diffmom_b200 import EFIEDevice, build_rwg, make_rect_plate
+    mesh = make_rect_plate(0.06, 0.06, 18, 20)  # 17.4 MB
+    rwg = build_rwg(mesh)
+    k = 2 * math.pi / 0.1
+    devs = [EFIEDevice(mesh, rwg) for _ in range(12)]
+    for dev in devs:
+        dev.assemble(k)
+    ref = [devs[0].assemble(k, copy_out=True) for _ in range(4)][-1]
+    free = torch.cuda.mem_get_info()[0]
+    for dev in devs:
+        np.testing.assert_array_equal(dev.assemble(k, copy_out=True), ref)
+    assert free - torch.cuda.mem_get_info()[0] < 32 << 20  # a chunk set per context would take 8 MB each
+    for precision in ("fp64", "mixed"):
+        ref = devs[0].assemble(k, precision=precision, copy_out=True)
+        with ThreadPoolExecutor(len(devs)) as pool:
+            for Z in pool.map(lambda d: d.assemble(k, precision=precision, copy_out=True), devs):
+                np.testing.assert_array_equal(Z, ref)
+    for dev in devs:
+        dev.close()
+    # kept for a context that follows; given back by one that did not use
+    # them, and made again
+    for calls in (1, 0, 4):
+        dev = EFIEDevice(mesh, rwg)
+        for _ in range(calls):
+            np.testing.assert_array_equal(dev.assemble(k, precision="mixed", copy_out=True), ref)
+        dev.close()
