@@ -1016,27 +1016,31 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
   unsigned *step_sync = err + 4;
   DMB_CUDA(cudaMemsetAsync(err, 0, 4 * flag_words, c->stream));
   const bool use_tc = std::is_same<C, float2>::value && dmb::tc_available(c);
-  double *bal = nullptr;  // column scales of the int8 updates
-  if (std::is_same<C, double2>::value && dmb::oz64_available(c, NBO)) {
-    c->oz64.bal.ensure(sizeof(double) * 2 * N);
-    bal = c->oz64.bal.as<double>();
-  }
+  // complex128 updates on the int8 tensor cores: a first run through the schedule
+  // only notes what each stream's largest update needs
+  double *bal = nullptr;  // column scales of the int8 updates; null: FP64 pipe
+  bool planning = std::is_same<C, double2>::value && dmb::oz64_available(c, NBO);
+  size_t need[3] = {0, 0, 0};
   // trailing update F[r][cc] -= W[r][woff..woff+K) L[cc][jcol..jcol+K) on
   // rows >= r0, columns [r0, c_hi); slot: the packed-operand buffers of the
   // issuing stream (0 main, 1 stream2, 2 stream3)
   auto update = [&](int64_t r0, int64_t c_hi, int64_t jcol, int K, const C *Wb, int woff, int slot) {
     const int64_t rest = N - r0;
     if (rest <= 0 || c_hi <= r0) return;
+    if (planning) {
+      need[slot] = std::max(need[slot], dmb::oz64_bytes(rest, c_hi - r0, K));
+      return;
+    }
     kt_begin(c);
     if (use_tc) {
       dmb::tc_ldlt_update_c64(c, N, r0, c_hi, jcol, K, (float2 *)F, (const float2 *)Wb, NBW, woff, slot);
     } else if constexpr (std::is_same<C, double2>::value) {
       const double2 *Wk = (const double2 *)Wb + r0 * NBW + woff, *Lk = (const double2 *)F + r0 * N + jcol;
-      if (dmb::oz64_available(c, K) && dmb::oz64_reserve(c, rest, c_hi - r0, K, slot))
+      if (bal && dmb::oz64_available(c, K))
         dmb::oz64_lower_update(c, rest, c_hi - r0, K, Wk, NBW, Lk, N, bal + jcol, bal + N + jcol,
                                (double2 *)F + r0 * N + r0, N, slot, err);
       else
-        // the FP64-pipe GEMM (128 x 64 tiles, lower triangle)
+        // the FP64-pipe GEMM (lower triangle)
         dmb::zgemm64_lower_update(c, rest, c_hi - r0, K, Wk, NBW, Lk, N, (double2 *)F + r0 * N + r0, N);
     } else {
       dim3 g(blocks_for(rest, 64), blocks_for(c_hi - r0, 64));
@@ -1068,6 +1072,7 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
   // everything issued so far on the main stream
   auto side = [&](int which, int64_t lo, int64_t hi, int64_t jcol, int K, const C *Wb, int woff) {
     if (lo >= hi || lo >= N) return;
+    if (planning) return update(lo, hi, jcol, K, Wb, woff, which);
     cudaStream_t s = which == 1 ? c->stream2 : c->stream3;
     cudaEvent_t start = c->la_ev[which == 1 ? 0 : 2], done = c->la_ev[which == 1 ? 1 : 3];
     DMB_CUDA(cudaEventRecord(start, c->stream));
@@ -1109,19 +1114,27 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
     side(1, c1, c2, jcol, K, Wb, 0);
     side(2, c2, N, jcol, K, Wb, 0);
   };
-  int64_t bc = 0;
-  for (int64_t J2 = 0; J2 < N; J2 += NBW, bc++) {
-    C *Wb = c->d_W.as<C>() + (bc & 1) * N * NBW;
-    const int64_t J2E = std::min<int64_t>(N, J2 + NBW);
-    for (int64_t J = J2; J < J2E; J += NBO) {
-      const int64_t JE = std::min<int64_t>(J2E, J + NBO);
-      DMB_LAUNCH(c, k_ldlt_mid<C>, blocks_for(N - J, NB), 256, DiagSmem<C>::bytes, N, J, (int)(JE - J), F, Linv,
-                 Wb + (J - J2), NBW, bal, step_sync + MID_WORDS * (J / NBO), err,
-                 c->spin_limit);
-      update_block_column(JE, J2E, J, (int)(JE - J), Wb, (int)(J - J2));
+  auto schedule = [&] {
+    int64_t bc = 0;
+    for (int64_t J2 = 0; J2 < N; J2 += NBW, bc++) {
+      C *Wb = c->d_W.as<C>() + (bc & 1) * N * NBW;
+      const int64_t J2E = std::min<int64_t>(N, J2 + NBW);
+      for (int64_t J = J2; J < J2E; J += NBO) {
+        const int64_t JE = std::min<int64_t>(J2E, J + NBO);
+        if (!planning)
+          DMB_LAUNCH(c, k_ldlt_mid<C>, blocks_for(N - J, NB), 256, DiagSmem<C>::bytes, N, J, (int)(JE - J), F, Linv,
+                     Wb + (J - J2), NBW, bal, step_sync + MID_WORDS * (J / NBO), err, c->spin_limit);
+        update_block_column(JE, J2E, J, (int)(JE - J), Wb, (int)(J - J2));
+      }
+      update_trailing(J2E, J2, (int)(J2E - J2), Wb);
     }
-    update_trailing(J2E, J2, (int)(J2E - J2), Wb);
+  };
+  if (planning) {
+    schedule();
+    planning = false;
+    if (need[0] > 0 && dmb::oz64_reserve(c, N, need)) bal = c->oz64.buf.as<double>();
   }
+  schedule();
   join2();
   join3();
   unsigned h_err = 0;

@@ -179,11 +179,12 @@ struct FarTileState {
   DevBuf d_panels, d_cnt, d_tasks, d_job, d_err;
 };
 
-// Operand planes, scales and residue planes of the complex128 factor updates on
-// the INT8 tensor cores (dmb_oz64.cu), one set per issuing stream.
+// Buffer of the complex128 factor updates on the INT8 tensor cores
+// (dmb_oz64.cu): per factor column 2^-e (scales W) and 2^e (scales L), then a
+// part per issuing stream
 struct Oz64State {
-  DevBuf planes[3], scale[3], res[3];
-  DevBuf bal;  // per factor column 2^-e (scales W) and 2^e (scales L)
+  DevBuf buf;
+  size_t part[3] = {0, 0, 0};
   bool attr = false;
 };
 
@@ -448,10 +449,12 @@ void zgemm64_sub(dmb_ctx *c, bool a_transposed, int64_t M, int64_t R, int64_t K,
 void zgemm64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int64_t K, const double2 *W, int64_t ldw,
                           const double2 *Lrows, int64_t ldl, double2 *F, int64_t ldf);
 // the same update on the INT8 tensor cores (dmb_oz64.cu), K 256 or 1024, with
-// the buffers of `slot`; err gets bit 8 when a pipeline wait expires.
-// oz64_reserve: false when the buffers cannot be allocated
+// the part of `slot` of the buffer; err gets bit 8 when a pipeline wait expires.
+// oz64_reserve: room for N columns' scales and the largest updates of the three
+// slots, false when it cannot be had
 bool oz64_available(dmb_ctx *c, int K);
-bool oz64_reserve(dmb_ctx *c, int64_t M, int64_t C, int K, int slot);
+size_t oz64_bytes(int64_t M, int64_t C, int K);
+bool oz64_reserve(dmb_ctx *c, int64_t N, const size_t (&bytes)[3]);
 void oz64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int K, const double2 *W, int64_t ldw, const double2 *L,
                        int64_t ldl, const double *balW, const double *balL, double2 *F, int64_t ldf, int slot,
                        unsigned *err);

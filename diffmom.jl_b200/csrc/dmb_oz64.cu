@@ -455,8 +455,19 @@ const Sched64 &sched64() {
 int64_t up(int64_t v, int64_t m) { return ((v + m - 1) / m) * m; }
 
 // Operand and residue planes are made for at most this many rows / columns at
-// a time (multiples of 128): 0.5 GB a slot whatever the matrix size.
+// a time (multiples of 128): 0.8 GB a stream whatever the matrix size.
 constexpr int64_t O6_ROWS_1024 = 4096, O6_ROWS_256 = 16384, O6_COLS = 4096;
+
+// A stream's part of the buffer: operand planes, row scales of both operands,
+// residue planes of `tiles` tiles, for padded sizes mp x cp
+struct Part64 {
+  size_t scale, res, end;
+  Part64(int64_t mp, int64_t cp, int64_t tiles, int K) {
+    scale = up((int64_t)OZ_NMOD64 * 2 * (mp + cp) * K, 1024);
+    res = scale + up(sizeof(double) * (mp + cp), 1024);
+    end = res + (size_t)tiles * O6_RES_TILE;
+  }
+};
 
 }  // namespace
 
@@ -464,14 +475,25 @@ namespace dmb {
 
 bool oz64_available(dmb_ctx *c, int K) { return tc_available(c) && (K == 256 || K == 1024); }
 
-bool oz64_reserve(dmb_ctx *c, int64_t M, int64_t C, int K, int slot) {
-  Oz64State &st = c->oz64;
+// bytes an update of M rows and C columns needs of its stream's part
+size_t oz64_bytes(int64_t M, int64_t C, int K) {
   const int64_t mc = up(std::min(M, K == 1024 ? O6_ROWS_1024 : O6_ROWS_256), O6_BM), cc = up(std::min(C, O6_COLS), O6_BN);
   const Tiles64 tl{(int)(mc / O6_BM), (int)(cc / O6_BN), M > mc ? cc / O6_BN : 0};
+  return Part64(mc, cc, tl.count(), K).end;
+}
+
+// One buffer for a factorisation's three streams and its column scales: an
+// allocation takes 0.33 ms and a release 0.3, whatever their size, so nothing grows on
+// the way (nine buffers that did cost the first factorisation of a context 5 ms)
+bool oz64_reserve(dmb_ctx *c, int64_t N, const size_t (&bytes)[3]) {
+  Oz64State &st = c->oz64;
+  size_t at = up(sizeof(double) * 2 * N, 1024);
+  for (int s = 0; s < 3; s++) {
+    st.part[s] = at;
+    at += up(bytes[s], 1024);
+  }
   try {
-    st.planes[slot].ensure((size_t)OZ_NMOD64 * 2 * (mc + cc) * K);
-    st.scale[slot].ensure(sizeof(double) * (mc + cc));
-    st.res[slot].ensure((size_t)tl.count() * O6_RES_TILE);
+    st.buf.ensure(at);
   } catch (const DmbError &) {
     (void)cudaGetLastError();  // no room: the caller keeps to the FP64 pipe
     return false;
@@ -495,8 +517,11 @@ void oz64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int K, const double2 *W
       const Tiles64 tl{(int)(nmp / O6_BM), (int)(ncp / O6_BN), (m0 - c0) / O6_BN};
       const int64_t ntiles = tl.count();
       if (ntiles == 0) continue;
-      double *rs = st.scale[slot].as<double>(), *cs = rs + nmp;
-      signed char *PA = st.planes[slot].as<signed char>(), *PB = PA + (size_t)OZ_NMOD64 * 2 * nmp * K;
+      const Part64 part(nmp, ncp, ntiles, K);
+      char *base = st.buf.as<char>() + st.part[slot];
+      double *rs = (double *)(base + part.scale), *cs = rs + nmp;
+      signed char *PA = (signed char *)base, *PB = PA + (size_t)OZ_NMOD64 * 2 * nmp * K;
+      unsigned char *res = (unsigned char *)(base + part.res);
       const Operand64 A{W + m0 * ldw, ldw, nm, nmp, balW, rs, PA}, B{L + c0 * ldl, ldl, nc, ncp, balL, cs, PB};
       const unsigned g = (unsigned)((nmp + ncp) / (1024 / K));
       if (K == 1024)
@@ -510,17 +535,13 @@ void oz64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int K, const double2 *W
                      OZ_BK, OZ_BN);
       const int64_t G = std::min<int64_t>(ntiles * OZ_NMOD64, c->sm_count);
       DMB_LAUNCH(c, k_oz64_gemm, (unsigned)G, O6_THREADS, O6_SMEM, mA, mB, sched64(), K / OZ_BK, tl, ntiles,
-                 (int)(2 * nmp), (int)(2 * ncp), st.res[slot].as<unsigned char>(), err);
+                 (int)(2 * nmp), (int)(2 * ncp), res, err);
       DMB_LAUNCH(c, k_oz64_crt, (unsigned)(ntiles * 8), 256, 0, sched64(), tl, nm, nc, m0, c0, (const double *)rs,
-                 (const double *)cs, F + m0 * ldf + c0, ldf, st.res[slot].as<unsigned char>());
+                 (const double *)cs, F + m0 * ldf + c0, ldf, res);
     }
   }
 }
 
-void oz64_release(dmb_ctx *c) {
-  for (int s = 0; s < 3; s++)
-    for (DevBuf *b : {&c->oz64.planes[s], &c->oz64.scale[s], &c->oz64.res[s]}) b->release();
-  c->oz64.bal.release();
-}
+void oz64_release(dmb_ctx *c) { c->oz64.buf.release(); }
 
 }  // namespace dmb
