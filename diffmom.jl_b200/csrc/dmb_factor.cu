@@ -600,7 +600,7 @@ __device__ __forceinline__ bool wait_word(volatile unsigned *flag, unsigned *err
       atomicOr(err, 4u);
       return false;
     }
-    if ((it & 15) == 0 && (*(volatile unsigned *)err & 4u)) return false;
+    if ((it & 255) == 0 && (*(volatile unsigned *)err & 4u)) return false;
     __nanosleep(32);
   }
   __threadfence();
