@@ -989,12 +989,21 @@ template <class C> void set_smem_attrs() {
 constexpr int NBO = 256;
 constexpr int NBW = 1024;
 
+// W is free once a factorisation is done.  Until the next one it holds the
+// 256-row block inverses of the few-column sweeps and, behind them, the products
+// of prepare_block_inverses: two allocations less for a context's first solve.
+size_t inverse_products_at(int64_t N) { return sizeof(double2) * N * 256; }
+size_t inverse_bytes(int64_t N) {
+  const size_t few = sizeof(double2) * ((N + 255) / 256) * 256 * 64, many = sizeof(float2) * ((N + 1023) / 1024) * 1024 * 256;
+  return inverse_products_at(N) + std::max(few, many);
+}
+
 template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
   c->f_version++;  // F changes from here on: packed copies are stale
   const int64_t N = c->n;
   set_smem_attrs<C>();
   const int nblk = (int)((N + NB - 1) / NB);
-  c->d_W.ensure(sizeof(C) * N * NBW * 2);
+  c->d_W.ensure(std::max(sizeof(C) * N * NBW * 2, inverse_bytes(N)));
   c->d_dinv.ensure(sizeof(C) * (size_t)nblk * NB * NB);  // Linv blocks
   // err word, then the tickets and flags of each middle panel
   const size_t flag_words = 4 + MID_WORDS * (size_t)((N + NBO - 1) / NBO);
@@ -1445,23 +1454,17 @@ __global__ void __launch_bounds__(256) k_inv_level(int64_t N, int s, const FC *_
     }
 }
 
-// Pack the complex64 factor for the tensor-core sweeps (once per
-// factorisation): L'' and (L^T)'', and the inverses of the 1024-row diagonal
-// blocks of L (recursive doubling, k_inv_init / k_inv_level).
 // The block inverses of L (once per factorisation): 1024-row ones by FP32
 // products into d_trsm_id for the tensor-core sweeps (which round them to TF32
-// anyway), 256-row ones by FP64 products into d_sv_inv for the few-column
-// sweeps (as accurate as substitution with the stored 64-block inverses).
+// anyway), 256-row ones by FP64 products into W for the few-column sweeps (as
+// accurate as substitution with the stored 64-block inverses).
 template <int OB, class FC, class TC>
-void prepare_block_inverses(dmb_ctx *c, const FC *F, DevBuf &dst, uint64_t &ver) {
+void prepare_block_inverses(dmb_ctx *c, const FC *F, double2 *Xid, uint64_t &ver) {
   if (ver == c->f_version) return;
   const int64_t N = c->n;
-  dst.ensure(sizeof(double2) * N * OB);
-  double2 *Xid = dst.as<double2>();
   const int64_t nout = (N + OB - 1) / OB;
-  // scratch for the products T: (pair slots) x s x s <= nout x OB x OB / 4
-  c->d_trsm_t.ensure(sizeof(TC) * nout * OB * (OB / 4));
-  TC *T = c->d_trsm_t.as<TC>();
+  // the products T: (pair slots) x s x s <= nout x OB x OB / 4
+  TC *T = reinterpret_cast<TC *>(c->d_W.as<char>() + inverse_products_at(N));
   DMB_LAUNCH(c, (k_inv_init<OB, FC>), blocks_for(N * OB, 256), 256, 0, N, c->d_dinv.as<FC>(), Xid);
   for (int s = NB; s < OB && s < N; s *= 2) {
     const int nt = (s + 63) / 64;
@@ -1472,13 +1475,16 @@ void prepare_block_inverses(dmb_ctx *c, const FC *F, DevBuf &dst, uint64_t &ver)
   ver = c->f_version;
 }
 
+// Pack the complex64 factor for the tensor-core sweeps (once per
+// factorisation): L'' and (L^T)'', and the 1024-row block inverses.
 void prepare_packed_factor(dmb_ctx *c, const float2 *F) {
   if (c->f_packed == c->f_version) return;
   const int64_t N = c->n;
   trsm_panel_attrs<float2>();
   dmb::tc_trsm_pack_factor(c, F, N);
-  prepare_block_inverses<TP_OUTER, float2, float2>(c, F, c->d_trsm_id, c->f_inv);
+  c->d_trsm_id.ensure(sizeof(double2) * N * TP_OUTER);
   double2 *Xid = c->d_trsm_id.as<double2>();
+  prepare_block_inverses<TP_OUTER, float2, float2>(c, F, Xid, c->f_inv);
   const int64_t nout = (N + TP_OUTER - 1) / TP_OUTER;
   for (int64_t o = 0; o < nout; o++) {
     const int64_t o0 = o * TP_OUTER, o1 = std::min<int64_t>(N, o0 + TP_OUTER);
@@ -1710,8 +1716,8 @@ __global__ void __launch_bounds__(256, 2) k_sweep_bwd(int64_t N, const FC *__res
 
 template <class C> void ldlt_solve(dmb_ctx *c, const C *F, double2 *x, int64_t R) {
   const int64_t N = c->n;
-  prepare_block_inverses<SV, C, double2>(c, F, c->d_sv_inv, c->f_inv64);
-  const double2 *X = c->d_sv_inv.as<double2>();
+  double2 *X = c->d_W.as<double2>();
+  prepare_block_inverses<SV, C, double2>(c, F, X, c->f_inv64);
   static std::once_flag once;
   std::call_once(once, [] {
     DMB_CUDA(cudaFuncSetAttribute(k_sweep_fwd<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SweepSmem)));
@@ -1868,9 +1874,9 @@ void pc_prepare_dev(dmb_ctx *c, int64_t nrhs) {
     return;
   }
   if (c->pc_prec == DMB_PREC_FP64)
-    prepare_block_inverses<SV, double2, double2>(c, c->d_F.as<double2>(), c->d_sv_inv, c->f_inv64);
+    prepare_block_inverses<SV, double2, double2>(c, c->d_F.as<double2>(), c->d_W.as<double2>(), c->f_inv64);
   else
-    prepare_block_inverses<SV, float2, double2>(c, c->d_F.as<float2>(), c->d_sv_inv, c->f_inv64);
+    prepare_block_inverses<SV, float2, double2>(c, c->d_F.as<float2>(), c->d_W.as<double2>(), c->f_inv64);
 }
 
 void pc_apply_dev(dmb_ctx *c, double *x, int64_t nrhs) {

@@ -256,7 +256,7 @@ struct dmb_ctx {
   int pc_prec = -1;
   DevBuf d_F;         // factor storage (N x N, L strictly lower + D diagonal)
   DevBuf d_dinv;      // Jacobi inverse diagonal
-  DevBuf d_W;         // LDL^T panel workspace
+  DevBuf d_W;         // LDL^T panel workspace; then 256-row block inverses of the factor
   DevBuf d_flags;     // triangular-solve progress flags / error word
   Oz64State oz64;
   double nnz_ratio = 0;
@@ -322,13 +322,12 @@ struct dmb_ctx {
   uint64_t f_version = 0;        // bumped by every LDL^T factorisation
   uint64_t f_packed = ~0ull;     // factor version packed for the batched triangular solves
   uint64_t f_inv = ~0ull;        // factor version whose 1024-row block inverses are in d_trsm_id
-  uint64_t f_inv64 = ~0ull;      // ... whose 256-row block inverses (FP64 products) are in d_sv_inv
-  DevBuf d_sv_acc, d_sv_inv;     // the few-column sweeps: scratch and block inverses
+  uint64_t f_inv64 = ~0ull;      // ... whose 256-row block inverses (FP64 products) are in d_W
+  DevBuf d_sv_acc;               // exchange buffers of the few-column sweeps
   // inputs of the current host topology (build_host_topology)
   bool topo_valid = false;
   std::vector<int32_t> topo_tri, topo_tplus, topo_tminus;
   DevBuf d_trsm_id;              // scratch: inverses of the 1024-row diagonal blocks of L
-  DevBuf d_trsm_t;               // scratch: products of the recursive-doubling levels
   int gm_kcap = 0;              // cached GMRES basis capacity
   int64_t gm_key_n = 0, gm_key_r = 0;
   int gm_key_maxiter = 0;
