@@ -540,6 +540,7 @@ __global__ void __launch_bounds__(256) k_mf_far(int nt, int nq, const TriCache *
 // distance is taken once per triangle pair (phase_exp).  Bound by the FP64 pipe.
 // Chunks give the parallelism; their partial sums are added in order.
 constexpr int MF_TB = 32;     // source triangles per shared tile
+constexpr int MF_CHUNK = 4;   // fewest source triangles per chunk
 constexpr int MF_F = 11;      // per source point: position, current (3 complex), charge (complex)
 
 // source points of every triangle: src[(q MF_F + f) nt + t]
@@ -845,9 +846,17 @@ void matvec_free_dev(dmb_ctx *c, const double *x, double *y) {
   DMB_REQUIRE(c->cache_valid && c->k != 0.0, DMB_ERR_STATE, "operator not prepared");
   const int64_t N = c->n;
   const int nt = (int)c->nt, nq = c->nq, qt = std::min(nq, 4), nz = (nq + qt - 1) / qt;
-  // source chunks (multiples of the shared tile) for about four CTAs per SM
-  const int gx = (nt + 127) / 128, want = std::max(1, (4 * c->sm_count + gx * nz - 1) / (gx * nz));
-  const int chunk = std::max(MF_TB, (nt + want - 1) / want / MF_TB * MF_TB), nchunk = (nt + chunk - 1) / chunk;
+  // source chunks for about four CTAs per SM, multiples of the shared tile; where
+  // that leaves less than a tile, two CTAs per SM and as little as MF_CHUNK: a
+  // CTA walks its chunk alone (280 unknowns, 7 points: 242 us with whole tiles, 105
+  // with chunks of 4; 1,026 unknowns: 288 with tiles, 320 with chunks for four CTAs)
+  const int gx = (nt + 127) / 128;
+  auto per_sm = [&](int ctas) {
+    const int want = std::max(1, (ctas * c->sm_count + gx * nz - 1) / (gx * nz));
+    return (nt + want - 1) / want;
+  };
+  const int chunk = per_sm(4) >= MF_TB ? per_sm(4) / MF_TB * MF_TB : std::min(MF_TB, std::max(MF_CHUNK, per_sm(2)));
+  const int nchunk = (nt + chunk - 1) / chunk;
   const size_t src_bytes = sizeof(double) * MF_F * nq * nt;
   c->d_mf.ensure(src_bytes + sizeof(double2) * 3 * nt * nchunk * nz + 16);
   double *src = c->d_mf.as<double>();

@@ -31,6 +31,14 @@ def test_matrix_free_matches_dense(nx, ny, quad_order):
     _check(make_rect_plate(0.01 * nx, 0.01 * ny, nx, ny), quad_order)
 
 
+# chunks of 4, of an odd size between, and of a whole tile (4, 392 and 1,250 triangles)
+@pytest.mark.parametrize("quad_order", [1, 7])
+@pytest.mark.parametrize("nx,ny", [(1, 2), (14, 14), (25, 25)])
+def test_matrix_free_chunks(nx, ny, quad_order):
+    from diffmom_b200 import make_rect_plate
+    _check(make_rect_plate(0.01 * nx, 0.01 * ny, nx, ny), quad_order)
+
+
 def test_matrix_free_junction():
     from diffmom_b200 import TriMesh, make_rect_plate
     m = make_rect_plate(0.1, 0.1, 4, 4)
