@@ -390,7 +390,6 @@ struct AcaGeo {
   const int *ptri;    // their triangles, [2][np]
   const int *ipos;    // basis function -> position
   int64_t np;
-  const int *rslot;
   const int *aoff, *anb;
   const int2 *near_mn;
   const int64_t *near_off;
@@ -1137,10 +1136,8 @@ __global__ void k_aca_diag_inv(int64_t N, const double2 *__restrict__ d, const d
     default: { constexpr int NQ = 7; CALL; } break; \
   }
 
-// the entries' geometry over the positions of `ids` (device, np of them), whose
-// points go to the buffers given; ipos may be null
-AcaGeo make_geo(dmb_ctx *c, int64_t np, const int *ids, DevBuf &pts, DevBuf &ptri, int *ipos) {
-  AcaGeo g;
+// quadrature data of the basis functions `ids` (device, np of them); ipos may be null
+void make_points(dmb_ctx *c, int64_t np, const int *ids, DevBuf &pts, DevBuf &ptri, int *ipos) {
   ACA_NQ_DISPATCH(c->nq, {
     pts.ensure(sizeof(double) * 2 * std::max<int64_t>(np, 1) * aca_fields<NQ>());
     ptri.ensure(sizeof(int) * 2 * std::max<int64_t>(np, 1));
@@ -1148,11 +1145,14 @@ AcaGeo make_geo(dmb_ctx *c, int64_t np, const int *ids, DevBuf &pts, DevBuf &ptr
       DMB_LAUNCH(c, k_aca_points<NQ>, blocks_for(2 * np, 128), 128, 0, np, ids, c->d_tcache.as<TriCache>(),
                  c->d_rwg_slot.as<int>(), pts.as<double>(), ptri.as<int>(), ipos);
   });
+}
+// the entries' geometry over np positions whose points are given
+AcaGeo make_geo(dmb_ctx *c, int64_t np, const DevBuf &pts, const DevBuf &ptri, const int *ipos) {
+  AcaGeo g;
   g.pts = pts.as<double>();
   g.ptri = ptri.as<int>();
   g.ipos = ipos;
   g.np = np;
-  g.rslot = c->d_rwg_slot.as<int>();
   g.aoff = c->d_adj_off.as<int>();
   g.anb = c->d_adj_nb.as<int>();
   g.near_mn = c->d_near_entry_mn.as<int2>();
@@ -1164,11 +1164,15 @@ AcaGeo make_geo(dmb_ctx *c, int64_t np, const int *ids, DevBuf &pts, DevBuf &ptr
   g.omega_mu0 = c->aca.k * c->aca.eta0;
   return g;
 }
-// ... of the context's operator, in tree order
+// ... of the context's operator, in tree order; the points are made once per build
 AcaGeo make_geo(dmb_ctx *c) {
   AcaState &A = c->aca;
-  A.d_ipos.ensure(sizeof(int) * std::max<int64_t>(A.n, 1));
-  return make_geo(c, A.n, A.d_perm.as<int>(), A.d_pts, A.d_ptri, A.d_ipos.as<int>());
+  if (!A.points) {
+    A.d_ipos.ensure(sizeof(int) * std::max<int64_t>(A.n, 1));
+    make_points(c, A.n, A.d_perm.as<int>(), A.d_pts, A.d_ptri, A.d_ipos.as<int>());
+    A.points = true;
+  }
+  return make_geo(c, A.n, A.d_pts, A.d_ptri, A.d_ipos.as<int>());
 }
 
 template <class T> void upload(dmb_ctx *c, DevBuf &b, const std::vector<T> &v) {
@@ -1254,7 +1258,7 @@ void aca_build(dmb_ctx *c, double k, double eta0, int quad_order, int leaf_size,
   DMB_REQUIRE(std::isfinite(inv_k2) && std::isfinite(k * eta0) && k * eta0 != 0.0, DMB_ERR_OVERFLOW,
               "EFIE prefactors are not representable");
   AcaState &A = c->aca;
-  A.valid = false;  // the buffers stay for the new operator
+  A.valid = A.points = false;  // the buffers stay for the new operator
   c->op_kind = 0;
   prepare_operator(c, k, eta0, quad_order);  // triangle cache + near records for this k
   const int64_t N = c->n;
@@ -1558,7 +1562,7 @@ void aca_nf_build(dmb_ctx *c, int kind, int precision) {
     // admissible against itself); evaluate them directly
     std::vector<int> mn(2 * N);
     for (int64_t i = 0; i < N; i++) mn[2 * i] = mn[2 * i + 1] = (int)i;
-    ScratchBuf d_mn, d_diag, tmp;
+    DevBuf &d_mn = c->d_tmp[0], &d_diag = c->d_tmp[1], &tmp = c->d_tmp[2];
     upload(c, d_mn, mn);
     d_diag.ensure(sizeof(double2) * N);
     tmp.ensure(16);
@@ -1668,7 +1672,8 @@ int aca_lowrank_one(dmb_ctx *c, double k, double eta0, int quad_order, const std
   d_out.ensure(sizeof(int) * 3);
   DMB_CUDA(cudaMemsetAsync(d_out.p, 0, sizeof(int) * 3, c->stream));
   ScratchBuf d_pts, d_ptri;
-  AcaGeo g = make_geo(c, m + n, d_idx.as<int>(), d_pts, d_ptri, nullptr);
+  make_points(c, m + n, d_idx.as<int>(), d_pts, d_ptri, nullptr);
+  AcaGeo g = make_geo(c, m + n, d_pts, d_ptri, nullptr);
   g.k = k;
   g.inv_k2 = 1.0 / (k * k);
   g.omega_mu0 = k * eta0;

@@ -144,6 +144,7 @@ struct AcaState {
   DevBuf d_row_zbase, d_col_zbase;        // per leaf item: partial offset minus the block's first row / column
   DevBuf d_ids, d_foff, d_soff, d_flags, d_scr, d_status, d_conv;  // the build's workspace
   DevBuf d_pts, d_ptri, d_ipos;           // quadrature data of the basis functions in tree order
+  bool points = false;                    // ... are those of the operator being built or built
   int64_t n_leaves = 0, n_lr = 0, t_total = 0;
   double k = 0, eta0 = 0;
   int quad_order = 3;
@@ -153,7 +154,7 @@ struct AcaState {
                    &d_row_zbase, &d_col_zbase, &d_ids, &d_foff, &d_soff, &d_flags, &d_scr, &d_status, &d_conv,
                    &d_pts, &d_ptri, &d_ipos};
     for (DevBuf *x : b) x->release();
-    valid = false;
+    valid = points = false;
   }
 };
 
