@@ -434,7 +434,7 @@ __global__ void k_aca_points(int64_t np, const int *__restrict__ ids, const TriC
   }
   double r2 = 0;
   for (int v = 0; v < 3; v++) {
-    const double x = T.p[v][0] - T.cen[0], y = T.p[v][1] - T.cen[1], z = T.p[v][2] - T.cen[2];
+    const double x = T.v[v][0] - T.cen[0], y = T.v[v][1] - T.cen[1], z = T.v[v][2] - T.cen[2];
     r2 = fmax(r2, x * x + y * y + z * z);
   }
   for (int c = 0; c < 3; c++) o[(7 * NQ + c) * np] = T.cen[c];

@@ -7,7 +7,8 @@ import math
 import numpy as np
 import pytest
 
-from diffmom_b200 import (EFIEDevice, make_rect_plate, build_rwg, build_aca_operator, build_efie_cache, aca_lowrank)
+from diffmom_b200 import (EFIEDevice, RWGData, TriMesh, aca_lowrank, build_aca_operator, build_efie_cache, build_rwg,
+                          make_rect_plate)
 
 pytestmark = pytest.mark.gpu
 
@@ -59,3 +60,31 @@ def test_lowrank_of_index_lists(m_rows, n_cols):
     S = Z[np.ix_(rows, cols)]
     assert U.shape[1] == V.shape[1] <= q
     assert np.linalg.norm(U @ V.conj().T - S) <= 100 * (q * q + 30) * EPS * np.linalg.norm(S)
+
+
+def test_neighbours_without_a_common_basis_function():
+    """Two slender triangles with a common edge that carries no basis function;
+    all slots of each belong to another edge, where three triangles are
+    attached.  Their entries take the near terms as the dense matrix does."""
+    L, e = 0.01, 0.001
+    v1, v2, v3, w = [-L, 3 * e, 0], [0, e, 0], [0, -e, 0], [L, -3 * e, 0]
+    tips = [[x, 0, z] for x in (-L / 2, L / 2) for z in (0.004, -0.005, 0.007)]
+    xyz = np.array([v1, v2, v3, w] + tips)
+    tri = np.array([[1, 2, 3], [4, 3, 2]] + [[1, 3, 5 + i] for i in range(3)] + [[4, 2, 8 + i] for i in range(3)])
+    mesh = TriMesh(xyz, tri)
+    one, edge = np.repeat([1, 2], 3), np.repeat([[1, 3], [2, 4]], 3, axis=0)
+    length = np.linalg.norm(xyz[edge[:, 0] - 1] - xyz[edge[:, 1] - 1], axis=1)
+    T = xyz[tri - 1]
+    area = 0.5 * np.linalg.norm(np.cross(T[:, 1] - T[:, 0], T[:, 2] - T[:, 0]), axis=1)
+    tminus = np.arange(3, 9)
+    rwg = RWGData(mesh=mesh, nedges=6, tplus=one, tminus=tminus, evert=edge, vplus_opp=np.repeat([2, 3], 3),
+                  vminus_opp=np.arange(5, 11), len=length, area_plus=area[one - 1], area_minus=area[tminus - 1],
+                  coeff_plus=np.ones(6), coeff_minus=np.ones(6))
+    dev = EFIEDevice(mesh, rwg)
+    Z = dev.assemble(K, copy_out=True)
+    dev.close()
+    A = build_aca_operator(mesh, rwg, K)
+    i, j = np.divmod(np.arange(36), 6)
+    E = A.entries(i + 1, j + 1).reshape(6, 6)
+    A.close()
+    assert np.abs(E - Z).max() <= _bound(Z, 3)
