@@ -969,13 +969,6 @@ __global__ void k_scale_vec(int64_t N, int64_t R, const double2 *__restrict__ d,
   x[i] = cmul(x[i], d[i % N]);
 }
 
-template <class C> void set_smem_attrs() {
-  static bool done = false;
-  if (done) return;
-  DMB_CUDA(cudaFuncSetAttribute(k_ldlt_mid<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DiagSmem<C>::bytes));
-  done = true;
-}
-
 // Three-level right-looking LDL^T.  Block columns of NBW = 1024 are factored
 // as 256-wide middle panels (one launch each).  After each middle panel the rest of the 1024-wide block column
 // receives one K = 256 update, and after the block column the whole trailing
@@ -1001,7 +994,7 @@ size_t inverse_bytes(int64_t N) {
 template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
   c->f_version++;  // F changes from here on: packed copies are stale
   const int64_t N = c->n;
-  set_smem_attrs<C>();
+  raise_smem(c, k_ldlt_mid<C>, DiagSmem<C>::bytes);
   const int nblk = (int)((N + NB - 1) / NB);
   c->d_W.ensure(std::max(sizeof(C) * N * NBW * 2, inverse_bytes(N)));
   c->d_dinv.ensure(sizeof(C) * (size_t)nblk * NB * NB);  // Linv blocks
@@ -1296,13 +1289,12 @@ __global__ void __launch_bounds__(256) k_gemm_sub(int64_t M, int64_t R, int K, c
     }
 }
 
-template <class C> void trsm_panel_attrs() {
-  static bool done = false;
-  if (done) return;
-  const int sm = (int)(sizeof(C) * 64 * 65 + sizeof(double2) * TP * (TP_COLS + 1));
-  DMB_CUDA(cudaFuncSetAttribute(k_trsm_panel<C, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-  DMB_CUDA(cudaFuncSetAttribute(k_trsm_panel<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-  done = true;
+template <class C> constexpr size_t trsm_panel_smem() {
+  return sizeof(C) * 64 * 65 + sizeof(double2) * TP * (TP_COLS + 1);
+}
+template <class C> void trsm_panel_attrs(dmb_ctx *c) {
+  raise_smem(c, k_trsm_panel<C, false>, trsm_panel_smem<C>());
+  raise_smem(c, k_trsm_panel<C, true>, trsm_panel_smem<C>());
 }
 
 // X[r_lo : r_hi] -= L[r_lo : r_hi, k_lo : k_lo + w] X[k_lo : k_lo + w]   (forward)
@@ -1340,7 +1332,7 @@ constexpr int TP_OUTER = 1024;
 // forward solve restricted to rows [o0, o1): L[o0:o1, o0:o1] y = x
 template <class C> void forward_block(dmb_ctx *c, const C *F, int64_t o0, int64_t o1, double2 *X, int64_t R) {
   const int64_t N = c->n;
-  const size_t sm = sizeof(C) * 64 * 65 + sizeof(double2) * TP * (TP_COLS + 1);
+  const size_t sm = trsm_panel_smem<C>();
   for (int64_t p0 = o0; p0 < o1; p0 += TP) {
     const int w = (int)std::min<int64_t>(TP, o1 - p0);
     DMB_LAUNCH(c, (k_trsm_panel<C, false>), blocks_for(R, TP_COLS), 256, sm, N, R, p0, w, F, c->d_dinv.as<C>(), X);
@@ -1480,7 +1472,7 @@ void prepare_block_inverses(dmb_ctx *c, const FC *F, double2 *Xid, uint64_t &ver
 void prepare_packed_factor(dmb_ctx *c, const float2 *F) {
   if (c->f_packed == c->f_version) return;
   const int64_t N = c->n;
-  trsm_panel_attrs<float2>();
+  trsm_panel_attrs<float2>(c);
   dmb::tc_trsm_pack_factor(c, F, N);
   c->d_trsm_id.ensure(sizeof(double2) * N * TP_OUTER);
   double2 *Xid = c->d_trsm_id.as<double2>();
@@ -1718,11 +1710,8 @@ template <class C> void ldlt_solve(dmb_ctx *c, const C *F, double2 *x, int64_t R
   const int64_t N = c->n;
   double2 *X = c->d_W.as<double2>();
   prepare_block_inverses<SV, C, double2>(c, F, X, c->f_inv64);
-  static std::once_flag once;
-  std::call_once(once, [] {
-    DMB_CUDA(cudaFuncSetAttribute(k_sweep_fwd<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SweepSmem)));
-    DMB_CUDA(cudaFuncSetAttribute(k_sweep_bwd<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SweepSmem)));
-  });
+  raise_smem(c, k_sweep_fwd<C>, sizeof(SweepSmem));
+  raise_smem(c, k_sweep_bwd<C>, sizeof(SweepSmem));
   // a and y of the forward sweep, a and x of the backward one, all empty
   c->d_sv_acc.ensure(sizeof(double2) * 4 * N * R);
   double2 *buf = c->d_sv_acc.as<double2>();
@@ -1741,7 +1730,7 @@ template <class C> void ldlt_solve(dmb_ctx *c, const C *F, double2 *x, int64_t R
 template <class C> void ldlt_solve_batched(dmb_ctx *c, const C *F, double2 *X, int64_t R) {
   const int64_t N = c->n;
   const C *Linv = c->d_dinv.as<C>();
-  trsm_panel_attrs<C>();
+  trsm_panel_attrs<C>(c);
   if (std::is_same<C, float2>::value && R >= c->tc_min_rhs && dmb::tc_available(c)) {
     // tensor cores: every step is a GEMM on operands packed once per factor
     prepare_packed_factor(c, (const float2 *)F);
@@ -1750,7 +1739,7 @@ template <class C> void ldlt_solve_batched(dmb_ctx *c, const C *F, double2 *X, i
     dmb::tc_trsm_sweep(c, N, X, R, true);
     return;
   }
-  const size_t sm = sizeof(C) * 64 * 65 + sizeof(double2) * TP * (TP_COLS + 1);
+  const size_t sm = trsm_panel_smem<C>();
   const unsigned gcols = blocks_for(R, TP_COLS);
   const int64_t nout = (N + TP_OUTER - 1) / TP_OUTER;
   for (int64_t o = 0; o < nout; o++) {

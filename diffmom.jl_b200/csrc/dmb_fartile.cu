@@ -388,10 +388,7 @@ size_t far_smem_bytes() {
 template <int NQ, int T, bool F64>
 void far_launch_t(dmb_ctx *c, const FarJob *d_jobs, const int4 *d_tasks, int64_t ntasks, unsigned *err) {
   const size_t smem = far_smem_bytes<NQ, T, F64>();
-  static std::once_flag once;
-  std::call_once(once, [&] {
-    cudaFuncSetAttribute(k_far_tile<NQ, T, F64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  });
+  raise_smem(c, k_far_tile<NQ, T, F64>, smem);
   DMB_LAUNCH(c, (k_far_tile<NQ, T, F64>), (unsigned)ntasks, FarThreads<F64>::value, smem, d_jobs, d_tasks, err);
 }
 

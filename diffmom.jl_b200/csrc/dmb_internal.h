@@ -186,7 +186,6 @@ struct FarTileState {
 struct Oz64State {
   DevBuf buf;
   size_t part[3] = {0, 0, 0};
-  bool attr = false;
 };
 
 struct HostCopy;
@@ -339,6 +338,7 @@ struct dmb_ctx {
   // timings
   dmb_timings tm{};
   int64_t launches = 0;
+  std::vector<const void *> smem_raised;  // kernels whose shared-memory limit is raised (raise_smem)
   bool kt_enabled = false;     // dominant-kernel event timing
   // per family: 0 3xTF32 Krylov / sweep GEMMs, 1 int8 GEMMs, 2 factor updates,
   // 3 H-matrix products (one right-hand side, work in bytes), 4 FP64-pipe
@@ -389,6 +389,16 @@ inline void kt_collect(dmb_ctx *c) {
   c->kt_used = 0;
   c->kt_pending.clear();
   c->kt_family.clear();
+}
+
+// A kernel's limit of dynamic shared memory belongs to a device: raised once per
+// context (a process may have contexts on several devices)
+template <class K> void raise_smem(dmb_ctx *c, K *kernel, size_t bytes) {
+  const void *f = reinterpret_cast<const void *>(kernel);
+  for (const void *k : c->smem_raised)
+    if (k == f) return;
+  DMB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  c->smem_raised.push_back(f);
 }
 
 // Runs the enclosed launches of a context on another stream (the context is

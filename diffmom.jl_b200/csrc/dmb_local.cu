@@ -770,17 +770,8 @@ LocalState &lstate(dmb_ctx *c) {
 template <int KM, class CT> void launch_local_inverse(dmb_ctx *c, const int *idx, const int *cnt, double2 *rows,
                                                       unsigned *err) {
   const size_t sm = sizeof(CT) * (KM * (KM + 1) + KM);
-  static bool attr = false;
-  if (!attr) {
-    if (c->z_prec == DMB_PREC_FP64)
-      DMB_CUDA(cudaFuncSetAttribute(k_local_inverse<KM, CT, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)sm));
-    DMB_CUDA(cudaFuncSetAttribute(k_local_inverse<KM, CT, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sm));
-    DMB_CUDA(cudaFuncSetAttribute(k_local_inverse<KM, CT, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sm));
-    attr = true;
-  }
+  raise_smem(c, k_local_inverse<KM, CT, float2>, sm);
+  raise_smem(c, k_local_inverse<KM, CT, double2>, sm);
   if (c->z_prec == DMB_PREC_FP64)
     DMB_LAUNCH(c, (k_local_inverse<KM, CT, double2>), (unsigned)c->n, 256, sm, c->n, c->d_Z.as<double2>(), idx, cnt,
                KM, rows, err);
@@ -793,11 +784,7 @@ void build_neighbors(dmb_ctx *c, double radius, int kmax, DevBuf &idx, DevBuf &c
   idx.ensure(sizeof(int) * c->n * kmax);
   cnt.ensure(sizeof(int) * c->n);
   const size_t sm = (sizeof(int) + sizeof(float)) * NCAND * NB_WARPS;
-  static bool attr = false;
-  if (!attr) {
-    DMB_CUDA(cudaFuncSetAttribute(k_neighbors, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    attr = true;
-  }
+  raise_smem(c, k_neighbors, sm);
   DMB_LAUNCH(c, k_neighbors, blocks_for(c->n, NB_WARPS), 32 * NB_WARPS, sm, c->n, c->d_centers.as<double>(), radius,
              kmax, idx.as<int>(), cnt.as<int>());
 }
@@ -1027,12 +1014,8 @@ void ls_rows(dmb_ctx *c, double radius) {
   e.p = c->d_small.p;
   DMB_CUDA(cudaMemsetAsync(e.p, 0, 4, c->stream));
   const size_t sm = sizeof(double2) * (KS * (KS + 1) + KS) + sizeof(float2) * KL * KS;
-  static bool attr = false;
-  if (!attr) {
-    DMB_CUDA(cudaFuncSetAttribute(k_spai_target<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    DMB_CUDA(cudaFuncSetAttribute(k_spai_target<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    attr = true;
-  }
+  raise_smem(c, k_spai_target<float2>, sm);
+  raise_smem(c, k_spai_target<double2>, sm);
   if (c->z_prec == DMB_PREC_FP64)
     DMB_LAUNCH(c, k_spai_target<double2>, (unsigned)N, 256, sm, N, c->d_Z.as<double2>(), st.idx_s.as<int>(),
                st.cnt_s.as<int>(), st.idx_l.as<int>(), st.cnt_l.as<int>(), st.rows_l.as<double2>(), e.as<unsigned>());

@@ -505,10 +505,7 @@ void oz64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int K, const double2 *W
                        int64_t ldl, const double *balW, const double *balL, double2 *F, int64_t ldf, int slot,
                        unsigned *err) {
   Oz64State &st = c->oz64;
-  if (!st.attr) {
-    DMB_CUDA(cudaFuncSetAttribute(k_oz64_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, O6_SMEM));
-    st.attr = true;
-  }
+  raise_smem(c, k_oz64_gemm, O6_SMEM);
   const int64_t mstep = K == 1024 ? O6_ROWS_1024 : O6_ROWS_256;
   for (int64_t c0 = 0; c0 < C; c0 += O6_COLS) {
     const int64_t nc = std::min(O6_COLS, C - c0), ncp = up(nc, O6_BN);

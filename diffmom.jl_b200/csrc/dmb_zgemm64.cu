@@ -124,12 +124,7 @@ template <int ALAY, int YLAY, int OP, bool LOWER>
 void launch(dmb_ctx *c, int64_t M, int64_t R, int64_t K, const double2 *A, int64_t lda, const double2 *B, int64_t ldb,
             double2 *Y, int64_t ldy) {
   if (M <= 0 || R <= 0) return;
-  static bool attr = false;  // one instantiation per template: set once per process
-  if (!attr) {
-    DMB_CUDA(cudaFuncSetAttribute(k_zgemm64<ALAY, YLAY, OP, LOWER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)ZG_SMEM));
-    attr = true;
-  }
+  raise_smem(c, k_zgemm64<ALAY, YLAY, OP, LOWER>, ZG_SMEM);
   dim3 g((unsigned)((M + ZG_BM - 1) / ZG_BM), (unsigned)((R + ZG_BN - 1) / ZG_BN));
   DMB_LAUNCH(c, (k_zgemm64<ALAY, YLAY, OP, LOWER>), g, 256, ZG_SMEM, M, R, K, A, lda, B, ldb, Y, ldy);
 }
