@@ -159,10 +159,10 @@ __global__ void k_init_state(int64_t R, const double *__restrict__ nrm, double t
 }
 
 // Givens update of column j of one system by one thread; col: the column's
-// first j entries in shared memory, rotated by the rotations rc, rs (shared)
-__device__ void givens_column(int j, double hnext, double2 *col, const double *rc, const double2 *rs,
-                              double2 *__restrict__ Hc, double *__restrict__ c, double2 *__restrict__ sv,
-                              double2 *__restrict__ gr, SysState &s) {
+// first j entries, rotated by the rotations rc, rs -- in shared memory, or, for a
+// column too long for it, Hc, c and sv themselves
+__device__ void givens_column(int j, double hnext, double2 *col, const double *rc, const double2 *rs, double2 *Hc,
+                              double *c, double2 *sv, double2 *__restrict__ gr, SysState &s) {
   // the rotations [c s; -conj(s) c] in order; only the running entry b feeds
   // the next one
   double2 a = col[0];
