@@ -606,8 +606,23 @@ def run_ours(args):
         if c2_results:
             line["c2_eval"] = c2_evaluation(c2_results)
     if rank == 0:
+        line, detail = split_line(line)
+        print(json.dumps({"detail": detail}), file=sys.stderr, flush=True)
         print(json.dumps(line), flush=True)
     replicas.finalize()
+
+
+DETAIL_KEYS = ("variants", "parity_vs_oracle", "c2_eval", "roofline_tc", "roofline_assembly", "fp64_peaks_measured")
+
+
+def split_line(line):
+    """The line of standard output, a few kilobytes whatever was run, and the
+    detail for standard error.  Of each variant the line keeps rate and time:
+    whole, the line outgrew what a reader of the output's end gets to see."""
+    short = {k: v for k, v in line.items() if k not in DETAIL_KEYS}
+    short["variants"] = {name: {k: v[k] for k in ("solves_per_s", "ms_per_step", "error") if k in v}
+                         for name, v in line.get("variants", {}).items()}
+    return short, {k: line[k] for k in DETAIL_KEYS if k in line}
 
 
 def clean(v):
