@@ -128,15 +128,6 @@ __global__ void k_diag_inv(int64_t N, const ZC *__restrict__ Z, const double *__
 // ---------------------------------------------------------------------------
 // LDL^T kernels; C is the storage and compute type (double2 or float2)
 // ---------------------------------------------------------------------------
-// Diagonal block: factor in shared memory, write L (strict lower) and D back,
-// and write Linv = L11^-1 (unit lower, b x b, row-major NB stride).
-//
-// 256 threads as 16 x 16; thread (tx, ty) keeps entries (ty + 16p, tx + 16q),
-// p, q in 0..3, of the block and of X = L^-1 in registers.  Elimination step k
-// broadcasts column k of the block and row k of X through shared memory and
-// applies both updates: L = L_0 L_1 ... with L_k = I + l_k e_k^T, so
-// X = ... (I - l_1 e_1^T)(I - l_0 e_0^T), and row k of X is final once steps
-// 0..k-1 have run.  One barrier pair per step covers both.
 // 1 / x for a positive normal float: the hardware approximation refined by
 // one Newton-Raphson step, r <- r (2 - x r)
 __device__ __forceinline__ float rcp_nr(float x) {
@@ -970,14 +961,13 @@ __global__ void k_scale_vec(int64_t N, int64_t R, const double2 *__restrict__ d,
 }
 
 // Three-level right-looking LDL^T.  Block columns of NBW = 1024 are factored
-// as 256-wide middle panels (one launch each).  After each middle panel the rest of the 1024-wide block column
-// receives one K = 256 update, and after the block column the whole trailing
-// matrix receives one K = 1024 update -- on the tensor cores (complex64: split
-// operands, complex128: int8 residues).
+// as 256-wide middle panels (one launch each).  After each middle panel the rest
+// of the 1024-wide block column receives one K = 256 update, and after the block
+// column the whole trailing matrix receives one K = 1024 update -- on the tensor
+// cores (complex64: split operands, complex128: int8 residues).
 //
-// Lookahead (details at update_block_column / update_trailing): the next
-// panel's latency-bound diagonal/panel/strip kernels run on the main stream
-// while the rest of each update streams through the tensor cores on two side
+// Lookahead (details at update_block_column / update_trailing): the next panel's
+// latency-bound launch and the update before it run on the main stream while the rest of each update streams through the tensor cores on two side
 // streams, always on columns disjoint from the main stream's.
 constexpr int NBO = 256;
 constexpr int NBW = 1024;

@@ -391,7 +391,7 @@ void gradient_impedance_dev(dmb_ctx *c, int64_t R, const double2 *I_dev, const d
   DMB_CUDA(cudaMemcpyAsync(btri.p, tri.data(), sizeof(int) * c->nt, cudaMemcpyHostToDevice, c->stream));
   DMB_LAUNCH(c, k_grad_impedance, dim3((unsigned)P, (unsigned)R), 128, 0, c->n, P, c->d_tcache.as<TriCache>(),
              c->nq, c->d_wq.as<double>(), boff.as<int>(), btri.as<int>(), I_dev, L_dev, reactive, g_dev);
-  DMB_CUDA(cudaStreamSynchronize(c->stream));  // the staging buffers are released on return
+  DMB_CUDA(cudaStreamSynchronize(c->stream));  // the host lists are released on return
 }
 
 void matvec_dev(dmb_ctx *c, const void *x, void *y, int64_t nrhs) {

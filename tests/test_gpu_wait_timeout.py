@@ -1,7 +1,7 @@
-"""The bounded-wait error path, exercised without any GPU fault: the chained
-triangular sweeps of a complex128 near-field factor wait on flags published by
-earlier CTAs; with DMB_OPT_SPIN_LIMIT = 0 a waiting CTA gives up at its first
-poll, records the error bit and returns.  The call must fail with
+"""The bounded-wait error path, exercised without any GPU fault: the triangular
+sweeps of a near-field factor wait for values published by earlier CTAs, and the
+tiles of a factorisation panel for its diagonal tiles; with DMB_OPT_SPIN_LIMIT = 0
+a waiting CTA gives up at its first poll, records the error bit and returns.  The call must fail with
 DMB_ERR_TIMEOUT (DeviceWaitTimeout), and the next call on the same context,
 with the default limit, must give the right answer."""
 import math
@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 
 
 def test_chain_wait_expires_and_context_recovers():
-    m = make_rect_plate(0.1, 0.1, 24, 24)   # 1,680 RWG: 27 chained 64-row blocks
+    m = make_rect_plate(0.1, 0.1, 24, 24)   # 1,680 RWG: seven 256-row blocks of a sweep
     r = build_rwg(m)
     k = 2 * math.pi / 0.1
     dev = EFIEDevice(m, r)
