@@ -802,7 +802,7 @@ __device__ __forceinline__ void mid_substitute(float2 (*Tw)[LD], const float2 (*
 template <class C>
 __global__ void __launch_bounds__(256, sizeof(C) == 16 ? 1 : 2) k_ldlt_mid(int64_t N, int64_t J, int w, C *__restrict__ F,
                                                                            C *__restrict__ Linv, C *__restrict__ W,
-                                                                           int wstride, double *__restrict__ bal,
+                                                                           int wstride, short *__restrict__ bal,
                                                                            unsigned *sync, unsigned *err,
                                                                            long long limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -870,13 +870,12 @@ __global__ void __launch_bounds__(256, sizeof(C) == 16 ? 1 : 2) k_ldlt_mid(int64
           Lb[(16 * q + i) * 64 + 16 * q + c] = sm.Xd[q][i][c];
         }
       publish(diag_flag + s);
-      // 2^-e and 2^e of the panel's columns, 4^e about |D|: what balances W and L
-      // for the int8 updates
+      // e of the panel's columns, 4^e about |D|: what balances W and L for the
+      // int8 updates
       if (bal && ok && t < b) {
         int e;
         frexp(fmax(fabs((double)As[t][t].x), fabs((double)As[t][t].y)), &e);
-        bal[jc + t] = ldexp(1.0, -(e >> 1));
-        bal[N + jc + t] = ldexp(1.0, e >> 1);
+        bal[jc + t] = (short)(e >> 1);
       }
       if (ok) ldlt_diag_phase2<C>(Lb, smem_raw);
       return;
@@ -1010,7 +1009,7 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
   const bool use_tc = std::is_same<C, float2>::value && dmb::tc_available(c);
   // complex128 updates on the int8 tensor cores: a first run through the schedule
   // only notes what each stream's largest update needs
-  double *bal = nullptr;  // column scales of the int8 updates; null: FP64 pipe
+  short *bal = nullptr;  // column exponents of the int8 updates; null: FP64 pipe
   bool planning = std::is_same<C, double2>::value && dmb::oz64_available(c, NBO);
   size_t need[3] = {0, 0, 0};
   // trailing update F[r][cc] -= W[r][woff..woff+K) L[cc][jcol..jcol+K) on
@@ -1029,8 +1028,8 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
     } else if constexpr (std::is_same<C, double2>::value) {
       const double2 *Wk = (const double2 *)Wb + r0 * NBW + woff, *Lk = (const double2 *)F + r0 * N + jcol;
       if (bal && dmb::oz64_available(c, K))
-        dmb::oz64_lower_update(c, rest, c_hi - r0, K, Wk, NBW, Lk, N, bal + jcol, bal + N + jcol,
-                               (double2 *)F + r0 * N + r0, N, slot, err);
+        dmb::oz64_lower_update(c, rest, c_hi - r0, K, Wk, NBW, Lk, N, bal + jcol, (double2 *)F + r0 * N + r0, N,
+                               slot, err);
       else
         // the FP64-pipe GEMM (lower triangle)
         dmb::zgemm64_lower_update(c, rest, c_hi - r0, K, Wk, NBW, Lk, N, (double2 *)F + r0 * N + r0, N);
@@ -1124,7 +1123,7 @@ template <class C> void ldlt_factor(dmb_ctx *c, C *F) {
   if (planning) {
     schedule();
     planning = false;
-    if (need[0] > 0 && dmb::oz64_reserve(c, N, need)) bal = c->oz64.buf.as<double>();
+    if (need[0] > 0 && dmb::oz64_reserve(c, N, need)) bal = c->oz64.buf.as<short>();
   }
   schedule();
   join2();

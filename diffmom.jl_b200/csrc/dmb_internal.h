@@ -181,8 +181,7 @@ struct FarTileState {
 };
 
 // Buffer of the complex128 factor updates on the INT8 tensor cores
-// (dmb_oz64.cu): per factor column 2^-e (scales W) and 2^e (scales L), then a
-// part per issuing stream
+// (dmb_oz64.cu): an exponent per factor column, then a part per issuing stream
 struct Oz64State {
   DevBuf buf;
   size_t part[3] = {0, 0, 0};
@@ -460,14 +459,14 @@ void zgemm64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int64_t K, const dou
                           const double2 *Lrows, int64_t ldl, double2 *F, int64_t ldf);
 // the same update on the INT8 tensor cores (dmb_oz64.cu), K 256 or 1024, with
 // the part of `slot` of the buffer; err gets bit 8 when a pipeline wait expires.
-// oz64_reserve: room for N columns' scales and the largest updates of the three
+// bal: exponents e of the K columns, W is scaled by 2^-e and L by 2^e.
+// oz64_reserve: room for N columns' exponents and the largest updates of the three
 // slots, false when it cannot be had
 bool oz64_available(dmb_ctx *c, int K);
 size_t oz64_bytes(int64_t M, int64_t C, int K);
 bool oz64_reserve(dmb_ctx *c, int64_t N, const size_t (&bytes)[3]);
 void oz64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int K, const double2 *W, int64_t ldw, const double2 *L,
-                       int64_t ldl, const double *balW, const double *balL, double2 *F, int64_t ldf, int slot,
-                       unsigned *err);
+                       int64_t ldl, const short *bal, double2 *F, int64_t ldf, int slot, unsigned *err);
 void oz64_release(dmb_ctx *c);
 unsigned read_err_word(dmb_ctx *c);  // error word of the triangular solves (bit 2: a wait expired)
 void matvec_dev(dmb_ctx *c, const void *x, void *y, int64_t nrhs);  // device buffers, c128

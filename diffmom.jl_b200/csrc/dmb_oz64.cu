@@ -326,7 +326,8 @@ struct Mods64 {
 struct Operand64 {
   const double2 *S;   // rows x K, row-major
   int64_t ld, rows, padded;
-  const double *bal;  // scales of the K columns, powers of two
+  const short *bal;   // exponents of the K columns, and their sign for this operand
+  int sign;
   double *scale;      // padded
   signed char *P;     // OZ_NMOD64 planes of 2 padded rows of K bytes
 };
@@ -356,15 +357,22 @@ __global__ void __launch_bounds__(64) k_oz64_planes(Operand64 A, Operand64 B, co
   for (int u = 0; u < 16; u++) {
     const int e = t + 64 * u;
     const int64_t rr = r0 + e / K;
-    st[e + (e >> 4)] = rr < O.rows ? cscale(O.S[rr * O.ld + e % K], O.bal[e % K]) : make_double2(0, 0);
+    st[e + (e >> 4)] = rr < O.rows ? O.S[rr * O.ld + e % K] : make_double2(0, 0);
   }
+  // this thread's columns: exponents two to a word, |e| < 540
+  const uint4 b0 = reinterpret_cast<const uint4 *>(O.bal + 16 * kt)[0], b1 = reinterpret_cast<const uint4 *>(O.bal + 16 * kt)[1];
+  const unsigned be[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
   __syncthreads();
   const double2 *my = st + 17 * t;
+  auto value = [&](int u) {  // balanced: times 2^(sign e), exact
+    const int e = (short)(u & 1 ? be[u >> 1] >> 16 : be[u >> 1] & 0xffffu);
+    return cscale(my[u], __hiloint2double((1023 + O.sign * e) << 20, 0));
+  };
   double mx = 0.0;
   bool finite = true;
 #pragma unroll
   for (int u = 0; u < 16; u++) {
-    const double2 v = my[u];
+    const double2 v = value(u);
     mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
     finite = finite && isfinite(v.x) && isfinite(v.y);
   }
@@ -387,7 +395,7 @@ __global__ void __launch_bounds__(64) k_oz64_planes(Operand64 A, Operand64 B, co
     unsigned lo[16], hi[16];
 #pragma unroll
     for (int u = 0; u < 16; u++) {
-      const double v = c == 0 ? my[u].x : my[u].y;
+      const double v = c == 0 ? value(u).x : value(u).y;
       const unsigned long long a = (unsigned long long)(__double2ll_rn(nan ? 0.0 : v * f) + (1ll << 56));
       lo[u] = (unsigned)a;
       hi[u] = (unsigned)(a >> 32);
@@ -482,12 +490,12 @@ size_t oz64_bytes(int64_t M, int64_t C, int K) {
   return Part64(mc, cc, tl.count(), K).end;
 }
 
-// One buffer for a factorisation's three streams and its column scales: an
+// One buffer for a factorisation's three streams and its column exponents: an
 // allocation takes 0.33 ms and a release 0.3, whatever their size, so nothing grows on
 // the way (nine buffers that did cost the first factorisation of a context 5 ms)
 bool oz64_reserve(dmb_ctx *c, int64_t N, const size_t (&bytes)[3]) {
   Oz64State &st = c->oz64;
-  size_t at = up(sizeof(double) * 2 * N, 1024);
+  size_t at = up(sizeof(short) * N, 1024);
   for (int s = 0; s < 3; s++) {
     st.part[s] = at;
     at += up(bytes[s], 1024);
@@ -502,8 +510,7 @@ bool oz64_reserve(dmb_ctx *c, int64_t N, const size_t (&bytes)[3]) {
 }
 
 void oz64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int K, const double2 *W, int64_t ldw, const double2 *L,
-                       int64_t ldl, const double *balW, const double *balL, double2 *F, int64_t ldf, int slot,
-                       unsigned *err) {
+                       int64_t ldl, const short *bal, double2 *F, int64_t ldf, int slot, unsigned *err) {
   Oz64State &st = c->oz64;
   raise_smem(c, k_oz64_gemm, O6_SMEM);
   const int64_t mstep = K == 1024 ? O6_ROWS_1024 : O6_ROWS_256;
@@ -519,7 +526,7 @@ void oz64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int K, const double2 *W
       double *rs = (double *)(base + part.scale), *cs = rs + nmp;
       signed char *PA = (signed char *)base, *PB = PA + (size_t)OZ_NMOD64 * 2 * nmp * K;
       unsigned char *res = (unsigned char *)(base + part.res);
-      const Operand64 A{W + m0 * ldw, ldw, nm, nmp, balW, rs, PA}, B{L + c0 * ldl, ldl, nc, ncp, balL, cs, PB};
+      const Operand64 A{W + m0 * ldw, ldw, nm, nmp, bal, -1, rs, PA}, B{L + c0 * ldl, ldl, nc, ncp, bal, 1, cs, PB};
       const unsigned g = (unsigned)((nmp + ncp) / (1024 / K));
       if (K == 1024)
         DMB_LAUNCH(c, k_oz64_planes<1024>, g, 64, 0, A, B, mods64());
