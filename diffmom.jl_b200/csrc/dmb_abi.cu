@@ -430,6 +430,7 @@ dmb_status dmb_nf_apply(dmb_ctx *c, const double *x, double *y, int64_t nrhs) {
     DevBuf &bx = c->d_io[0];
     bx.ensure(bytes);
     DMB_CUDA(cudaMemcpyAsync(bx.p, x, bytes, cudaMemcpyHostToDevice, c->stream));
+    dmb::clear_err_word(c);
     dmb::pc_apply_dev(c, bx.as<double>(), nrhs);
     dmb::copy_out(c, y, bx.p, (int64_t)(bytes / sizeof(double2)));
     DMB_REQUIRE((dmb::read_err_word(c) & 4u) == 0, DMB_ERR_TIMEOUT, "triangular solve wait expired");

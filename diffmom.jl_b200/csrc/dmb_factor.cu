@@ -1548,10 +1548,10 @@ __device__ __forceinline__ void rows2_fma(const double2 *m, const double2 *v, in
   }
 }
 
-__global__ void k_sweep_clear(int64_t n, ulonglong2 *buf, int words, unsigned *err) {
+__global__ void k_sweep_clear(int64_t n, ulonglong2 *buf, int ntickets, unsigned *tickets) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e < n) buf[e] = make_ulonglong2(SV_EMPTY, SV_EMPTY);
-  if (e < words) err[e] = 0u;
+  if (e < ntickets) tickets[e] = 0u;
 }
 
 struct SweepSmem {
@@ -1704,12 +1704,12 @@ template <class C> void ldlt_solve(dmb_ctx *c, const C *F, double2 *x, int64_t R
   // a and y of the forward sweep, a and x of the backward one, all empty
   c->d_sv_acc.ensure(sizeof(double2) * 4 * N * R);
   double2 *buf = c->d_sv_acc.as<double2>();
-  // the error word, a ticket counter per column and sweep
-  const size_t words = 1 + 2 * R;
-  c->d_flags.ensure(std::max<size_t>(64, 4 * words));
+  // the error word, then a ticket counter per column and sweep (at most 14; the
+  // factorisation made room).  The error word stays: a solve's later sweeps must
+  // not hide that an earlier one gave up (clear_err_word at the solve's start)
   unsigned *err = c->d_flags.as<unsigned>(), *tickets = err + 1;
   DMB_LAUNCH(c, k_sweep_clear, blocks_for(4 * N * R, 256), 256, 0, 4 * N * R, reinterpret_cast<ulonglong2 *>(buf),
-             (int)words, err);
+             (int)(2 * R), tickets);
   const dim3 g((unsigned)((N + SW - 1) / SW), (unsigned)R);
   DMB_LAUNCH(c, k_sweep_fwd<C>, g, 256, sizeof(SweepSmem), N, F, X, x, buf, buf + N * R, tickets, err, c->spin_limit);
   DMB_LAUNCH(c, k_sweep_bwd<C>, g, 256, sizeof(SweepSmem), N, F, X, buf + N * R, buf + 2 * N * R, buf + 3 * N * R, x,
@@ -1753,6 +1753,10 @@ template <class C> void ldlt_solve_batched(dmb_ctx *c, const C *F, double2 *X, i
 }  // namespace
 
 namespace dmb {
+
+void clear_err_word(dmb_ctx *c) {
+  if (c->d_flags.p) DMB_CUDA(cudaMemsetAsync(c->d_flags.p, 0, 4, c->stream));
+}
 
 unsigned read_err_word(dmb_ctx *c) {
   unsigned e = 0;

@@ -355,6 +355,7 @@ void gmres_dev(dmb_ctx *c, const double *b_dev, double *x_dev, int64_t R, double
   DMB_REQUIRE(precond_kind == DMB_PRECOND_NONE || precond_kind == c->pc_kind, DMB_ERR_STATE,
               "requested preconditioner kind differs from the one built");
   if (precond_kind == DMB_PRECOND_NF_LU) pc_prepare_dev(c, R);
+  clear_err_word(c);
   if (matvec_op_inexact(c, R)) tc_zx_prepare(c);
   // basis capacity: maxiter vectors, bounded by a 40% share of free memory
   // (decided once per problem shape; repeated solves reuse the buffers); the

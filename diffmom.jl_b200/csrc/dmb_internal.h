@@ -468,7 +468,10 @@ bool oz64_reserve(dmb_ctx *c, int64_t N, const size_t (&bytes)[3]);
 void oz64_lower_update(dmb_ctx *c, int64_t M, int64_t C, int K, const double2 *W, int64_t ldw, const double2 *L,
                        int64_t ldl, const short *bal, double2 *F, int64_t ldf, int slot, unsigned *err);
 void oz64_release(dmb_ctx *c);
-unsigned read_err_word(dmb_ctx *c);  // error word of the triangular solves (bit 2: a wait expired)
+// error word of the triangular solves (bit 2: a wait expired): cleared at the
+// start of a call that applies a factor, kept by its sweeps, read at its end
+void clear_err_word(dmb_ctx *c);
+unsigned read_err_word(dmb_ctx *c);
 void matvec_dev(dmb_ctx *c, const void *x, void *y, int64_t nrhs);  // device buffers, c128
 void conj_dev(dmb_ctx *c, double2 *x, int64_t count);
 void nf_build(dmb_ctx *c, double cutoff, int kind);

@@ -43,6 +43,34 @@ def test_chain_wait_expires_and_context_recovers():
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_no_expired_wait_is_lost(precision):
+    """Limits at which some of a solve's sweeps expire and others do not: the
+    solve fails, or gives what it gives without a limit."""
+    m = make_rect_plate(0.1, 0.1, 18, 20)
+    dev = EFIEDevice(m, build_rwg(m))
+    dev.assemble(2 * math.pi / 0.1, precision=precision)
+    P = dev.build_nearfield(0.03, "lu")
+    dev.set_option("true_residual", 0)
+    b = np.random.default_rng(3).standard_normal(dev.N) + 0j
+
+    def solve():
+        return dev.gmres(b, tol=1e-6, maxiter=60, preconditioner=P, check_gmres_convergence=False)[0]
+
+    ref, expired = solve(), 0
+    for limit in [int(1.25 ** e) for e in range(8, 44)]:  # 5 to 14,000 polls
+        for _ in range(3):
+            dev.set_option("spin_limit", limit)
+            try:
+                np.testing.assert_array_equal(solve(), ref)
+            except DeviceWaitTimeout:
+                expired += 1
+    dev.set_option("spin_limit", -1)
+    np.testing.assert_array_equal(solve(), ref)
+    dev.close()
+    assert expired > 0
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_factorisation_wait_expires_and_context_recovers(precision):
     """The tiles of a 256-wide panel wait for its diagonal tiles."""
     m = make_rect_plate(0.1, 0.1, 20, 23)   # 1,337 RWG: six panels, two block columns
