@@ -139,11 +139,20 @@ static bool copy_staged(dmb_ctx *c, HostCopy &h, void *dst, const void *src, int
   return ok;
 }
 
+// memory of the caller's that the device does not reach by itself; pinned memory is
+// copied to at the bus rate without a detour
+static bool pageable(const void *dst) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, dst) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
+  (void)cudaGetLastError();
+  return true;
+}
+
 // dst (complex128, host) <- src (device, complex64 when widen) after the work
 // issued on the context's stream; returns when dst is written
 void copy_out(dmb_ctx *c, void *dst, const void *src, int64_t count, bool widen) {
   const size_t bytes = sizeof(double2) * (size_t)count;
-  if (bytes >= HC_MIN) {
+  if (bytes >= HC_MIN && pageable(dst)) {
     c->copied += bytes;
     const bool make = bytes >= HC_MAKE || c->copied >= 2 * HC_MAKE;
     if (!c->hostcopy || !c->hostcopy->usable) c->hostcopy = hostcopy_of(c->device, make);
