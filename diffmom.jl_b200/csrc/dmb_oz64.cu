@@ -15,10 +15,11 @@
 // are balanced first: column k of W = L D is scaled by 2^-e, column k of L by
 // 2^e, 4^e about |D_k| (exact).  Both rows are then rows of about L sqrt(|D|),
 // whose elements do not carry the scales of the basis functions of their
-// columns.  Without it an error grew with the spread of these scales: largest
-// |A - L D L^T| over the diagonal scales of a graded plate, 519 unknowns, scales
-// over 1.6e3: 2e-11, balanced 1e-13, FP64 sums 1e-13; over 3e6: 0.4, 3e-9 and 2e-9;
-// on plates and disks of even meshes 1e-15 to 3e-15 in all three.
+// columns.  Without it the error grew with the spread of these scales.  Largest
+// |A - L D L^T| over the diagonal scales, updates of 64 columns emulated on the
+// host, plates of 519 unknowns with graded cells: scales over 1.6e3 2e-11, balanced
+// 1e-13, FP64 sums 1e-13; over 3e6 0.4, 3e-9 and 2e-9; even plates and disks 1e-15 to
+// 3e-15 in all three.
 //
 // Why: B200 has no FP64 tcgen05 kind, and an FP64-pipe GEMM stops at 36.8
 // TFLOP/s (a complex MAC = 8 flops); 16 int8 products at the nominal int8
